@@ -128,8 +128,8 @@ typedef struct tnsr_b200_config {
      * multiple of 16 that divides capacity.  kv_pool_pages = 0 sizes the pool
      * for the worst case (batch * capacity / kv_page_rows).  A step that needs a
      * page when none is free fails with TNSR_B200_ERR_CAPACITY and changes
-     * nothing.  Multi-token chunks run on the non-tiled attention scan in this
-     * mode. */
+     * nothing.  Multi-token chunks run on the warp-level tiled attention kernel in
+     * this mode. */
     uint32_t kv_page_rows;
     uint32_t kv_pool_pages;
     /* Single-token steps of at most 32 sessions (bf16 weights, SwiGLU, width <=

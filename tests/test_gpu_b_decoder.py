@@ -683,6 +683,42 @@ def test_paged_kv_cache_gives_the_same_bits_as_the_contiguous_one():
     assert np.array_equal(divided.view(np.uint32), reference.view(np.uint32))
 
 
+@pytest.mark.parametrize("heads,paged,batch", [(4, True, 3), (8, True, 1), (8, False, 2), (2, False, 3), (16, False, 2)])
+def test_multi_token_chunks_off_the_tiled_prefill_kernels(heads, paged, batch):
+    """Paged caches, and heads of other widths than 64 (here 32, 64, 128 and 16): chunks of 2 .. 130 ids at any position run on the
+    grouped kernels.  Against the same handle on the non-tiled scan (prefill mode Scalar): weights enter the value product with
+    16 bits instead of 24 and scores are summed in another order, far below the bf16 rounding (2^-9) of the rows both store, which
+    is what two layers and the head pass on; and against the CPU checker."""
+    from oracle import oracle
+    cfg = GptConfig(vocab_size=320, max_sequence_length=288, embed_dim=256, num_heads=heads, feed_forward_dim=512, num_layers=2,
+                    layer_norm_epsilon=1e-5, activation="swiglu", weight_dtype="bf16")
+    arrays = normal_model_arrays(cfg, seed=85, std=0.05)
+    chunks = [2, 63, 64, 17, 130]                                  # the last one ends at 276, inside a page
+    ids = np.random.default_rng(86).integers(0, cfg.vocab_size, size=(batch, sum(chunks))).astype(np.uint32)
+
+    def run(mode, **kw):
+        s = B200Session(cfg, batch, 288, GptDecoderOptions(prefill=mode), logits_mode="all", **kw)
+        for i, a in enumerate(arrays):
+            s.refresh(i, a)
+        out, at = [], 0
+        for n in chunks:
+            out.append(s.decode_full(ids[:, at:at + n], at)[0].reshape(batch, n, -1))
+            at += n
+        caches = [s.read_cache(i) for i in range(4)]
+        s.close()
+        return np.concatenate(out, axis=1), caches
+
+    got, caches = run(GptPrefillMode.Auto, **({"kv_page_rows": 32} if paged else {}))
+    want, plain = run(GptPrefillMode.Scalar)
+    assert rel_err(got, want) <= 1e-2
+    for a, b in zip(caches, plain):
+        assert np.max(np.abs(a - b)) <= max(1.0, float(np.max(np.abs(b)))) / 64
+    ref = oracle.OracleModel(cfg.vocab_size, cfg.max_sequence_length, cfg.embed_dim, cfg.num_heads, cfg.feed_forward_dim,
+                             cfg.num_layers, cfg.layer_norm_epsilon, "swiglu")
+    ref.set_params([oracle.bf16_round_np(a) if a.ndim == 2 else a for a in arrays])
+    assert rel_err(got, ref.forward(ids)) <= 2e-2
+
+
 def test_paged_kv_pool_smaller_than_the_worst_case():
     """A pool of 7 pages for 4 sessions x 64 rows (worst case 16 pages): short sessions fit, a step that would need an
     eighth page is refused with ERR_CAPACITY and changes nothing, releasing a session makes room again."""

@@ -83,6 +83,9 @@ struct tnsr_b200_decoder {
     uint32_t split_rows = 0;
     uint32_t split_pending = 0;   // partial sums of the last layer's down projection, for the final LayerNorm to add
     uint64_t attn_ws_bytes = 0;
+    // multi-token chunks that the tiled prefill kernels do not take (grouped_attention.cu)
+    void* grouped_ws = nullptr;
+    uint64_t grouped_ws_bytes = 0;
     cudaStream_t side_stream[3] = {nullptr, nullptr, nullptr};   // forked from and joined to `stream` by events
     cudaEvent_t ev_fork = nullptr, ev_join[3] = {nullptr, nullptr, nullptr};
     uint32_t parts = 1;
