@@ -111,6 +111,18 @@ def test_strict_matmul_keeps_rounded_products_and_k_order(oracle):
     assert np.array_equal(run_strict(a, np.ascontiguousarray(b.T), transposed=True).view(np.uint32), expected.view(np.uint32))
 
 
+@pytest.mark.parametrize("shape", [(65, 128, 128), (64 * 37 + 1, 129, 257), (1000, 31, 640), (66, 33, 31), (4801, 8, 130), (130, 513, 1024), (67, 30, 33)])
+def test_strict_matmul_tiles_bit_exact(oracle, shape):
+    """More than 64 rows run on 32 x 32 or (from 148 tiles on) 64 x 64 output tiles with packed instructions: sizes at the edges of both,
+    of the 32-deep shared tiles and of 16-byte loads, against the CPU order bit for bit, weights in either layout."""
+    m, k, n = shape
+    rng = np.random.default_rng(m + k + n)
+    a, b, bias = (rng.standard_normal(x).astype(np.float32) for x in ((m, k), (k, n), (n,)))
+    expected = oracle.linear(a, b, bias).view(np.uint32)
+    assert np.array_equal(run_strict(a, b, bias).view(np.uint32), expected)
+    assert np.array_equal(run_strict(a, np.ascontiguousarray(b.T), bias, transposed=True).view(np.uint32), expected)
+
+
 @pytest.mark.parametrize("shape", [(1, 128, 128), (16, 128, 512), (7, 13, 8), (33, 37, 35), (3, 512, 96)])
 def test_strict_matmul_random_shapes_bit_exact(oracle, shape):
     m, k, n = shape

@@ -648,6 +648,31 @@ def test_session_sampler_draws_what_the_cpu_restatement_draws(logits_mode):
     assert np.array_equal(got, greedy)
 
 
+@pytest.mark.parametrize("heads,width,batch", [(4, 128, 1), (4, 128, 16), (3, 72, 2), (1, 64, 40), (2, 200, 3)])
+@pytest.mark.parametrize("precision", [GptAttentionPrecision.F32, GptAttentionPrecision.Bf16])
+def test_strict_chunks_have_the_bits_of_single_tokens(heads, width, batch, precision):
+    """f32 weights: every output is a chain of rounded operations in a stated order, so a chunk of any length -- 32 or 8 queries per block,
+    keys 64 at a time, rows of LayerNorm 32 at a time -- gives the bits of its tokens one by one.  Heads of 32, 24, 64 and 100."""
+    cfg = GptConfig(vocab_size=70, max_sequence_length=160, embed_dim=width, num_heads=heads, feed_forward_dim=2 * width + 3, num_layers=2,
+                    layer_norm_epsilon=1e-5)
+    model = Gpt(cfg)
+    set_model_arrays(model, normal_model_arrays(cfg, seed=31, std=0.2, bias_std=0.1))
+    ids = np.random.default_rng(32).integers(0, 70, size=(batch, 134)).astype(np.uint32)
+    decoder = gpu_decoder(model, batch, 160, GptDecoderOptions(attention_precision=precision))
+
+    def logits(cuts):
+        decoder.reset()
+        parts, at = [], 0
+        for n in cuts:
+            parts.append(decoder.decode(ids[:, at:at + n].reshape(-1).tolist()).reshape(batch, n, -1))
+            at += n
+        return np.concatenate(parts, axis=1).view(np.uint32)
+
+    single = logits([1] * 134)
+    for cuts in ([134], [65, 2, 67], [33, 31, 70]):
+        assert np.array_equal(logits(cuts), single)
+
+
 def test_paged_kv_cache_gives_the_same_bits_as_the_contiguous_one():
     """kv_page_rows > 0: every cache tensor is a pool of pages handed to sessions on demand.  Same kernels, other
     addresses: prefill (non-tiled scan in both handles), graph-replayed steps, ragged steps and the cache read back in

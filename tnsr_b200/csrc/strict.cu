@@ -8,101 +8,138 @@
 // in increasing index order from a zero start.  exp/ln go through the f64
 // routines and are rounded once to f32, which is the nearest-f32 result the
 // host libm delivers in all but rare last-bit cases.
-#include "common.cuh"
+#include <algorithm>
+
+#include "strict.cuh"
 
 namespace tb {
 
-__device__ __forceinline__ float strict_expf(float x) { return (float)exp((double)x); }
-__device__ __forceinline__ float strict_logf(float x) { return (float)log((double)x); }
-
-// nn::sigmoid op by op (src/nn/activations.rs:5-14).
-__device__ __forceinline__ float strict_sigmoid(float x) {
-    float negative = (-x > 0.0f) ? 1.0f : 0.0f;
-    float nonnegative = 1.0f - negative;
-    float magnitude = x * (1.0f - negative * 2.0f);
-    float z = strict_expf(-magnitude);
-    float denominator = z + 1.0f;
-    float a = (nonnegative != 0.0f) ? (1.0f / denominator) : 0.0f;
-    float b = (negative != 0.0f) ? (z / denominator) : 0.0f;
-    return a + b;
-}
-
-// nn::gelu op by op (src/nn/activations.rs:29-47).
-__device__ __forceinline__ float strict_gelu(float x) {
-    float negative = (-x > 0.0f) ? 1.0f : 0.0f;
-    float nonnegative = 1.0f - negative;
-    float magnitude = (x * (1.0f - negative * 2.0f)) * 0.70710678118654752440f;
-    float t = 1.0f / (magnitude * 0.3275911f + 1.0f);
-    float polynomial =
-        ((((t * 1.0614054f - 1.4531521f) * t + 1.4214138f) * t - 0.28449672f) * t + 0.2548296f) * t;
-    float tail = (polynomial * strict_expf(-(magnitude * magnitude))) * 0.5f;
-    float a = (nonnegative != 0.0f) ? (1.0f - tail) : 0.0f;
-    float b = (negative != 0.0f) ? tail : 0.0f;
-    return x * (a + b);
-}
-
-// tanh form of gelu in f32 with the full-precision tanh.
-__device__ __forceinline__ float strict_gelu_tanh(float x) {
-    return 0.5f * x * (1.0f + tanhf(0.79788456080286536f * (x + 0.044715f * (x * x * x))));
-}
-
 // ---------------------------------------------------------------------------
-// GEMM: one thread per output element, K walked in order through 16-wide
-// shared tiles.  The tiling changes which thread loads what, not the order in
-// which any output's products are added.
+// GEMM: a block of 256 threads owns a T x T tile of the output, a thread R x R of its elements (R = T / 16), K is walked in
+// order through 32-deep shared tiles.  An output is one chain of rounded products and rounded sums; the R * R chains of a
+// thread are independent of each other and hide each other's latency.  Two columns go through one packed instruction whose halves
+// round as the scalar ones do: mul.rn.f32x2, then fma.rn.f32x2 with a factor of one that only the launch knows, because the
+// assembler joins a packed product and a packed sum into one operation with one rounding.  The rows' values are stored twice side
+// by side so that a pair of them is loaded and not made.  The next tile's global loads are in flight while a tile is worked on.
 // ---------------------------------------------------------------------------
-constexpr int ST = 16;
+constexpr uint32_t SK = 32;
 
-template <bool BT>
-__global__ void __launch_bounds__(ST* ST)
-gemm_strict_kernel(const float* __restrict__ a, const float* __restrict__ b, void* __restrict__ out,
-                   uint32_t ldc, uint32_t m, uint32_t k, uint32_t n, GemmEpilogue ep) {
-    __shared__ float as[ST][ST + 1];
-    __shared__ float bs[ST][ST + 1];
-    const uint32_t tx = threadIdx.x, ty = threadIdx.y;
-    const uint32_t row = blockIdx.y * ST + ty, col = blockIdx.x * ST + tx;
-    float sum = 0.0f;
-    for (uint32_t k0 = 0; k0 < k; k0 += ST) {
-        uint32_t ka = k0 + tx;
-        as[ty][tx] = (row < m && ka < k) ? a[(size_t)row * k + ka] : 0.0f;
-        if (BT) {
-            // b is [n, k]: element (p, j) lives at b[j * k + p]
-            uint32_t j = blockIdx.x * ST + ty, p = k0 + tx;
-            bs[tx][ty] = (j < n && p < k) ? b[(size_t)j * k + p] : 0.0f;
-        } else {
-            uint32_t p = k0 + ty;
-            bs[ty][tx] = (p < k && col < n) ? b[(size_t)p * n + col] : 0.0f;
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+// sum + p, as p * one + sum
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t sum, uint64_t p, uint64_t one) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(p), "l"(one), "l"(sum));
+    return d;
+}
+
+// Four values src[0 .. 3] along a row of `limit` values from `at` on; zeros past the end or for a row that is not there.
+__device__ __forceinline__ float4 strict_load4(const float* row, uint32_t at, uint32_t limit, bool live, bool vec) {
+    if (vec) return live && at < limit ? *reinterpret_cast<const float4*>(row + at) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 v;
+    v.x = live && at < limit ? row[at] : 0.0f;
+    v.y = live && at + 1 < limit ? row[at + 1] : 0.0f;
+    v.z = live && at + 2 < limit ? row[at + 2] : 0.0f;
+    v.w = live && at + 3 < limit ? row[at + 3] : 0.0f;
+    return v;
+}
+
+template <int T, bool BT>
+__global__ void __launch_bounds__(256)
+gemm_strict_tile_kernel(const float* __restrict__ a, const float* __restrict__ b, void* __restrict__ out, uint32_t ldc, uint32_t m,
+                        uint32_t k, uint32_t n, bool vec_a, bool vec_b, float one, GemmEpilogue ep) {
+    constexpr uint32_t R = T / 16, LOADS = T * SK / 4 / 256;      // float4 loads per thread and operand tile (1 or 2)
+    __shared__ __align__(16) float as[SK][2 * T];                 // every value twice
+    __shared__ __align__(16) float bs[SK][T];
+    const uint32_t tid = threadIdx.x, tx = tid % 16, ty = tid / 16, row0 = blockIdx.y * T, col0 = blockIdx.x * T;
+    float4 ra[LOADS], rb[LOADS];
+    auto fetch = [&](uint32_t k0) {
+#pragma unroll
+        for (uint32_t i = 0; i < LOADS; ++i) {
+            const uint32_t e = tid + i * 256, r = e % T, q = e / T;      // along k: lanes on different rows, so that stores do not collide
+            ra[i] = strict_load4(a + (size_t)(row0 + r) * k, k0 + 4 * q, k, row0 + r < m, vec_a);
+            if (BT) {
+                rb[i] = strict_load4(b + (size_t)(col0 + r) * k, k0 + 4 * q, k, col0 + r < n, vec_b);
+            } else {
+                const uint32_t p = e / (T / 4), c = e % (T / 4);
+                rb[i] = strict_load4(b + (size_t)(k0 + p) * n, col0 + 4 * c, n, k0 + p < k, vec_b);
+            }
+        }
+    };
+    uint64_t acc[R][R / 2];
+#pragma unroll
+    for (uint32_t i = 0; i < R; ++i)
+#pragma unroll
+        for (uint32_t j = 0; j < R / 2; ++j) acc[i][j] = 0;
+    const uint64_t one2 = (uint64_t)__float_as_uint(one) << 32 | __float_as_uint(one);
+    fetch(0);
+    for (uint32_t k0 = 0; k0 < k; k0 += SK) {
+        __syncthreads();
+#pragma unroll
+        for (uint32_t i = 0; i < LOADS; ++i) {
+            const uint32_t e = tid + i * 256, r = e % T, q = e / T;
+            const float va[4] = {ra[i].x, ra[i].y, ra[i].z, ra[i].w}, vb[4] = {rb[i].x, rb[i].y, rb[i].z, rb[i].w};
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) {
+                *reinterpret_cast<float2*>(&as[4 * q + j][2 * r]) = make_float2(va[j], va[j]);
+                if (BT) bs[4 * q + j][r] = vb[j];
+            }
+            if (!BT) *reinterpret_cast<float4*>(&bs[e / (T / 4)][4 * (e % (T / 4))]) = rb[i];
         }
         __syncthreads();
-        const uint32_t lim = min((uint32_t)ST, k - k0);
-        for (uint32_t p = 0; p < lim; ++p) sum = sum + as[ty][p] * bs[p][tx];
-        __syncthreads();
+        if (k0 + SK < k) fetch(k0 + SK);
+        auto step = [&](uint32_t p) {
+            uint64_t av[R], bv[R / 2];
+            const ulonglong2* ap = reinterpret_cast<const ulonglong2*>(&as[p][2 * R * ty]);
+#pragma unroll
+            for (uint32_t i = 0; i < R / 2; ++i) { const ulonglong2 v = ap[i]; av[2 * i] = v.x; av[2 * i + 1] = v.y; }
+            if (R == 2) {
+                bv[0] = *reinterpret_cast<const uint64_t*>(&bs[p][2 * tx]);
+            } else {
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&bs[p][R * tx]);
+                bv[0] = v.x;
+                bv[R / 2 - 1] = v.y;
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < R; ++i)
+#pragma unroll
+                for (uint32_t j = 0; j < R / 2; ++j) acc[i][j] = add_f32x2(acc[i][j], mul_f32x2(av[i], bv[j]), one2);
+        };
+        if (k - k0 >= SK) {
+#pragma unroll 8
+            for (uint32_t p = 0; p < SK; ++p) step(p);
+        } else {
+            for (uint32_t p = 0; p < k - k0; ++p) step(p);     // never a product past the end: it would be a rounded sum more
+        }
     }
-    if (row >= m || col >= n) return;
-    float v = sum;
-    if (ep.bias) v = v + ep.bias[col];
-    if (ep.activation == ACT_RELU) v = fmaxf(v, 0.0f);
-    else if (ep.activation == ACT_GELU) v = strict_gelu(v);
-    else if (ep.activation == ACT_GELU_TANH) v = strict_gelu_tanh(v);
-    if (ep.scale) v = v * ep.scale[col];
-    if (ep.residual) v = ep.residual[(size_t)row * ep.ldr + col] + v;
-    if (ep.round_bf16) v = round_to_bf16(v);
-    size_t orow = row;
-    if (ep.rows_per_session) {
-        uint32_t off = ep.d_row_offset ? *ep.d_row_offset : ep.row_offset;
-        orow = (size_t)(row / ep.rows_per_session) * ep.out_session_rows + off + row % ep.rows_per_session;
-    }
-    if (ep.out_dtype == TNSR_B200_BF16)
-        reinterpret_cast<bf16*>(out)[orow * ldc + col] = __float2bfloat16_rn(v);
-    else
-        reinterpret_cast<float*>(out)[orow * ldc + col] = v;
+#pragma unroll
+    for (uint32_t i = 0; i < R; ++i)
+#pragma unroll
+        for (uint32_t j = 0; j < R; ++j) {
+            const uint32_t row = row0 + R * ty + i, col = col0 + R * tx + j;
+            const uint32_t bits = (uint32_t)(acc[i][j / 2] >> (j % 2 ? 32 : 0));
+            if (row < m && col < n) strict_finish(ep, __uint_as_float(bits), row, col, out, ldc);
+        }
+}
+
+template <int T>
+static void launch_strict_tile(const float* a, const float* b, void* out, uint32_t ldc, uint32_t m, uint32_t k, uint32_t n, bool b_transposed,
+                               const GemmEpilogue& ep, cudaStream_t stream) {
+    const bool vec_a = k % 4 == 0 && reinterpret_cast<uintptr_t>(a) % 16 == 0;
+    const bool vec_b = (b_transposed ? k : n) % 4 == 0 && reinterpret_cast<uintptr_t>(b) % 16 == 0;
+    const dim3 grid(ceil_div(n, (uint32_t)T), ceil_div(m, (uint32_t)T));
+    if (b_transposed) gemm_strict_tile_kernel<T, true><<<grid, 256, 0, stream>>>(a, b, out, ldc, m, k, n, vec_a, vec_b, 1.0f, ep);
+    else gemm_strict_tile_kernel<T, false><<<grid, 256, 0, stream>>>(a, b, out, ldc, m, k, n, vec_a, vec_b, 1.0f, ep);
 }
 
 // Few rows (decode steps, short prefills): one block per (row, 32 output columns).  The sum of an output is
 // still ONE sequential chain in increasing k -- that is the reference's arithmetic -- but the terms are
 // independent of the chain, so all 512 threads first form the rounded products a[row,p] * b[p,col] side by
 // side into shared memory (every global load of the block is in flight at once), and then one lane per column
-// walks its K products in order.  Same values, same order of additions as gemm_strict_kernel.
+// walks its K products in order.  Same values, same order of additions as gemm_strict_tile_kernel.
 constexpr int SR_COLS = 32, SR_THREADS = 512;
 
 template <bool BT>
@@ -130,23 +167,7 @@ gemm_strict_rows_kernel(const float* __restrict__ a, const float* __restrict__ b
     float sum = 0.0f;
 #pragma unroll 8
     for (uint32_t p = 0; p < k; ++p) sum = sum + prod[p * SR_COLS + threadIdx.x];
-    float v = sum;
-    if (ep.bias) v = v + ep.bias[col];
-    if (ep.activation == ACT_RELU) v = fmaxf(v, 0.0f);
-    else if (ep.activation == ACT_GELU) v = strict_gelu(v);
-    else if (ep.activation == ACT_GELU_TANH) v = strict_gelu_tanh(v);
-    if (ep.scale) v = v * ep.scale[col];
-    if (ep.residual) v = ep.residual[(size_t)row * ep.ldr + col] + v;
-    if (ep.round_bf16) v = round_to_bf16(v);
-    size_t orow = row;
-    if (ep.rows_per_session) {
-        uint32_t off = ep.d_row_offset ? *ep.d_row_offset : ep.row_offset;
-        orow = (size_t)(row / ep.rows_per_session) * ep.out_session_rows + off + row % ep.rows_per_session;
-    }
-    if (ep.out_dtype == TNSR_B200_BF16)
-        reinterpret_cast<bf16*>(out)[orow * ldc + col] = __float2bfloat16_rn(v);
-    else
-        reinterpret_cast<float*>(out)[orow * ldc + col] = v;
+    strict_finish(ep, sum, row, col, out, ldc);
 }
 
 int launch_gemm_strict(const float* a, const float* b, void* out, uint32_t ldc, uint32_t m, uint32_t k,
@@ -170,15 +191,14 @@ int launch_gemm_strict(const float* a, const float* b, void* out, uint32_t ldc, 
         count_launch();
         return check_launch("gemm_strict_rows");
     }
-    dim3 grid(ceil_div(n, ST), ceil_div(m, ST)), block(ST, ST);
-    if (grid.y > 65535u) {
+    // 64 x 64 tiles if there are enough of them for every SM, else 32 x 32
+    const uint64_t tiles = (uint64_t)ceil_div(m, 64u) * ceil_div(n, 64u);
+    if (ceil_div(m, 16u) > 65535u) {
         set_thread_error("strict GEMM: too many rows for one launch");
         return TNSR_B200_ERR_UNSUPPORTED;
     }
-    if (b_transposed)
-        gemm_strict_kernel<true><<<grid, block, 0, stream>>>(a, b, out, ldc, m, k, n, ep);
-    else
-        gemm_strict_kernel<false><<<grid, block, 0, stream>>>(a, b, out, ldc, m, k, n, ep);
+    if (tiles >= 148) launch_strict_tile<64>(a, b, out, ldc, m, k, n, b_transposed, ep, stream);
+    else launch_strict_tile<32>(a, b, out, ldc, m, k, n, b_transposed, ep, stream);
     count_launch();
     return check_launch("gemm_strict");
 }
@@ -235,9 +255,70 @@ layernorm_strict_kernel(const float* __restrict__ x, const float* __restrict__ w
     }
 }
 
+// Many rows: a block owns 32 of them, all threads form the terms of all rows, and the 32 lanes of one warp then walk a row's
+// chain each -- 32 chains in the time of one.
+constexpr uint32_t LR = 32;
+__global__ void __launch_bounds__(256)
+layernorm_strict_rows_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b, float* __restrict__ y,
+                             uint32_t rows, uint32_t width, float eps) {
+    extern __shared__ float smem[];    // [LR][width + 1] values, then as many terms
+    __shared__ float stats[2][LR];
+    const uint32_t pitch = width | 1, row0 = blockIdx.x * LR, n = min(LR, rows - row0), lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+    float* term = smem + LR * pitch;
+    const float nf = (float)width;
+    for (uint32_t r = warp; r < n; r += 8)
+        for (uint32_t c = lane; c < width; c += 32) {
+            const float v = x[(size_t)(row0 + r) * width + c];
+            smem[r * pitch + c] = v;
+            term[r * pitch + c] = v / nf;
+        }
+    __syncthreads();
+    if (threadIdx.x < n) {
+        float mean = 0.0f;
+#pragma unroll 8
+        for (uint32_t c = 0; c < width; ++c) mean = mean + term[threadIdx.x * pitch + c];
+        stats[0][threadIdx.x] = mean;
+    }
+    __syncthreads();
+    for (uint32_t r = warp; r < n; r += 8) {
+        const float mean = stats[0][r];
+        for (uint32_t c = lane; c < width; c += 32) {
+            const float d = smem[r * pitch + c] - mean;
+            const float sq = d * d;
+            term[r * pitch + c] = sq / nf;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < n) {
+        float var = 0.0f;
+#pragma unroll 8
+        for (uint32_t c = 0; c < width; ++c) var = var + term[threadIdx.x * pitch + c];
+        stats[1][threadIdx.x] = strict_expf(strict_logf(var + eps) * -0.5f);
+    }
+    __syncthreads();
+    for (uint32_t r = warp; r < n; r += 8) {
+        const float mean = stats[0][r], inv = stats[1][r];
+        for (uint32_t c = lane; c < width; c += 32) {
+            const float d = smem[r * pitch + c] - mean;
+            y[(size_t)(row0 + r) * width + c] = ((d * inv) * w[c]) + b[c];
+        }
+    }
+}
+
+// From this many rows on blocks of 32 give every SM more than a row's chain at a time.
+constexpr uint32_t LR_MIN_ROWS = 1024;
+
 int launch_layernorm_strict(const float* x, const float* w, const float* b, float* out, uint32_t rows,
                             uint32_t width, float eps, cudaStream_t stream) {
     if (rows == 0) return TNSR_B200_OK;
+    const size_t rows_smem = 2 * (size_t)LR * (width | 1) * sizeof(float);
+    if (rows >= LR_MIN_ROWS && rows_smem <= 100 * 1024) {     // two blocks per SM at least
+        if (rows_smem > 48 * 1024)
+            cudaFuncSetAttribute(layernorm_strict_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem);
+        layernorm_strict_rows_kernel<<<ceil_div(rows, LR), 256, rows_smem, stream>>>(x, w, b, out, rows, width, eps);
+        count_launch();
+        return check_launch("layernorm_strict_rows");
+    }
     size_t smem = 2 * (size_t)width * sizeof(float);
     if (smem > 200 * 1024) {
         set_thread_error("strict LayerNorm: row does not fit shared memory");
@@ -277,13 +358,6 @@ int launch_swiglu_strict(const float* gate, const float* up, float* out, size_t 
 // in the cache, so every key is read from it.  One block per (session, head,
 // query).
 // ---------------------------------------------------------------------------
-template <typename KV>
-__device__ __forceinline__ float kv_load(const KV* p, size_t i);
-template <>
-__device__ __forceinline__ float kv_load<float>(const float* p, size_t i) { return p[i]; }
-template <>
-__device__ __forceinline__ float kv_load<bf16>(const bf16* p, size_t i) { return __bfloat162float(p[i]); }
-
 template <typename KV>
 __global__ void __launch_bounds__(128)
 attention_strict_kernel(const float* __restrict__ q, const KV* __restrict__ kc, const KV* __restrict__ vc,
@@ -343,6 +417,193 @@ attention_strict_kernel(const float* __restrict__ q, const KV* __restrict__ kc, 
     }
 }
 
+// Chunks of new rows: a block owns QT queries of one (session, head).  The keys pass through shared memory 64 at a time, once for
+// the scores and once (the values) for the outputs; every (query, key) and (query, column) is a chain of its own in the reference's
+// order, with HP = head width padded to 32, 64 or 128 deciding how outputs spread over threads: a thread's NI outputs share their
+// column, so a value is loaded once for all of them.  The sums over the keys of a row are walked by one lane per query.
+constexpr uint32_t AT_KEYS = 64;
+
+template <typename KV, int HP, int QT>
+__global__ void __launch_bounds__(256)
+attention_strict_tile_kernel(const float* __restrict__ q, const KV* __restrict__ kc, const KV* __restrict__ vc, float* __restrict__ out,
+                             uint32_t chunk, uint32_t position, const uint32_t* __restrict__ d_position, uint32_t capacity, uint32_t heads,
+                             uint32_t hd, float scale, int round_bf16, uint32_t pitch) {
+    constexpr uint32_t NI = QT * HP / 256, QG = QT / 4;       // outputs of a thread; queries of a thread's scores
+    extern __shared__ __align__(16) float smem[];
+    float* qs = smem;                            // [QT][HP]
+    float* kv = qs + QT * HP;                    // [AT_KEYS][HP + 1]
+    float* sc = kv + AT_KEYS * (HP + 1);         // [QT][pitch]
+    __shared__ float denom[QT];
+    const uint32_t tid = threadIdx.x, lane = tid % 32, warp = tid / 32;
+    // queries with the most keys first
+    const uint32_t t0 = (gridDim.x - 1 - blockIdx.x) * QT, h = blockIdx.y, s = blockIdx.z, n = min((uint32_t)QT, chunk - t0), d = heads * hd;
+    const uint32_t past = d_position ? *d_position : position;
+    const uint32_t total = min(past + t0 + n, capacity);     // keys of the last query; never past the cache
+    auto keys_of = [&](uint32_t i) { return min(past + t0 + min(i, n - 1) + 1, capacity); };
+    const float* qr = q + ((size_t)s * chunk + t0) * d + (size_t)h * hd;
+    for (uint32_t i = tid; i < QT * HP; i += 256) {
+        const uint32_t r = i / HP, c = i % HP;
+        qs[i] = r < n && c < hd ? qr[(size_t)r * d + c] : 0.0f;
+    }
+    const KV* kb = kc + (size_t)s * capacity * d + (size_t)h * hd;
+    const KV* vb = vc + (size_t)s * capacity * d + (size_t)h * hd;
+    auto stage = [&](const KV* base, uint32_t j0) {
+        for (uint32_t i = tid; i < AT_KEYS * HP; i += 256) {
+            const uint32_t r = i / HP, c = i % HP;
+            if (c < hd) kv[r * (HP + 1) + c] = j0 + r < total ? kv_load<KV>(base, (size_t)(j0 + r) * d + c) : 0.0f;
+        }
+    };
+    {
+        const uint32_t key = tid % AT_KEYS, q0 = (tid / AT_KEYS) * QG;
+        for (uint32_t j0 = 0; j0 < total; j0 += AT_KEYS) {
+            __syncthreads();
+            stage(kb, j0);
+            __syncthreads();
+            float sum[QG];
+#pragma unroll
+            for (uint32_t i = 0; i < QG; ++i) sum[i] = 0.0f;
+            uint32_t c = 0;
+            for (; c + 4 <= hd; c += 4) {
+                float kr[4];
+#pragma unroll
+                for (uint32_t e = 0; e < 4; ++e) kr[e] = kv[key * (HP + 1) + c + e];
+#pragma unroll
+                for (uint32_t i = 0; i < QG; ++i) {
+                    const float4 v = *reinterpret_cast<const float4*>(qs + (q0 + i) * HP + c);
+                    sum[i] = sum[i] + v.x * kr[0];
+                    sum[i] = sum[i] + v.y * kr[1];
+                    sum[i] = sum[i] + v.z * kr[2];
+                    sum[i] = sum[i] + v.w * kr[3];
+                }
+            }
+            for (; c < hd; ++c)
+#pragma unroll
+                for (uint32_t i = 0; i < QG; ++i) sum[i] = sum[i] + qs[(q0 + i) * HP + c] * kv[key * (HP + 1) + c];
+            if (j0 + key < total)
+#pragma unroll
+                for (uint32_t i = 0; i < QG; ++i) {
+                    float v = sum[i] * scale;
+                    v = v + 0.0f;  // the mask term of visible keys
+                    sc[(q0 + i) * pitch + j0 + key] = v;
+                }
+        }
+    }
+    __syncthreads();
+    for (uint32_t i = warp; i < n; i += 8) {
+        const uint32_t keys = keys_of(i);
+        float mx = -INFINITY;
+        for (uint32_t j = lane; j < keys; j += 32) mx = fmaxf(mx, sc[i * pitch + j]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        for (uint32_t j = lane; j < keys; j += 32) sc[i * pitch + j] = strict_expf(sc[i * pitch + j] - mx);
+    }
+    __syncthreads();
+    if (tid < n) {
+        const uint32_t keys = keys_of(tid);
+        const float* row = sc + tid * pitch;
+        float sum = 0.0f;
+        uint32_t j = 0;
+        for (; j + 4 <= keys; j += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(row + j);
+            sum = sum + v.x;
+            sum = sum + v.y;
+            sum = sum + v.z;
+            sum = sum + v.w;
+        }
+        for (; j < keys; ++j) sum = sum + row[j];
+        denom[tid] = sum;
+    }
+    __syncthreads();
+    for (uint32_t i = warp; i < n; i += 8) {
+        const uint32_t keys = keys_of(i);
+        for (uint32_t j = lane; j < keys; j += 32) sc[i * pitch + j] = sc[i * pitch + j] / denom[i];
+    }
+    float acc[NI];
+    uint32_t keys[NI];
+#pragma unroll
+    for (uint32_t i = 0; i < NI; ++i) {
+        acc[i] = 0.0f;
+        keys[i] = keys_of(tid / HP + i * (256 / HP));
+    }
+    const uint32_t col = tid % HP, qi = tid / HP;
+    const uint32_t least = keys_of(0);           // every query of the block sees these
+    for (uint32_t j0 = 0; j0 < total; j0 += AT_KEYS) {
+        __syncthreads();
+        stage(vb, j0);
+        __syncthreads();
+        const uint32_t end = min(AT_KEYS, total - j0);
+        uint32_t j = 0;
+        for (; j + 4 <= end && j0 + j + 4 <= least; j += 4) {
+            float v[4];
+#pragma unroll
+            for (uint32_t e = 0; e < 4; ++e) v[e] = kv[(j + e) * (HP + 1) + col];
+#pragma unroll
+            for (uint32_t i = 0; i < NI; ++i) {
+                const float4 p = *reinterpret_cast<const float4*>(sc + (qi + i * (256 / HP)) * pitch + j0 + j);
+                acc[i] = acc[i] + p.x * v[0];
+                acc[i] = acc[i] + p.y * v[1];
+                acc[i] = acc[i] + p.z * v[2];
+                acc[i] = acc[i] + p.w * v[3];
+            }
+        }
+        for (; j < end; ++j) {
+            const float v = kv[j * (HP + 1) + col];
+#pragma unroll
+            for (uint32_t i = 0; i < NI; ++i)
+                if (j0 + j < keys[i]) acc[i] = acc[i] + sc[(qi + i * (256 / HP)) * pitch + j0 + j] * v;
+        }
+    }
+    if (col >= hd) return;
+#pragma unroll
+    for (uint32_t i = 0; i < NI; ++i) {
+        const uint32_t r = qi + i * (256 / HP);
+        if (r < n) out[((size_t)s * chunk + t0 + r) * d + (size_t)h * hd + col] = round_bf16 ? round_to_bf16(acc[i]) : acc[i];
+    }
+}
+
+// Shared memory of a block, or 0 if the scores of its queries do not fit.
+template <int HP, int QT>
+static size_t strict_tile_smem(uint32_t longest, uint32_t* pitch) {
+    *pitch = (longest + 3) / 4 * 4 + 4;          // 16-byte rows that do not all start in the same bank
+    const size_t bytes = ((size_t)QT * HP + AT_KEYS * (HP + 1) + (size_t)QT * *pitch) * sizeof(float);
+    return bytes <= 200 * 1024 ? bytes : 0;
+}
+
+template <typename KV, int HP, int QT>
+static bool launch_strict_tile_attention(const float* q, const void* kc, const void* vc, float* out, uint32_t sessions, uint32_t chunk, uint32_t position,
+                                         const uint32_t* d_position, uint32_t capacity, uint32_t heads, uint32_t hd, float scale, int round_bf16,
+                                         cudaStream_t stream) {
+    uint32_t pitch;
+    const size_t smem = strict_tile_smem<HP, QT>(d_position ? capacity : std::min(capacity, position + chunk), &pitch);
+    if (!smem) return false;
+    if (smem > 48 * 1024)
+        cudaFuncSetAttribute(attention_strict_tile_kernel<KV, HP, QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    attention_strict_tile_kernel<KV, HP, QT><<<dim3(ceil_div(chunk, (uint32_t)QT), heads, sessions), 256, smem, stream>>>(
+        q, (const KV*)kc, (const KV*)vc, out, chunk, position, d_position, capacity, heads, hd, scale, round_bf16, pitch);
+    return true;
+}
+
+// 32 queries per block, or 8 where the scores of 32 do not fit (contexts from about 1400 keys) or too few blocks would run.
+template <typename KV, int HP>
+static bool launch_strict_tile_width(const float* q, const void* kc, const void* vc, float* out, uint32_t sessions, uint32_t chunk, uint32_t position,
+                                     const uint32_t* d_position, uint32_t capacity, uint32_t heads, uint32_t hd, float scale, int round_bf16,
+                                     cudaStream_t stream) {
+    if ((uint64_t)ceil_div(chunk, 32u) * heads * sessions >= 148 &&
+        launch_strict_tile_attention<KV, HP, 32>(q, kc, vc, out, sessions, chunk, position, d_position, capacity, heads, hd, scale, round_bf16, stream))
+        return true;
+    return launch_strict_tile_attention<KV, HP, 8>(q, kc, vc, out, sessions, chunk, position, d_position, capacity, heads, hd, scale, round_bf16, stream);
+}
+
+template <typename KV>
+static bool launch_strict_tile_any(const float* q, const void* kc, const void* vc, float* out, uint32_t sessions, uint32_t chunk, uint32_t position,
+                                   const uint32_t* d_position, uint32_t capacity, uint32_t heads, uint32_t hd, float scale, int round_bf16,
+                                   cudaStream_t stream) {
+    if (chunk < 2 || hd > 128 || heads > 65535u || sessions > 65535u) return false;
+    if (hd <= 32) return launch_strict_tile_width<KV, 32>(q, kc, vc, out, sessions, chunk, position, d_position, capacity, heads, hd, scale, round_bf16, stream);
+    if (hd <= 64) return launch_strict_tile_width<KV, 64>(q, kc, vc, out, sessions, chunk, position, d_position, capacity, heads, hd, scale, round_bf16, stream);
+    return launch_strict_tile_width<KV, 128>(q, kc, vc, out, sessions, chunk, position, d_position, capacity, heads, hd, scale, round_bf16, stream);
+}
+
 int launch_attention_strict(const float* q, const void* k_cache, const void* v_cache, float* out,
                             uint32_t sessions, uint32_t chunk, uint32_t position,
                             const uint32_t* d_position, uint32_t capacity, uint32_t heads,
@@ -359,6 +620,12 @@ int launch_attention_strict(const float* q, const void* k_cache, const void* v_c
     if (blocks > 0x7fffffffull) {
         set_thread_error("strict attention: too many queries for one launch");
         return TNSR_B200_ERR_UNSUPPORTED;
+    }
+    if (kv_dtype == TNSR_B200_BF16
+            ? launch_strict_tile_any<bf16>(q, k_cache, v_cache, out, sessions, chunk, position, d_position, capacity, heads, head_dim, scale, round_bf16, stream)
+            : launch_strict_tile_any<float>(q, k_cache, v_cache, out, sessions, chunk, position, d_position, capacity, heads, head_dim, scale, round_bf16, stream)) {
+        count_launch();
+        return check_launch("attention_strict_tile");
     }
     if (kv_dtype == TNSR_B200_BF16) {
         if (smem > 48 * 1024)
