@@ -673,6 +673,34 @@ def test_strict_chunks_have_the_bits_of_single_tokens(heads, width, batch, preci
         assert np.array_equal(logits(cuts), single)
 
 
+@pytest.mark.parametrize("vocab,batch,width,hidden", [(2100, 3, 128, 520), (130, 9, 256, 1024), (50, 1, 16, 4)])
+def test_strict_step_in_one_launch_has_the_bits_of_the_operators(vocab, batch, width, hidden):
+    """Small f32 sessions take a step (here 1 to 5 rows per session) as one launch of a cluster of 16 CTAs: heads beyond its output
+    head's vocabulary, phases of more than 32 columns per CTA, of fewer than one, logits of the last rows only and greedy ids, against
+    one long chunk, which runs operator by operator."""
+    cfg = GptConfig(vocab_size=vocab, max_sequence_length=96, embed_dim=width, num_heads=2, feed_forward_dim=hidden, num_layers=3,
+                    layer_norm_epsilon=1e-5, activation="gelu")
+    arrays = normal_model_arrays(cfg, seed=41, std=0.2, bias_std=0.1)
+    ids = np.random.default_rng(42).integers(0, vocab, size=(batch, 60)).astype(np.uint32)
+
+    def session(mode):
+        s = B200Session(cfg, batch, 96, logits_mode=mode)
+        for i, a in enumerate(arrays):
+            s.refresh(i, a)
+        return s
+
+    s = session("all")
+    want = s.decode_full(ids, 0)[0].reshape(batch, 60, vocab)
+    s.close()
+    s, at = session("last"), 0
+    for n in [1, 1, 2, 3, 5, 1, 17, 4, 1, 1]:
+        logits, greedy = s.decode_full(ids[:, at:at + n], at)
+        at += n
+        assert np.array_equal(logits.reshape(batch, vocab).view(np.uint32), want[:, at - 1].view(np.uint32))
+        assert greedy.tolist() == [argmax_last(r) for r in want[:, at - 1]]
+    s.close()
+
+
 def test_paged_kv_cache_gives_the_same_bits_as_the_contiguous_one():
     """kv_page_rows > 0: every cache tensor is a pool of pages handed to sessions on demand.  Same kernels, other
     addresses: prefill (non-tiled scan in both handles), graph-replayed steps, ragged steps and the cache read back in

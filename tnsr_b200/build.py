@@ -4,8 +4,8 @@
 
 Every ``.cu`` file is compiled with ``-gencode arch=compute_100a,code=sm_100a``
 and linked into one shared library whose only exports are the ``extern "C"``
-entry points of ``include/tnsr_b200.h``.  ``strict.cu`` and ``encoder.cu`` are
-compiled with ``--fmad=false``: their kernels must round every product before
+entry points of ``include/tnsr_b200.h``.  ``strict.cu``, ``strict_step.cu`` and
+``encoder.cu`` are compiled with ``--fmad=false``: their kernels must round every product before
 adding it.
 """
 from __future__ import annotations
@@ -23,11 +23,11 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "build")
 LIB = os.path.join(CSRC, "libtnsr_b200.so")
 
-SOURCES = ["decoder.cu", "ops_api.cu", "elementwise.cu", "strict.cu", "gemm.cu", "gemm_skinny.cu", "attention.cu", "prefill.cu", "prefill_tc.cu",
+SOURCES = ["decoder.cu", "ops_api.cu", "elementwise.cu", "strict.cu", "strict_step.cu", "gemm.cu", "gemm_skinny.cu", "attention.cu", "prefill.cu", "prefill_tc.cu",
            "decode_attention_static.cu", "sampler.cu", "encoder.cu", "decode_tail.cu", "gemm_stream.cu",
            "layer_stack.cu", "mixer_attention.cu", "grouped_attention.cu", "mixer_mamba2.cu", "ssd_scan.cu", "mixer_hgrn2.cu", "hgrn2_scan.cu",
            "mixer_rglru.cu", "feed_forward.cu", "gemm_grouped.cu"]
-EXTRA = {"strict.cu": ["--fmad=false"], "encoder.cu": ["--fmad=false"]}
+EXTRA = {name: ["--fmad=false"] for name in ("strict.cu", "strict_step.cu", "encoder.cu")}
 
 BASE_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

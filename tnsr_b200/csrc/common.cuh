@@ -293,6 +293,27 @@ int launch_attention_strict(const float* q, const void* k_cache, const void* v_c
                             const uint32_t* d_position, uint32_t capacity, uint32_t heads,
                             uint32_t head_dim, int kv_dtype, int round_bf16, cudaStream_t stream);
 
+// A whole step of a small f32 session (relu or gelu blocks) in one launch (strict_step.cu).  logits: [sessions, vocab] of the last
+// rows (last_only) or [sessions * chunk, vocab]; nullptr: the launch ends with the last layer, rows in h.
+constexpr uint32_t SS_MAX_LAYERS = 20;     // their pointers travel as kernel parameters
+struct StrictStepLayer {
+    const float *ln1w, *ln1b, *wq, *bq, *wk, *bk, *wv, *bv, *wo, *bo, *ln2w, *ln2b, *w_in, *b_in, *w_out, *b_out;
+    void *kcache, *vcache;
+};
+struct StrictStepArgs {
+    const float *tok, *pos, *fnw, *fnb;
+    const uint32_t* ids;
+    float *h, *logits;                     // h: the last layer's rows, if logits is null
+    int* d_status;
+    uint32_t sessions, chunk, position, capacity, vocab, d, f, heads, num_layers;
+    float eps, scale;
+    int activation, round_bf16, last_only;
+    StrictStepLayer layers[SS_MAX_LAYERS];
+};
+bool strict_step_supported(const StrictStepArgs& a, bool kv_bf16);
+bool strict_step_has_head(uint32_t vocab);
+int launch_strict_step(const StrictStepArgs& a, bool kv_bf16, cudaStream_t stream);
+
 // bf16 attention for any head_dim and chunk (online softmax, one warp per query/head).
 int launch_attention_generic(const bf16* q, const bf16* k_cache, const bf16* v_cache, bf16* out,
                              uint32_t sessions, uint32_t chunk, uint32_t position,

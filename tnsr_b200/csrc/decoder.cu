@@ -224,9 +224,37 @@ int reserve_uniform(tnsr_b200_decoder* dec, uint32_t rows_needed) {
 }
 
 // ---- one step on the strict f32 path -----------------------------------------
-// `d_position` (optional): the position as a device scalar, for replay from a captured graph.
-int step_strict(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chunk, uint32_t position,
-                const uint32_t* d_position, uint32_t logit_rows) {
+// The step as one launch, if the session is small enough for that (strict_step.cu); its position comes from the host.
+bool fused_strict_args(const tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chunk, uint32_t position, uint32_t logit_rows, StrictStepArgs* a) {
+    const tnsr_b200_config& c = dec->cfg;
+    if (dec->bf16_path || dec->stack || dec->swiglu || dec->layers.size() > SS_MAX_LAYERS || debug_sync_enabled()) return false;
+    a->tok = (const float*)dec->tok; a->pos = (const float*)dec->pos; a->fnw = dec->fnw; a->fnb = dec->fnb;
+    a->ids = d_tokens;
+    a->h = dec->h;
+    a->logits = strict_step_has_head(c.vocab_size) ? dec->logits : nullptr;
+    a->d_status = dec->d_status;
+    a->sessions = c.batch; a->chunk = chunk; a->position = position; a->capacity = c.capacity; a->vocab = c.vocab_size;
+    a->d = c.embed_dim; a->f = c.feed_forward_dim; a->heads = c.num_heads; a->num_layers = c.num_layers;
+    a->eps = c.layer_norm_epsilon;
+    a->scale = 1.0f / sqrtf((float)c.embed_dim / (float)c.num_heads);
+    a->activation = c.activation == TNSR_B200_ACT_GELU ? ACT_GELU : ACT_RELU;
+    a->round_bf16 = dec->kv_bf16;
+    a->last_only = logit_rows != c.batch * chunk;
+    for (uint32_t l = 0; l < c.num_layers; ++l) {
+        const Layer& L = dec->layers[l];
+        StrictStepLayer& o = a->layers[l];
+        o.ln1w = L.ln1w; o.ln1b = L.ln1b; o.ln2w = L.ln2w; o.ln2b = L.ln2b;
+        o.wq = (const float*)L.wq; o.wk = (const float*)L.wk; o.wv = (const float*)L.wv; o.wo = (const float*)L.wo;
+        o.bq = L.bq; o.bk = L.bk; o.bv = L.bv; o.bo = L.bo;
+        o.w_in = (const float*)L.w_in; o.b_in = L.b_in; o.w_out = (const float*)L.w_out; o.b_out = L.b_out;
+        o.kcache = L.kcache; o.vcache = L.vcache;
+    }
+    return strict_step_supported(*a, dec->kv_bf16);
+}
+
+// Embedding and all layers, one launch per operator.  `d_position` (optional): the position as a device scalar, for replay from a
+// captured graph.
+int strict_layers(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chunk, uint32_t position, const uint32_t* d_position) {
     const tnsr_b200_config& c = dec->cfg;
     const uint32_t d = c.embed_dim, f = c.feed_forward_dim, H = c.num_heads, B = c.batch, rows = B * chunk;
     cudaStream_t st = dec->stream;
@@ -268,6 +296,23 @@ int step_strict(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chunk
         GemmEpilogue ef; ef.bias = L.b_out; ef.residual = dec->h; ef.ldr = d;
         RUN(dec, launch_gemm_strict(ff, (const float*)L.w_out, dec->h, d, rows, f, d, false, ef, st));
     }
+    return TNSR_B200_OK;
+}
+
+int step_strict(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chunk, uint32_t position,
+                const uint32_t* d_position, uint32_t logit_rows) {
+    const tnsr_b200_config& c = dec->cfg;
+    const uint32_t d = c.embed_dim, B = c.batch, rows = B * chunk;
+    cudaStream_t st = dec->stream;
+    StrictStepArgs fused;
+    const bool one_launch = !d_position && fused_strict_args(dec, d_tokens, chunk, position, logit_rows, &fused);
+    if (one_launch) {
+        RUN(dec, launch_strict_step(fused, dec->kv_bf16, st));
+        if (fused.logits) return TNSR_B200_OK;
+    } else {
+        RUN(dec, strict_layers(dec, d_tokens, chunk, position, d_position));
+    }
+    float* n = (float*)dec->n;
     const float* src = dec->h;
     if (logit_rows != rows) {
         RUN(dec, launch_gather_last_rows(dec->h, dec->hl, B, chunk, d, st));
@@ -562,7 +607,9 @@ int run_step_direct(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t c
 // One step.  Single-token steps are captured once per (ids pointer, output pointer) pair and replayed: the
 // kernels read the position from dec->d_pos, which a one-thread kernel sets before each replay.
 int run_step(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chunk, uint32_t position, uint32_t* d_argmax_out) {
-    const bool graphable = dec->use_graphs && chunk == 1 && !dec->profile_attention && dec->stepped_once && !debug_sync_enabled();
+    bool graphable = dec->use_graphs && chunk == 1 && !dec->profile_attention && dec->stepped_once && !debug_sync_enabled();
+    StrictStepArgs fused;   // a step that is one launch anyway: a graph and the launch that sets its position would be two
+    if (graphable && !dec->bf16_path && !dec->stack) graphable = !fused_strict_args(dec, d_tokens, 1, position, dec->cfg.batch, &fused);
     if (!graphable) {
         int rc = run_step_direct(dec, d_tokens, chunk, position, nullptr, d_argmax_out);
         if (rc == TNSR_B200_OK && chunk == 1) dec->stepped_once = true;

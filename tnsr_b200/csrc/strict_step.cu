@@ -1,0 +1,460 @@
+// A whole step of a small f32 session in one launch: embedding, every layer, final LayerNorm and output head.
+//
+// A step of the character model (4 layers of 128 columns) is 38 short kernels one behind the other, each about 3 us of launch, of one
+// or two dependent trips to L2 and of one chain of additions (the reference's order allows no other: 128 to 512 sums of 4 cycles).
+// Here a cluster of 16 CTAs takes whole sessions through the step: a layer is five phases (LayerNorm and q/k/v, attention, output
+// projection, LayerNorm and first feed-forward matrix, second matrix), every CTA owns a sixteenth of a phase's output columns and
+// stores them into the shared memory of all sixteen, and the phases meet at the cluster's hardware barrier (180 cycles; through global
+// memory the stores took 1100 cycles to be visible and the loads 1500 to come back).  The weights of a CTA's next columns are on
+// their way while it waits there.  Sessions do not depend on each other, so clusters never wait for one another.
+//
+// Arithmetic is strict.cu's, operation by operation: all threads form the rounded products of an output side by side in shared
+// memory, one lane per output adds them up in order.  What is left is chains: sums, and the f64 exp and log of a LayerNorm and of the
+// scores.  One step of one session at 4 x 128 columns and 60 keys, ids in to logits out, B200: 197 us in 38 launches, 125 us here; 48
+// sessions 246 and 154 us.
+#include <algorithm>
+
+#include "strict.cuh"
+
+namespace tb {
+
+namespace {
+
+constexpr uint32_t SS_CTAS = 16, SS_THREADS = 512, SS_WARPS = SS_THREADS / 32;
+constexpr uint32_t SS_COLS = 32;            // columns a CTA works on at a time: one lane each
+constexpr uint32_t SS_MAX_D = 256;
+constexpr uint32_t SS_SMEM = 200 * 1024;
+constexpr uint32_t SS_VALUES = 8192;        // weight x value products of a head in shared memory at a time
+
+struct SsParams {
+    StrictStepArgs a;
+    uint32_t sessions_per_cluster;
+};
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
+// Stores v where `local` lies, in the shared memory of every CTA of the cluster.
+__device__ __forceinline__ void store_to_all(float* local, float v) {
+    const uint32_t at = (uint32_t)__cvta_generic_to_shared(local);
+#pragma unroll
+    for (uint32_t peer = 0; peer < SS_CTAS; ++peer) {
+        uint32_t remote;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at), "r"(peer));
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
+    }
+}
+
+// The matrix of a phase: [k, n] row-major; q, k and v are three of `width` columns each side by side.
+struct Matrix {
+    const float *w0, *w1, *w2;
+    uint32_t k, n, width;
+    __device__ __forceinline__ const float* column(uint32_t j) const { return j < width ? w0 + j : j < 2 * width ? w1 + (j - width) : w2 + (j - 2 * width); }
+};
+
+// A CTA's share of a phase: columns [col0, col0 + cols) of n, at most SS_COLS of them at a time; in shared memory there is room for
+// 1 << log2_pad of them, each with its k products in order (row pitch k + 4: 16-byte accesses of neighbouring lanes do not collide).
+struct Share {
+    uint32_t col0, cols, log2_pad;
+};
+__device__ __forceinline__ uint32_t per_cta(uint32_t n) { return (n + SS_CTAS - 1) / SS_CTAS; }
+__device__ __forceinline__ Share share_of(uint32_t n, uint32_t rank, uint32_t round) {
+    const uint32_t per = per_cta(n), first = rank * per + round * SS_COLS, end = min(n, (rank + 1) * per), room = min(per, SS_COLS);
+    return {first, first < end ? min(SS_COLS, end - first) : 0u, room <= 1 ? 0u : 32u - __clz(room - 1)};
+}
+
+// Four weights of one column, one below the other.
+__device__ __forceinline__ float4 weights4(const float* w, uint32_t ld) { return make_float4(__ldg(w), __ldg(w + ld), __ldg(w + 2 * (size_t)ld), __ldg(w + 3 * (size_t)ld)); }
+
+// Thread t forms the products of column t % pad, four rows of the matrix at a time, groups of four dealt over the threads.  The first
+// two groups are asked for before the phase's barrier.
+__device__ __forceinline__ void ask_weights(const Matrix& m, const Share& s, float4 (&ahead)[2]) {
+    const uint32_t c = threadIdx.x & ((1u << s.log2_pad) - 1), g = threadIdx.x >> s.log2_pad, groups = SS_THREADS >> s.log2_pad;
+    if (c >= s.cols) return;
+    const float* w = m.column(s.col0 + c);
+#pragma unroll
+    for (uint32_t i = 0; i < 2; ++i)
+        if (4 * (g + i * groups) < m.k) ahead[i] = weights4(w + (size_t)4 * (g + i * groups) * m.width, m.width);
+}
+__device__ __forceinline__ void form_products(const Matrix& m, const Share& s, const float4 (&ahead)[2], bool use_ahead, const float* xs, float* prod,
+                                              uint32_t rows) {
+    const uint32_t c = threadIdx.x & ((1u << s.log2_pad) - 1), g = threadIdx.x >> s.log2_pad, groups = SS_THREADS >> s.log2_pad, k = m.k;
+    if (c >= s.cols) return;
+    const float* w = m.column(s.col0 + c);
+    float* mine = prod + c * (k + 4);
+    const uint32_t row_pitch = (k + 4) << s.log2_pad;
+    auto put = [&](uint32_t p, const float4& v) {
+        for (uint32_t r = 0; r < rows; ++r) {
+            const float4 x = *reinterpret_cast<const float4*>(xs + r * k + p);
+            *reinterpret_cast<float4*>(mine + r * row_pitch + p) = make_float4(x.x * v.x, x.y * v.y, x.z * v.z, x.w * v.w);
+        }
+    };
+    uint32_t p = 4 * g;
+    if (use_ahead) {
+#pragma unroll
+        for (uint32_t i = 0; i < 2; ++i, p += 4 * groups)
+            if (p < k) put(p, ahead[i]);
+    }
+    for (; p < k; p += 4 * groups) put(p, weights4(w + (size_t)p * m.width, m.width));
+}
+
+// sum of terms[0 .. n) in order from a zero start, n a multiple of 4 (16-byte aligned): sixteen loads ahead of sixteen sums.
+__device__ __forceinline__ float add_up(const float* terms, uint32_t n) {
+    const float4* t = reinterpret_cast<const float4*>(terms);
+    float sum = 0.0f;
+    float4 v[4];
+    const uint32_t quads = n / 4, whole = quads & ~3u;
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i) v[i] = t[min(i, quads - 1)];
+    for (uint32_t q = 0; q < whole; q += 4) {
+        float4 u[4];
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) u[i] = t[min(q + 4 + i, quads - 1)];
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) {
+            sum = sum + v[i].x;
+            sum = sum + v[i].y;
+            sum = sum + v[i].z;
+            sum = sum + v[i].w;
+            v[i] = u[i];
+        }
+    }
+    for (uint32_t q = whole; q < quads; ++q) {
+        const float4 x = t[q];
+        sum = sum + x.x;
+        sum = sum + x.y;
+        sum = sum + x.z;
+        sum = sum + x.w;
+    }
+    return sum;
+}
+
+// LayerNorm of row r (x + r * d) by warp r, in strict.cu's order, into xs; `term`: d floats per row.
+__device__ __forceinline__ void norm_rows(float* xs, float* term, const float* x, uint32_t stride, const float* __restrict__ w, const float* __restrict__ b,
+                                          uint32_t rows, uint32_t d, float eps) {
+    const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    if (warp >= rows) return;
+    constexpr uint32_t V = SS_MAX_D / 32;
+    const float nf = (float)d;
+    float v[V], wv[V], bv[V];
+    float* mine = term + warp * d;
+#pragma unroll
+    for (uint32_t i = 0; i < V; ++i) {
+        const uint32_t c = lane + 32 * i;
+        wv[i] = c < d ? __ldg(w + c) : 0.0f;
+        bv[i] = c < d ? __ldg(b + c) : 0.0f;
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < V; ++i)
+        if (lane + 32 * i < d) {
+            v[i] = x[warp * stride + lane + 32 * i];
+            mine[lane + 32 * i] = v[i] / nf;
+        }
+    __syncwarp();
+    const float mean = __shfl_sync(0xffffffffu, lane == 0 ? add_up(mine, d) : 0.0f, 0);
+    __syncwarp();
+#pragma unroll
+    for (uint32_t i = 0; i < V; ++i)
+        if (lane + 32 * i < d) {
+            const float c = v[i] - mean;
+            const float sq = c * c;
+            mine[lane + 32 * i] = sq / nf;
+        }
+    __syncwarp();
+    const float var = __shfl_sync(0xffffffffu, lane == 0 ? add_up(mine, d) : 0.0f, 0);
+    const float inv = strict_expf(strict_logf(var + eps) * -0.5f);
+#pragma unroll
+    for (uint32_t i = 0; i < V; ++i)
+        if (lane + 32 * i < d) {
+            const float c = v[i] - mean;
+            xs[warp * d + lane + 32 * i] = ((c * inv) * wv[i]) + bv[i];
+        }
+}
+
+__device__ __forceinline__ float4 load_kv4(const float* p) { return __ldcg(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ float4 load_kv4(const bf16* p) {
+    const uint2 v = __ldcg(reinterpret_cast<const uint2*>(p));
+    return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+}
+
+// Attention of one (row, head) by the whole CTA, in the order of attention_strict_kernel: thread c < head width returns output c.
+// `scratch`: scores, then products.
+template <typename KV>
+__device__ __forceinline__ float attend(const StrictStepArgs& a, const KV* kb, const KV* vb, const float* qs, uint32_t total, float* scratch) {
+    __shared__ float red[SS_WARPS + 1];
+    const uint32_t tid = threadIdx.x, lane = tid % 32, warp = tid / 32, hd = a.d / a.heads, quads = hd / 4, d = a.d;
+    float* sc = scratch;
+    float* prod = sc + (total + 3) / 4 * 4;
+    const uint32_t tile = SS_VALUES / hd;            // keys whose products fit
+    // the first values are asked for before anything else
+    float4 early[2];
+#pragma unroll
+    for (uint32_t i = 0; i < 2; ++i) {
+        const uint32_t e = tid + i * SS_THREADS;
+        if (e < min(total, tile) * quads) early[i] = load_kv4(vb + (size_t)(e / quads) * d + 4 * (e % quads));
+    }
+    float mx = -INFINITY;
+    for (uint32_t j = tid; j < total; j += SS_THREADS) {
+        float sum = 0.0f;
+        const KV* row = kb + (size_t)j * d;
+#pragma unroll 8
+        for (uint32_t c = 0; c < hd; c += 4) {
+            const float4 k = load_kv4(row + c), v = *reinterpret_cast<const float4*>(qs + c);
+            sum = sum + v.x * k.x;
+            sum = sum + v.y * k.y;
+            sum = sum + v.z * k.z;
+            sum = sum + v.w * k.w;
+        }
+        float v = sum * a.scale;
+        v = v + 0.0f;  // the mask term of visible keys
+        sc[j] = v;
+        mx = fmaxf(mx, v);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if (lane == 0) red[warp] = mx;
+    __syncthreads();
+    mx = red[0];
+#pragma unroll
+    for (uint32_t w = 1; w < SS_WARPS; ++w) mx = fmaxf(mx, red[w]);
+    for (uint32_t j = tid; j < total; j += SS_THREADS) sc[j] = strict_expf(sc[j] - mx);
+    __syncthreads();
+    if (tid == 0) {
+        float sum = total >= 4 ? add_up(sc, total & ~3u) : 0.0f;
+        for (uint32_t j = total & ~3u; j < total; ++j) sum = sum + sc[j];
+        red[SS_WARPS] = sum;
+    }
+    __syncthreads();
+    const float denom = red[SS_WARPS];
+    for (uint32_t j = tid; j < total; j += SS_THREADS) sc[j] = sc[j] / denom;
+    __syncthreads();
+    float acc = 0.0f;
+    for (uint32_t j0 = 0; j0 < total; j0 += tile) {
+        const uint32_t keys = min(tile, total - j0);
+        if (j0) __syncthreads();
+        auto put = [&](uint32_t e, const float4& v) {
+            const float p = sc[j0 + e / quads];
+            reinterpret_cast<float4*>(prod)[e] = make_float4(p * v.x, p * v.y, p * v.z, p * v.w);
+        };
+        uint32_t e = tid;
+        if (j0 == 0) {
+#pragma unroll
+            for (uint32_t i = 0; i < 2; ++i, e += SS_THREADS)
+                if (e < keys * quads) put(e, early[i]);
+        }
+        for (; e < keys * quads; e += SS_THREADS) put(e, load_kv4(vb + (size_t)(j0 + e / quads) * d + 4 * (e % quads)));
+        __syncthreads();
+        if (tid < hd) {
+            float v[16];
+#pragma unroll
+            for (uint32_t i = 0; i < 16; ++i) v[i] = prod[min(i, keys - 1) * hd + tid];
+            uint32_t j = 0;
+            for (; j + 16 <= keys; j += 16) {
+                float u[16];
+#pragma unroll
+                for (uint32_t i = 0; i < 16; ++i) u[i] = prod[min(j + 16 + i, keys - 1) * hd + tid];
+#pragma unroll
+                for (uint32_t i = 0; i < 16; ++i) { acc = acc + v[i]; v[i] = u[i]; }
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < 16; ++i)
+                if (j + i < keys) acc = acc + v[i];
+        }
+    }
+    __syncthreads();
+    return a.round_bf16 ? round_to_bf16(acc) : acc;
+}
+
+// Shared floats of one row: residual, queries, attention output, normalised row, its terms, hidden row.
+__host__ __device__ __forceinline__ uint32_t floats_per_row(uint32_t d, uint32_t f) { return 5 * d + f; }
+
+template <typename KV>
+__global__ void __launch_bounds__(SS_THREADS, 1)
+strict_step_kernel(const __grid_constant__ SsParams P) {
+    extern __shared__ __align__(16) float smem[];
+    const StrictStepArgs& a = P.a;
+    const uint32_t rank = blockIdx.x % SS_CTAS, cluster = blockIdx.x / SS_CTAS, tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+    const uint32_t s0 = cluster * P.sessions_per_cluster, ns = min(P.sessions_per_cluster, a.sessions - s0);
+    const uint32_t row0 = s0 * a.chunk, rows = ns * a.chunk, d = a.d, f = a.f, hd = d / a.heads;
+    float* h = smem;                         // [rows][d] each
+    float* q = h + rows * d;
+    float* att = q + rows * d;
+    float* xs = att + rows * d;
+    float* term = xs + rows * d;
+    float* ff = term + rows * d;             // [rows][f]
+    float* prod = ff + rows * f;
+    float4 ahead[2];
+
+    for (uint32_t r = 0; r < rows; ++r) {    // every CTA keeps the residual rows
+        const uint32_t id = a.ids[row0 + r], position = a.position + r % a.chunk;
+        if (id >= a.vocab && tid == 0 && rank == 0) atomicCAS(a.d_status, DEV_OK, DEV_TOKEN_RANGE);
+        for (uint32_t c = tid; c < d; c += SS_THREADS) h[r * d + c] = id < a.vocab ? a.tok[(size_t)id * d + c] + a.pos[(size_t)position * d + c] : 0.0f;
+    }
+    __syncthreads();
+    cluster_arrive();
+    // One phase: rows of k values (the LayerNorm of h, or `src`) times the CTA's columns; `store` takes the sums.
+    auto phase = [&](const Matrix& m, const float* src, const float* lnw, const float* lnb, auto&& store) {
+        ask_weights(m, share_of(m.n, rank, 0), ahead);
+        cluster_wait();
+        if (lnw) norm_rows(xs, term, h, d, lnw, lnb, rows, d, a.eps);
+        const float* x = lnw ? xs : src;
+        const uint32_t rounds = (per_cta(m.n) + SS_COLS - 1) / SS_COLS;
+        for (uint32_t round = 0; round < rounds; ++round) {
+            const Share s = share_of(m.n, rank, round);
+            __syncthreads();
+            form_products(m, s, ahead, round == 0, x, prod, rows);
+            __syncthreads();
+            if (warp < rows && lane < s.cols) store(warp, s.col0 + lane, add_up(prod + (((warp << s.log2_pad) + lane) * (m.k + 4)), m.k));
+        }
+        cluster_arrive();
+    };
+    for (uint32_t l = 0; l < a.num_layers; ++l) {
+        const StrictStepLayer& L = P.a.layers[l];
+        KV* kcache = reinterpret_cast<KV*>(L.kcache);
+        KV* vcache = reinterpret_cast<KV*>(L.vcache);
+        phase(Matrix{L.wq, L.wk, L.wv, d, 3 * d, d}, nullptr, L.ln1w, L.ln1b, [&](uint32_t r, uint32_t col, float sum) {
+            const uint32_t part = col < d ? 0 : col < 2 * d ? 1 : 2, c = col - part * d;
+            float v = sum + (part == 0 ? L.bq : part == 1 ? L.bk : L.bv)[c];
+            if (a.round_bf16) v = round_to_bf16(v);
+            if (part == 0) {
+                store_to_all(q + r * d + c, v);
+            } else {
+                KV* cache = part == 1 ? kcache : vcache;
+                const size_t at = ((size_t)(s0 + r / a.chunk) * a.capacity + a.position + r % a.chunk) * d + c;
+                if constexpr (sizeof(KV) == 2) cache[at] = __float2bfloat16_rn(v);
+                else cache[at] = v;
+            }
+        });
+        cluster_wait();
+        for (uint32_t i = rank; i < rows * a.heads; i += SS_CTAS) {
+            const uint32_t r = i / a.heads, head = i % a.heads;
+            const size_t base = (size_t)(s0 + r / a.chunk) * a.capacity * d + (size_t)head * hd;
+            const uint32_t at = r * d + head * hd;
+            const float v = attend<KV>(a, kcache + base, vcache + base, q + at, min(a.position + r % a.chunk + 1, a.capacity), prod);
+            if (tid < hd) store_to_all(att + at + tid, v);
+        }
+        cluster_arrive();
+        auto add_to_residual = [&](const float* bias) {
+            return [&, bias](uint32_t r, uint32_t col, float sum) {
+                const float v = sum + bias[col];
+                store_to_all(h + r * d + col, h[r * d + col] + v);
+            };
+        };
+        phase(Matrix{L.wo, nullptr, nullptr, d, d, d}, att, nullptr, nullptr, add_to_residual(L.bo));
+        phase(Matrix{L.w_in, nullptr, nullptr, d, f, f}, nullptr, L.ln2w, L.ln2b, [&](uint32_t r, uint32_t col, float sum) {
+            const float v = sum + L.b_in[col];
+            store_to_all(ff + r * f + col, a.activation == ACT_GELU ? strict_gelu(v) : fmaxf(v, 0.0f));
+        });
+        phase(Matrix{L.w_out, nullptr, nullptr, f, d, d}, ff, nullptr, nullptr, add_to_residual(L.b_out));
+    }
+    cluster_wait();
+    if (!a.logits) {                        // a large vocabulary: the head is a launch of its own
+        for (uint32_t i = rank * SS_THREADS + tid; i < rows * d; i += SS_CTAS * SS_THREADS) a.h[(size_t)row0 * d + i] = h[i];
+        return;
+    }
+    // the tied head: rows of the token table [vocab, d], so lanes run along d; every row, or the last one of each session
+    const uint32_t wanted = a.last_only ? ns : rows, per = per_cta(a.vocab), col0 = rank * per, cols = col0 < a.vocab ? min(per, a.vocab - col0) : 0u;
+    norm_rows(xs, term, a.last_only ? h + (a.chunk - 1) * d : h, a.last_only ? a.chunk * d : d, a.fnw, a.fnb, wanted, d, a.eps);
+    for (uint32_t c0 = 0; c0 < cols; c0 += SS_COLS) {
+        const uint32_t nc = min(SS_COLS, cols - c0);
+        __syncthreads();
+        for (uint32_t c = warp; c < nc; c += SS_WARPS)
+            for (uint32_t p = 4 * lane; p < d; p += 128) {
+                const float* w = a.tok + (size_t)(col0 + c0 + c) * d + p;
+                const float4 v = make_float4(__ldg(w), __ldg(w + 1), __ldg(w + 2), __ldg(w + 3));
+                for (uint32_t r = 0; r < wanted; ++r) {
+                    const float4 x = *reinterpret_cast<const float4*>(xs + r * d + p);
+                    *reinterpret_cast<float4*>(prod + (r * SS_COLS + c) * (d + 4) + p) = make_float4(x.x * v.x, x.y * v.y, x.z * v.z, x.w * v.w);
+                }
+            }
+        __syncthreads();
+        if (warp < wanted && lane < nc)
+            a.logits[(size_t)((a.last_only ? s0 : row0) + warp) * a.vocab + col0 + c0 + lane] = add_up(prod + (warp * SS_COLS + lane) * (d + 4), d);
+    }
+}
+
+// Rows that fit a cluster's shared memory: their values, their products in the widest phase, and a head's scores and products.
+uint32_t rows_that_fit(const StrictStepArgs& a) {
+    auto room = [](uint32_t n) {
+        const uint32_t per = std::min(ceil_div(n, SS_CTAS), SS_COLS);
+        uint32_t p = 1;
+        while (p < per) p *= 2;
+        return p;
+    };
+    const uint32_t products = std::max({(a.d + 4) * room(3 * a.d), (a.d + 4) * room(a.f), (a.f + 4) * room(a.d), (a.d + 4) * SS_COLS});
+    const uint32_t floats = SS_SMEM / 4, head = a.capacity + 4 + SS_VALUES, each = floats_per_row(a.d, a.f);
+    if (head + each > floats) return 0;
+    return std::min({SS_WARPS, floats / (each + products), (floats - head) / each});
+}
+
+template <typename KV>
+int clusters_at_once() {
+    static int known[64] = {};              // per device: clusters of 16 CTAs that run side by side, -1: none
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    if (known[dev] == 0) {
+        int n = 0;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(SS_CTAS);
+        cfg.blockDim = dim3(SS_THREADS);
+        cfg.dynamicSmemBytes = SS_SMEM;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = SS_CTAS;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        const bool fits = cudaFuncSetAttribute(strict_step_kernel<KV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SS_SMEM) == cudaSuccess &&
+                          cudaFuncSetAttribute(strict_step_kernel<KV>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                          cudaOccupancyMaxActiveClusters(&n, strict_step_kernel<KV>, &cfg) == cudaSuccess && n > 0;
+        if (!fits) cudaGetLastError();
+        known[dev] = fits ? n : -1;
+    }
+    return std::max(0, known[dev]);
+}
+
+}  // namespace
+
+// Most rows that one cluster takes through a step: a warp each.  Up to there it is the faster form at every size measured (4 x 128: 8 rows 152
+// against 298 us, 4 x 256: 2 rows 170 against 370 us); what ends it earlier is shared memory (rows_that_fit).
+constexpr uint32_t SS_MAX_ROWS = 16;
+// A cluster reads every weight through 16 SMs: beyond this many bytes of one layer the launches of strict.cu, which use all SMs, are faster.
+constexpr uint64_t SS_MAX_LAYER_BYTES = 4u << 20;
+
+bool strict_step_supported(const StrictStepArgs& a, bool kv_bf16) {
+    if (!a.num_layers || a.num_layers > SS_MAX_LAYERS || a.d > SS_MAX_D || a.d % 4 || a.f % 4 || a.d % a.heads || (a.d / a.heads) % 4) return false;
+    if ((4ull * a.d * a.d + 2ull * a.d * a.f) * 4 > SS_MAX_LAYER_BYTES || a.capacity > 16384) return false;
+    const int at_once = kv_bf16 ? clusters_at_once<bf16>() : clusters_at_once<float>();
+    return at_once > 0 && (uint64_t)ceil_div(a.sessions, (uint32_t)at_once) * a.chunk <= std::min(SS_MAX_ROWS, rows_that_fit(a));
+}
+
+// Largest vocabulary whose output head is part of the launch.
+bool strict_step_has_head(uint32_t vocab) { return vocab <= 2048; }
+
+template <typename KV>
+static int launch_strict_step_kind(const StrictStepArgs& a, cudaStream_t stream) {
+    SsParams P;
+    P.a = a;
+    const int at_once = std::max(1, clusters_at_once<KV>());
+    P.sessions_per_cluster = ceil_div(a.sessions, (uint32_t)at_once);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ceil_div(a.sessions, P.sessions_per_cluster) * SS_CTAS);
+    cfg.blockDim = dim3(SS_THREADS);
+    cfg.dynamicSmemBytes = SS_SMEM;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = SS_CTAS;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, strict_step_kernel<KV>, P);
+    count_launch();
+    return check_launch("strict_step");
+}
+
+int launch_strict_step(const StrictStepArgs& a, bool kv_bf16, cudaStream_t stream) {
+    return kv_bf16 ? launch_strict_step_kind<bf16>(a, stream) : launch_strict_step_kind<float>(a, stream);
+}
+
+}  // namespace tb
