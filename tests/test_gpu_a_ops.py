@@ -206,6 +206,31 @@ def test_gemm_bf16_epilogues(engine):
     assert rel_err(gelu, orc.gelu(z.astype(np.float32))) <= 1 / 128
 
 
+@pytest.mark.parametrize("shape", [(1, 512, 16), (3, 40, 80), (16, 768, 768), (17, 771, 1040), (24, 768, 4608), (48, 768, 2048), (49, 768, 3072),
+                                   (33, 4096, 768), (65, 768, 768), (128, 250, 1072), (9, 20000, 512)])
+def test_gemm_bf16_register_engine_matches_f64(shape):
+    """Few rows, k a multiple of 16: 16 to 64 rows and 8 to 32 columns per CTA, k in blocks of 64 over eight warps and, for a narrow matrix with
+    a long k, over the two CTAs of a cluster; ragged rows, columns and k, several column tiles per CTA.  f32 sums of exact products: 4e-6 k.
+    A row's bits do not depend on the rows beside it."""
+    m, n, k = shape
+    a, bt, ref = gemm_case(m, n, k, seed=21)
+    rng = np.random.default_rng(22)
+    bias, resid = rng.standard_normal(n).astype(np.float32), rng.standard_normal((m, n)).astype(np.float32)
+    da, dbt, dbias, dres = dev(a, torch.bfloat16), dev(bt, torch.bfloat16), dev(bias), dev(resid)
+    tol = 4e-6 * k
+    plain = gemm_bf16(da, dbt)
+    assert np.max(np.abs(plain.cpu().numpy() - ref)) <= tol
+    assert torch.equal(plain[:1], gemm_bf16(da[:1].contiguous(), dbt))
+    fused = gemm_bf16(da, dbt, bias=dbias, residual=dres).cpu().numpy()
+    assert np.max(np.abs(fused - (ref + bias + resid))) <= tol + 1e-5
+    relu = gemm_bf16(da, dbt, bias=dbias, activation=0, out_dtype=BF16).float().cpu().numpy()
+    assert rel_err(relu, np.maximum(ref + bias, 0)) <= 1 / 128
+    in_place = dres.clone()
+    ok(lib().tnsr_b200_gemm_bf16(ptr(da), ptr(dbt), ptr(dbias), ptr(in_place), ptr(in_place), m, n, k, -1, 0, stream()))
+    torch.cuda.synchronize()
+    assert np.array_equal(in_place.cpu().numpy(), fused)
+
+
 @pytest.mark.parametrize("shape", [(1, 4096, 4096), (8, 4096, 4096), (64, 4096, 4096), (17, 768, 768), (32, 768, 2048),
                                    (64, 2304, 768), (5, 100, 72), (33, 129, 520), (16, 32000, 768), (1, 128, 64)])
 def test_gemm_bf16_few_rows_engine_matches_f64_with_and_without_split_k(shape):

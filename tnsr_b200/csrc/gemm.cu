@@ -19,82 +19,13 @@
 #include <mutex>
 #include <unordered_map>
 
+#include "gemm_epilogue.cuh"
 #include "tc_common.cuh"
 
 namespace tb {
 
 int g_gemm_engine = 0;
 thread_local uint32_t t_lose_gemm_stage = 0;
-struct EpiParams {
-    GemmEpilogue ep;
-    GemmQkvTargets qkv;
-    GemmSegments seg;
-    void* out;
-    uint32_t ldc;
-    uint32_t m, n;  // n = columns of the accumulator (packed width for SWIGLU)
-};
-
-// ---- epilogue: scalar forms ---------------------------------------------------
-__device__ __forceinline__ size_t map_out_row(const GemmEpilogue& ep, uint32_t row) {
-    if (!ep.rows_per_session) return row;
-    uint32_t off = ep.d_row_offset ? *ep.d_row_offset : ep.row_offset;
-    return (size_t)(row / ep.rows_per_session) * ep.out_session_rows + off + row % ep.rows_per_session;
-}
-
-__device__ __forceinline__ void store_plain(const EpiParams& P, uint32_t row, uint32_t col, float acc) {
-    float v = acc;
-    if (P.ep.bias) v += P.ep.bias[col];
-    v = apply_activation(v, P.ep.activation);
-    size_t orow = map_out_row(P.ep, row);
-    if (P.ep.out_dtype == TNSR_B200_BF16) {
-        reinterpret_cast<bf16*>(P.out)[orow * P.ldc + col] = __float2bfloat16_rn(v);
-    } else {
-        if (P.ep.scale) v *= P.ep.scale[col];
-        if (P.ep.residual) v += P.ep.residual[(size_t)row * P.ep.ldr + col];
-        reinterpret_cast<float*>(P.out)[orow * P.ldc + col] = v;
-    }
-}
-
-__device__ __forceinline__ void store_qkv(const EpiParams& P, uint32_t row, uint32_t col, float acc) {
-    float v = acc;
-    if (P.ep.bias) v += P.ep.bias[col];
-    const uint32_t d = P.qkv.d, which = col / d, c = col % d;
-    if (which == 0) {
-        P.qkv.q[(size_t)row * d + c] = __float2bfloat16_rn(v);
-    } else {
-        const uint32_t session = row / P.qkv.chunk;
-        uint32_t pos = P.qkv.d_position ? P.qkv.d_position[session * P.qkv.position_stride] : P.qkv.position;
-        size_t crow = kv_row(P.qkv.paging, session, pos + row % P.qkv.chunk, P.qkv.capacity);
-        (which == 1 ? P.qkv.k_cache : P.qkv.v_cache)[crow * d + c] = __float2bfloat16_rn(v);
-    }
-}
-
-// Range of column `col` (GEMM_SEGMENTS).
-__device__ __forceinline__ uint32_t segment_of(const EpiParams& P, uint32_t col) {
-    uint32_t i = 0;
-    if (P.seg.count > 1 && col >= P.seg.s[1].col0) i = 1;
-    if (P.seg.count > 2 && col >= P.seg.s[2].col0) i = 2;
-    return i;
-}
-
-__device__ __forceinline__ void store_segment(const EpiParams& P, uint32_t row, uint32_t col, float acc) {
-    const GemmSegment& g = P.seg.s[segment_of(P, col)];
-    const float v = apply_activation(P.ep.bias ? acc + P.ep.bias[col] : acc, g.activation);
-    const size_t o = (size_t)row * g.ld + (col - g.col0);
-    if (g.out_dtype == TNSR_B200_BF16) reinterpret_cast<bf16*>(g.out)[o] = __float2bfloat16_rn(v);
-    else reinterpret_cast<float*>(g.out)[o] = v;
-}
-
-// g, u: accumulators of packed columns pc and pc + 16; output column oc.
-__device__ __forceinline__ void store_swiglu(const EpiParams& P, uint32_t row, uint32_t pc, uint32_t oc,
-                                             float g, float u) {
-    if (P.ep.bias) {
-        g += P.ep.bias[pc];
-        u += P.ep.bias[pc + 16];
-    }
-    reinterpret_cast<bf16*>(P.out)[(size_t)row * P.ldc + oc] = __float2bfloat16_rn(fast_silu(g) * u);
-}
-
 // ===========================================================================
 // CUDA-core engine: 64x64 tile, 16x16 threads, 4x4 outputs per thread.
 // ===========================================================================
@@ -931,6 +862,9 @@ static int launch_gemm_impl(const bf16* a, const bf16* bt, void* out, uint32_t l
             return TNSR_B200_ERR_INVALID_ARGUMENT;
         }
     }
+    // Few rows: operands straight into registers (gemm_few.cu; not where a test asks this engine to lose a stage).
+    if (!split_req && mode != GEMM_ARGMAX && g_gemm_engine == 0 && !ep.round_bf16 && !t_lose_gemm_stage && gemm_few_pays(a, bt, m, n, k))
+        return launch_gemm_few(a, bt, P, k, mode, stream);
     // A handful of rows against a large weight matrix: stream the weights with the operands swapped (gemm_skinny.cu)
     // when that engine can fill the GPU, i.e. with split-K scratch lent by the caller or with at least half as many
     // 128-column tiles as SMs.  Measured inside a CUDA graph, 4096 x 4096 weights: 14.8 / 16.3 us at 1 / 8 rows against
@@ -1062,6 +996,7 @@ static int launch_gemm_impl(const bf16* a, const bf16* bt, void* out, uint32_t l
 uint32_t gemm_split_k(const bf16* a, const bf16* bt, uint32_t m, uint32_t n, uint32_t k) {
     if (g_gemm_engine == 1 || !tc_eligible(a, k, bt, k)) return 0;
     if (m == 0 || m > 256 || k % BK != 0) return 0;
+    if (g_gemm_engine == 0 && gemm_few_pays(a, bt, m, n, k)) return 0;
     if (m <= 64 && (uint64_t)n * k >= (4ull << 20)) return 0;   // the few-row engines take these shapes
     const uint32_t num_kb = k / BK, tiles_n = ceil_div(n, 32u);
     for (uint32_t s = 4; s >= 2; --s)

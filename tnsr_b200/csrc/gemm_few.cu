@@ -1,0 +1,325 @@
+// bf16 GEMM for few activation rows, every epilogue of a decode step: out[m, n] = epilogue(a[m, :] . w[n, :]).
+//
+// A projection of a single-token step is a few MB of weights against a few dozen rows: neither the tensor cores nor HBM are what it
+// waits for, but the chain of latencies behind the previous kernel -- tensor-map fetch, a ring of TMA copies (one SM takes in 128
+// padded rows at about 70 GB/s), TMEM and the epilogue's transposes came to 7 to 22 us a launch.  Here nothing is staged: a thread's
+// weights are 32-byte loads straight into registers (whole 128-byte lines per row), asked for before the previous kernel has ended
+// (they do not depend on it), the activation rows follow the same way from L2, and warp-level products consume both where they land.
+// The order of k inside a block of 64 is free as long as both operands agree, so lane t of a row takes k = 16t .. 16t + 15 and feeds
+// four m16n8k16 products.
+//
+//  * a CTA owns 16 MT rows x 8 NT columns at a time, its eight warps divide K; partial tiles are added in warp order through shared
+//    memory.  With more column tiles than CTAs the next tile's weights are on their way while this one is added up and written;
+//  * K may be divided over a cluster of CTAs (ck): each takes in 1 / ck of the rows' and the weights' bytes, the partial tiles meet
+//    through distributed shared memory, added in rank order.
+// How K is divided depends on n and k only, so the bits of an element do not depend on how many rows share the call.
+#include <algorithm>
+#include <atomic>
+
+#include "gemm_epilogue.cuh"
+
+namespace tb {
+
+namespace {
+
+constexpr uint32_t FW_THREADS = 256, FW_WARPS = FW_THREADS / 32, FW_BLOCK = 64;
+
+struct FewParams {
+    const bf16* a;         // [m, k]
+    const bf16* w;         // [n, k]
+    EpiParams epi;
+    uint32_t k;
+    uint32_t ck;           // CTAs of a cluster, each with its range of k
+    uint32_t tiles;        // column tiles
+    int mode;
+};
+
+struct Words { uint32_t x[8]; };
+
+__device__ __forceinline__ Words fw_zero() { return {{0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u}}; }
+__device__ __forceinline__ Words fw_load_weights(const bf16* p) {
+    Words v;
+    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v.x[0]), "=r"(v.x[1]), "=r"(v.x[2]), "=r"(v.x[3]), "=r"(v.x[4]), "=r"(v.x[5]), "=r"(v.x[6]), "=r"(v.x[7]) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ Words fw_load_rows(const bf16* p) {
+    Words v;
+    asm volatile("ld.global.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v.x[0]), "=r"(v.x[1]), "=r"(v.x[2]), "=r"(v.x[3]), "=r"(v.x[4]), "=r"(v.x[5]), "=r"(v.x[6]), "=r"(v.x[7]) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void fw_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ float fw_load_peer(const float* local, uint32_t rank) {
+    const uint32_t at = (uint32_t)__cvta_generic_to_shared(local);
+    uint32_t remote;
+    float v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
+    return v;
+}
+__device__ __forceinline__ void fw_cluster_sync() { asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory"); }
+
+// MT: 16-row tiles, NT: 8-column tiles of a CTA, S: k blocks whose weights a warp has in registers at a time.
+template <int MT, int NT, int S>
+__global__ void __launch_bounds__(FW_THREADS, MT == 1 ? 2 : 1)
+gemm_few_kernel(const __grid_constant__ FewParams P) {
+    constexpr uint32_t ROWS = 16 * MT, COLS = 8 * NT, TILE = ROWS * COLS;
+    constexpr int AHEAD = MT == 1 ? 2 : 1;                      // k blocks whose rows are asked for at a time
+    constexpr int MINE = (TILE + FW_THREADS - 1) / FW_THREADS;
+    extern __shared__ __align__(16) float fw_smem[];            // [8 warps][TILE]; then this CTA's sums over warp 0's
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const uint32_t rank = blockIdx.x % P.ck, row0 = blockIdx.y * ROWS;
+    const uint32_t m = P.epi.m, n = P.epi.n, k = P.k, tile_step = gridDim.x / P.ck;
+    const bool swiglu = P.mode == GEMM_SWIGLU;
+    const uint32_t blocks = (k + FW_BLOCK - 1) / FW_BLOCK, slices = P.ck * FW_WARPS;
+    const uint32_t per = (blocks + slices - 1) / slices, b0 = min(blocks, (rank * FW_WARPS + warp) * per), b1 = min(blocks, b0 + per);
+    // first column of a tile and the distance of its 8-column parts: side by side, or (packed gate / up, NT = 2) a gate part and its up part
+    const uint32_t col_step = swiglu && NT == 2 ? 16 : 8;
+    auto first_col = [&](uint32_t tile) { return swiglu && NT == 2 ? (tile >> 1) * 32 + (tile & 1) * 8 : tile * COLS; };
+
+    Words w[NT][S];
+    auto load_w = [&](int s, uint32_t tile, uint32_t b) {
+        const uint32_t col = first_col(tile) + g;
+        const bool ok = tile < P.tiles && b < b1 && b * FW_BLOCK + 16 * t < k;
+        const bf16* p = P.w + (size_t)col * k + b * FW_BLOCK + 16 * t;
+#pragma unroll
+        for (int j = 0; j < NT; ++j) w[j][s] = ok && col + j * col_step < n ? fw_load_weights(p + (size_t)j * col_step * k) : fw_zero();
+    };
+    uint32_t tile = blockIdx.x / P.ck;
+#pragma unroll
+    for (int s = 0; s < S; ++s) load_w(s, tile, b0 + s);
+    // A thread finishes elements tid, tid + 256, ... of the (ck = 1) tile, all of one column: its bias and scale
+    const uint32_t threads = FW_THREADS * P.ck, tid = rank * FW_THREADS + threadIdx.x;
+    const uint32_t my_cols = swiglu ? COLS / 2 : COLS, my_col = tid % my_cols;
+
+    pdl_wait();
+    pdl_trigger();
+    const bf16* ap = P.a + (size_t)(row0 + g) * k + 16 * t;       // rows g, g + 8, g + 16 ... of the tile
+    for (; tile < P.tiles; tile += tile_step) {
+        const uint32_t col0 = first_col(tile), col = col0 + my_col;
+        float bias = 0.0f, bias_up = 0.0f;
+        if (P.epi.ep.bias && col < n) {
+            bias = __ldg(P.epi.ep.bias + col);
+            if (swiglu) bias_up = __ldg(P.epi.ep.bias + col + 16);
+        }
+        // what the end of the tile reads from memory per element: the residual, or the row of the cache
+        uint32_t early[MINE];
+#pragma unroll
+        for (int i = 0; i < MINE; ++i) {
+            const uint32_t e = tid + i * threads, row = row0 + e / COLS;
+            early[i] = 0u;
+            if (e >= TILE || row >= m || col >= n) continue;
+            if (P.mode == GEMM_PLAIN && P.epi.ep.residual) early[i] = __float_as_uint(__ldcg(P.epi.ep.residual + (size_t)row * P.epi.ep.ldr + col));
+            if (P.mode == GEMM_QKV && col >= P.epi.qkv.d) {
+                const GemmQkvTargets& q = P.epi.qkv;
+                const uint32_t session = row / q.chunk, at = q.d_position ? q.d_position[session * q.position_stride] : q.position;
+                early[i] = (uint32_t)kv_row(q.paging, session, at + row % q.chunk, q.capacity);
+            }
+        }
+        float acc[MT][NT][4];
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.0f;
+        for (uint32_t b = b0; b < b1; b += S) {
+            const bool more = b + S < b1;
+#pragma unroll
+            for (int s0 = 0; s0 < S; s0 += AHEAD) {
+                Words a[AHEAD][2 * MT];
+#pragma unroll
+                for (int s = 0; s < AHEAD; ++s) {
+                    const uint32_t at = (b + s0 + s) * FW_BLOCK;
+                    const bool ok = b + s0 + s < b1 && at + 16 * t < k;
+#pragma unroll
+                    for (int i = 0; i < 2 * MT; ++i) a[s][i] = ok && row0 + 8 * i + g < m ? fw_load_rows(ap + (size_t)i * 8 * k + at) : fw_zero();
+                }
+#pragma unroll
+                for (int s = 0; s < AHEAD; ++s) {
+                    if (b + s0 + s < b1) {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+#pragma unroll
+                            for (int j = 0; j < NT; ++j)
+#pragma unroll
+                                for (int i = 0; i < MT; ++i)
+                                    fw_mma(acc[i][j], a[s][2 * i].x[2 * q], a[s][2 * i + 1].x[2 * q], a[s][2 * i].x[2 * q + 1], a[s][2 * i + 1].x[2 * q + 1],
+                                           w[j][s0 + s].x[2 * q], w[j][s0 + s].x[2 * q + 1]);
+                    }
+                    // the place is free: the same block of the next round, or of the next tile
+                    if (more) load_w(s0 + s, tile, b + S + s0 + s);
+                    else load_w(s0 + s, tile + tile_step, b0 + s0 + s);
+                }
+            }
+        }
+        float* mine = fw_smem + warp * TILE;
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+                *reinterpret_cast<float2*>(mine + (16 * i + g) * COLS + 8 * j + 2 * t) = make_float2(acc[i][j][0], acc[i][j][1]);
+                *reinterpret_cast<float2*>(mine + (16 * i + g + 8) * COLS + 8 * j + 2 * t) = make_float2(acc[i][j][2], acc[i][j][3]);
+            }
+        __syncthreads();
+        auto sum_of = [&](uint32_t e) {
+            float v = fw_smem[e];
+#pragma unroll
+            for (uint32_t i = 1; i < FW_WARPS; ++i) v += fw_smem[i * TILE + e];
+            return v;
+        };
+        if (P.ck > 1) {
+            for (uint32_t e = threadIdx.x; e < TILE; e += FW_THREADS) fw_smem[e] = sum_of(e);     // a thread reads and writes its own elements
+            fw_cluster_sync();
+        }
+        auto total = [&](uint32_t e) {
+            if (P.ck == 1) return sum_of(e);
+            float v = fw_load_peer(fw_smem + e, 0);
+            for (uint32_t r = 1; r < P.ck; ++r) v += fw_load_peer(fw_smem + e, r);
+            return v;
+        };
+        if (swiglu) {
+            constexpr uint32_t HALF = COLS / 2;      // gate columns of the tile, then their up columns
+#pragma unroll
+            for (int i = 0; i < (MINE + 1) / 2; ++i) {
+                const uint32_t e = tid + i * threads, r = e / HALF, c = e % HALF, row = row0 + r;
+                if (e >= ROWS * HALF || row >= m || col >= n) continue;
+                const float gate = total(r * COLS + c) + bias, up = total(r * COLS + HALF + c) + bias_up;
+                reinterpret_cast<bf16*>(P.epi.out)[(size_t)row * P.epi.ldc + (col / 32 * 16 + col % 32)] = __float2bfloat16_rn(fast_silu(gate) * up);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < MINE; ++i) {
+                const uint32_t e = tid + i * threads, row = row0 + e / COLS;
+                if (e >= TILE || row >= m || col >= n) continue;
+                float v = total(e);
+                if (P.mode == GEMM_QKV) {
+                    const GemmQkvTargets& q = P.epi.qkv;
+                    const uint32_t part = col / q.d, c = col - part * q.d;
+                    const size_t at = part == 0 ? row : early[i];
+                    (part == 0 ? q.q : part == 1 ? q.k_cache : q.v_cache)[at * q.d + c] = __float2bfloat16_rn(v + bias);
+                } else if (P.mode == GEMM_SEGMENTS) {
+                    const GemmSegment& s = P.epi.seg.s[segment_of(P.epi, col)];
+                    v = apply_activation(v + bias, s.activation);
+                    const size_t o = (size_t)row * s.ld + (col - s.col0);
+                    if (s.out_dtype == TNSR_B200_BF16) reinterpret_cast<bf16*>(s.out)[o] = __float2bfloat16_rn(v);
+                    else reinterpret_cast<float*>(s.out)[o] = v;
+                } else {
+                    const GemmEpilogue& ep = P.epi.ep;
+                    v = apply_activation(v + bias, ep.activation);
+                    const size_t o = map_out_row(ep, row) * P.epi.ldc + col;
+                    if (ep.out_dtype == TNSR_B200_BF16) {
+                        reinterpret_cast<bf16*>(P.epi.out)[o] = __float2bfloat16_rn(v);
+                    } else {
+                        if (ep.scale) v *= __ldg(ep.scale + col);
+                        if (ep.residual) v += __uint_as_float(early[i]);
+                        reinterpret_cast<float*>(P.epi.out)[o] = v;
+                    }
+                }
+            }
+        }
+        if (P.ck > 1) fw_cluster_sync();       // peers may still read this CTA's sums
+        else if (tile + tile_step < P.tiles) __syncthreads();
+    }
+}
+
+template <int MT, int NT, int S>
+int launch_shape(FewParams P, cudaStream_t stream) {
+    constexpr uint32_t bytes = FW_WARPS * 16 * MT * 8 * NT * 4;
+    static std::atomic<int> per_sm[64] = {};            // CTAs that fit an SM, 0: not asked yet
+    int dev = 0;
+    cudaGetDevice(&dev);
+    dev = dev < 0 || dev >= 64 ? 63 : dev;
+    int resident = per_sm[dev].load(std::memory_order_relaxed);
+    if (!resident) {
+        prefer_max_shared_carveout(reinterpret_cast<const void*>(gemm_few_kernel<MT, NT, S>));
+        if (bytes > 48 * 1024 && cudaFuncSetAttribute(gemm_few_kernel<MT, NT, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
+            return check_launch("gemm_few attribute");
+        int sms = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, gemm_few_kernel<MT, NT, S>, FW_THREADS, bytes) != cudaSuccess ||
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || resident < 1)
+            return check_launch("gemm_few occupancy");
+        resident *= sms;
+        per_sm[dev].store(resident, std::memory_order_relaxed);
+    }
+    P.tiles = ceil_div(P.epi.n, 8u * NT);
+    const uint32_t row_tiles = ceil_div(P.epi.m, 16u * MT);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(std::min(P.tiles, std::max(1u, (uint32_t)resident / (row_tiles * P.ck))) * P.ck, row_tiles);
+    cfg.blockDim = dim3(FW_THREADS);
+    cfg.dynamicSmemBytes = bytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    uint32_t count = 0;
+    if (t_pdl) {
+        attr[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[count++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (P.ck > 1) {
+        attr[count].id = cudaLaunchAttributeClusterDimension;
+        attr[count].val.clusterDim.x = P.ck;
+        attr[count].val.clusterDim.y = 1;
+        attr[count++].val.clusterDim.z = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = count;
+    cudaLaunchKernelEx(&cfg, gemm_few_kernel<MT, NT, S>, P);
+    count_launch();
+    return check_launch("gemm_few");
+}
+
+template <int NT, int S>
+int launch_rows(const FewParams& P, cudaStream_t stream) {
+    const uint32_t m = P.epi.m;
+    if (m <= 16) return launch_shape<1, NT, S>(P, stream);
+    if (m <= 32) return launch_shape<2, NT, S>(P, stream);
+    if (m <= 48) return launch_shape<3, NT, S>(P, stream);
+    return launch_shape<4, NT, S>(P, stream);
+}
+
+}  // namespace
+
+// Whether this engine is the faster one.  Measured on B200 as chains of 48 dependent launches over 420 MB of weights, us per launch here /
+// in the tcgen05 engine (at most 16 rows and 4 M weights: the streaming engine), by rows:
+//     n x k            1           24          48          64          128
+//     768 x 768     1.8 / 7.0   2.6 / 7.0   3.6 / 7.1   4.0 / 7.1   5.3 / 7.2
+//     768 x 2048    3.1 / 12.5  4.6 / 12.5  5.4 / 12.5  6.1 / 12.5  10.1 / 12.6   (split-K of that engine: about 7 and a fold)
+//     768 x 4608    7.5 / 22.4  8.0 / 22.4  9.4 / 22.4  10.9 / 22.5 16.1 / 22.6
+//     2304 x 768    2.0 / 7.4   3.3 / 7.0   4.3 / 7.1   5.4 / 7.1   9.4 / 7.3
+//     4096 x 768    2.8 / 8.8   5.5 / 8.4   7.0 / 8.0   8.0 / 7.5   14.3 / 6.7
+//     4096 x 4096   9.8 / 12.6  16.2 / 20.1 20.0 / 20.3 21.7 / 20.4 39 / 20.6
+//     32000 x 768   17.3 / 26.1 31 / 18.1   51 / 18.2   62 / 19.1   118 / 17.3
+// Every column tile takes in all rows, so what ends it is rows x columns; only a small matrix still gains past 64 rows.
+bool gemm_few_pays(const bf16* a, const bf16* w, uint32_t m, uint32_t n, uint32_t k) {
+    if (m == 0 || m > 128 || n == 0 || k % 16 != 0 || k == 0) return false;
+    if (reinterpret_cast<uintptr_t>(a) % 32 != 0 || reinterpret_cast<uintptr_t>(w) % 32 != 0) return false;
+    const uint64_t weights = (uint64_t)n * k;
+    if (m <= 16) return true;
+    if (m <= 32) return weights <= (17ull << 20);
+    if (m <= 48 && weights <= (3ull << 20)) return true;
+    if (m <= 64 && (weights <= (2ull << 20) || n <= 1024)) return true;
+    return weights <= (3ull << 18);
+}
+
+int launch_gemm_few(const bf16* a, const bf16* w, const EpiParams& epi, uint32_t k, GemmMode mode, cudaStream_t stream) {
+    FewParams P;
+    P.a = a; P.w = w; P.epi = epi; P.k = k; P.mode = mode; P.tiles = 0;
+    const uint32_t m = epi.m, n = epi.n;
+    // a narrow matrix with a long k (an output or down projection) has fewer column tiles than SMs: two CTAs share its k
+    P.ck = k > 1024 && n <= 1024 ? 2 : 1;
+    // up to 16 rows 16 columns per CTA were the fastest throughout; with more rows as few CTAs as still make a wave
+    uint32_t nt = 2;
+    if (m > 16) {
+        const uint32_t row_tiles = ceil_div(m, 64u);
+        nt = mode == GEMM_SWIGLU ? 2 : 1;
+        while (nt < 4 && ceil_div(n, 8 * nt) * P.ck * row_tiles > 148) nt *= 2;
+    }
+    const uint32_t per = ceil_div(ceil_div(k, FW_BLOCK), P.ck * FW_WARPS);
+    if (nt == 4) return launch_rows<4, 2>(P, stream);
+    if (nt == 2) return per <= 2 ? launch_rows<2, 2>(P, stream) : launch_rows<2, 4>(P, stream);
+    return per <= 2 ? launch_rows<1, 2>(P, stream) : launch_rows<1, 4>(P, stream);
+}
+
+}  // namespace tb
