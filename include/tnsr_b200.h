@@ -132,11 +132,9 @@ typedef struct tnsr_b200_config {
      * this mode. */
     uint32_t kv_page_rows;
     uint32_t kv_pool_pages;
-    /* Single-token steps of at most 32 sessions (bf16 weights, SwiGLU, width <=
-     * 1024): 0 = everything between two attention scans runs as one persistent
-     * kernel with grid-wide barriers (the default), 1 = one kernel per operator
-     * as at larger batches.  No reference counterpart; the two differ by rounding
-     * only. */
+    /* 0 or 1; chose between two forms of a small single-token step.  Both are
+     * the same launches now: one kernel per operator, the faster form since
+     * few-row products take their operands straight into registers. */
     uint32_t small_batch_mode;
 } tnsr_b200_config;
 

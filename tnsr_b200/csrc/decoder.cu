@@ -324,11 +324,6 @@ int step_strict(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chunk
     return TNSR_B200_OK;
 }
 
-// Largest batch whose single-token step runs each layer's projections as one persistent kernel (decode_tail.cu): the
-// kernel keeps 32 session rows per CTA (LayerNorm rows in registers, activation ring in shared memory).
-// Measured on B200 with the 12-layer d768 model, ms per step fused / operator by operator: 32 sessions 0.55 / 0.74.
-constexpr uint32_t kTailMaxSessions = 32;
-
 // ---- one step on the bf16 tensor-core path -----------------------------------
 // The part of a step that belongs to a range of sessions [s0, s0 + ns): embedding and all layers, on stream `st`.
 // Nothing in it couples two sessions, so disjoint ranges may run on different streams at the same time.
@@ -356,48 +351,6 @@ int layers_bf16(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chunk
     const bool fast_decode = chunk == 1 && ws && decode_attention_supported(H, hd);
     if (ragged && !fast_decode) return fail(dec, TNSR_B200_ERR_UNSUPPORTED, "ragged decode needs the split-KV attention kernel (head width 32, 64 or 128)");
     bool planned = false;
-    // Small batch: everything between two attention scans is one persistent kernel (decode_tail.cu).
-    if (fast_decode && !lean && dec->fused_gu && dec->tail_ws && dec->use_tail && ns <= kTailMaxSessions &&
-        decode_tail_supported(ns, d, f)) {
-        const size_t layers = dec->layers.size();
-        auto tail = [&](size_t prev, bool with_prev, bool with_next) -> int {
-            DecodeTailArgs a;
-            a.rows = ns; a.d = d; a.f = f; a.eps = c.layer_norm_epsilon;
-            a.h = h; a.att = att; a.ff = ff; a.q = q;
-            a.workspace = dec->tail_ws; a.d_status = dec->d_status;
-            if (with_prev) {
-                const Layer& L = dec->layers[prev];
-                a.run_o = a.run_ffn = true;
-                a.wo = (const bf16*)L.wo; a.bo = L.bo; a.ln2w = L.ln2w; a.ln2b = L.ln2b; a.wgu = L.wgu; a.bgu = L.bgu;
-                a.wdown = (const bf16*)L.w_out; a.bdown = L.b_out;
-            }
-            if (with_next) {
-                const Layer& N = dec->layers[with_prev ? prev + 1 : prev];
-                a.run_qkv = true;
-                a.ln1w = N.ln1w; a.ln1b = N.ln1b; a.wqkv = N.wqkv; a.bqkv = N.bqkv;
-                a.k_cache = (bf16*)N.kcache + cache0; a.v_cache = (bf16*)N.vcache + cache0;
-                a.capacity = c.capacity; a.d_position = pos_arg; a.position = position; a.position_stride = ragged ? 1u : 0u;
-                a.paging = &pg;
-            }
-            return launch_decode_tail(a, st);
-        };
-        RUN(dec, tail(0, false, true));
-        for (size_t l = 0; l < layers; ++l) {
-            Layer& L = dec->layers[l];
-            bf16* kcache = (bf16*)L.kcache + cache0;
-            bf16* vcache = (bf16*)L.vcache + cache0;
-            if (ragged)
-                RUN(dec, launch_decode_attention_ex(q, kcache, vcache, pos_arg, nullptr, 1, att, ws, dec->attn_ws_bytes, ns,
-                                                    c.capacity, H, hd, !planned, dec->d_status, st, false, &pg));
-            else
-                RUN(dec, launch_decode_attention_ex(q, kcache, vcache, nullptr, d_position, d_position ? 1 : position + 1, att,
-                                                    ws, dec->attn_ws_bytes, ns, c.capacity, H, hd, !planned, dec->d_status,
-                                                    st, false, &pg));
-            planned = true;
-            RUN(dec, tail(l, true, l + 1 < layers));
-        }
-        return TNSR_B200_OK;
-    }
     // Single-token steps of up to 256 rows: the two narrow projections (attention output, FFN down) divide their K extent
     // over several CTAs per tile; the partial sums are added to the residual, in a fixed order, by the LayerNorm that
     // follows (for the last layer's down projection that is the final LayerNorm in step_bf16: dec->split_pending).
@@ -826,10 +779,6 @@ static int create_decoder(const tnsr_b200_config* config, const tnsr_b200_stack*
             if ((rc = dev_alloc(dec, (void**)&dec->split_ws, (size_t)4 * dec->split_rows * config->embed_dim * sizeof(float), true)))
                 return bail(rc);
         }
-        if (config->batch <= kTailMaxSessions) {
-            if ((rc = dev_alloc(dec, &dec->tail_ws, decode_tail_workspace_bytes(), true))) return bail(rc);
-            dec->use_tail = config->small_batch_mode == 0;
-        }
     }
     if (!stack && dec->bf16_path && config->prefill_mode != TNSR_B200_PREFILL_SCALAR) {   // multi-token chunks off the tiled prefill kernels
         const uint32_t hd = config->embed_dim / config->num_heads;
@@ -1010,7 +959,6 @@ int tnsr_b200_decoder_reset(tnsr_b200_decoder* dec) {
         CU(dec, cudaMemsetAsync(L.vcache, 0, cache_bytes, dec->stream));
     }
     CU(dec, cudaMemsetAsync(dec->d_status, 0, 16, dec->stream));
-    if (dec->tail_ws) CU(dec, cudaMemsetAsync(dec->tail_ws, 0, decode_tail_workspace_bytes(), dec->stream));
     CU(dec, cudaStreamSynchronize(dec->stream));
     dec->failed = false;
     return TNSR_B200_OK;

@@ -89,9 +89,6 @@ struct tnsr_b200_decoder {
     cudaStream_t side_stream[3] = {nullptr, nullptr, nullptr};   // forked from and joined to `stream` by events
     cudaEvent_t ev_fork = nullptr, ev_join[3] = {nullptr, nullptr, nullptr};
     uint32_t parts = 1;
-    // small batches: one persistent kernel per layer between the attention scans (decode_tail.cu); its barrier words
-    void* tail_ws = nullptr;
-    bool use_tail = true;
     // paged K/V: every cache tensor is a pool [pool_pages, page_rows, d]; h_table[s * pps + i] is the pool page of
     // session s's i-th page, kNoPage while unassigned (the device copy is refreshed before the step that needs it)
     bool paged = false;
