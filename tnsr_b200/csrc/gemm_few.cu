@@ -291,7 +291,9 @@ int launch_rows(const FewParams& P, cudaStream_t stream) {
 //     4096 x 768    2.8 / 8.8   5.5 / 8.4   7.0 / 8.0   8.0 / 7.5   14.3 / 6.7
 //     4096 x 4096   9.8 / 12.6  16.2 / 20.1 20.0 / 20.3 21.7 / 20.4 39 / 20.6
 //     32000 x 768   17.3 / 26.1 31 / 18.1   51 / 18.2   62 / 19.1   118 / 17.3
-// Every column tile takes in all rows, so what ends it is rows x columns; only a small matrix still gains past 64 rows.
+// Every column tile takes in all rows, so what ends it is rows x columns; past 64 rows only a matrix that is small altogether gains.  (The
+// 768 x 768 projection of 128 rows does alone, but not inside a step of two ranges of sessions: its CTAs do not fit beside the other
+// range's attention.)
 bool gemm_few_pays(const bf16* a, const bf16* w, uint32_t m, uint32_t n, uint32_t k) {
     if (m == 0 || m > 128 || n == 0 || k % 16 != 0 || k == 0) return false;
     if (reinterpret_cast<uintptr_t>(a) % 32 != 0 || reinterpret_cast<uintptr_t>(w) % 32 != 0) return false;
@@ -300,7 +302,7 @@ bool gemm_few_pays(const bf16* a, const bf16* w, uint32_t m, uint32_t n, uint32_
     if (m <= 32) return weights <= (17ull << 20);
     if (m <= 48 && weights <= (3ull << 20)) return true;
     if (m <= 64 && (weights <= (2ull << 20) || n <= 1024)) return true;
-    return weights <= (3ull << 18);
+    return weights <= (300u << 10);
 }
 
 int launch_gemm_few(const bf16* a, const bf16* w, const EpiParams& epi, uint32_t k, GemmMode mode, cudaStream_t stream) {
