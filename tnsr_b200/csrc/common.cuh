@@ -49,7 +49,7 @@ struct KernelTimer {
 };
 extern thread_local KernelTimer* t_attention_timer;
 
-// Programmatic dependent launch: while t_pdl is set (the session sets it around single-token steps) kernels are
+// Programmatic dependent launch: while t_pdl is set (the session sets it around its shorter steps with bf16 weights) kernels are
 // launched with programmatic stream serialization, i.e. a kernel may be scheduled while its predecessor in the
 // stream is still draining.  Every kernel launched this way starts with pdl_wait(), which blocks until the
 // predecessor has completed and its writes are visible, so only launch latency overlaps, never data.
