@@ -676,6 +676,36 @@ def test_unequal_sessions_slots_and_pages_used_again(paged, dtype):
     sess.close()
 
 
+@pytest.mark.parametrize("shape", [(3, 64, 64), (2, 128, 64), (1, 64, 128), (5, 5, 7), (2, 136, 200), (1, 250, 30)])
+@pytest.mark.parametrize("sessions,tokens", [(1, 500), (2, 193), (3, 769)])
+def test_prompts_divided_in_time(shape, sessions, tokens):
+    """A prompt of 192 tokens and more for few sessions is scanned in segments side by side.  Against the same model on portions too short to
+    be divided, which makes the same projections (their sums do not depend on the rows beside them): the state differs by the 16 bits
+    that a written k R keeps (other chunk borders) and by f32 sums in another order, the logits by bf16 roundings that fall the other way."""
+    cfg = config(128, 160, [parallel((2, 1, 16, 16, 8, 20, 0.2), shape)])
+    _, _, model = build(cfg, "bf16")
+    ids = np.stack([tokens_for(cfg, tokens + 40, seed=30 + b) for b in range(sessions)])
+
+    def run(portions):
+        sess = B200Session(model.config(), sessions, 1024, logits_mode="all")
+        for i, p in enumerate(model.parameters()):
+            sess.refresh(i, p.values())
+        out, at = [], 0
+        for n in portions:
+            out.append(sess.decode_full(ids[:, at:at + n], at)[0].reshape(sessions, n, -1))
+            at += n
+        state = [sess.read_cache(i) for i in range(sess.cache_count())]
+        sess.close()
+        return np.concatenate(out, axis=1), state
+
+    got, states = run([40, tokens])                                 # the long portion starts from a state
+    want, expected = run([40] + [160] * (tokens // 160) + ([tokens % 160] if tokens % 160 else []))
+    a, b = states[-1], expected[-1]                                 # keys, values, state
+    assert a.shape[1] == shape[0] * shape[1] * shape[2]
+    assert np.max(np.abs(a - b)) <= 2.0 ** -9 * np.max(np.abs(b))
+    assert np.linalg.norm(got - want) <= 2.0 ** -7 * np.linalg.norm(want)
+
+
 def test_paged_prompts():
     cfg, tensors, model = build("even", "bf16")
     ids = tokens_for(cfg, 150)

@@ -15,6 +15,12 @@
 // operands of the next chunk (gates, running products, silu), so one barrier per chunk is enough.  The RMS norm of the
 // output waits in registers for the next chunk's barrier, behind which the other warps' sums of squares are in place.
 //
+// A long prompt of few sessions leaves most SMs without a sequence of their own.  The recurrence is linear in the state, so time is
+// divided then: a first launch (SC_STATES) takes every segment from a zero state to what it adds and to its product of gates, a
+// second one (SC_OUTPUTS) starts every segment from those before it, S = D_j S + L_j in order, all in f32.  One session of 1792 tokens
+// through 8 such mixers of 12 heads of 64 x 64 (and 4 recurrent units, 6 steps), B200: 7.9 ms with 12 CTAs for 254 us each, 6.2 ms
+// with 23 segments (first launch 27 us).
+//
 // The state, the written k R, k / P and the inner weights enter the products as two bf16 halves (split_bf16x2), so that they
 // keep 16 bits; the readout's q P is rounded to bf16 like q itself, v is bf16.
 #include <algorithm>
@@ -44,17 +50,30 @@ __device__ __forceinline__ void hs_gate(float z2, float lower, float rest, float
     k = rest * (t * s);
 }
 
+enum : int { SC_WHOLE = 0, SC_STATES = 1, SC_OUTPUTS = 2 };
+// Segments of a divided scan.  Per (session, head): the states [segments][dim][vdim] they add, the state before the first one, and
+// their products of gates [segments][dim].
+struct HsSegments {
+    uint32_t count, tokens;      // tokens: a multiple of 16
+    float* space;
+    __host__ __device__ size_t unit_floats(uint32_t dim, uint32_t vdim) const { return (size_t)(count + 1) * dim * vdim + (size_t)count * dim; }
+};
+
 // NP: channels padded to a multiple of 64; WARPS: 16 columns each.
-template <int NP, int WARPS>
+template <int NP, int WARPS, int PHASE>
 __global__ void __launch_bounds__(WARPS * 32, NP <= 64 ? (WARPS == 4 ? 4 : 2) : NP <= 128 ? (WARPS == 4 ? 2 : 1) : 1)
-hgrn2_scan_kernel(Hgrn2 m, StepPlace place, uint32_t vec) {
+hgrn2_scan_kernel(Hgrn2 m, StepPlace place, uint32_t vec, HsSegments segments) {
     using S = HsShape<NP, WARPS>;
     constexpr int NT = NP / 8, GROUPS = NP / 16, MINE = (GROUPS + WARPS - 1) / WARPS;    // 16-channel groups, per warp
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ float s_sq[2][WARPS][HS_Q];
     __shared__ uint32_t s_tiny[4];            // by chunk modulo 4: one is set, one read and one cleared between two barriers
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g8 = lane >> 2, t4 = lane & 3;
-    const uint32_t c_first = blockIdx.x * (WARPS * 16), h = blockIdx.y, s = blockIdx.z;
+    const uint32_t c_first = blockIdx.x * (WARPS * 16), h = blockIdx.y;
+    // SC_STATES leaves the last segment out: nothing follows it
+    const uint32_t per_session = PHASE == SC_WHOLE ? 1 : PHASE == SC_STATES ? segments.count - 1 : segments.count;
+    const uint32_t s = blockIdx.z / per_session, segment = blockIdx.z % per_session;
+    const uint32_t begin = PHASE == SC_WHOLE ? 0 : segment * segments.tokens, end = PHASE == SC_WHOLE ? place.chunk : min(place.chunk, begin + segments.tokens);
     const uint32_t width = min((uint32_t)(WARPS * 16), m.vdim - c_first);
     const uint32_t pw = warp * 16;              // the warp's columns
     const bool owner = pw < width, fused = m.vdim <= HGRN2_FUSED_VDIM;
@@ -66,7 +85,14 @@ hgrn2_scan_kernel(Hgrn2 m, StepPlace place, uint32_t vec) {
     const float* fb = m.f + row_base * m.f_ld + h * m.dim;
     const bf16* qb = reinterpret_cast<const bf16*>(m.q) + row_base * m.ld + h * m.dim;
     const bf16* vb = reinterpret_cast<const bf16*>(m.v) + row_base * m.ld + h * m.vdim + c_first;
-    float* state = m.state + (((size_t)s * m.heads + h) * m.dim) * m.vdim + c_first;
+    const size_t unit = (size_t)s * m.heads + h, matrix = (size_t)m.dim * m.vdim;
+    float* state = m.state + unit * matrix + c_first;
+    float* added = segments.space + (PHASE == SC_WHOLE ? 0 : unit * segments.unit_floats(m.dim, m.vdim));     // [count + 1][dim][vdim]
+    float* decays = added + (segments.count + 1) * matrix;                                                    // [count][dim]
+    constexpr int DEC = (NP + WARPS * 32 - 1) / (WARPS * 32);
+    float decay[DEC];           // SC_STATES: products of the channels tid, tid + threads ..
+#pragma unroll
+    for (int i = 0; i < DEC; ++i) decay[i] = 1.0f;
 
     // ---- operands of a chunk: a lane owns two channels of four tokens of a 16-channel group ----
     const uint32_t p8 = lane & 7, tq = lane >> 3;
@@ -89,12 +115,12 @@ hgrn2_scan_kernel(Hgrn2 m, StepPlace place, uint32_t vec) {
                 const uint32_t c = (warp + i * WARPS) * 16 + p8 * 2, t = t0 + tq * 4 + j;
                 raw_f[i][j] = make_float2(0.0f, 0.0f);
                 raw_q[i][j] = 0u;
-                if (t < place.chunk && c < m.dim) {
+                if (t < end && c < m.dim) {
                     const float* f = fb + (size_t)t * m.f_ld + c;
                     const bf16* q = qb + (size_t)t * m.ld + c;
                     if (vec) {
                         raw_f[i][j] = *reinterpret_cast<const float2*>(f);
-                        raw_q[i][j] = *reinterpret_cast<const uint32_t*>(q);
+                        if (PHASE != SC_STATES) raw_q[i][j] = *reinterpret_cast<const uint32_t*>(q);
                     } else {
                         const bool second = c + 1 < m.dim;
                         raw_f[i][j] = make_float2(f[0], second ? f[1] : 0.0f);
@@ -105,25 +131,25 @@ hgrn2_scan_kernel(Hgrn2 m, StepPlace place, uint32_t vec) {
     };
     auto load_v = [&](uint32_t t0, uint8_t* stage) {
         uint8_t* dst = stage + 5 * S::OP;
-        if (t0 < place.chunk) {
+        if (t0 < end) {
             if (vec) {
                 for (uint32_t i = tid; i < HS_Q * WARPS * 2; i += WARPS * 32) {
                     const uint32_t r = i / (WARPS * 2), c = (i % (WARPS * 2)) * 8;
-                    const bool real = t0 + r < place.chunk && c < width;
+                    const bool real = t0 + r < end && c < width;
                     mx_cp16(dst + r * S::VPITCH + c * 2, real ? vb + (size_t)(t0 + r) * m.ld + c : vb, real);
                 }
             } else {
                 for (uint32_t i = tid; i < HS_Q * WARPS * 16; i += WARPS * 32) {
                     const uint32_t r = i / (WARPS * 16), c = i % (WARPS * 16);
                     *reinterpret_cast<bf16*>(dst + r * S::VPITCH + c * 2) =
-                        t0 + r < place.chunk && c < width ? vb[(size_t)(t0 + r) * m.ld + c] : __float2bfloat16_rn(0.0f);
+                        t0 + r < end && c < width ? vb[(size_t)(t0 + r) * m.ld + c] : __float2bfloat16_rn(0.0f);
                 }
             }
         }
         mx_commit();
     };
     auto prepare = [&](uint32_t t0, uint8_t* stage) {
-        const bool whole = t0 + HS_Q <= place.chunk;
+        const bool whole = t0 + HS_Q <= end;
 #pragma unroll
         for (int i = 0; i < MINE; ++i) {
             const uint32_t grp = warp + i * WARPS, c = grp * 16 + p8 * 2;
@@ -138,7 +164,7 @@ hgrn2_scan_kernel(Hgrn2 m, StepPlace place, uint32_t vec) {
                     hs_gate(fmaf(z[e], -HS_LOG2E, bias2[i][e]), lower[i][e], 1.0f - lower[i][e], f[j][e], k[j][e]);
                     q[j][e] = mx_silu(qq[e]);      // 0 past the end and past the last channel
                 }
-                if (!whole && t0 + tq * 4 + j >= place.chunk) { f[j][0] = f[j][1] = 1.0f; k[j][0] = k[j][1] = 0.0f; }
+                if (!whole && t0 + tq * 4 + j >= end) { f[j][0] = f[j][1] = 1.0f; k[j][0] = k[j][1] = 0.0f; }
             }
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
@@ -198,7 +224,7 @@ hgrn2_scan_kernel(Hgrn2 m, StepPlace place, uint32_t vec) {
 #pragma unroll
                 for (int n = 0; n < NP / 32; ++n) {
                     const uint32_t c = lane + 32 * n, t = t0 + i;
-                    if (c >= m.dim || t >= place.chunk) continue;
+                    if (c >= m.dim || t >= end) continue;
                     const float lo = m.lower[h * m.dim + c];
                     float f, k;
                     hs_gate(-HS_LOG2E * (fb[(size_t)t * m.f_ld + c] + m.f_bias[h * m.dim + c]), lo, 1.0f - lo, f, k);
@@ -225,19 +251,39 @@ hgrn2_scan_kernel(Hgrn2 m, StepPlace place, uint32_t vec) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const uint32_t p = pw + g8 + (e >> 1) * 8, n = nt * 8 + t4 * 2 + (e & 1);
-            acc[nt][e] = p0 > 0 && n < m.dim && p < width ? state[(size_t)n * m.vdim + p] : 0.0f;
+            const bool real = n < m.dim && p < width;
+            const size_t at = (size_t)n * m.vdim + p;
+            if (PHASE == SC_OUTPUTS) {
+                acc[nt][e] = real ? __ldcg(added + (segment ? 0 : segments.count) * matrix + c_first + at) : 0.0f;
+            } else {
+                acc[nt][e] = p0 > 0 && segment == 0 && real ? state[at] : 0.0f;
+                if (PHASE == SC_STATES && segment == 0 && real) added[segments.count * matrix + c_first + at] = acc[nt][e];
+            }
         }
+    if (PHASE == SC_OUTPUTS) {
+        for (uint32_t j = 1; j < segment; ++j) {
+            const float* add = added + j * matrix + c_first;
+            const float* d = decays + j * m.dim;
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const uint32_t p = pw + g8 + (e >> 1) * 8, n = nt * 8 + t4 * 2 + (e & 1);
+                    if (n < m.dim && p < width) acc[nt][e] = fmaf(__ldcg(d + n), acc[nt][e], __ldcg(add + (size_t)n * m.vdim + p));
+                }
+        }
+    }
     float nw[4];       // norm weights of the lane's output columns pw + t4 * 2 (+ 1, + 8, + 9)
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         const uint32_t p = pw + (e >> 1) * 8 + t4 * 2 + (e & 1);
         nw[e] = fused && p < width ? m.norm_w[p] * m.gain : 0.0f;
     }
-    fetch(0);
-    load_v(0, smem);
+    fetch(begin);
+    load_v(begin, smem);
     __syncthreads();       // s_tiny is clear
-    prepare(0, smem);
-    fetch(HS_Q);
+    prepare(begin, smem);
+    fetch(begin + HS_Q);
 
     const uint32_t a_off = ((lane & 7) + ((lane >> 3) & 1) * 8) * S::NPITCH + (lane >> 4) * 16;     // A operand, [token][channel]
     const uint32_t b_off = ((lane & 7) + (lane >> 4) * 8) * S::NPITCH + ((lane >> 3) & 1) * 16;     // B operand, [n = token][k = channel]
@@ -251,7 +297,7 @@ hgrn2_scan_kernel(Hgrn2 m, StepPlace place, uint32_t vec) {
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
             const uint32_t t = t0 + g8 + half * 8;
-            if (t >= place.chunk || !owner) continue;
+            if (t >= end || !owner) continue;
             if (!fused) {
                 float* raw = m.raw + (row_base + t) * ((size_t)m.heads * m.vdim) + h * m.vdim + c_first;
 #pragma unroll
@@ -277,13 +323,13 @@ hgrn2_scan_kernel(Hgrn2 m, StepPlace place, uint32_t vec) {
     };
 
     uint32_t buf = 0;
-    for (uint32_t t0 = 0; t0 < place.chunk; t0 += HS_Q, buf ^= 1) {
+    for (uint32_t t0 = begin; t0 < end; t0 += HS_Q, buf ^= 1) {
         uint8_t* stage = smem + buf * S::STAGE;
         uint8_t* next = smem + (buf ^ 1) * S::STAGE;
         const uint32_t sb = mx_smem(stage), sv = sb + 5 * S::OP;
         mx_wait<0>();
         __syncthreads();       // this chunk's operands and the last one's sums are in place, the last one's operands used up
-        if (t0 > 0) finish(t0 - HS_Q);
+        if (PHASE != SC_STATES && t0 > begin) finish(t0 - HS_Q);
         load_v(t0 + HS_Q, next);
         const uint32_t turn = t0 / HS_Q;
         const bool slow = s_tiny[turn & 3] != 0;
@@ -292,7 +338,13 @@ hgrn2_scan_kernel(Hgrn2 m, StepPlace place, uint32_t vec) {
         for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
             for (int e = 0; e < 4; ++e) y[nt][e] = 0.0f;
-        if (owner) {
+        if (PHASE == SC_STATES && blockIdx.x == 0) {
+            const float* all = reinterpret_cast<const float*>(stage + 5 * S::OP + S::V_BYTES);
+#pragma unroll
+            for (int i = 0; i < DEC; ++i)
+                if (tid + i * WARPS * 32 < NP) decay[i] *= all[tid + i * WARPS * 32];
+        }
+        if (PHASE != SC_STATES && owner) {
             // ---- q P . S_in and the inner weights q P . k / P ----
             float yl[2][4] = {}, gm[2][4] = {};        // yl: a second accumulator, shorter chains of dependent products
 #pragma unroll
@@ -332,6 +384,8 @@ hgrn2_scan_kernel(Hgrn2 m, StepPlace place, uint32_t vec) {
             for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) y[nt][e] += yl[nt][e];
+        }
+        if (owner) {
             // ---- S^T: decayed, plus v^T . (k R) ----
             uint32_t va[4];
             mx_ldsm_t(sv + vt_off, va);
@@ -352,6 +406,7 @@ hgrn2_scan_kernel(Hgrn2 m, StepPlace place, uint32_t vec) {
                 mx_mma(acc[2 * n + 1], va, kl[2], kl[3]);
             }
         }
+        if (PHASE != SC_STATES) {
         float sq0 = 0.0f, sq1 = 0.0f;
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {      // columns past the width are zero: v is
@@ -363,15 +418,24 @@ hgrn2_scan_kernel(Hgrn2 m, StepPlace place, uint32_t vec) {
         sq1 += __shfl_xor_sync(0xffffffffu, sq1, 1);
         sq1 += __shfl_xor_sync(0xffffffffu, sq1, 2);
         if (t4 == 0) { s_sq[turn & 1][warp][g8] = sq0; s_sq[turn & 1][warp][g8 + 8] = sq1; }
-        if (t0 + HS_Q < place.chunk) {
+        }
+        if (t0 + HS_Q < end) {
             prepare(t0 + HS_Q, next);
             fetch(t0 + 2 * HS_Q);       // a whole chunk ahead of its use
         }
     }
     mx_wait<0>();
     __syncthreads();
-    finish((place.chunk - 1) / HS_Q * HS_Q);
-    if (owner) {
+    if (PHASE == SC_STATES) {
+        if (blockIdx.x == 0)
+#pragma unroll
+            for (int i = 0; i < DEC; ++i)
+                if (tid + i * WARPS * 32 < m.dim) decays[segment * m.dim + tid + i * WARPS * 32] = decay[i];
+        state = added + segment * matrix + c_first;
+    } else {
+        finish((end - 1) / HS_Q * HS_Q);
+    }
+    if (owner && (PHASE != SC_OUTPUTS || segment + 1 == segments.count)) {
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -380,27 +444,57 @@ hgrn2_scan_kernel(Hgrn2 m, StepPlace place, uint32_t vec) {
                 if (n < m.dim && p < width) state[(size_t)n * m.vdim + p] = acc[nt][e];
             }
     }
-    if (fused && h + 1 == m.heads && m.out_cols > m.heads * m.vdim) {
+    if (PHASE != SC_STATES && fused && h + 1 == m.heads && m.out_cols > m.heads * m.vdim) {
         const uint32_t pad = m.out_cols - m.heads * m.vdim;
-        for (uint64_t i = tid; i < (uint64_t)pad * place.chunk; i += WARPS * 32)
-            reinterpret_cast<bf16*>(m.out)[(row_base + i / pad) * m.out_ld + m.heads * m.vdim + i % pad] = __float2bfloat16_rn(0.0f);
+        for (uint64_t i = tid; i < (uint64_t)pad * (end - begin); i += WARPS * 32)
+            reinterpret_cast<bf16*>(m.out)[(row_base + begin + i / pad) * m.out_ld + m.heads * m.vdim + i % pad] = __float2bfloat16_rn(0.0f);
     }
 }
 
-template <int NP, int WARPS>
-static int launch_scan(const Hgrn2& m, const StepPlace& place, uint32_t vec, cudaStream_t stream) {
+template <int NP, int WARPS, int PHASE>
+static int launch_phase(const Hgrn2& m, const StepPlace& place, uint32_t vec, const HsSegments& segments, cudaStream_t stream) {
     static bool configured[64] = {};
     const uint32_t bytes = HsShape<NP, WARPS>::BYTES;
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !configured[dev]) {
-        if (cudaFuncSetAttribute(hgrn2_scan_kernel<NP, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
+        if (cudaFuncSetAttribute(hgrn2_scan_kernel<NP, WARPS, PHASE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
             return check_launch("hgrn2_scan attribute");
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    launch_kernel(hgrn2_scan_kernel<NP, WARPS>, dim3(ceil_div(m.vdim, WARPS * 16u), m.heads, place.sessions), dim3(WARPS * 32), bytes, stream, m, place, vec);
+    const uint32_t per_session = PHASE == SC_WHOLE ? 1 : PHASE == SC_STATES ? segments.count - 1 : segments.count;
+    launch_kernel(hgrn2_scan_kernel<NP, WARPS, PHASE>, dim3(ceil_div(m.vdim, WARPS * 16u), m.heads, place.sessions * per_session), dim3(WARPS * 32), bytes,
+                  stream, m, place, vec, segments);
     count_launch();
     return check_launch("hgrn2_scan");
+}
+
+// Segments for so many sequences: two CTAs per SM (they wait for each other little), at least four chunks each so that a segment is longer
+// than its part of the second pass, and only where there are three segments, since every token is taken through the gates twice.
+constexpr uint32_t HS_CTAS = 296, HS_LEAST_CHUNKS = 4;
+static uint32_t most_segments(uint32_t heads, uint32_t vdim, uint32_t sessions, uint32_t chunk) {
+    const uint64_t ctas = (uint64_t)sessions * heads * ceil_div(vdim, vdim <= 64 ? 64u : 128u);
+    return (uint32_t)std::min<uint64_t>(ceil_div(chunk, (uint32_t)HS_Q) / HS_LEAST_CHUNKS, HS_CTAS / std::max<uint64_t>(1, ctas));
+}
+static HsSegments divide(uint32_t most, uint32_t chunk) {
+    const uint32_t chunks = ceil_div(chunk, (uint32_t)HS_Q), each = ceil_div(chunks, most);
+    return {ceil_div(chunks, each), each * HS_Q, nullptr};
+}
+// Grows with the chunk, so that scratch for the longest one serves the others.
+uint64_t hgrn2_scan_workspace_bytes(uint32_t sessions, uint32_t chunk, uint32_t heads, uint32_t dim, uint32_t vdim) {
+    const uint32_t most = most_segments(heads, vdim, sessions, chunk);
+    return most < 3 ? 0 : (uint64_t)sessions * heads * HsSegments{most, 0, nullptr}.unit_floats(dim, vdim) * 4;
+}
+
+template <int NP, int WARPS>
+static int launch_scan(const Hgrn2& m, const StepPlace& place, uint32_t vec, cudaStream_t stream) {
+    const uint32_t most = most_segments(m.heads, m.vdim, place.sessions, place.chunk);
+    if (most < 3 || m.segment_bytes < hgrn2_scan_workspace_bytes(place.sessions, place.chunk, m.heads, m.dim, m.vdim))
+        return launch_phase<NP, WARPS, SC_WHOLE>(m, place, vec, HsSegments{1, 0, nullptr}, stream);
+    HsSegments g = divide(most, place.chunk);
+    g.space = m.segment_space;
+    int rc = launch_phase<NP, WARPS, SC_STATES>(m, place, vec, g, stream);
+    return rc ? rc : launch_phase<NP, WARPS, SC_OUTPUTS>(m, place, vec, g, stream);
 }
 
 int launch_hgrn2_scan(const Hgrn2& m, const StepPlace& place, cudaStream_t stream) {

@@ -100,6 +100,8 @@ struct LayerStack {
     void* attention_ws = nullptr;
     uint64_t attention_ws_bytes = 0;
     float* raw = nullptr;     // [rows, rec_heads * rec_vdim] of hgrn2 with wide heads
+    float* segments = nullptr;          // of a prompt whose hgrn2 scan is divided in time
+    uint64_t segments_bytes = 0;
     void* u = nullptr;        // [rows, width] of rglru
     float* gates = nullptr;   // [rows, 2 width]
     void* ff_z = nullptr;     // [rows, ff]: up before polynorm
@@ -537,7 +539,7 @@ bool stack_cache(const tnsr_b200_decoder* dec, uint32_t index, void** ptr, uint6
 int stack_alloc_rows(tnsr_b200_decoder* dec, uint32_t rows) {
     LayerStack* S = dec->stack;
     const size_t e = elt(dec);
-    uint64_t proj = 0, tail = 0, cat = 0, q = 0, xbc = 0, gated = 0, raw = 0, u = 0, ff_z = 0, ff_act = 0, router = 0, experts = 0;
+    uint64_t proj = 0, tail = 0, cat = 0, q = 0, xbc = 0, gated = 0, raw = 0, u = 0, ff_z = 0, ff_act = 0, router = 0, experts = 0, segments = 0;
     for (const StackLayer& L : S->layers) {
         const tnsr_b200_layer& l = L.cfg;
         proj = std::max<uint64_t>(proj, L.proj_cols);
@@ -549,6 +551,8 @@ int stack_alloc_rows(tnsr_b200_decoder* dec, uint32_t rows) {
             gated = std::max<uint64_t>(gated, L.mixer_width);
         }
         if (l.mixer == TNSR_B200_MIXER_ATTENTION_HGRN2 && l.rec_vdim > HGRN2_FUSED_VDIM) raw = std::max<uint64_t>(raw, (uint64_t)l.rec_heads * l.rec_vdim);
+        if (l.mixer == TNSR_B200_MIXER_ATTENTION_HGRN2 && dec->bf16_path)
+            segments = std::max(segments, hgrn2_scan_workspace_bytes(dec->cfg.batch, rows / dec->cfg.batch, l.rec_heads, l.rec_dim, l.rec_vdim));
         if (l.mixer == TNSR_B200_MIXER_RGLRU) u = std::max<uint64_t>(u, l.width);
         if (!sequential(l) || !l.feed_forward) continue;
         if (l.feed_forward_kind == TNSR_B200_FF_EXPERTS) {
@@ -560,9 +564,10 @@ int stack_alloc_rows(tnsr_b200_decoder* dec, uint32_t rows) {
         }
     }
     S->experts_ws_bytes = experts;
+    S->segments_bytes = segments;
     struct { void** p; uint64_t bytes; } want[] = {{&S->proj, proj * e * rows}, {(void**)&S->tail, tail * 4 * rows}, {&S->cat, cat * e * rows},
                                                    {&S->q, q * e * rows}, {&S->xbc, xbc * e * rows}, {&S->gated, gated * e * rows},
-                                                   {(void**)&S->raw, raw * 4 * rows}, {&S->u, u * e * rows}, {(void**)&S->gates, 2 * u * 4 * rows},
+                                                   {(void**)&S->raw, raw * 4 * rows}, {(void**)&S->segments, segments}, {&S->u, u * e * rows}, {(void**)&S->gates, 2 * u * 4 * rows},
                                                    {&S->ff_z, ff_z * e * rows}, {&S->ff_act, ff_act * e * rows}, {(void**)&S->router, router * 4 * rows},
                                                    {&S->experts_ws, experts}};
     for (auto& w : want) {
@@ -701,7 +706,7 @@ int stack_step(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chunk,
             m.q = (const uint8_t*)S->proj + (size_t)L.rec_q_col * e; m.v = (const uint8_t*)S->proj + (size_t)L.rec_v_col * e; m.ld = L.proj_cols;
             m.f = S->tail; m.f_ld = L.tail_cols; m.heads = l.rec_heads; m.dim = l.rec_dim; m.vdim = l.rec_vdim;
             m.f_bias = W.f_bias; m.lower = W.lower; m.norm_w = W.norm_w; m.eps = eps; m.gain = (float)l.recurrent_gain;
-            m.state = L.ssm; m.raw = S->raw;
+            m.state = L.ssm; m.raw = S->raw; m.segment_space = S->segments; m.segment_bytes = S->segments_bytes;
             m.out = (uint8_t*)S->cat + (size_t)L.rec_col * e; m.out_ld = L.k_out; m.out_cols = L.mixer_cols - L.rec_col;
             m.engine = plain_prefill ? 1 : 0;
             RUN(dec, launch_hgrn2(m, place, dtype, st));

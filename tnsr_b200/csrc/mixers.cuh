@@ -139,7 +139,10 @@ struct Hgrn2 {
     void* out = nullptr;               // [rows, out_ld]; columns [heads * vdim, out_cols) are zeroed
     uint32_t out_ld = 0, out_cols = 0;
     int engine = 0;                    // 0: best kernel for the shape, 1: token by token
+    float* segment_space = nullptr;    // hgrn2_scan_workspace_bytes() of scratch: a long prompt of few sessions is divided in time
+    uint64_t segment_bytes = 0;
 };
+uint64_t hgrn2_scan_workspace_bytes(uint32_t sessions, uint32_t chunk, uint32_t heads, uint32_t dim, uint32_t vdim);
 constexpr uint32_t HGRN2_FUSED_VDIM = 128;   // value width up to which the kernels norm their own output
 bool hgrn2_supported(uint32_t heads, uint32_t dim, uint32_t vdim);
 int launch_hgrn2(const Hgrn2& m, const StepPlace& place, int dtype, cudaStream_t stream);
