@@ -6,7 +6,10 @@
 // part] matrix per block (r rows, then i rows), f32 out.
 //  * rglru_scan_kernel   many tokens: a block owns a strip of channels of one session; its eight warps take consecutive
 //                        segments of 8 tokens each, which are scanned side by side from zero, joined through shared memory
-//                        (each segment is S -> A S + H) and finished from registers: every value is read once.
+//                        (each segment is S -> A S + H) and finished from registers: every value is read once.  Few sessions leave
+//                        SMs idle: then a cluster of up to 8 blocks takes consecutive runs of 64 tokens of a strip side by side,
+//                        joined the same way through distributed shared memory (1792 tokens x 1024 channels of one session, B200:
+//                        97 us without, 29 us with clusters of 8).
 //  * rglru_fused_step_kernel  single-token steps, bf16, parts of a multiple of 32 channels up to 256: convolution, both gates
 //                        and the recurrence in one launch.  The gates of a part need its own channels only, so nothing
 //                        passes between parts.
@@ -61,16 +64,29 @@ __device__ __forceinline__ float2 rg_values(float2 v) { return v; }
 __device__ __forceinline__ float2 rg_values(bf16 v) { return make_float2(__bfloat162float(v), 0.0f); }
 __device__ __forceinline__ float2 rg_values(float v) { return make_float2(v, 0.0f); }
 
-template <typename T, int VEC>
-__global__ void __launch_bounds__(RG_WARPS * 32, 3)
-rglru_scan_kernel(Rglru m, StepPlace place) {
+__device__ __forceinline__ void rg_cluster_sync() { asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ float4 rg_load_peer(const float4* local, uint32_t rank) {
+    const uint32_t at = (uint32_t)__cvta_generic_to_shared(local);
+    uint32_t remote;
+    float4 v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
+    return v;
+}
+
+// CLUSTER: `cluster_size` blocks share a strip, each with every cluster_size-th run of 64 tokens.
+template <typename T, int VEC, bool CLUSTER>
+__global__ void __launch_bounds__(RG_WARPS * 32, CLUSTER ? 2 : 3)
+rglru_scan_kernel(Rglru m, StepPlace place, uint32_t cluster_size) {
+    const uint32_t cluster = CLUSTER ? cluster_size : 1;
     constexpr uint32_t STRIP = 32 * VEC;
     typedef typename RgRaw<T, VEC>::type Raw;
     __shared__ float4 seg[2][RG_WARPS][32];          // per lane: A of its channels, H of its channels
+    __shared__ float4 run[2][32];                    // the same of the block's run
     pdl_wait();
     pdl_trigger();
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, s = blockIdx.y;
-    const uint32_t c = blockIdx.x * STRIP + lane * VEC;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, s = blockIdx.y, strip = blockIdx.x / cluster, rank = blockIdx.x % cluster;
+    const uint32_t c = strip * STRIP + lane * VEC;
     const bool live = c < m.width;
     const uint32_t part = m.width / m.blocks, rows = place.sessions * place.chunk;
     const uint32_t cc = live ? c : 0, blk = cc / part, local = cc % part;
@@ -87,8 +103,8 @@ rglru_scan_kernel(Rglru m, StepPlace place) {
         carry[e] = place.pos(s) > 0 ? m.state[(size_t)s * m.width + cc + e] : 0.0f;
     }
     uint32_t buf = 0;
-    for (uint32_t t0 = 0; t0 < place.chunk; t0 += RG_WARPS * RG_SEG, buf ^= 1) {
-        const uint32_t first = t0 + warp * RG_SEG;
+    for (uint32_t t0 = 0; t0 < place.chunk; t0 += cluster * RG_WARPS * RG_SEG, buf ^= 1) {
+        const uint32_t first = t0 + (rank * RG_WARPS + warp) * RG_SEG;
         float a[RG_SEG][VEC], b[RG_SEG][VEC];
         Raw yy[RG_SEG], uu[RG_SEG];
 #pragma unroll
@@ -125,7 +141,29 @@ rglru_scan_kernel(Rglru m, StepPlace place) {
         }
         seg[buf][warp][lane] = make_float4(A[0], A[VEC - 1], H[0], H[VEC - 1]);
         __syncthreads();       // the other buffer is rewritten only after the next barrier
-        float S[VEC];
+        float S[VEC], next[VEC];
+        if (CLUSTER) {
+            if (warp == 0) {
+                float4 r = make_float4(1.0f, 1.0f, 0.0f, 0.0f);
+#pragma unroll
+                for (uint32_t w = 0; w < RG_WARPS; ++w) {
+                    const float4 q = seg[buf][w][lane];
+                    r = make_float4(q.x * r.x, q.y * r.y, fmaf(q.x, r.z, q.z), fmaf(q.y, r.w, q.w));
+                }
+                run[buf][lane] = r;
+            }
+            rg_cluster_sync();     // a block rewrites this buffer two rounds on, behind the next round's barrier
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) next[e] = carry[e];
+            for (uint32_t r = 0; r < cluster; ++r) {
+                const float4 q = rg_load_peer(&run[buf][lane], r);
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) {
+                    if (r == rank) carry[e] = next[e];
+                    next[e] = e ? fmaf(q.y, next[e], q.w) : fmaf(q.x, next[e], q.z);
+                }
+            }
+        }
 #pragma unroll
         for (uint32_t w = 0; w < RG_WARPS; ++w) {
             const float4 q = seg[buf][w][lane];
@@ -134,6 +172,10 @@ rglru_scan_kernel(Rglru m, StepPlace place) {
                 if (w == warp) S[e] = carry[e];
                 carry[e] = e ? fmaf(q.y, carry[e], q.w) : fmaf(q.x, carry[e], q.z);
             }
+        }
+        if (CLUSTER) {
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) carry[e] = next[e];
         }
 #pragma unroll
         for (uint32_t i = 0; i < RG_SEG; ++i) {
@@ -147,10 +189,11 @@ rglru_scan_kernel(Rglru m, StepPlace place) {
             else out[(size_t)t * m.out_ld] = from_f32<T>(o[0]);
         }
     }
-    if (warp == 0 && live)
+    if (warp == 0 && live && rank == 0)
 #pragma unroll
         for (int e = 0; e < VEC; ++e) m.state[(size_t)s * m.width + c + e] = carry[e];
-    if (blockIdx.x == 0 && m.out_cols > m.width) {
+    if (CLUSTER) rg_cluster_sync();       // peers still read this block's run
+    if (strip == 0 && rank == 0 && m.out_cols > m.width) {
         const uint32_t pad = m.out_cols - m.width;
         for (uint64_t i = threadIdx.x; i < (uint64_t)pad * place.chunk; i += blockDim.x)
             reinterpret_cast<T*>(m.out)[(row0 + i / pad) * m.out_ld + m.width + i % pad] = from_f32<T>(0.0f);
@@ -322,8 +365,32 @@ static void rglru_typed(const Rglru& m, const StepPlace& place, cudaStream_t str
     const uint32_t part = m.width / m.blocks;
     const bool pairs = part % 2 == 0 && m.ld % 2 == 0 && m.out_ld % 2 == 0 && even(m.proj) && even(m.u) && even(m.out) &&
                        reinterpret_cast<uintptr_t>(m.gates) % 8 == 0;
-    if (pairs) launch_kernel(rglru_scan_kernel<T, 2>, dim3(ceil_div(m.width, 64u), place.sessions), dim3(RG_WARPS * 32), 0, stream, m, place);
-    else launch_kernel(rglru_scan_kernel<T, 1>, dim3(ceil_div(m.width, 32u), place.sessions), dim3(RG_WARPS * 32), 0, stream, m, place);
+    // as many blocks per strip as have a run of their own and find room, two per SM
+    const uint32_t strips = ceil_div(m.width, pairs ? 64u : 32u), runs = ceil_div(place.chunk, RG_WARPS * RG_SEG);
+    uint32_t cluster = 1;
+    while (cluster < 8 && cluster < runs && (uint64_t)strips * place.sessions * cluster * 2 <= 296) cluster *= 2;
+    auto scan = cluster > 1 ? (pairs ? rglru_scan_kernel<T, 2, true> : rglru_scan_kernel<T, 1, true>)
+                            : (pairs ? rglru_scan_kernel<T, 2, false> : rglru_scan_kernel<T, 1, false>);
+    prefer_max_shared_carveout(reinterpret_cast<const void*>(scan));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(strips * cluster, place.sessions);
+    cfg.blockDim = dim3(RG_WARPS * 32);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    uint32_t count = 0;
+    if (t_pdl) {
+        attr[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[count++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[count].id = cudaLaunchAttributeClusterDimension;
+        attr[count].val.clusterDim.x = cluster;
+        attr[count].val.clusterDim.y = attr[count].val.clusterDim.z = 1;
+        ++count;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = count;
+    cudaLaunchKernelEx(&cfg, scan, m, place, cluster);
 }
 
 int launch_rglru(const Rglru& m, const StepPlace& place, int dtype, cudaStream_t stream) {
