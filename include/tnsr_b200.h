@@ -341,6 +341,12 @@ TNSR_B200_API int tnsr_b200_decoder_decode(tnsr_b200_decoder* dec, const uint32_
                                            uint32_t chunk, uint32_t position, float* logits_out,
                                            uint32_t* argmax_out);
 
+/* Page-locked host memory for results (no reference counterpart): logits that
+ * are copied there skip the driver's detour through a staging buffer.  NULL if
+ * there is none to be had. */
+TNSR_B200_API void* tnsr_b200_host_alloc(uint64_t bytes);
+TNSR_B200_API void tnsr_b200_host_free(void* p);
+
 /* Ragged single-token step (no reference counterpart: the reference's sessions
  * advance together; its documentation lists ragged batches as future work,
  * docs/kv-cache.md:94-95).  Session b consumes tokens[b] at its own position

@@ -741,8 +741,8 @@ static int create_decoder(const tnsr_b200_config* config, const tnsr_b200_stack*
     if ((rc = stack ? stack_create(dec, stack) : allocate_weights(dec))) return bail(rc);
     const uint64_t d = config->embed_dim;
     if ((rc = dev_alloc(dec, (void**)&dec->hl, (size_t)config->batch * d * 4, false))) return bail(rc);
-    if ((rc = dev_alloc(dec, (void**)&dec->d_argmax, (size_t)config->batch * 4, true))) return bail(rc);
-    if ((rc = dev_alloc(dec, (void**)&dec->d_status, 16, true))) return bail(rc);
+    if ((rc = dev_alloc(dec, (void**)&dec->d_status, 16 + (size_t)config->batch * 4, true))) return bail(rc);
+    dec->d_argmax = (uint32_t*)(dec->d_status + 4);     // status word and greedy ids come down in one copy
     if ((rc = dev_alloc(dec, (void**)&dec->d_pos, 16, true))) return bail(rc);
     if (dec->bf16_path && config->logits_mode == TNSR_B200_LOGITS_NONE)
         if ((rc = dev_alloc(dec, &dec->lm_candidates, lm_head_argmax_scratch_bytes(config->batch, config->vocab_size), false)))
@@ -754,9 +754,10 @@ static int create_decoder(const tnsr_b200_config* config, const tnsr_b200_stack*
         if (v && v[0] == '1') dec->use_pdl = false;
 
     }
-    if (cudaMallocHost((void**)&dec->h_argmax, (size_t)config->batch * 4) != cudaSuccess ||
-        cudaMallocHost((void**)&dec->h_status, 16) != cudaSuccess)
+    if (cudaMallocHost((void**)&dec->h_status, 16 + (size_t)config->batch * 4) != cudaSuccess ||
+        cudaMallocHost((void**)&dec->h_logits, kStagedLogitBytes) != cudaSuccess)
         return bail(cuda_fail(dec, cudaGetLastError(), "cudaMallocHost"));
+    dec->h_argmax = (uint32_t*)(dec->h_status + 4);
     *dec->h_status = 0;
     if (!stack && dec->bf16_path && decode_attention_supported(config->num_heads, config->embed_dim / config->num_heads)) {
         dec->attn_ws_bytes = decode_attention_workspace_bytes(config->batch, config->capacity, config->num_heads,
@@ -815,7 +816,7 @@ void tnsr_b200_decoder_destroy(tnsr_b200_decoder* dec) {
     stack_destroy(dec);
     for (void* p : dec->allocations) cudaFree(p);
     if (dec->h_tokens) cudaFreeHost(dec->h_tokens);
-    if (dec->h_argmax) cudaFreeHost(dec->h_argmax);
+    if (dec->h_logits) cudaFreeHost(dec->h_logits);
     if (dec->h_positions) cudaFreeHost(dec->h_positions);
     if (dec->h_status) cudaFreeHost(dec->h_status);
     if (dec->h_stage) cudaFreeHost(dec->h_stage);
@@ -986,6 +987,26 @@ static int device_status_to_code(tnsr_b200_decoder* dec, int status) {
     }
 }
 
+// Results of the queued step to the host.  A copy to pageable memory waits for everything before it and holds up what is queued behind
+// it: status and ids come first, in one copy, and logits of up to kStagedLogitBytes go through page-locked memory of the handle, so that
+// there is one wait.  Larger logits go straight to the caller, whose memory may be page-locked (tnsr_b200_host_alloc).
+static int finish_step(tnsr_b200_decoder* dec, float* logits_out, size_t logit_bytes, uint32_t* argmax_out) {
+    const size_t id_bytes = argmax_out ? (size_t)dec->cfg.batch * 4 : 0;
+    const bool staged = logits_out && logit_bytes <= kStagedLogitBytes;
+    CU(dec, cudaMemcpyAsync(dec->h_status, dec->d_status, 16 + id_bytes, cudaMemcpyDeviceToHost, dec->stream));
+    if (logits_out) CU(dec, cudaMemcpyAsync(staged ? dec->h_logits : logits_out, dec->logits, logit_bytes, cudaMemcpyDeviceToHost, dec->stream));
+    CU(dec, cudaStreamSynchronize(dec->stream));
+    if (*dec->h_status != DEV_OK) {
+        int status = *dec->h_status;
+        cudaMemsetAsync(dec->d_status, 0, 16, dec->stream);
+        return device_status_to_code(dec, status);
+    }
+    if (staged) std::memcpy(logits_out, dec->h_logits, logit_bytes);
+    if (argmax_out) std::memcpy(argmax_out, dec->h_argmax, id_bytes);
+    dec->failed = false;
+    return TNSR_B200_OK;
+}
+
 int tnsr_b200_decoder_decode(tnsr_b200_decoder* dec, const uint32_t* tokens, uint32_t chunk, uint32_t position,
                              float* logits_out, uint32_t* argmax_out) {
     if (!dec) return fail(nullptr, TNSR_B200_ERR_INVALID_ARGUMENT, "null decoder");
@@ -1006,20 +1027,7 @@ int tnsr_b200_decoder_decode(tnsr_b200_decoder* dec, const uint32_t* tokens, uin
     std::memcpy(dec->h_tokens, tokens, (size_t)rows * 4);
     CU(dec, cudaMemcpyAsync(dec->d_tokens, dec->h_tokens, (size_t)rows * 4, cudaMemcpyHostToDevice, dec->stream));
     if ((rc = run_step(dec, dec->d_tokens, chunk, position, argmax_out ? dec->d_argmax : nullptr))) return rc;
-    if (logits_out)
-        CU(dec, cudaMemcpyAsync(logits_out, dec->logits, (size_t)logit_rows * c.vocab_size * 4, cudaMemcpyDeviceToHost, dec->stream));
-    if (argmax_out)
-        CU(dec, cudaMemcpyAsync(dec->h_argmax, dec->d_argmax, (size_t)c.batch * 4, cudaMemcpyDeviceToHost, dec->stream));
-    CU(dec, cudaMemcpyAsync(dec->h_status, dec->d_status, 4, cudaMemcpyDeviceToHost, dec->stream));
-    CU(dec, cudaStreamSynchronize(dec->stream));
-    if (*dec->h_status != DEV_OK) {
-        int status = *dec->h_status;
-        cudaMemsetAsync(dec->d_status, 0, 16, dec->stream);
-        return device_status_to_code(dec, status);
-    }
-    if (argmax_out) std::memcpy(argmax_out, dec->h_argmax, (size_t)c.batch * 4);
-    dec->failed = false;
-    return TNSR_B200_OK;
+    return finish_step(dec, logits_out, (size_t)logit_rows * c.vocab_size * 4, argmax_out);
 }
 
 // One new token per session, every session at its own position (no reference counterpart: the reference's
@@ -1070,20 +1078,7 @@ int tnsr_b200_decoder_decode_ragged(tnsr_b200_decoder* dec, const uint32_t* toke
                       : launch_argmax(dec->logits, dec->d_argmax, c.batch, c.vocab_size, c.vocab_size, dec->stream);
         if (rc) { dec->error = thread_error(); return rc; }
     }
-    if (logits_out)
-        CU(dec, cudaMemcpyAsync(logits_out, dec->logits, (size_t)c.batch * c.vocab_size * 4, cudaMemcpyDeviceToHost, dec->stream));
-    if (argmax_out)
-        CU(dec, cudaMemcpyAsync(dec->h_argmax, dec->d_argmax, (size_t)c.batch * 4, cudaMemcpyDeviceToHost, dec->stream));
-    CU(dec, cudaMemcpyAsync(dec->h_status, dec->d_status, 4, cudaMemcpyDeviceToHost, dec->stream));
-    CU(dec, cudaStreamSynchronize(dec->stream));
-    if (*dec->h_status != DEV_OK) {
-        int status = *dec->h_status;
-        cudaMemsetAsync(dec->d_status, 0, 16, dec->stream);
-        return device_status_to_code(dec, status);
-    }
-    if (argmax_out) std::memcpy(argmax_out, dec->h_argmax, (size_t)c.batch * 4);
-    dec->failed = false;
-    return TNSR_B200_OK;
+    return finish_step(dec, logits_out, (size_t)c.batch * c.vocab_size * 4, argmax_out);
 }
 
 int tnsr_b200_decoder_decode_device(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chunk, uint32_t position,
@@ -1099,6 +1094,20 @@ int tnsr_b200_decoder_decode_device(tnsr_b200_decoder* dec, const uint32_t* d_to
     if ((rc = ensure_rows(dec, rows, logit_rows))) return rc;
     if ((rc = reserve_uniform(dec, position + chunk))) return rc;
     return run_step(dec, d_tokens, chunk, position, d_argmax_out);
+}
+
+void* tnsr_b200_host_alloc(uint64_t bytes) {
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, bytes, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return p;
+}
+
+void tnsr_b200_host_free(void* p) {
+    if (p) cudaFreeHost(p);
+    cudaGetLastError();
 }
 
 int tnsr_b200_decoder_set_sampler(tnsr_b200_decoder* dec, float temperature, uint32_t top_k, uint64_t seed) {

