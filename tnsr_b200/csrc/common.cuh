@@ -253,6 +253,15 @@ int launch_decode_attention_ex(const bf16* q, const bf16* k_cache, const bf16* v
                                const KvPaging* paging = nullptr);
 int launch_pack_gate_up(const bf16* wg, const bf16* wu, const float* bg, const float* bu, bf16* w_out,
                         float* b_out, uint32_t d, uint32_t f, cudaStream_t stream);
+// Zeroes the listed regions (16-byte aligned) in one launch; regions past kClearAlone bytes keep a memset of their own.
+constexpr uint32_t kClearRegions = 128;
+constexpr uint64_t kClearAlone = 4u << 20;
+struct ClearList {
+    void* at[kClearRegions];
+    uint64_t bytes[kClearRegions];
+    uint32_t count = 0;
+};
+int launch_clear(const ClearList& list, cudaStream_t stream);
 int launch_fill_u32(uint32_t* p, uint32_t value, uint32_t n, cudaStream_t stream);
 int launch_add_u32(uint32_t* p, uint32_t delta, cudaStream_t stream);
 

@@ -955,15 +955,15 @@ int tnsr_b200_decoder_reset(tnsr_b200_decoder* dec) {
         std::fill(dec->h_table_shadow.begin(), dec->h_table_shadow.end(), kNoPage);
         dec->table_dirty = true;
     }
-    if (dec->stack) {
-        int rc = stack_reset(dec);
-        if (rc) return rc;
-    }
+    Clearing clear(dec);
+    int rc;
+    if (dec->stack && (rc = stack_reset(dec, clear))) return rc;
     for (Layer& L : dec->layers) {
-        CU(dec, cudaMemsetAsync(L.kcache, 0, cache_bytes, dec->stream));
-        CU(dec, cudaMemsetAsync(L.vcache, 0, cache_bytes, dec->stream));
+        if ((rc = clear.add(L.kcache, cache_bytes))) return rc;
+        if ((rc = clear.add(L.vcache, cache_bytes))) return rc;
     }
-    CU(dec, cudaMemsetAsync(dec->d_status, 0, 16, dec->stream));
+    if ((rc = clear.add(dec->d_status, 16))) return rc;
+    if ((rc = clear.finish())) return rc;
     CU(dec, cudaStreamSynchronize(dec->stream));
     dec->failed = false;
     return TNSR_B200_OK;

@@ -166,6 +166,31 @@ inline int cuda_fail(tnsr_b200_decoder* dec, cudaError_t e, const char* what) {
         }                                                               \
     } while (0)
 
+// Collects regions to zero on the handle's stream: the small ones in one launch, the large ones as memsets.
+struct Clearing {
+    tnsr_b200_decoder* dec;
+    ClearList list;
+    explicit Clearing(tnsr_b200_decoder* d) : dec(d) {}
+    int add(void* p, uint64_t bytes) {
+        if (bytes > kClearAlone) {
+            CU(dec, cudaMemsetAsync(p, 0, bytes, dec->stream));
+            return TNSR_B200_OK;
+        }
+        if (list.count == kClearRegions) {
+            int rc = finish();
+            if (rc) return rc;
+        }
+        list.at[list.count] = p;
+        list.bytes[list.count++] = bytes;
+        return TNSR_B200_OK;
+    }
+    int finish() {
+        RUN(dec, launch_clear(list, dec->stream));
+        list.count = 0;
+        return TNSR_B200_OK;
+    }
+};
+
 inline void drop_graphs(tnsr_b200_decoder* dec) {
     for (auto& g : dec->graphs) cudaGraphExecDestroy(g.exec);
     dec->graphs.clear();
@@ -207,7 +232,7 @@ void stack_destroy(tnsr_b200_decoder* dec);
 uint32_t stack_param_count(const tnsr_b200_decoder* dec);
 uint64_t stack_param_elems(const tnsr_b200_decoder* dec, uint32_t index);
 int stack_upload(tnsr_b200_decoder* dec, uint32_t index, const float* host);
-int stack_reset(tnsr_b200_decoder* dec);                                  // queues zeroing of every cache and state
+int stack_reset(tnsr_b200_decoder* dec, Clearing& clear);                 // queues zeroing of every cache and state
 int stack_alloc_rows(tnsr_b200_decoder* dec, uint32_t rows);             // (re)allocates the activation buffers for `rows` rows
 // One step: embedding, all layers, final norm, and logits or (fused_ids) greedy ids.
 int stack_step(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chunk, uint32_t position, const uint32_t* d_position,

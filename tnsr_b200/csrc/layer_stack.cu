@@ -521,11 +521,11 @@ int stack_upload(tnsr_b200_decoder* dec, uint32_t index, const float* host) {
     return TNSR_B200_OK;
 }
 
-int stack_reset(tnsr_b200_decoder* dec) {
+int stack_reset(tnsr_b200_decoder* dec, Clearing& clear) {
+    int rc;
     for (const StackCache& t : dec->stack->caches)
-        CU(dec, cudaMemsetAsync(t.ptr, 0, t.elems * (t.dtype == TNSR_B200_BF16 ? 2 : 4), dec->stream));
-    if (dec->stack->attention_ws) CU(dec, cudaMemsetAsync(dec->stack->attention_ws, 0, dec->stack->attention_ws_bytes, dec->stream));
-    return TNSR_B200_OK;
+        if ((rc = clear.add(t.ptr, t.elems * (t.dtype == TNSR_B200_BF16 ? 2 : 4)))) return rc;
+    return dec->stack->attention_ws ? clear.add(dec->stack->attention_ws, dec->stack->attention_ws_bytes) : TNSR_B200_OK;
 }
 
 uint32_t stack_cache_count(const tnsr_b200_decoder* dec) { return (uint32_t)dec->stack->caches.size(); }
