@@ -108,8 +108,6 @@ grouped_split_kernel(GaParams P) {
     const GroupedAttention& a = P.a;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g8 = lane >> 2, t4 = lane & 3;
     const uint32_t split = blockIdx.x, tile = blockIdx.y % P.row_tiles, kvh = blockIdx.y / P.row_tiles, s = blockIdx.z;
-    pdl_wait();
-    pdl_trigger();
     const uint32_t p0 = P.place.pos(s), row0 = tile * 16;
     const uint32_t n_rows = min(16u, P.rows - row0);
     const uint32_t keys = min(p0 + (row0 + n_rows - 1) / P.per + 1, a.capacity);    // visible to the tile's last row
@@ -127,7 +125,7 @@ grouped_split_kernel(GaParams P) {
 
     uint8_t* ring = smem + warp * (STAGES * S::STAGE);
     const size_t k_ld = (size_t)a.kv_heads * a.dim, v_ld = (size_t)a.kv_heads * a.vdim;
-    auto load = [&](uint32_t i, uint32_t stage) {     // tile i of the session; the pages of a tile's 16 keys are one page
+    auto copy = [&](uint32_t i, uint32_t stage) {     // tile i of the session; the pages of a tile's 16 keys are one page
         if (i < tile1) {
             const size_t kr = kv_row(a.paging, s, i * 16, a.capacity);
             const uint32_t live = min(16u, keys - i * 16);
@@ -136,10 +134,23 @@ grouped_split_kernel(GaParams P) {
             ga_copy<DV>(dst + 16 * S::KP, reinterpret_cast<const bf16*>(a.v_cache) + kr * v_ld + (size_t)kvh * a.vdim, v_ld, 16, live, a.vdim,
                         P.vec, lane, 32);
         }
+    };
+    auto load = [&](uint32_t i, uint32_t stage) {
+        copy(i, stage);
         mx_commit();
     };
+    // tiles that earlier steps wrote are asked for before the previous kernel has ended (see load_pair_l2; these copies pass L1 by)
+    auto old_tile = [&](int i) { return P.vec && (tile0 + warp + i * GA_WARPS + 1) * 16 <= p0; };
 #pragma unroll
-    for (int i = 0; i < STAGES - 1; ++i) load(tile0 + warp + i * GA_WARPS, i);
+    for (int i = 0; i < STAGES - 1; ++i)
+        if (old_tile(i)) copy(tile0 + warp + i * GA_WARPS, i);
+    pdl_wait();
+    pdl_trigger();
+#pragma unroll
+    for (int i = 0; i < STAGES - 1; ++i) {
+        if (!old_tile(i)) copy(tile0 + warp + i * GA_WARPS, i);
+        mx_commit();
+    }
     // query fragments straight from global memory: rows g8 and g8 + 8
     uint32_t qa[DK / 16][4];
     const bf16* q = reinterpret_cast<const bf16*>(a.q);

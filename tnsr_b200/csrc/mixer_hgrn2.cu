@@ -25,8 +25,6 @@ template <typename T, int ROWS, int VEC>
 __global__ void __launch_bounds__(HG_THREADS, ROWS * VEC <= 32 ? 4 : ROWS * VEC <= 64 ? 2 : 1)
 hgrn2_token_kernel(Hgrn2 m, StepPlace place) {
     __shared__ float sf[HG_MAX_DIM], sk[HG_MAX_DIM], sq[HG_MAX_DIM], sv[HG_SLICE], red[HG_THREADS * VEC], ssum[HG_SLICE / 32];
-    pdl_wait();
-    pdl_trigger();
     const uint32_t tid = threadIdx.x;
     const uint32_t c_first = blockIdx.x * HG_SLICE, h = blockIdx.y, s = blockIdx.z;
     const uint32_t width = min(HG_SLICE, m.vdim - c_first);
@@ -41,15 +39,18 @@ hgrn2_token_kernel(Hgrn2 m, StepPlace place) {
         const uint32_t n = k + ng * i;
         const bool have = live && n < m.dim && p0 > 0;
         if (VEC == 4) {
-            const float4 v = have ? *reinterpret_cast<const float4*>(state + (size_t)n * m.vdim) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4 v = have ? __ldcg(reinterpret_cast<const float4*>(state + (size_t)n * m.vdim)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             S[i][0] = v.x; S[i][VEC > 1 ? 1 : 0] = v.y; S[i][VEC > 2 ? 2 : 0] = v.z; S[i][VEC > 3 ? 3 : 0] = v.w;
         } else {
-            S[i][0] = have ? state[(size_t)n * m.vdim] : 0.0f;
+            S[i][0] = have ? __ldcg(state + (size_t)n * m.vdim) : 0.0f;
         }
     }
     const bool fused = m.vdim <= HGRN2_FUSED_VDIM;
     const float lower = tid < m.dim ? m.lower[h * m.dim + tid] : 0.0f, bias = tid < m.dim ? m.f_bias[h * m.dim + tid] : 0.0f;
     const float nw = fused && tid < width ? m.norm_w[tid] * m.gain : 0.0f;
+    // the state, most of what this kernel reads, is on its way while the previous kernel ends (see load_pair_l2)
+    pdl_wait();
+    pdl_trigger();
     for (uint32_t t = 0; t < place.chunk; ++t) {
         const size_t row = (size_t)s * place.chunk + t;
         if (tid < m.dim) {

@@ -33,10 +33,11 @@ __global__ void __launch_bounds__(128)
 short_conv_kernel(const T* __restrict__ rows, uint32_t ld, uint32_t channels, uint32_t taps, const float* __restrict__ conv_w,
                   const float* __restrict__ conv_b, T* __restrict__ ring, T* __restrict__ out, uint32_t part, StepPlace place,
                   uint32_t run, uint32_t vec) {
-    pdl_wait();
-    pdl_trigger();
     const uint32_t c = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
-    if (c >= channels) return;
+    if (c >= channels) {
+        pdl_wait();
+        return;
+    }
     const bool second = c + 1 < channels;
     const uint32_t s = blockIdx.z, t0 = blockIdx.y * run, t1 = min(place.chunk, t0 + run);
     const uint32_t p0 = place.pos(s);
@@ -51,6 +52,8 @@ short_conv_kernel(const T* __restrict__ rows, uint32_t ld, uint32_t channels, ui
         dst[(size_t)t * part] = from_f32<T>(y.x);
         if (second) dst1[(size_t)t * part] = from_f32<T>(y.y);
     };
+    // weights, and the ring that earlier steps filled, are asked for before the previous kernel has ended
+    if (t0 > 0) pdl_wait();
     float2 w[TAPS], win[TAPS];
     const float* cw = conv_w + (size_t)c * taps;
     if (TAPS == 4 && taps == 4) {
@@ -73,10 +76,12 @@ short_conv_kernel(const T* __restrict__ rows, uint32_t ld, uint32_t channels, ui
         if (j > 0 && (int)t0 - t < (int)taps) {
             const long long pos = (long long)p0 + t;
             if (t >= 0) win[j] = load_pair<T>(in + (size_t)t * ld, vec, second);
-            else if (pos >= 0) win[j] = load_pair<T>(ring + ((size_t)s * taps + pos % taps) * channels + c, vec, second);
+            else if (pos >= 0) win[j] = load_pair_l2<T>(ring + ((size_t)s * taps + pos % taps) * channels + c, vec, second);
         }
     }
     const float2 b = make_float2(conv_b[c], second ? conv_b[c + 1] : 0.0f);
+    if (t0 == 0) pdl_wait();
+    pdl_trigger();
     if (place.chunk == 1) {
         // the slot of this position held the oldest row, which no single-token step reads
         const float2 now = load_pair<T>(in, vec, second);
@@ -152,8 +157,6 @@ template <typename T, int ROWS, int VEC>
 __global__ void __launch_bounds__(SSD_THREADS, ROWS * VEC <= 32 ? 4 : 2)
 ssd_token_kernel(Mamba2 m, StepPlace place) {
     __shared__ float sb[SSD_MAX_STATE], sc[SSD_MAX_STATE], sx[SSD_SLICE], red[SSD_THREADS * VEC];
-    pdl_wait();
-    pdl_trigger();
     const uint32_t tid = threadIdx.x;
     const uint32_t p_first = blockIdx.x * SSD_SLICE, h = blockIdx.y, s = blockIdx.z;
     const uint32_t width = min(SSD_SLICE, m.vdim - p_first);
@@ -170,15 +173,18 @@ ssd_token_kernel(Mamba2 m, StepPlace place) {
         const uint32_t n = k + ng * i;
         const bool have = live && n < m.state && p0 > 0;
         if (VEC == 4) {
-            const float4 v = have ? *reinterpret_cast<const float4*>(state + (size_t)n * m.vdim) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4 v = have ? __ldcg(reinterpret_cast<const float4*>(state + (size_t)n * m.vdim)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             S[i][0] = v.x; S[i][VEC > 1 ? 1 : 0] = v.y; S[i][VEC > 2 ? 2 : 0] = v.z; S[i][VEC > 3 ? 3 : 0] = v.w;
         } else {
-            S[i][0] = have ? state[(size_t)n * m.vdim] : 0.0f;
+            S[i][0] = have ? __ldcg(state + (size_t)n * m.vdim) : 0.0f;
         }
     }
     const T* xbc = reinterpret_cast<const T*>(m.xbc) + (size_t)s * place.chunk * channels;
     const T* zrow = reinterpret_cast<const T*>(m.proj) + (size_t)s * place.chunk * m.ld + h * m.vdim + p_first;
     const float a_log = m.a_log[h], dt_bias = m.dt_bias[h], skip = m.d_skip[h];
+    // the state, most of what this kernel reads, is on its way while the previous kernel ends (see load_pair_l2)
+    pdl_wait();
+    pdl_trigger();
     for (uint32_t t = 0; t < place.chunk; ++t) {
         const size_t row = (size_t)s * place.chunk + t;
         const float dt_raw = m.dt[row * m.dt_ld + h];

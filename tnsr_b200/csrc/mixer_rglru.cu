@@ -249,16 +249,20 @@ rglru_fused_step_kernel(Rglru m, StepPlace place) {
     }
     const uint32_t c = n0 + t4 * 2, ch = c_first + c;
     const RgChannel ca = rg_channel(m, ch), cb = rg_channel(m, ch + 1);
-    pdl_wait();
-    pdl_trigger();
     const bf16* proj = reinterpret_cast<const bf16*>(m.proj);
     bf16* ring = reinterpret_cast<bf16*>(m.ring);
     float2 old[2], y[2];
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
         const uint32_t s = s0 + g8 + half * 8;
+        old[half] = s < place.sessions && place.pos(s) > 0 ? load_pair_l2(m.state + (size_t)s * m.width + ch, true, true) : make_float2(0.0f, 0.0f);
+    }
+    pdl_wait();
+    pdl_trigger();
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const uint32_t s = s0 + g8 + half * 8;
         const bool here = s < place.sessions;
-        old[half] = here && place.pos(s) > 0 ? *reinterpret_cast<const float2*>(m.state + (size_t)s * m.width + ch) : make_float2(0.0f, 0.0f);
         y[half] = here ? bf16x2_to_f32(*reinterpret_cast<const uint32_t*>(proj + (size_t)s * m.ld + ch)) : make_float2(0.0f, 0.0f);
     }
     // ---- convolution: a thread owns two neighbouring channels and asks for eight sessions' rows at a time ----

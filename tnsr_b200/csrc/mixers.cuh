@@ -186,6 +186,21 @@ __device__ __forceinline__ float2 load_pair<bf16>(const bf16* p, bool vec, bool 
     if (vec) return bf16x2_to_f32(*reinterpret_cast<const uint32_t*>(p));
     return make_float2(__bfloat162float(p[0]), second ? __bfloat162float(p[1]) : 0.0f);
 }
+// The same past L1: for what an earlier step left behind and a kernel asks for before its pdl_wait().  Its predecessor's predecessor has
+// ended by then (the predecessor lets it start behind a wait of its own), and with it everything before; L1 alone might still hold
+// the lines of a step further back.
+template <typename T>
+__device__ __forceinline__ float2 load_pair_l2(const T* p, bool vec, bool second);
+template <>
+__device__ __forceinline__ float2 load_pair_l2<float>(const float* p, bool vec, bool second) {
+    if (vec) return __ldcg(reinterpret_cast<const float2*>(p));
+    return make_float2(__ldcg(p), second ? __ldcg(p + 1) : 0.0f);
+}
+template <>
+__device__ __forceinline__ float2 load_pair_l2<bf16>(const bf16* p, bool vec, bool second) {
+    if (vec) return bf16x2_to_f32(__ldcg(reinterpret_cast<const uint32_t*>(p)));
+    return make_float2(__bfloat162float(__ldcg(p)), second ? __bfloat162float(__ldcg(p + 1)) : 0.0f);
+}
 template <typename T>
 __device__ __forceinline__ void store_pair(T* p, float2 v, bool vec, bool second);
 template <>
