@@ -435,6 +435,20 @@ def test_grouped_products(counts, n, k):
         assert rel_err(grouped(a, w, None, -1, BF16, F32), equal.reshape(rows, n)) < 2e-6
 
 
+@pytest.mark.parametrize("counts", [[1], [0, 16, 17, 0, 1], [3] * 40, [0] * 70 + [5, 2], [128]])
+@pytest.mark.parametrize("n,k", [(16, 16), (40, 80), (50, 1040), (33, 2064)])
+def test_grouped_products_of_few_rows(counts, n, k):
+    """At most 128 rows: 16-row tiles found from the offsets (32 groups at a time), k in blocks of 64 over eight warps, two at a time.  f32 sums
+    of exact products of order k^-1/2: 1e-7 sqrt(k)."""
+    rng = np.random.default_rng(n + k + len(counts))
+    rows, offsets = sum(counts), np.concatenate([[0], np.cumsum(counts)])
+    a = bf16_exact(rng.normal(size=(rows, k)).astype(np.float32))
+    w = bf16_exact((rng.normal(size=(len(counts), n, k)) * k ** -0.5).astype(np.float32))
+    want = np.concatenate([a[offsets[g]:offsets[g + 1]].astype(np.float64) @ w[g].astype(np.float64).T for g in range(len(counts))])
+    assert rel_err(grouped(a, w, offsets, -1, BF16, F32), want) < 1e-7 * max(k, 400) ** 0.5
+    assert rel_err(grouped(a, w, offsets, 4, BF16, BF16), np.maximum(want, 0.0) ** 2) < 5e-3
+
+
 def test_grouped_product_refuses_what_it_cannot_address():
     a, w = np.zeros((10, 64), np.float32), np.zeros((3, 32, 64), np.float32)
     out = torch.zeros((10, 32), device="cuda")

@@ -20,6 +20,9 @@ struct GroupedGemm {
 };
 // dtype: element type of a and w.
 int launch_gemm_grouped(const GroupedGemm& g, int dtype, cudaStream_t stream);
+// bf16, few rows, groups by offsets: operands straight into registers (gemm_few.cu).
+bool gemm_grouped_few_pays(const GroupedGemm& g);
+int launch_gemm_grouped_few(const GroupedGemm& g, cudaStream_t stream);
 
 // ---- PolyNorm ---------------------------------------------------------------------
 // out[r] = a N(z) + b N(z^2) + c N(z^3) + e, N(v) = v / sqrt(mean(v^2) + eps) over the row; act = {a, b, c, e} on the device.

@@ -16,6 +16,7 @@
 #include <algorithm>
 #include <atomic>
 
+#include "feed_forward.cuh"
 #include "gemm_epilogue.cuh"
 
 namespace tb {
@@ -322,6 +323,116 @@ int launch_gemm_few(const bf16* a, const bf16* w, const EpiParams& epi, uint32_t
     if (nt == 4) return launch_rows<4, 2>(P, stream);
     if (nt == 2) return per <= 2 ? launch_rows<2, 2>(P, stream) : launch_rows<2, 4>(P, stream);
     return per <= 2 ? launch_rows<1, 2>(P, stream) : launch_rows<1, 4>(P, stream);
+}
+
+// ---- grouped products of few rows -------------------------------------------------------------
+// The experts of a step: groups of a few rows each, which ones only the device knows.  Block (x, y) = 16 columns of the y-th 16-row tile of
+// the groups in turn; it finds its group from the offsets, a trip that the weights have to wait for, and then works as above.
+namespace {
+
+struct GroupedFewParams {
+    const bf16* a;             // [rows, k], group after group
+    const bf16* w;             // [groups, n, k]
+    void* out;                 // [rows, n]
+    const uint32_t* offsets;   // [groups + 1]
+    uint32_t groups, n, k;
+    int activation, out_dtype;
+};
+
+__global__ void __launch_bounds__(FW_THREADS, 2)
+gemm_grouped_few_kernel(GroupedFewParams P) {
+    constexpr uint32_t COLS = 16, TILE = 16 * COLS;
+    constexpr int NT = 2, S = 2;             // k blocks whose operands a warp has in registers at a time
+    __shared__ float sums[FW_WARPS * TILE];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3, col0 = blockIdx.x * COLS;
+    pdl_wait();
+    pdl_trigger();
+    // the group of this block's tile: lanes count the tiles of 32 groups at a time
+    uint32_t group = 0, row0 = 0, row1 = 0, before = 0;
+    bool found = false;
+    for (uint32_t e0 = 0; e0 < P.groups && !found; e0 += 32) {
+        const uint32_t e = e0 + lane;
+        const uint32_t first = e < P.groups ? __ldcg(P.offsets + e) : 0u, last = e < P.groups ? __ldcg(P.offsets + e + 1) : 0u;
+        const uint32_t tiles = (last - first + 15) / 16;
+        uint32_t upto = tiles;
+#pragma unroll
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += u;
+        }
+        const uint32_t hit = __ballot_sync(0xffffffffu, blockIdx.y < before + upto);
+        if (hit) {
+            const uint32_t at = __ffs(hit) - 1;
+            group = e0 + at;
+            const uint32_t tile = blockIdx.y - before - __shfl_sync(0xffffffffu, upto - tiles, at);
+            row0 = __shfl_sync(0xffffffffu, first, at) + tile * 16;
+            row1 = __shfl_sync(0xffffffffu, last, at);
+            found = true;
+        }
+        before += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    if (!found) return;           // the same for the whole block
+    const uint32_t blocks = (P.k + FW_BLOCK - 1) / FW_BLOCK, per = (blocks + FW_WARPS - 1) / FW_WARPS;
+    const uint32_t b0 = min(blocks, warp * per), b1 = min(blocks, b0 + per);
+    const bf16* wp = P.w + ((size_t)group * P.n + col0 + g) * P.k + 16 * t;
+    const bf16* ap = P.a + (size_t)(row0 + g) * P.k + 16 * t;
+    float acc[NT][4] = {};
+    for (uint32_t b = b0; b < b1; b += S) {
+        Words w[NT][S], a[2][S];
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            const uint32_t at = (b + s) * FW_BLOCK;
+            const bool ok = b + s < b1 && at + 16 * t < P.k;
+#pragma unroll
+            for (int j = 0; j < NT; ++j) w[j][s] = ok && col0 + 8 * j + g < P.n ? fw_load_weights(wp + (size_t)j * 8 * P.k + at) : fw_zero();
+#pragma unroll
+            for (int i = 0; i < 2; ++i) a[i][s] = ok && row0 + 8 * i + g < row1 ? fw_load_rows(ap + (size_t)i * 8 * P.k + at) : fw_zero();
+        }
+#pragma unroll
+        for (int s = 0; s < S; ++s)
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int j = 0; j < NT; ++j)
+                    fw_mma(acc[j], a[0][s].x[2 * q], a[1][s].x[2 * q], a[0][s].x[2 * q + 1], a[1][s].x[2 * q + 1], w[j][s].x[2 * q], w[j][s].x[2 * q + 1]);
+    }
+    float* mine = sums + warp * TILE;
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+        *reinterpret_cast<float2*>(mine + g * COLS + 8 * j + 2 * t) = make_float2(acc[j][0], acc[j][1]);
+        *reinterpret_cast<float2*>(mine + (g + 8) * COLS + 8 * j + 2 * t) = make_float2(acc[j][2], acc[j][3]);
+    }
+    __syncthreads();
+    const uint32_t row = row0 + threadIdx.x / COLS, col = col0 + threadIdx.x % COLS;
+    if (row >= row1 || col >= P.n) return;
+    float v = sums[threadIdx.x];
+#pragma unroll
+    for (uint32_t i = 1; i < FW_WARPS; ++i) v += sums[i * TILE + threadIdx.x];
+    if (P.activation == ACT_RELU_SQUARED) {
+        v = fmaxf(v, 0.0f);
+        v *= v;
+    } else {
+        v = apply_activation(v, P.activation);
+    }
+    if (P.out_dtype == TNSR_B200_BF16) reinterpret_cast<bf16*>(P.out)[(size_t)row * P.n + col] = __float2bfloat16_rn(v);
+    else reinterpret_cast<float*>(P.out)[(size_t)row * P.n + col] = v;
+}
+
+}  // namespace
+
+// At most 128 rows in groups of 16 on average: with more, a group's weights are read for several tiles and the tcgen05 tiles are the better ones.
+bool gemm_grouped_few_pays(const GroupedGemm& g) {
+    return g.offsets && g.rows <= 128 && g.k % 16 == 0 && reinterpret_cast<uintptr_t>(g.a) % 32 == 0 && reinterpret_cast<uintptr_t>(g.w) % 32 == 0;
+}
+
+int launch_gemm_grouped_few(const GroupedGemm& g, cudaStream_t stream) {
+    GroupedFewParams P;
+    P.a = (const bf16*)g.a; P.w = (const bf16*)g.w; P.out = g.out; P.offsets = g.offsets; P.groups = g.groups; P.n = g.n; P.k = g.k;
+    P.activation = g.activation; P.out_dtype = g.out_dtype;
+    const dim3 grid(ceil_div(g.n, 16u), g.rows / 16 + std::min(g.groups, g.rows));      // every group may end in a ragged tile
+    launch_kernel(gemm_grouped_few_kernel, grid, dim3(FW_THREADS), 0, stream, P);
+    count_launch();
+    return check_launch("gemm_grouped_few");
 }
 
 }  // namespace tb

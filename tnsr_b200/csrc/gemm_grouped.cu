@@ -341,6 +341,7 @@ int launch_gemm_grouped(const GroupedGemm& g, int dtype, cudaStream_t stream) {
         set_thread_error("grouped gemm: too many rows");
         return TNSR_B200_ERR_UNSUPPORTED;
     }
+    if (dtype == TNSR_B200_BF16 && g.engine == 0 && g_gemm_engine == 0 && gemm_grouped_few_pays(g)) return launch_gemm_grouped_few(g, stream);
     GgParams prm;
     prm.out = g.out; prm.offsets = g.offsets; prm.groups = g.groups; prm.rows = g.rows; prm.n = g.n; prm.k = g.k;
     prm.activation = g.activation; prm.out_dtype = g.out_dtype; prm.d_status = g.d_status;
