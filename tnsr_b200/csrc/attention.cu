@@ -577,51 +577,92 @@ decode_attention_kernel(DaParams P) {
                         constexpr int DPL = HD / 32;  // output dims per lane
                         const float* base = P.partial + ((size_t)mt.first_slot * P.heads + h) * (HD + 2);
                         const size_t step = (size_t)P.heads * (HD + 2);
-                        // Sums go in a fixed order of the pieces.  Lane i holds maximum and sum of pieces i, i + 32, ...; the numerators are
-                        // asked for up to sixteen pieces at a time, so a merge costs a few trips to L2 however the session was cut (one
-                        // session of 1000 keys is 63 pieces; a piece after the other took most of a launch: a step of 12 layers 448 ->
-                        // 409 us).
+                        // Sums go in a fixed order of the pieces, f32.
                         float o[DPL], mx = -INFINITY, lt = 0.0f;
 #pragma unroll
                         for (int e = 0; e < DPL; ++e) o[e] = 0.0f;
-                        constexpr uint32_t LOTS = DA_MAX_CTAS / 32, TOGETHER = HD == 128 ? 4 : HPW == 2 ? 8 : 16;
-                        float pm[LOTS], pl[LOTS];
+                        constexpr uint32_t FEW = 4;
+                        if (n_parts <= FEW) {
+                            // the usual case of a full GPU (a session cut in two to four pieces): every value of every piece is
+                            // requested before the first is used, one L2 round trip
+                            float pm[FEW], pl[FEW], pn[FEW][DPL];
 #pragma unroll
-                        for (uint32_t r = 0; r < LOTS; ++r) {
-                            const bool have = r * 32 + lane < n_parts;
-                            const float* pp = base + (size_t)(r * 32 + lane) * step;
-                            const float2 v = have ? __ldcg(reinterpret_cast<const float2*>(pp + HD)) : make_float2(-INFINITY, 0.0f);
-                            pm[r] = v.x;
-                            pl[r] = v.y;
-                            mx = fmaxf(mx, v.x);
-                        }
+                            for (uint32_t i = 0; i < FEW; ++i) {
+                                const float* pp = base + i * step;
+                                const bool have = i < n_parts;
+                                pm[i] = have ? __ldcg(pp + HD) : -INFINITY;
+                                pl[i] = have ? __ldcg(pp + HD + 1) : 0.0f;
 #pragma unroll
-                        for (uint32_t x = 16; x > 0; x >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
-                        const float ms = (mx == -INFINITY) ? 0.0f : mx;
+                                for (int e = 0; e < DPL; ++e) pn[i][e] = have ? __ldcg(pp + lane * DPL + e) : 0.0f;
+                            }
 #pragma unroll
-                        for (uint32_t r = 0; r < LOTS; ++r) {
-                            pm[r] = ex2(pm[r] - ms);           // the piece's weight
-                            lt = fmaf(pl[r], pm[r], lt);
-                        }
+                            for (uint32_t i = 0; i < FEW; ++i) mx = fmaxf(mx, pm[i]);
+                            const float ms = (mx == -INFINITY) ? 0.0f : mx;
 #pragma unroll
-                        for (uint32_t x = 16; x > 0; x >>= 1) lt += __shfl_xor_sync(0xffffffffu, lt, x);
-#pragma unroll
-                        for (uint32_t r = 0; r < LOTS; ++r) {
-                            if (r * 32 >= n_parts) continue;   // warp-uniform
-#pragma unroll
-                            for (uint32_t i0 = 0; i0 < 32; i0 += TOGETHER) {
-                                if (r * 32 + i0 >= n_parts) continue;
-                                float pn[TOGETHER][DPL];
-#pragma unroll
-                                for (uint32_t i = 0; i < TOGETHER; ++i)
-#pragma unroll
-                                    for (int e = 0; e < DPL; ++e)
-                                        pn[i][e] = r * 32 + i0 + i < n_parts ? __ldcg(base + (size_t)(r * 32 + i0 + i) * step + lane * DPL + e) : 0.0f;
-#pragma unroll
-                                for (uint32_t i = 0; i < TOGETHER; ++i) {
-                                    const float w = __shfl_sync(0xffffffffu, pm[r], i0 + i);
+                            for (uint32_t i = 0; i < FEW; ++i) {
+                                if (i < n_parts) {
+                                    const float w = ex2(pm[i] - ms);
+                                    lt = fmaf(pl[i], w, lt);
 #pragma unroll
                                     for (int e = 0; e < DPL; ++e) o[e] = fmaf(pn[i][e], w, o[e]);
+                                }
+                            }
+                        } else if (KS == DA_KS_LEAN) {
+                            // a range of a large batch: sessions in more pieces are rare, and the code below makes the scan itself 3 %
+                            // slower here (256 sessions 1.23 -> 1.27 ms per step)
+                            for (uint32_t i = 0; i < n_parts; ++i) mx = fmaxf(mx, __ldcg(base + i * step + HD));
+                            const float ms = (mx == -INFINITY) ? 0.0f : mx;
+                            for (uint32_t i = 0; i < n_parts; ++i) {
+                                const float* pp = base + i * step;
+                                const float w = ex2(__ldcg(pp + HD) - ms);
+                                lt = fmaf(__ldcg(pp + HD + 1), w, lt);
+#pragma unroll
+                                for (int e = 0; e < DPL; ++e) o[e] = fmaf(__ldcg(pp + lane * DPL + e), w, o[e]);
+                            }
+                        } else {
+                            // Few sessions on many SMs: lane i holds maximum and sum of pieces i, i + 32, ...; the numerators are asked for up
+                            // to eight pieces at a time, so a merge costs a few trips to L2 however the session was cut (one session
+                            // of 1000 keys is 63 pieces; a piece after the other took most of a launch: a step of 12 layers 448 ->
+                            // 409 us).
+                            constexpr uint32_t LOTS = DA_MAX_CTAS / 32, TOGETHER = HD == 128 ? 4 : 8;
+                            float pm[LOTS], pl[LOTS];
+#pragma unroll
+                            for (uint32_t r = 0; r < LOTS; ++r) {
+                                const bool have = r * 32 + lane < n_parts;
+                                const float* pp = base + (size_t)(r * 32 + lane) * step;
+                                const float2 v = have ? __ldcg(reinterpret_cast<const float2*>(pp + HD)) : make_float2(-INFINITY, 0.0f);
+                                pm[r] = v.x;
+                                pl[r] = v.y;
+                                mx = fmaxf(mx, v.x);
+                            }
+#pragma unroll
+                            for (uint32_t x = 16; x > 0; x >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
+                            const float ms = (mx == -INFINITY) ? 0.0f : mx;
+#pragma unroll
+                            for (uint32_t r = 0; r < LOTS; ++r) {
+                                pm[r] = ex2(pm[r] - ms);           // the piece's weight
+                                lt = fmaf(pl[r], pm[r], lt);
+                            }
+#pragma unroll
+                            for (uint32_t x = 16; x > 0; x >>= 1) lt += __shfl_xor_sync(0xffffffffu, lt, x);
+#pragma unroll
+                            for (uint32_t r = 0; r < LOTS; ++r) {
+                                if (r * 32 >= n_parts) continue;   // warp-uniform
+#pragma unroll
+                                for (uint32_t i0 = 0; i0 < 32; i0 += TOGETHER) {
+                                    if (r * 32 + i0 >= n_parts) continue;
+                                    float pn[TOGETHER][DPL];
+#pragma unroll
+                                    for (uint32_t i = 0; i < TOGETHER; ++i)
+#pragma unroll
+                                        for (int e = 0; e < DPL; ++e)
+                                            pn[i][e] = r * 32 + i0 + i < n_parts ? __ldcg(base + (size_t)(r * 32 + i0 + i) * step + lane * DPL + e) : 0.0f;
+#pragma unroll
+                                    for (uint32_t i = 0; i < TOGETHER; ++i) {
+                                        const float w = __shfl_sync(0xffffffffu, pm[r], i0 + i);
+#pragma unroll
+                                        for (int e = 0; e < DPL; ++e) o[e] = fmaf(pn[i][e], w, o[e]);
+                                    }
                                 }
                             }
                         }
