@@ -232,8 +232,9 @@ da_plan_kernel(const uint32_t* __restrict__ lengths, const uint32_t* __restrict_
     if (tid == 0) {
         sstart[batch] = total;
         const uint32_t ctas = total < grid ? (total ? total : 1) : grid;
-        s_quota = (total + ctas - 1) / ctas;
-        if (s_quota == 0) s_quota = 1;
+        // two stages at least: with one per CTA a session of 1000 keys is 63 pieces, whose merge costs more than the second stage (one
+        // session's attention, 12 heads: 21.1 -> 19.2 us with the plan)
+        s_quota = max(2u, (total + ctas - 1) / ctas);
         s_total = total;
     }
     __syncthreads();
@@ -368,6 +369,7 @@ struct DaParams {
     int* d_status;
     uint64_t wait_limit_ns;   // bound of every mbarrier wait (tnsr_b200_set_wait_limit_ns)
     KvPaging paging;          // page pools instead of per-session slabs (page_rows is a multiple of the stage size)
+    uint32_t early;           // the item list is older than the previous kernel, which wrote no key but every session's last
 };
 
 // HD: head width; LPK = HD / 8 lanes share one (key, head) row slice, each lane
@@ -395,10 +397,13 @@ decode_attention_kernel(DaParams P) {
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    pdl_wait();
-    pdl_trigger();
     __syncthreads();
-    const uint32_t item_begin = P.cta_begin[blockIdx.x], item_end = P.cta_begin[blockIdx.x + 1];
+    const bool early = KS != DA_KS_LEAN && P.early;
+    if (!(early && warp == consumers)) {
+        pdl_wait();
+        pdl_trigger();
+    }
+    const uint32_t item_begin = __ldcg(P.cta_begin + blockIdx.x), item_end = __ldcg(P.cta_begin + blockIdx.x + 1);
 
     if (warp == consumers) {
         // ---------------- producer ----------------
@@ -409,34 +414,72 @@ decode_attention_kernel(DaParams P) {
             asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(once));
             // item records and the per-session piece counts are fetched one item ahead, so their latency
             // hides behind the copies of the current item
-            DaItem nxt = {};
-            if (item_begin < item_end) nxt = P.items[item_begin];
-            for (uint32_t item = item_begin; ok && item < item_end; ++item) {
-                const DaItem it = nxt;
-                if (item + 1 < item_end) nxt = P.items[item + 1];
+            auto item_at = [&](uint32_t i) {
+                const uint4 a = __ldcg(reinterpret_cast<const uint4*>(P.items + i)), b = __ldcg(reinterpret_cast<const uint4*>(P.items + i) + 1);
+                return DaItem{a.x, a.y, a.z, a.w, b.x, b.y, {0u, 0u}};
+            };
+            // stage s of item `it` into the ring; `with_q`: also the session's query row, which the item's first stage carries
+            auto fill = [&](const DaItem& it, uint32_t s, uint32_t n_stages, bool with_q) {
+                const uint32_t nk = min((uint32_t)KS, it.nkeys - s * KS);
+                uint8_t* sk = ring + (size_t)stage * stage_bytes;
+                DaStageMeta mt;
+                mt.slot = it.slot;
+                mt.nk = nk;
+                mt.flags = (s == 0 ? 1u : 0u) | (s + 1 == n_stages ? 2u : 0u);
+                mt.session = it.session;
+                mt.n_parts = it.n_parts;
+                mt.first_slot = it.first_slot;
+                meta[stage] = mt;
+                const uint32_t bytes = nk * row_bytes;
+                da_mbar_expect_tx(full_bar + stage, 2 * bytes + (s == 0 ? row_bytes : 0));
+                // a stage never straddles pages: key0 and the page size are multiples of the stage size
+                const size_t base = kv_row(P.paging, it.session, it.key0 + s * KS, P.capacity) * d;
+                da_bulk_load_once(sk, P.kc + base, bytes, full_bar + stage, once);
+                da_bulk_load_once(sk + k_bytes, P.vc + base, bytes, full_bar + stage, once);
+                if (s == 0 && with_q) da_bulk_load(sk + 2 * k_bytes, P.q + (size_t)it.session * d, row_bytes, full_bar + stage);
+            };
+            DaItem it = {}, nxt = {};
+            if (item_begin < item_end) it = nxt = item_at(item_begin);
+            uint32_t item = item_begin, s = 0;
+            if (early) {
+                // The previous kernel writes the queries and every session's last key; the keys before it are whole steps old.  Up to a ring
+                // of them is asked for now, the query rows follow once that kernel has ended (12 layers, us per step without / with: one
+                // session at 1000 341 / 332, 48 at 1000 700 / 692, 64 at 512 652 / 640).
+                uint32_t filled = 0, waiting = 0;
+                while (item < item_end && filled < P.stages) {
+                    const uint32_t n_stages = (it.nkeys + KS - 1) / KS;
+                    if (s + 1 == n_stages && (it.slot == DA_DIRECT || it.slot + 1 == it.first_slot + it.n_parts)) break;
+                    stage = filled;
+                    fill(it, s, n_stages, false);
+                    if (s == 0) waiting |= 1u << filled;
+                    ++filled;
+                    if (++s == n_stages) {
+                        s = 0;
+                        if (++item < item_end) it = item_at(item);
+                    }
+                }
+                nxt = it;
+                pdl_wait();
+                for (uint32_t i = 0; i < filled; ++i)
+                    if (waiting >> i & 1u)
+                        da_bulk_load(ring + (size_t)i * stage_bytes + 2 * k_bytes, P.q + (size_t)meta[i].session * d, row_bytes, full_bar + i);
+                stage = filled == P.stages ? 0 : filled;
+                phase = filled == P.stages ? 1 : 0;
+            }
+            for (; ok && item < item_end; ++item, s = 0) {
+                it = nxt;
+                if (item + 1 < item_end) nxt = item_at(item + 1);
                 const uint32_t n_stages = (it.nkeys + KS - 1) / KS;
-                for (uint32_t s = 0; s < n_stages; ++s) {
+                for (; s < n_stages; ++s) {
                     if (!da_mbar_wait(empty_bar + stage, phase ^ 1, abort_flag, P.wait_limit_ns)) { ok = false; break; }
-                    const uint32_t nk = min((uint32_t)KS, it.nkeys - s * KS);
-                    uint8_t* sk = ring + (size_t)stage * stage_bytes;
-                    DaStageMeta mt;
-                    mt.slot = it.slot;
-                    mt.nk = nk;
-                    mt.flags = (s == 0 ? 1u : 0u) | (s + 1 == n_stages ? 2u : 0u);
-                    mt.session = it.session;
-                    mt.n_parts = it.n_parts;
-                    mt.first_slot = it.first_slot;
-                    meta[stage] = mt;
-                    const uint32_t bytes = nk * row_bytes;
-                    da_mbar_expect_tx(full_bar + stage, 2 * bytes + (s == 0 ? row_bytes : 0));
-                    // a stage never straddles pages: key0 and the page size are multiples of the stage size
-                    const size_t base = kv_row(P.paging, it.session, it.key0 + s * KS, P.capacity) * d;
-                    da_bulk_load_once(sk, P.kc + base, bytes, full_bar + stage, once);
-                    da_bulk_load_once(sk + k_bytes, P.vc + base, bytes, full_bar + stage, once);
-                    if (s == 0) da_bulk_load(sk + 2 * k_bytes, P.q + (size_t)it.session * d, row_bytes, full_bar + stage);
+                    fill(it, s, n_stages, true);
                     if (++stage == P.stages) { stage = 0; phase ^= 1; }
                 }
             }
+        }
+        if (early) {
+            pdl_wait();
+            pdl_trigger();
         }
     } else {
         // ---------------- consumers ----------------
@@ -622,7 +665,7 @@ decode_attention_kernel(DaParams P) {
                         } else {
                             // Few sessions on many SMs: lane i holds maximum and sum of pieces i, i + 32, ...; the numerators are asked for up
                             // to eight pieces at a time, so a merge costs a few trips to L2 however the session was cut (one session
-                            // of 1000 keys is 63 pieces; a piece after the other took most of a launch: a step of 12 layers 448 ->
+                            // of 1000 keys is 32 pieces; a piece after the other took most of a launch: a step of 12 layers 448 ->
                             // 409 us).
                             constexpr uint32_t LOTS = DA_MAX_CTAS / 32, TOGETHER = HD == 128 ? 4 : 8;
                             float pm[LOTS], pl[LOTS];
@@ -807,6 +850,7 @@ int launch_decode_attention_ex(const bf16* q, const bf16* k_cache, const bf16* v
     P.scale_log2 = (1.0f / sqrtf((float)head_dim)) * 1.4426950408889634f;
     P.d_status = d_status;
     P.wait_limit_ns = g_wait_limit_ns.load(std::memory_order_relaxed);
+    P.early = !plan && t_pdl;
     if (paging && paging->table) {
         if (paging->page_rows == 0 || paging->page_rows % DA_KS != 0) {
             set_thread_error("decode attention: the page size must be a multiple of 16 rows");
