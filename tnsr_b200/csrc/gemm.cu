@@ -883,11 +883,16 @@ static int launch_gemm_impl(const bf16* a, const bf16* bt, void* out, uint32_t l
         if (pays || g_gemm_engine == 3)
             return launch_gemm_skinny(a, bt, out, ldc, m, n, k, ep, ep.skinny_ws, ep.skinny_ws_bytes, d_status, stream);
     }
-    // tile width: the widest that still gives every SM a tile (32 at the narrowest)
+    // Tile width: a tile takes what its operands take to come in, BM + bn rows of k, and tiles run in waves of one per SM: the fewest rows
+    // through one SM, the wider tile where it is the same.  (The widest that still gives every SM a tile, the rule before, ran 186 tiles of 128
+    // columns in two waves where 93 of 256 are one.)
     const uint32_t tiles_m = ceil_div(m, BM);
     uint32_t bn = 256;
-    while (bn > 64 && (uint64_t)tiles_m * ceil_div(n, bn) < (uint64_t)sm_count()) bn >>= 1;
-    if (bn == 64 && 2ull * tiles_m * ceil_div(n, 64) <= (uint64_t)sm_count()) bn = 32;  // very few tiles: halve once more
+    uint64_t least = ~0ull;
+    for (uint32_t w = 256; w >= 32; w >>= 1) {
+        const uint64_t rows = ceil_div64((uint64_t)tiles_m * ceil_div(n, w), (uint64_t)sm_count()) * (BM + w);
+        if (rows < least) { least = rows; bn = w; }
+    }
     while (bn > 32 && bn / 2 >= n) bn >>= 1;      // no wider than the matrix (a router's few columns)
     if (split_req) bn = 32;   // many small tiles: every CTA takes in as little of both operands as possible
     TcParams prm;
