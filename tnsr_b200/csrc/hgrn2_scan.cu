@@ -16,10 +16,10 @@
 // output waits in registers for the next chunk's barrier, behind which the other warps' sums of squares are in place.
 //
 // A long prompt of few sessions leaves most SMs without a sequence of their own.  The recurrence is linear in the state, so time is
-// divided then: a first launch (SC_STATES) takes every segment from a zero state to what it adds and to its product of gates, a
-// second one (SC_OUTPUTS) starts every segment from those before it, S = D_j S + L_j in order, all in f32.  One session of 1792 tokens
-// through 8 such mixers of 12 heads of 64 x 64 (and 4 recurrent units, 6 steps), B200: 7.9 ms with 12 CTAs for 254 us each, 6.2 ms
-// with 23 segments (first launch 27 us).
+// divided then: a first launch (SC_STATES) takes every segment from a zero state to what it adds and to its product of gates, a second
+// one (hgrn2_join_kernel) joins these to the state before every segment, S = D_j S + L_j in order, a third (SC_OUTPUTS) starts from
+// them; all in f32.  1792 tokens, 12 heads of 64 x 64, one session, B200: 254 us in 12 CTAs; in 23 segments 40 us for the three (14 us for the
+// first launch), 127 us while every CTA of the third launch joined the segments before it by itself.
 //
 // The state, the written k R, k / P and the inner weights enter the products as two bf16 halves (split_bf16x2), so that they
 // keep 16 bits; the readout's q P is rounded to bf16 like q itself, v is bf16.
@@ -51,8 +51,8 @@ __device__ __forceinline__ void hs_gate(float z2, float lower, float rest, float
 }
 
 enum : int { SC_WHOLE = 0, SC_STATES = 1, SC_OUTPUTS = 2 };
-// Segments of a divided scan.  Per (session, head): the states [segments][dim][vdim] they add, the state before the first one, and
-// their products of gates [segments][dim].
+// Segments of a divided scan.  Per (session, head): the states [segments][dim][vdim] that they add (joined: those after them), the state
+// before the first one, and their products of gates [segments][dim].
 struct HsSegments {
     uint32_t count, tokens;      // tokens: a multiple of 16
     float* space;
@@ -254,25 +254,12 @@ hgrn2_scan_kernel(Hgrn2 m, StepPlace place, uint32_t vec, HsSegments segments) {
             const bool real = n < m.dim && p < width;
             const size_t at = (size_t)n * m.vdim + p;
             if (PHASE == SC_OUTPUTS) {
-                acc[nt][e] = real ? __ldcg(added + (segment ? 0 : segments.count) * matrix + c_first + at) : 0.0f;
+                acc[nt][e] = real ? __ldcg(added + (segment ? segment - 1 : segments.count) * matrix + c_first + at) : 0.0f;
             } else {
                 acc[nt][e] = p0 > 0 && segment == 0 && real ? state[at] : 0.0f;
                 if (PHASE == SC_STATES && segment == 0 && real) added[segments.count * matrix + c_first + at] = acc[nt][e];
             }
         }
-    if (PHASE == SC_OUTPUTS) {
-        for (uint32_t j = 1; j < segment; ++j) {
-            const float* add = added + j * matrix + c_first;
-            const float* d = decays + j * m.dim;
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const uint32_t p = pw + g8 + (e >> 1) * 8, n = nt * 8 + t4 * 2 + (e & 1);
-                    if (n < m.dim && p < width) acc[nt][e] = fmaf(__ldcg(d + n), acc[nt][e], __ldcg(add + (size_t)n * m.vdim + p));
-                }
-        }
-    }
     float nw[4];       // norm weights of the lane's output columns pw + t4 * 2 (+ 1, + 8, + 9)
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -451,6 +438,34 @@ hgrn2_scan_kernel(Hgrn2 m, StepPlace place, uint32_t vec, HsSegments segments) {
     }
 }
 
+// A thread per element of a state: what the segments add becomes the state after each of them.  What bounds it is the trips to L2, so eight
+// segments are asked for at a time.
+__global__ void __launch_bounds__(256)
+hgrn2_join_kernel(HsSegments segments, uint32_t dim, uint32_t vdim) {
+    pdl_wait();
+    pdl_trigger();
+    const uint32_t at = blockIdx.x * blockDim.x + threadIdx.x, matrix = dim * vdim, last = segments.count - 1;     // of that nothing is kept
+    if (at >= matrix) return;
+    float* added = segments.space + (size_t)blockIdx.y * segments.unit_floats(dim, vdim) + at;
+    const float* decays = added - at + (size_t)(segments.count + 1) * matrix + at / vdim;
+    constexpr uint32_t AHEAD = 8;
+    float S = __ldcg(added);
+    for (uint32_t j0 = 1; j0 < last; j0 += AHEAD) {
+        float l[AHEAD], d[AHEAD];
+#pragma unroll
+        for (uint32_t i = 0; i < AHEAD; ++i) {
+            const bool have = j0 + i < last;
+            l[i] = have ? __ldcg(added + (size_t)(j0 + i) * matrix) : 0.0f;
+            d[i] = have ? __ldcg(decays + (size_t)(j0 + i) * dim) : 0.0f;
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < AHEAD; ++i) {
+            S = fmaf(d[i], S, l[i]);
+            if (j0 + i < last) added[(size_t)(j0 + i) * matrix] = S;
+        }
+    }
+}
+
 template <int NP, int WARPS, int PHASE>
 static int launch_phase(const Hgrn2& m, const StepPlace& place, uint32_t vec, const HsSegments& segments, cudaStream_t stream) {
     static bool configured[64] = {};
@@ -494,7 +509,11 @@ static int launch_scan(const Hgrn2& m, const StepPlace& place, uint32_t vec, cud
     HsSegments g = divide(most, place.chunk);
     g.space = m.segment_space;
     int rc = launch_phase<NP, WARPS, SC_STATES>(m, place, vec, g, stream);
-    return rc ? rc : launch_phase<NP, WARPS, SC_OUTPUTS>(m, place, vec, g, stream);
+    if (rc) return rc;
+    launch_kernel(hgrn2_join_kernel, dim3(ceil_div(m.dim * m.vdim, 256u), place.sessions * m.heads), dim3(256), 0, stream, g, m.dim, m.vdim);
+    count_launch();
+    if ((rc = check_launch("hgrn2_join"))) return rc;
+    return launch_phase<NP, WARPS, SC_OUTPUTS>(m, place, vec, g, stream);
 }
 
 int launch_hgrn2_scan(const Hgrn2& m, const StepPlace& place, cudaStream_t stream) {
