@@ -865,7 +865,8 @@ static int launch_gemm_impl(const bf16* a, const bf16* bt, void* out, uint32_t l
     // Few rows: operands straight into registers (gemm_few.cu; not where a test asks this engine to lose a stage).
     if (!split_req && mode != GEMM_ARGMAX && g_gemm_engine == 0 && !ep.round_bf16 && !t_lose_gemm_stage && gemm_few_pays(a, bt, m, n, k))
         return launch_gemm_few(a, bt, P, k, mode, stream);
-    // A handful of rows against a large weight matrix: stream the weights with the operands swapped (gemm_skinny.cu)
+    // What is left of few rows (k no multiple of 16, pointers of 16-byte alignment, a lost stage to provoke):
+    // a handful of rows against a large weight matrix: stream the weights with the operands swapped (gemm_skinny.cu)
     // when that engine can fill the GPU, i.e. with split-K scratch lent by the caller or with at least half as many
     // 128-column tiles as SMs.  Measured inside a CUDA graph, 4096 x 4096 weights: 14.8 / 16.3 us at 1 / 8 rows against
     // 28 us for the engine below; at 64 rows (33.6 against 21.5 us) and for the small matrices of a decode step (the
