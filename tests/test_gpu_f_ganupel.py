@@ -449,6 +449,35 @@ def test_grouped_products_of_few_rows(counts, n, k):
     assert rel_err(grouped(a, w, offsets, 4, BF16, BF16), np.maximum(want, 0.0) ** 2) < 5e-3
 
 
+@pytest.mark.parametrize("offsets", [[0, 10, 40], [0, 4, 4, 3000000000], [12, 20, 3, 9], [30, 40, 50], [24, 0, 7]])
+@pytest.mark.parametrize("k", [64, 72])
+def test_grouped_products_cut_a_group_list_to_the_rows(offsets, k):
+    """24 rows and a list that runs past them, goes back or starts behind them: no row outside the buffers is read or written, rows that no
+    group owns stay as they are.  k = 64 is the kernel for few rows, 72 the tcgen05 one, engine 1 the one for CUDA cores."""
+    rows, n, groups = 24, 33, len(offsets) - 1
+    rng = np.random.default_rng(k + groups)
+    a = bf16_exact(rng.normal(size=(rows, k)).astype(np.float32))
+    w = bf16_exact((rng.normal(size=(groups, n, k)) * k ** -0.5).astype(np.float32))
+    want = np.full((rows, n), 7.0)
+    for g in range(groups):
+        first, last = (min(rows, o) for o in offsets[g:g + 2])
+        if last > first:
+            want[first:last] = a[first:last].astype(np.float64) @ w[g].astype(np.float64).T
+    spare = 64                                 # rows on either side of the operands: whatever leaves the 24 is seen there
+    wide = torch.full((rows + 2 * spare, n), 7.0, device="cuda")
+    out, status = wide[spare:spare + rows], torch.zeros(1, dtype=torch.int32, device="cuda")
+    around = torch.full((rows + 2 * spare, k), float("nan"), dtype=torch.bfloat16, device="cuda")
+    around[spare:spare + rows] = dev(a, torch.bfloat16)
+    off = dev(np.asarray(offsets, np.uint32).view(np.int32))
+    for engine in (0, 1):
+        wide.fill_(7.0)
+        ok(lib().tnsr_b200_gemm_grouped(ptr(around[spare:]), ptr(dev(w, torch.bfloat16)), ptr(out), ptr(off), groups, rows, n, k, -1, BF16, F32, engine,
+                                        ptr(status), stream()))
+        torch.cuda.synchronize()
+        assert int(status[0]) == 0 and rel_err(out.cpu().numpy(), want) < 2e-6
+        assert torch.all(wide[:spare] == 7.0) and torch.all(wide[spare + rows:] == 7.0)
+
+
 def test_grouped_product_refuses_what_it_cannot_address():
     a, w = np.zeros((10, 64), np.float32), np.zeros((3, 32, 64), np.float32)
     out = torch.zeros((10, 32), device="cuda")

@@ -335,7 +335,7 @@ struct GroupedFewParams {
     const bf16* w;             // [groups, n, k]
     void* out;                 // [rows, n]
     const uint32_t* offsets;   // [groups + 1]
-    uint32_t groups, n, k;
+    uint32_t groups, rows, n, k;
     int activation, out_dtype;
 };
 
@@ -347,13 +347,14 @@ gemm_grouped_few_kernel(GroupedFewParams P) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3, col0 = blockIdx.x * COLS;
     pdl_wait();
     pdl_trigger();
-    // the group of this block's tile: lanes count the tiles of 32 groups at a time
+    // the group of this block's tile: lanes count the tiles of 32 groups at a time.  A group list that does not fit the rows is cut to
+    // them, as in gemm_grouped.cu.
     uint32_t group = 0, row0 = 0, row1 = 0, before = 0;
     bool found = false;
     for (uint32_t e0 = 0; e0 < P.groups && !found; e0 += 32) {
         const uint32_t e = e0 + lane;
-        const uint32_t first = e < P.groups ? __ldcg(P.offsets + e) : 0u, last = e < P.groups ? __ldcg(P.offsets + e + 1) : 0u;
-        const uint32_t tiles = (last - first + 15) / 16;
+        const uint32_t first = e < P.groups ? min(P.rows, __ldcg(P.offsets + e)) : 0u, last = e < P.groups ? min(P.rows, __ldcg(P.offsets + e + 1)) : 0u;
+        const uint32_t tiles = last > first ? (last - first + 15) / 16 : 0u;
         uint32_t upto = tiles;
 #pragma unroll
         for (uint32_t o = 1; o < 32; o <<= 1) {
@@ -427,7 +428,7 @@ bool gemm_grouped_few_pays(const GroupedGemm& g) {
 
 int launch_gemm_grouped_few(const GroupedGemm& g, cudaStream_t stream) {
     GroupedFewParams P;
-    P.a = (const bf16*)g.a; P.w = (const bf16*)g.w; P.out = g.out; P.offsets = g.offsets; P.groups = g.groups; P.n = g.n; P.k = g.k;
+    P.a = (const bf16*)g.a; P.w = (const bf16*)g.w; P.out = g.out; P.offsets = g.offsets; P.groups = g.groups; P.rows = g.rows; P.n = g.n; P.k = g.k;
     P.activation = g.activation; P.out_dtype = g.out_dtype;
     const dim3 grid(ceil_div(g.n, 16u), g.rows / 16 + std::min(g.groups, g.rows));      // every group may end in a ragged tile
     launch_kernel(gemm_grouped_few_kernel, grid, dim3(FW_THREADS), 0, stream, P);
