@@ -701,6 +701,44 @@ def test_strict_step_in_one_launch_has_the_bits_of_the_operators(vocab, batch, w
     s.close()
 
 
+def test_two_f32_handles_on_two_threads():
+    """Chunks whose blocks ask for different amounts of shared memory (rows of 384 and 256 columns, 1200 and 300 keys) run from two threads at
+    once: what one launch asks for does not decide what another one may have.  Bits as of each handle alone."""
+    import threading
+
+    def handle(width, capacity, batch):
+        cfg = GptConfig(vocab_size=50, max_sequence_length=capacity, embed_dim=width, num_heads=width // 32, feed_forward_dim=64, num_layers=2,
+                        layer_norm_epsilon=1e-5)
+        s = B200Session(cfg, batch, capacity, logits_mode="none")
+        for i, a in enumerate(normal_model_arrays(cfg, seed=51, std=0.2, bias_std=0.1)):
+            s.refresh(i, a)
+        return s, np.random.default_rng(52).integers(0, 50, size=(batch, capacity)).astype(np.uint32)
+
+    def passes(s, ids, count):
+        chunk = 300
+        for _ in range(count):
+            for at in range(0, ids.shape[1], chunk):
+                s.decode_full(ids[:, at:at + chunk], at)
+        return [s.read_cache(i).view(np.uint32) for i in range(4)]
+
+    sessions = [handle(384, 1200, 4), handle(256, 300, 8)]
+    alone = [passes(s, ids, 1) for s, ids in sessions]
+    got = [None, None]
+
+    def work(i, count):
+        got[i] = passes(*sessions[i], count)
+
+    threads = [threading.Thread(target=work, args=(0, 25)), threading.Thread(target=work, args=(1, 100))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for want, have in zip(alone, got):
+        assert have is not None and all(np.array_equal(a, b) for a, b in zip(want, have))
+    for s, _ in sessions:
+        s.close()
+
+
 def test_paged_kv_cache_gives_the_same_bits_as_the_contiguous_one():
     """kv_page_rows > 0: every cache tensor is a pool of pages handed to sessions on demand.  Same kernels, other
     addresses: prefill (non-tiled scan in both handles), graph-replayed steps, ragged steps and the cache read back in

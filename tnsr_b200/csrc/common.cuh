@@ -41,6 +41,20 @@ inline int check_launch(const char* what) {
     return TNSR_B200_OK;
 }
 
+// Dynamic shared memory past 48 KB for a kernel: `most`, what its dispatch can ask for at the most, once per device.  The limit belongs to the
+// kernel and not to a launch: set to the bytes of one launch, it refuses the larger one that another handle's thread makes in between.
+template <auto KERNEL>
+int allow_shared(size_t most, const char* what) {
+    static std::atomic<bool> allowed[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const bool known = dev >= 0 && dev < 64;
+    if (known && allowed[dev].load(std::memory_order_acquire)) return TNSR_B200_OK;
+    if (cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) return check_launch(what);
+    if (known) allowed[dev].store(true, std::memory_order_release);
+    return TNSR_B200_OK;
+}
+
 // Optional per-thread sink: when set, the decode-attention launcher records an
 // event pair around its main kernel.
 struct KernelTimer {

@@ -136,8 +136,10 @@ int tnsr_b200_encoder_attention(const float* q, const float* k, const float* v, 
         set_thread_error("encoder_attention: sequence too long for shared memory or too many queries for one launch");
         return TNSR_B200_ERR_UNSUPPORTED;
     }
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(encoder_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) {
+        const int rc = allow_shared<encoder_attention_kernel>(200 * 1024, "encoder_attention attribute");
+        if (rc) return rc;
+    }
     // (head as f32).sqrt().recip()  -- examples/forty_five/mod.rs:377
     const float scale = 1.0f / sqrtf((float)head_dim);
     encoder_attention_kernel<<<(unsigned)blocks, 128, smem, reinterpret_cast<cudaStream_t>(stream)>>>(

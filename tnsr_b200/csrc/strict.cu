@@ -23,6 +23,7 @@ namespace tb {
 // by side so that a pair of them is loaded and not made.  The next tile's global loads are in flight while a tile is worked on.
 // ---------------------------------------------------------------------------
 constexpr uint32_t SK = 32;
+constexpr size_t SMOST = 200 * 1024;      // dynamic shared memory of a block of the kernels here, at the most
 
 __device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
     uint64_t d;
@@ -174,14 +175,11 @@ int launch_gemm_strict(const float* a, const float* b, void* out, uint32_t ldc, 
                        uint32_t n, bool b_transposed, const GemmEpilogue& ep, cudaStream_t stream) {
     if (m == 0 || n == 0) return TNSR_B200_OK;
     const size_t rows_smem = (size_t)k * SR_COLS * sizeof(float);
-    if (m <= 64 && k > 0 && rows_smem <= 200 * 1024) {
-        static bool configured[2] = {false, false};
-        if (rows_smem > 48 * 1024 && !configured[b_transposed]) {
-            cudaError_t e = b_transposed
-                ? cudaFuncSetAttribute(gemm_strict_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)
-                : cudaFuncSetAttribute(gemm_strict_rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            if (e != cudaSuccess) return check_launch("gemm_strict_rows attribute");
-            configured[b_transposed] = true;
+    if (m <= 64 && k > 0 && rows_smem <= SMOST) {
+        if (rows_smem > 48 * 1024) {
+            const int rc = b_transposed ? allow_shared<gemm_strict_rows_kernel<true>>(SMOST, "gemm_strict_rows attribute")
+                                        : allow_shared<gemm_strict_rows_kernel<false>>(SMOST, "gemm_strict_rows attribute");
+            if (rc) return rc;
         }
         dim3 grid(ceil_div(n, SR_COLS), m);
         if (b_transposed)
@@ -307,25 +305,25 @@ layernorm_strict_rows_kernel(const float* __restrict__ x, const float* __restric
 
 // From this many rows on blocks of 32 give every SM more than a row's chain at a time.
 constexpr uint32_t LR_MIN_ROWS = 1024;
+constexpr size_t LR_SMEM = 100 * 1024;     // two blocks per SM at least
 
 int launch_layernorm_strict(const float* x, const float* w, const float* b, float* out, uint32_t rows,
                             uint32_t width, float eps, cudaStream_t stream) {
     if (rows == 0) return TNSR_B200_OK;
     const size_t rows_smem = 2 * (size_t)LR * (width | 1) * sizeof(float);
-    if (rows >= LR_MIN_ROWS && rows_smem <= 100 * 1024) {     // two blocks per SM at least
-        if (rows_smem > 48 * 1024)
-            cudaFuncSetAttribute(layernorm_strict_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem);
+    int rc;
+    if (rows >= LR_MIN_ROWS && rows_smem <= LR_SMEM) {
+        if (rows_smem > 48 * 1024 && (rc = allow_shared<layernorm_strict_rows_kernel>(LR_SMEM, "layernorm_strict_rows attribute"))) return rc;
         layernorm_strict_rows_kernel<<<ceil_div(rows, LR), 256, rows_smem, stream>>>(x, w, b, out, rows, width, eps);
         count_launch();
         return check_launch("layernorm_strict_rows");
     }
     size_t smem = 2 * (size_t)width * sizeof(float);
-    if (smem > 200 * 1024) {
+    if (smem > SMOST) {
         set_thread_error("strict LayerNorm: row does not fit shared memory");
         return TNSR_B200_ERR_UNSUPPORTED;
     }
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(layernorm_strict_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024 && (rc = allow_shared<layernorm_strict_kernel>(SMOST, "layernorm_strict attribute"))) return rc;
     layernorm_strict_kernel<<<rows, 128, smem, stream>>>(x, w, b, out, width, eps);
     count_launch();
     return check_launch("layernorm_strict");
@@ -566,7 +564,7 @@ template <int HP, int QT>
 static size_t strict_tile_smem(uint32_t longest, uint32_t* pitch) {
     *pitch = (longest + 3) / 4 * 4 + 4;          // 16-byte rows that do not all start in the same bank
     const size_t bytes = ((size_t)QT * HP + AT_KEYS * (HP + 1) + (size_t)QT * *pitch) * sizeof(float);
-    return bytes <= 200 * 1024 ? bytes : 0;
+    return bytes <= SMOST ? bytes : 0;
 }
 
 template <typename KV, int HP, int QT>
@@ -576,8 +574,7 @@ static bool launch_strict_tile_attention(const float* q, const void* kc, const v
     uint32_t pitch;
     const size_t smem = strict_tile_smem<HP, QT>(d_position ? capacity : std::min(capacity, position + chunk), &pitch);
     if (!smem) return false;
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(attention_strict_tile_kernel<KV, HP, QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024 && allow_shared<attention_strict_tile_kernel<KV, HP, QT>>(SMOST, "attention_strict_tile attribute")) return false;
     attention_strict_tile_kernel<KV, HP, QT><<<dim3(ceil_div(chunk, (uint32_t)QT), heads, sessions), 256, smem, stream>>>(
         q, (const KV*)kc, (const KV*)vc, out, chunk, position, d_position, capacity, heads, hd, scale, round_bf16, pitch);
     return true;
@@ -612,7 +609,7 @@ int launch_attention_strict(const float* q, const void* k_cache, const void* v_c
     // (width as f32 / heads as f32).sqrt().recip()  -- src/nn/kv_cache/graph.rs:105
     const float scale = 1.0f / sqrtf((float)(heads * head_dim) / (float)heads);
     size_t smem = ((size_t)head_dim + capacity) * sizeof(float);
-    if (smem > 200 * 1024) {
+    if (smem > SMOST) {
         set_thread_error("strict attention: context does not fit shared memory");
         return TNSR_B200_ERR_UNSUPPORTED;
     }
@@ -627,15 +624,14 @@ int launch_attention_strict(const float* q, const void* k_cache, const void* v_c
         count_launch();
         return check_launch("attention_strict_tile");
     }
+    int rc;
     if (kv_dtype == TNSR_B200_BF16) {
-        if (smem > 48 * 1024)
-            cudaFuncSetAttribute(attention_strict_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (smem > 48 * 1024 && (rc = allow_shared<attention_strict_kernel<bf16>>(SMOST, "attention_strict attribute"))) return rc;
         attention_strict_kernel<bf16><<<(unsigned)blocks, 128, smem, stream>>>(
             q, (const bf16*)k_cache, (const bf16*)v_cache, out, chunk, position, d_position, capacity, heads,
             head_dim, scale, round_bf16);
     } else {
-        if (smem > 48 * 1024)
-            cudaFuncSetAttribute(attention_strict_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (smem > 48 * 1024 && (rc = allow_shared<attention_strict_kernel<float>>(SMOST, "attention_strict attribute"))) return rc;
         attention_strict_kernel<float><<<(unsigned)blocks, 128, smem, stream>>>(
             q, (const float*)k_cache, (const float*)v_cache, out, chunk, position, d_position, capacity, heads,
             head_dim, scale, round_bf16);

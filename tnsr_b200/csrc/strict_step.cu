@@ -389,11 +389,11 @@ uint32_t rows_that_fit(const StrictStepArgs& a) {
 
 template <typename KV>
 int clusters_at_once() {
-    static int known[64] = {};              // per device: clusters of 16 CTAs that run side by side, -1: none
+    static std::atomic<int> known[64];      // per device: clusters of 16 CTAs that run side by side, -1: none, 0: not asked yet
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-    if (known[dev] == 0) {
-        int n = 0;
+    int n = known[dev].load(std::memory_order_acquire);
+    if (n == 0) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(SS_CTAS);
         cfg.blockDim = dim3(SS_THREADS);
@@ -408,9 +408,10 @@ int clusters_at_once() {
                           cudaFuncSetAttribute(strict_step_kernel<KV>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
                           cudaOccupancyMaxActiveClusters(&n, strict_step_kernel<KV>, &cfg) == cudaSuccess && n > 0;
         if (!fits) cudaGetLastError();
-        known[dev] = fits ? n : -1;
+        n = fits ? n : -1;
+        known[dev].store(n, std::memory_order_release);
     }
-    return std::max(0, known[dev]);
+    return std::max(0, n);
 }
 
 }  // namespace
