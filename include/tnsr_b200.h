@@ -343,9 +343,14 @@ TNSR_B200_API int tnsr_b200_decoder_decode(tnsr_b200_decoder* dec, const uint32_
 
 /* Page-locked host memory for results (no reference counterpart): logits that
  * are copied there skip the driver's detour through a staging buffer.  NULL if
- * there is none to be had. */
+ * there is none to be had.  An asynchronous copy out of it does not wait: let it
+ * end before the memory takes another result or is freed. */
 TNSR_B200_API void* tnsr_b200_host_alloc(uint64_t bytes);
 TNSR_B200_API void tnsr_b200_host_free(void* p);
+/* The same for memory that the caller has: page-locked from register to
+ * unregister. */
+TNSR_B200_API int tnsr_b200_host_register(void* p, uint64_t bytes);
+TNSR_B200_API void tnsr_b200_host_unregister(void* p);
 
 /* Ragged single-token step (no reference counterpart: the reference's sessions
  * advance together; its documentation lists ragged batches as future work,

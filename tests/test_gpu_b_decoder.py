@@ -701,6 +701,28 @@ def test_strict_step_in_one_launch_has_the_bits_of_the_operators(vocab, batch, w
     s.close()
 
 
+def test_results_lie_on_ordinary_memory():
+    """A copy to the device that a caller starts from a result and does not wait for has to be staged before the call returns: the array may be
+    dropped, and its memory take the next result, while the copy is on its way.  The driver does so for memory that is not page-locked."""
+    cfg = GptConfig(vocab_size=32000, max_sequence_length=16, embed_dim=64, num_heads=1, feed_forward_dim=64, num_layers=1,
+                    layer_norm_epsilon=1e-5)
+    s = B200Session(cfg, 16, 16, logits_mode="last")
+    for i, a in enumerate(normal_model_arrays(cfg, seed=53)):
+        s.refresh(i, a)
+    ids = np.random.default_rng(54).integers(0, 32000, size=(16, 3)).astype(np.uint32)
+    want = [s.decode_full(ids[:, t:t + 1], t)[0].copy() for t in range(3)]
+    s.reset()
+    copies = []
+    for t in range(3):
+        logits = s.decode_full(ids[:, t:t + 1], t)[0]
+        assert not torch.from_numpy(logits).is_pinned()
+        copies.append(torch.from_numpy(logits).to("cuda", non_blocking=True))
+        del logits
+    for a, b in zip(copies, want):
+        assert np.array_equal(a.cpu().numpy().view(np.uint32), b.view(np.uint32))
+    s.close()
+
+
 def test_two_f32_handles_on_two_threads():
     """Chunks whose blocks ask for different amounts of shared memory (rows of 384 and 256 columns, 1200 and 300 keys) run from two threads at
     once: what one launch asks for does not decide what another one may have.  Bits as of each handle alone."""

@@ -1110,6 +1110,18 @@ void tnsr_b200_host_free(void* p) {
     cudaGetLastError();
 }
 
+int tnsr_b200_host_register(void* p, uint64_t bytes) {
+    if (cudaHostRegister(p, bytes, cudaHostRegisterPortable) == cudaSuccess) return TNSR_B200_OK;
+    cudaGetLastError();
+    set_thread_error("host_register: these pages cannot be locked");
+    return TNSR_B200_ERR_CUDA;
+}
+
+void tnsr_b200_host_unregister(void* p) {
+    if (p) cudaHostUnregister(p);
+    cudaGetLastError();
+}
+
 int tnsr_b200_decoder_set_sampler(tnsr_b200_decoder* dec, float temperature, uint32_t top_k, uint64_t seed) {
     if (!dec) return fail(nullptr, TNSR_B200_ERR_INVALID_ARGUMENT, "null decoder");
     if (temperature > 0.0f && (!std::isfinite(temperature) || top_k == 0 || top_k > 256))

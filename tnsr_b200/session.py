@@ -5,6 +5,8 @@ from __future__ import annotations
 
 import collections
 import ctypes as C
+import mmap
+import os
 import weakref
 
 import numpy as np
@@ -13,46 +15,73 @@ from . import _native
 from ._native import ACT, DTYPE, LOGITS, PREFILL, Config, NativeError, check, lib
 
 
-class _ResultBlocks:
-    """Page-locked memory under the larger logits arrays of a session whose results have one size.
+_forks = [0]       # how often this process was copied
+os.register_at_fork(before=lambda: _forks.__setitem__(0, _forks[0] + 1))
 
-    A fresh pageable array costs a page fault per 4 KB and a copy through the driver's staging buffer (48 x 32000 logits: 0.28 ms and the
-    faults, 0.11 ms from a block that was used before).  An array owns its block until the last view of it is gone; then the block serves
-    another result.  There are two (the array a caller still holds and the one being filled); further arrays are ordinary ones.
-    Locking pages takes about 1 ms per 2 MB, so that larger results keep to ordinary memory as well."""
+
+class _Block:
+    """The same pages under two addresses: `address` is page-locked, and where the device's copy engine writes; `seen` is ordinary memory to the
+    driver, and what an array lies on.  A caller's asynchronous copy out of the array is staged before it returns, as it is for any
+    array, so that dropping the array and using its pages again is safe."""
+
+    def __init__(self, size):
+        fd = os.memfd_create("results")
+        try:
+            os.ftruncate(fd, size)
+            self._locked = mmap.mmap(fd, size)
+            self.seen = mmap.mmap(fd, size, flags=mmap.MAP_SHARED | mmap.MAP_POPULATE)
+        finally:
+            os.close(fd)
+        self.address = C.addressof(C.c_char.from_buffer(self._locked))
+        if lib().tnsr_b200_host_register(self.address, size) != 0:
+            raise OSError("no page-locked memory")
+
+    def unlock(self):
+        lib().tnsr_b200_host_unregister(self.address)
+
+
+class _ResultBlocks:
+    """Memory under the larger logits arrays of a session whose results have one size.
+
+    A copy into ordinary memory goes through the driver's staging buffer (48 x 32000 logits: 0.36 ms, 0.11 ms into a block).  An array owns its
+    block until the last view of it is gone; then the block serves another result, unless the process was forked while the array
+    was held: a child may still read it.  There are two (the array a caller still holds and the one being filled); further arrays
+    are ordinary ones.  Locking pages takes about 1 ms per 2 MB, so that larger results keep to ordinary memory as well.  Finalizers
+    never call the driver: a closed session unlocks its blocks itself, and arrays that are still held keep the pages."""
     LEAST, MOST, BLOCKS = 1 << 20, 16 << 20, 2
 
     def __init__(self, floats):
         self._floats = floats
-        self._free = collections.deque()       # addresses; its operations are atomic, finalizers run anywhere
-        self._closed = False
+        self._blocks = []
         if self.LEAST <= 4 * floats <= self.MOST:
-            for _ in range(self.BLOCKS):
-                address = lib().tnsr_b200_host_alloc(4 * floats)
-                if address:
-                    self._free.append(address)
+            try:
+                for _ in range(self.BLOCKS):
+                    self._blocks.append(_Block(4 * floats))
+            except (OSError, AttributeError, ValueError):
+                pass
+        self._free = collections.deque(self._blocks)       # its operations are atomic, finalizers run anywhere
 
     def array(self, floats):
+        """(An array of so many floats, the address to copy them to.)"""
         try:
-            address = self._free.pop() if floats == self._floats else None
+            block = self._free.pop() if floats == self._floats else None
         except IndexError:
-            address = None
-        if address is None:
-            return np.empty(floats, dtype=np.float32)
-        owner = (C.c_float * floats).from_address(address)
-        weakref.finalize(owner, self._back, address).atexit = False
-        return np.frombuffer(owner, dtype=np.float32)
+            block = None
+        if block is None:
+            plain = np.empty(floats, dtype=np.float32)
+            return plain, plain.ctypes.data
+        owner = (C.c_float * floats).from_buffer(block.seen)
+        weakref.finalize(owner, self._back, block, _forks[0]).atexit = False
+        return np.frombuffer(owner, dtype=np.float32), block.address
 
-    def _back(self, address):
-        if self._closed:
-            lib().tnsr_b200_host_free(address)
-        else:
-            self._free.append(address)
+    def _back(self, block, forks):
+        if forks == _forks[0]:
+            self._free.append(block)
 
     def close(self):
-        self._closed = True
-        while self._free:
-            lib().tnsr_b200_host_free(self._free.pop())
+        self._free.clear()
+        while self._blocks:
+            self._blocks.pop().unlock()
 
 
 class B200Session:
@@ -127,11 +156,11 @@ class B200Session:
         logits = None
         lp = None
         if self.logits_mode == "all":
-            logits = self._blocks.array(batch * chunk * self.vocab)
+            logits, lp = self._blocks.array(batch * chunk * self.vocab)
         elif self.logits_mode == "last":
-            logits = self._blocks.array(batch * self.vocab)
-        if logits is not None:
-            lp = logits.ctypes.data_as(C.POINTER(C.c_float))
+            logits, lp = self._blocks.array(batch * self.vocab)
+        if lp is not None:
+            lp = C.cast(lp, C.POINTER(C.c_float))
         argmax = np.empty(batch, dtype=np.uint32) if want_argmax else None
         ap = argmax.ctypes.data_as(C.POINTER(C.c_uint32)) if want_argmax else None
         self._check(lib().tnsr_b200_decoder_decode(self.handle, tok.ctypes.data_as(C.POINTER(C.c_uint32)), chunk,
@@ -143,8 +172,9 @@ class B200Session:
         tok = np.ascontiguousarray(tokens, dtype=np.uint32).reshape(-1)
         pos = np.ascontiguousarray(positions, dtype=np.uint32).reshape(-1)
         assert tok.size == self.batch and pos.size == self.batch
-        logits = None if self.logits_mode == "none" else self._blocks.array(self.batch * self.vocab)
-        lp = logits.ctypes.data_as(C.POINTER(C.c_float)) if logits is not None else None
+        logits, lp = (None, None) if self.logits_mode == "none" else self._blocks.array(self.batch * self.vocab)
+        if lp is not None:
+            lp = C.cast(lp, C.POINTER(C.c_float))
         argmax = np.empty(self.batch, dtype=np.uint32) if want_argmax else None
         ap = argmax.ctypes.data_as(C.POINTER(C.c_uint32)) if want_argmax else None
         u32p = C.POINTER(C.c_uint32)
