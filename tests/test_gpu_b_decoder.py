@@ -701,6 +701,42 @@ def test_strict_step_in_one_launch_has_the_bits_of_the_operators(vocab, batch, w
     s.close()
 
 
+def test_pages_that_change_hands_between_steps():
+    """Sessions end and others take their slots and pages in another order.  Kernels of a step ask for keys ahead of the previous kernel's end,
+    through positions and page numbers of this step: the bits are those of a handle that never had the earlier sessions."""
+    cfg = GptConfig(vocab_size=300, max_sequence_length=256, embed_dim=128, num_heads=2, feed_forward_dim=256, num_layers=3,
+                    layer_norm_epsilon=1e-5, activation="swiglu", weight_dtype="bf16")
+    arrays = normal_model_arrays(cfg, seed=55, std=0.05)
+    rng = np.random.default_rng(56)
+    old, new = (rng.integers(0, cfg.vocab_size, size=(3, 140)).astype(np.uint32) for _ in range(2))
+
+    def session():
+        s = B200Session(cfg, 3, 256, logits_mode="last", kv_page_rows=16, kv_pool_pages=30)
+        for i, a in enumerate(arrays):
+            s.refresh(i, a)
+        return s
+
+    def requests(s, ids, prompt):
+        out = [s.decode_full(ids[:, :prompt], 0)[0].copy()]
+        at = np.asarray([prompt, prompt - 20, prompt - 3], dtype=np.uint32)
+        for t in range(24):
+            out.append(s.decode_ragged(ids[:, prompt + t], at)[0].copy())
+            at += 1
+        return np.stack(out).view(np.uint32)
+
+    fresh = session()
+    want = requests(fresh, new, 70)
+    fresh.close()
+    used = session()
+    requests(used, old, 110)
+    for order in ([2, 0, 1], [1, 2, 0]):
+        for b in order:
+            used.release(b)
+        assert used.free_pages() == 30
+        assert np.array_equal(requests(used, new, 70), want)
+    used.close()
+
+
 def test_results_lie_on_ordinary_memory():
     """A copy to the device that a caller starts from a result and does not wait for has to be staged before the call returns: the array may be
     dropped, and its memory take the next result, while the copy is on its way.  The driver does so for memory that is not page-locked."""

@@ -418,8 +418,9 @@ decode_attention_kernel(DaParams P) {
                 const uint4 a = __ldcg(reinterpret_cast<const uint4*>(P.items + i)), b = __ldcg(reinterpret_cast<const uint4*>(P.items + i) + 1);
                 return DaItem{a.x, a.y, a.z, a.w, b.x, b.y, {0u, 0u}};
             };
-            // stage s of item `it` into the ring; `with_q`: also the session's query row, which the item's first stage carries
-            auto fill = [&](const DaItem& it, uint32_t s, uint32_t n_stages, bool with_q) {
+            // stage s of item `it` into the ring, with the session's query row, which the item's first stage carries, unless that is still
+            // being written (`ahead`: the previous kernel may be running)
+            auto fill = [&](const DaItem& it, uint32_t s, uint32_t n_stages, bool ahead) {
                 const uint32_t nk = min((uint32_t)KS, it.nkeys - s * KS);
                 uint8_t* sk = ring + (size_t)stage * stage_bytes;
                 DaStageMeta mt;
@@ -433,10 +434,11 @@ decode_attention_kernel(DaParams P) {
                 const uint32_t bytes = nk * row_bytes;
                 da_mbar_expect_tx(full_bar + stage, 2 * bytes + (s == 0 ? row_bytes : 0));
                 // a stage never straddles pages: key0 and the page size are multiples of the stage size
-                const size_t base = kv_row(P.paging, it.session, it.key0 + s * KS, P.capacity) * d;
+                const uint32_t key = it.key0 + s * KS;
+                const size_t base = (ahead ? kv_row_l2(P.paging, it.session, key, P.capacity) : kv_row(P.paging, it.session, key, P.capacity)) * d;
                 da_bulk_load_once(sk, P.kc + base, bytes, full_bar + stage, once);
                 da_bulk_load_once(sk + k_bytes, P.vc + base, bytes, full_bar + stage, once);
-                if (s == 0 && with_q) da_bulk_load(sk + 2 * k_bytes, P.q + (size_t)it.session * d, row_bytes, full_bar + stage);
+                if (s == 0 && !ahead) da_bulk_load(sk + 2 * k_bytes, P.q + (size_t)it.session * d, row_bytes, full_bar + stage);
             };
             DaItem it = {}, nxt = {};
             if (item_begin < item_end) it = nxt = item_at(item_begin);
@@ -450,7 +452,7 @@ decode_attention_kernel(DaParams P) {
                     const uint32_t n_stages = (it.nkeys + KS - 1) / KS;
                     if (s + 1 == n_stages && (it.slot == DA_DIRECT || it.slot + 1 == it.first_slot + it.n_parts)) break;
                     stage = filled;
-                    fill(it, s, n_stages, false);
+                    fill(it, s, n_stages, true);
                     if (s == 0) waiting |= 1u << filled;
                     ++filled;
                     if (++s == n_stages) {
@@ -472,7 +474,7 @@ decode_attention_kernel(DaParams P) {
                 const uint32_t n_stages = (it.nkeys + KS - 1) / KS;
                 for (; s < n_stages; ++s) {
                     if (!da_mbar_wait(empty_bar + stage, phase ^ 1, abort_flag, P.wait_limit_ns)) { ok = false; break; }
-                    fill(it, s, n_stages, true);
+                    fill(it, s, n_stages, false);
                     if (++stage == P.stages) { stage = 0; phase ^= 1; }
                 }
             }

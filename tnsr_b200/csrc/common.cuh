@@ -186,6 +186,11 @@ __device__ __forceinline__ size_t kv_row(const KvPaging& pg, uint32_t s, uint32_
     if (!pg.table) return (size_t)s * capacity + r;
     return (size_t)pg.table[(size_t)s * pg.pages_per_session + r / pg.page_rows] * pg.page_rows + r % pg.page_rows;
 }
+// The same past L1, for a kernel that asks before its pdl_wait() (see load_pair_l2 in mixers.cuh): slots and pages change hands between steps.
+__device__ __forceinline__ size_t kv_row_l2(const KvPaging& pg, uint32_t s, uint32_t r, uint32_t capacity) {
+    if (!pg.table) return (size_t)s * capacity + r;
+    return (size_t)__ldcg(pg.table + (size_t)s * pg.pages_per_session + r / pg.page_rows) * pg.page_rows + r % pg.page_rows;
+}
 #endif
 
 struct GemmQkvTargets {

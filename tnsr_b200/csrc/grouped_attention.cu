@@ -125,9 +125,9 @@ grouped_split_kernel(GaParams P) {
 
     uint8_t* ring = smem + warp * (STAGES * S::STAGE);
     const size_t k_ld = (size_t)a.kv_heads * a.dim, v_ld = (size_t)a.kv_heads * a.vdim;
-    auto copy = [&](uint32_t i, uint32_t stage) {     // tile i of the session; the pages of a tile's 16 keys are one page
+    auto copy = [&](uint32_t i, uint32_t stage, bool early) {     // tile i of the session; the pages of a tile's 16 keys are one page
         if (i < tile1) {
-            const size_t kr = kv_row(a.paging, s, i * 16, a.capacity);
+            const size_t kr = early ? kv_row_l2(a.paging, s, i * 16, a.capacity) : kv_row(a.paging, s, i * 16, a.capacity);
             const uint32_t live = min(16u, keys - i * 16);
             uint8_t* dst = ring + stage * S::STAGE;
             ga_copy<DK>(dst, reinterpret_cast<const bf16*>(a.k_cache) + kr * k_ld + (size_t)kvh * a.dim, k_ld, 16, live, a.dim, P.vec, lane, 32);
@@ -136,19 +136,19 @@ grouped_split_kernel(GaParams P) {
         }
     };
     auto load = [&](uint32_t i, uint32_t stage) {
-        copy(i, stage);
+        copy(i, stage, false);
         mx_commit();
     };
     // tiles that earlier steps wrote are asked for before the previous kernel has ended (see load_pair_l2; these copies pass L1 by)
     auto old_tile = [&](int i) { return P.vec && (tile0 + warp + i * GA_WARPS + 1) * 16 <= p0; };
 #pragma unroll
     for (int i = 0; i < STAGES - 1; ++i)
-        if (old_tile(i)) copy(tile0 + warp + i * GA_WARPS, i);
+        if (old_tile(i)) copy(tile0 + warp + i * GA_WARPS, i, true);
     pdl_wait();
     pdl_trigger();
 #pragma unroll
     for (int i = 0; i < STAGES - 1; ++i) {
-        if (!old_tile(i)) copy(tile0 + warp + i * GA_WARPS, i);
+        if (!old_tile(i)) copy(tile0 + warp + i * GA_WARPS, i, false);
         mx_commit();
     }
     // query fragments straight from global memory: rows g8 and g8 + 8

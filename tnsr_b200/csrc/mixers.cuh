@@ -16,8 +16,9 @@ struct StepPlace {
     const uint32_t* d_position = nullptr;   // device scalar, or one entry per session (position_stride 1)
     uint32_t position_stride = 0;
 #ifdef __CUDACC__
+    // past L1: kernels ask for it before their pdl_wait() (see load_pair_l2)
     __device__ __forceinline__ uint32_t pos(uint32_t session) const {
-        return d_position ? d_position[session * position_stride] : position;
+        return d_position ? __ldcg(d_position + session * position_stride) : position;
     }
 #endif
 };
