@@ -449,6 +449,22 @@ def test_grouped_products_of_few_rows(counts, n, k):
     assert rel_err(grouped(a, w, offsets, 4, BF16, BF16), np.maximum(want, 0.0) ** 2) < 5e-3
 
 
+@pytest.mark.parametrize("counts,n,k", [([128], 3072, 768), ([8] * 16, 768, 768), ([0] * 31 + [64], 1536, 512), ([2] * 64, 144, 128)])
+def test_grouped_products_past_the_line_of_the_kernel_for_few_rows(counts, n, k):
+    """More than 444 blocks of 16 rows and columns: every group's weights would be read once per tile of its rows, and blocks without rows would
+    hold up the others.  The sums are those of the tcgen05 kernel, bit for bit (the kernel for few rows adds in another order)."""
+    rng = np.random.default_rng(n + k)
+    rows, offsets = sum(counts), np.concatenate([[0], np.cumsum(counts)])
+    a, w = rng.normal(size=(rows, k)).astype(np.float32), (rng.normal(size=(len(counts), n, k)) * k ** -0.5).astype(np.float32)
+    got = grouped(a, w, offsets, -1, BF16, F32)
+    lib().tnsr_b200_set_gemm_engine(2)
+    try:
+        want = grouped(a, w, offsets, -1, BF16, F32)
+    finally:
+        lib().tnsr_b200_set_gemm_engine(0)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
 @pytest.mark.parametrize("offsets", [[0, 10, 40], [0, 4, 4, 3000000000], [12, 20, 3, 9], [30, 40, 50], [24, 0, 7]])
 @pytest.mark.parametrize("k", [64, 72])
 def test_grouped_products_cut_a_group_list_to_the_rows(offsets, k):

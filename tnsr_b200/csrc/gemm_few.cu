@@ -421,16 +421,31 @@ gemm_grouped_few_kernel(GroupedFewParams P) {
 
 }  // namespace
 
-// At most 128 rows in groups of 16 on average: with more, a group's weights are read for several tiles and the tcgen05 tiles are the better ones.
+// Blocks of the launch: a column of them per 16 columns, in it one per 16-row tile that the groups can have (every group may end in a ragged one).
+static uint32_t grouped_few_tiles(const GroupedGemm& g) { return g.rows / 16 + std::min(g.groups, g.rows); }
+
+// Which groups have rows only the device knows, so there are blocks for the most tiles there can be, and each group's weights are read once per
+// tile of it.  Three blocks per SM are the line (two run at a time).  Measured on B200 as chains of launches, us here / in the tcgen05 kernel:
+//     groups, rows, n x k       blocks    rows even      all in one group
+//      4,  96,  256 x 2048       160     4.1 / 12.3      4.1 / 12.3
+//     16,   4,  768 x 768        192     4.1 /  7.0      3.5 /  7.2
+//     16,   8,  768 x 768        384     5.9 /  7.5      4.1 /  7.4
+//      4,  32, 1024 x 4096       384    12.2 / 21.1      7.1 / 20.2
+//     16,  32,  768 x 768        864     9.4 /  8.7      6.3 /  7.2
+//      8, 128, 3072 x 768       3072    22.2 / 12.8     17.8 / 10.9
+//     64, 128, 3072 x 768      13824     159 / 52        178 / 12
+// Of 1892 products (1 to 64 groups, 1 to 128 rows, 128 to 3072 columns, rows spread evenly, half of them in one group, all of them) 1167 are
+// within the line, 1164 of these more than 5 % faster here and none slower; past it the share of slower ones grows.
 bool gemm_grouped_few_pays(const GroupedGemm& g) {
-    return g.offsets && g.rows <= 128 && g.k % 16 == 0 && reinterpret_cast<uintptr_t>(g.a) % 32 == 0 && reinterpret_cast<uintptr_t>(g.w) % 32 == 0;
+    if (!g.offsets || g.rows > 128 || g.k % 16 != 0 || reinterpret_cast<uintptr_t>(g.a) % 32 != 0 || reinterpret_cast<uintptr_t>(g.w) % 32 != 0) return false;
+    return (uint64_t)ceil_div(g.n, 16u) * grouped_few_tiles(g) <= 3 * 148;
 }
 
 int launch_gemm_grouped_few(const GroupedGemm& g, cudaStream_t stream) {
     GroupedFewParams P;
     P.a = (const bf16*)g.a; P.w = (const bf16*)g.w; P.out = g.out; P.offsets = g.offsets; P.groups = g.groups; P.rows = g.rows; P.n = g.n; P.k = g.k;
     P.activation = g.activation; P.out_dtype = g.out_dtype;
-    const dim3 grid(ceil_div(g.n, 16u), g.rows / 16 + std::min(g.groups, g.rows));      // every group may end in a ragged tile
+    const dim3 grid(ceil_div(g.n, 16u), grouped_few_tiles(g));
     launch_kernel(gemm_grouped_few_kernel, grid, dim3(FW_THREADS), 0, stream, P);
     count_launch();
     return check_launch("gemm_grouped_few");
