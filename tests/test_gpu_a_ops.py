@@ -231,6 +231,23 @@ def test_gemm_bf16_register_engine_matches_f64(shape):
     assert np.array_equal(in_place.cpu().numpy(), fused)
 
 
+@pytest.mark.parametrize("engine,shape", [(2, (32, 6144, 512)), (2, (32, 8192, 2048)), (2, (24, 16384, 1024)), (2, (17, 32000, 256)), (2, (48, 3072, 512)),
+                                          (2, (64, 3072, 512)), (2, (56, 4096, 256)), (4, (1, 2048, 4096)), (4, (8, 1536, 4096)), (4, (4, 2304, 2048))])
+def test_gemm_bf16_sizes_that_keep_the_other_engines(engine, shape):
+    """Sizes at which operands on registers are the slower form: the sums of the tcgen05 engine, or of the one that streams the weights, bit for
+    bit (each of the three adds in another order)."""
+    m, n, k = shape
+    a, bt, _ = gemm_case(m, n, k, seed=23)
+    da, dbt = dev(a, torch.bfloat16), dev(bt, torch.bfloat16)
+    got = gemm_bf16(da, dbt)
+    lib().tnsr_b200_set_gemm_engine(engine)
+    try:
+        want = gemm_bf16(da, dbt)
+    finally:
+        lib().tnsr_b200_set_gemm_engine(0)
+    assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+
+
 @pytest.mark.parametrize("shape", [(1, 4096, 4096), (8, 4096, 4096), (64, 4096, 4096), (17, 768, 768), (32, 768, 2048),
                                    (64, 2304, 768), (5, 100, 72), (33, 129, 520), (16, 32000, 768), (1, 128, 64)])
 def test_gemm_bf16_few_rows_engine_matches_f64_with_and_without_split_k(shape):

@@ -862,10 +862,15 @@ static int launch_gemm_impl(const bf16* a, const bf16* bt, void* out, uint32_t l
             return TNSR_B200_ERR_INVALID_ARGUMENT;
         }
     }
-    // Few rows: operands straight into registers (gemm_few.cu; not where a test asks this engine to lose a stage).
-    if (!split_req && mode != GEMM_ARGMAX && g_gemm_engine == 0 && !ep.round_bf16 && !t_lose_gemm_stage && gemm_few_pays(a, bt, m, n, k))
+    const bool streams = !split_req && mode == GEMM_PLAIN && m <= 16 && (uint64_t)n * k >= (4ull << 20) && gemm_stream_eligible(a, bt, m, n, k, ep);
+    // Few rows: operands straight into registers (gemm_few.cu; not where a test asks this engine to lose a stage).  The exception is a narrow
+    // matrix with a long k, whose tiles do not give every SM one: outside a session's chain of launches, in which the weights are on their way
+    // before the previous kernel ends, streaming is the faster form (us here / there, 2048 x 4096: 1 row 9.8 / 8.7, 8 rows 9.9 / 9.5;
+    // 2048 x 5632: 12.9 / 11.2, 13.1 / 12.3; 2048 x 2048: 6.2 / 5.6, 6.2 / 6.4).
+    const bool narrow = streams && !t_pdl && m <= (k >= 4096 ? 8u : 4u) && n > 1024 && n <= 2304;
+    if (!split_req && mode != GEMM_ARGMAX && g_gemm_engine == 0 && !ep.round_bf16 && !t_lose_gemm_stage && !narrow && gemm_few_pays(a, bt, m, n, k))
         return launch_gemm_few(a, bt, P, k, mode, stream);
-    // What is left of few rows (k no multiple of 16, pointers of 16-byte alignment, a lost stage to provoke):
+    // What is left of few rows (k no multiple of 16, pointers of 16-byte alignment, the exception, a lost stage to provoke):
     // a handful of rows against a large weight matrix: stream the weights with the operands swapped (gemm_skinny.cu)
     // when that engine can fill the GPU, i.e. with split-K scratch lent by the caller or with at least half as many
     // 128-column tiles as SMs.  Measured inside a CUDA graph, 4096 x 4096 weights: 14.8 / 16.3 us at 1 / 8 rows against
@@ -874,8 +879,8 @@ static int launch_gemm_impl(const bf16* a, const bf16* bt, void* out, uint32_t l
     // Engine 3 (tests) takes it for every eligible shape up to 64 rows.
     // Up to 16 rows against at least 4 M weight elements: one pass over the weights with no split-K (gemm_stream.cu).
     // Engine 4 (tests) takes it for every eligible shape.
-    if (!split_req && mode == GEMM_PLAIN && m <= 16 && (g_gemm_engine == 0 || g_gemm_engine == 4) && gemm_stream_eligible(a, bt, m, n, k, ep) &&
-        ((uint64_t)n * k >= (4ull << 20) || g_gemm_engine == 4))
+    if ((streams && g_gemm_engine == 0) ||
+        (g_gemm_engine == 4 && !split_req && mode == GEMM_PLAIN && m <= 16 && gemm_stream_eligible(a, bt, m, n, k, ep)))
         return launch_gemm_stream(a, bt, out, ldc, m, n, k, ep, d_status, stream);
     if (!split_req && mode == GEMM_PLAIN && m <= 64 && g_gemm_engine != 1 && gemm_skinny_eligible(a, bt, m, n, k, ep)) {
         const bool pays = m <= 16 && (uint64_t)n * k >= (4ull << 20) &&
