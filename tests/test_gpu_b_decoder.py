@@ -701,6 +701,31 @@ def test_strict_step_in_one_launch_has_the_bits_of_the_operators(vocab, batch, w
     s.close()
 
 
+@pytest.mark.parametrize("batch,parts", [(128, 2), (192, 4)])
+def test_ranges_of_a_divided_step_keep_the_tcgen05_products(batch, parts):
+    """More than 32 rows in a range: products on register operands do not fit beside the other range's attention.  The sums are the tcgen05
+    engine's, bit for bit."""
+    from tnsr_b200 import _native
+    cfg = GptConfig(vocab_size=2048, max_sequence_length=64, embed_dim=256, num_heads=4, feed_forward_dim=512, num_layers=2,
+                    layer_norm_epsilon=1e-5, activation="swiglu", weight_dtype="bf16")
+    arrays = normal_model_arrays(cfg, seed=57, std=0.05)
+    ids = np.random.default_rng(58).integers(0, cfg.vocab_size, size=(batch, 12)).astype(np.uint32)
+
+    def run(engine):
+        _native.lib().tnsr_b200_set_gemm_engine(engine)
+        try:
+            s = B200Session(cfg, batch, 64, logits_mode="last", step_parts=parts)
+            for i, a in enumerate(arrays):
+                s.refresh(i, a)
+            out = [s.decode_full(ids[:, :9], 0)[0].copy()] + [s.decode_full(ids[:, t:t + 1], t)[0].copy() for t in range(9, 12)]
+            s.close()
+            return np.stack(out).view(np.uint32)
+        finally:
+            _native.lib().tnsr_b200_set_gemm_engine(0)
+
+    assert np.array_equal(run(0), run(2))
+
+
 def test_pages_that_change_hands_between_steps():
     """Sessions end and others take their slots and pages in another order.  Kernels of a step ask for keys ahead of the previous kernel's end,
     through positions and page numbers of this step: the bits are those of a handle that never had the earlier sessions."""

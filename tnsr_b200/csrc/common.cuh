@@ -140,6 +140,7 @@ struct GemmEpilogue {
     float* split_partials = nullptr;
     uint32_t split_k = 0;
     uint32_t split_rows = 0;
+    bool beside = false;              // another range of a divided step runs its attention on the same SMs meanwhile
 };
 
 // How many ways launch_gemm_bf16 can divide the k-blocks of a plain f32 residual GEMM with `m` rows (0: do not).  The

@@ -369,7 +369,7 @@ int layers_bf16(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chunk
             RUN(dec, launch_layernorm(h, L.ln1w, L.ln1b, n, rows, d, c.layer_norm_epsilon, TNSR_B200_BF16, false, st));
         pending = 0;
         GemmEpilogue eq;
-        eq.bias = L.bqkv;
+        eq.bias = L.bqkv; eq.beside = lean;
         GemmQkvTargets tg;
         tg.q = q; tg.k_cache = kcache; tg.v_cache = vcache;
         tg.d = d; tg.chunk = chunk; tg.capacity = c.capacity; tg.position = position; tg.d_position = pos_arg;
@@ -410,7 +410,7 @@ int layers_bf16(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chunk
             RUN(dec, launch_attention_generic(q, kcache, vcache, att, ns, chunk, position, d_position, c.capacity, H, hd, st, &pg));
         }
         GemmEpilogue eo;
-        eo.bias = L.bo; eo.residual = h; eo.ldr = d; eo.out_dtype = TNSR_B200_F32;
+        eo.beside = lean; eo.bias = L.bo; eo.residual = h; eo.ldr = d; eo.out_dtype = TNSR_B200_F32;
         const uint32_t split_o = splitk ? gemm_split_k(att, (const bf16*)L.wo, rows, d, d) : 0;
         if (split_o) { eo.split_k = split_o; eo.split_partials = part_ws; eo.split_rows = dec->split_rows; }
         RUN(dec, launch_gemm_bf16(att, (const bf16*)L.wo, h, d, rows, d, d, GEMM_PLAIN, eo, nullptr, dec->d_status, st));
@@ -420,21 +420,21 @@ int layers_bf16(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chunk
             RUN(dec, launch_layernorm(h, L.ln2w, L.ln2b, n, rows, d, c.layer_norm_epsilon, TNSR_B200_BF16, false, st));
         if (dec->swiglu) {
             if (dec->fused_gu) {
-                GemmEpilogue eg; eg.bias = L.bgu; eg.out_dtype = TNSR_B200_BF16;
+                GemmEpilogue eg; eg.beside = lean; eg.bias = L.bgu; eg.out_dtype = TNSR_B200_BF16;
                 RUN(dec, launch_gemm_bf16(n, L.wgu, ff, f, rows, 2 * f, d, GEMM_SWIGLU, eg, nullptr, dec->d_status, st));
             } else {
-                GemmEpilogue eg; eg.bias = L.b_gate; eg.out_dtype = TNSR_B200_BF16;
+                GemmEpilogue eg; eg.beside = lean; eg.bias = L.b_gate; eg.out_dtype = TNSR_B200_BF16;
                 RUN(dec, launch_gemm_bf16(n, (const bf16*)L.w_gate, ff, f, rows, f, d, GEMM_PLAIN, eg, nullptr, dec->d_status, st));
-                GemmEpilogue eu; eu.bias = L.b_up; eu.out_dtype = TNSR_B200_BF16;
+                GemmEpilogue eu; eu.beside = lean; eu.bias = L.b_up; eu.out_dtype = TNSR_B200_BF16;
                 RUN(dec, launch_gemm_bf16(n, (const bf16*)L.w_up, ff2, f, rows, f, d, GEMM_PLAIN, eu, nullptr, dec->d_status, st));
                 RUN(dec, launch_swiglu(ff, ff2, ff, (uint64_t)rows * f, st));
             }
         } else {
-            GemmEpilogue ei; ei.bias = L.b_in; ei.out_dtype = TNSR_B200_BF16;
+            GemmEpilogue ei; ei.beside = lean; ei.bias = L.b_in; ei.out_dtype = TNSR_B200_BF16;
             ei.activation = c.activation == TNSR_B200_ACT_GELU ? ACT_GELU : ACT_RELU;
             RUN(dec, launch_gemm_bf16(n, (const bf16*)L.w_in, ff, f, rows, f, d, GEMM_PLAIN, ei, nullptr, dec->d_status, st));
         }
-        GemmEpilogue ef; ef.bias = L.b_out; ef.residual = h; ef.ldr = d; ef.out_dtype = TNSR_B200_F32;
+        GemmEpilogue ef; ef.beside = lean; ef.bias = L.b_out; ef.residual = h; ef.ldr = d; ef.out_dtype = TNSR_B200_F32;
         const uint32_t split_d = splitk ? gemm_split_k(ff, (const bf16*)L.w_out, rows, d, f) : 0;
         if (split_d) { ef.split_k = split_d; ef.split_partials = part_ws; ef.split_rows = dec->split_rows; }
         RUN(dec, launch_gemm_bf16(ff, (const bf16*)L.w_out, h, d, rows, d, f, GEMM_PLAIN, ef, nullptr, dec->d_status, st));
