@@ -648,7 +648,7 @@ def test_session_sampler_draws_what_the_cpu_restatement_draws(logits_mode):
     assert np.array_equal(got, greedy)
 
 
-@pytest.mark.parametrize("heads,width,batch", [(4, 128, 1), (4, 128, 16), (3, 72, 2), (1, 64, 40), (2, 200, 3)])
+@pytest.mark.parametrize("heads,width,batch", [(4, 128, 1), (4, 128, 16), (3, 72, 2), (1, 64, 40), (2, 200, 3), (3, 72, 8), (2, 200, 9)])
 @pytest.mark.parametrize("precision", [GptAttentionPrecision.F32, GptAttentionPrecision.Bf16])
 def test_strict_chunks_have_the_bits_of_single_tokens(heads, width, batch, precision):
     """f32 weights: every output is a chain of rounded operations in a stated order, so a chunk of any length -- 32 or 8 queries per block,
@@ -671,6 +671,29 @@ def test_strict_chunks_have_the_bits_of_single_tokens(heads, width, batch, preci
     single = logits([1] * 134)
     for cuts in ([134], [65, 2, 67], [33, 31, 70]):
         assert np.array_equal(logits(cuts), single)
+
+
+def test_two_ids_of_an_f32_session_take_no_longer_than_two_steps():
+    """64 sessions of 8 heads of 8 columns behind 960 keys: a tile of 32 queries per block, of which a chunk of two ids has two, took four times
+    as long as a block per query (2750 us here; two single steps 820)."""
+    import time
+    cfg = GptConfig(vocab_size=96, max_sequence_length=1024, embed_dim=64, num_heads=8, feed_forward_dim=256, num_layers=4,
+                    layer_norm_epsilon=1e-5)
+    s = B200Session(cfg, 64, 1024, logits_mode="none")
+    for i, a in enumerate(normal_model_arrays(cfg, seed=61)):
+        s.refresh(i, a)
+    ids = np.random.default_rng(62).integers(0, 96, size=(64, 2)).astype(np.uint32)
+
+    def best(chunk):
+        times = []
+        for _ in range(30):
+            start = time.perf_counter()
+            s.decode_full(ids[:, :chunk], 960)
+            times.append(time.perf_counter() - start)
+        return min(times)
+
+    assert best(2) <= 1.5 * 2 * best(1)
+    s.close()
 
 
 @pytest.mark.parametrize("vocab,batch,width,hidden", [(2100, 3, 128, 520), (130, 9, 256, 1024), (50, 1, 16, 4)])

@@ -580,12 +580,29 @@ static bool launch_strict_tile_attention(const float* q, const void* kc, const v
     return true;
 }
 
-// 32 queries per block, or 8 where the scores of 32 do not fit (contexts from about 1400 keys) or too few blocks would run.
+// Queries of a block of the tiled kernel, or 0: the kernel above, with a block per query.  A tile reads every key once for its queries, but its
+// block walks all their chains: it pays when there are more queries than the GPU takes side by side, the more so the wider the head (below 32
+// columns most of a block's lanes idle; there long rows of scores, which leave room for a block or two per SM, lose at any number).  32
+// queries instead of 8 need shared memory for their scores and a chunk that fills them.  Measured on B200 over 2862 chunks (widths 8 to
+// 128, 1 to 64 sessions, 2 to 256 ids, up to 4096 keys): none more than 6 % slower than the other kernel.  Four layers, us per block and query /
+// in tiles of 8 / of 32:
+//     heads x width, sessions x ids, keys
+//     4 x 32    1 x   2  1024     452 /   582 /   660        4 x 32    16 x 64   1024    2885 /  969 /  975
+//     4 x 32    8 x  16  1024     764 /   705 /   812        4 x 32    32 x 64    320    1908 /  853 /  771
+//     8 x 8    64 x   8  1024    1277 /   933 /  2869        8 x 8     16 x 64   4096    8655 / 14925 / 14929
+//     4 x 64    8 x  64  1024    2869 /  1611 /  1916        6 x 16    32 x 16   1024    1671 /  968 /  1648
+static uint32_t strict_tile_queries(uint64_t units, uint32_t chunk, uint32_t hd, uint32_t longest) {
+    if (chunk < 2 || hd > 128) return 0;
+    const uint64_t queries = units * chunk;
+    if (hd >= 32 ? queries < (chunk >= 8 ? 1024 : 1536) : chunk < 8 || longest > 2048 || queries < (hd >= 16 ? 1536 : 2048)) return 0;
+    return chunk >= 32 && queries >= 8192 && longest <= 640 ? 32 : 8;
+}
+
 template <typename KV, int HP>
-static bool launch_strict_tile_width(const float* q, const void* kc, const void* vc, float* out, uint32_t sessions, uint32_t chunk, uint32_t position,
-                                     const uint32_t* d_position, uint32_t capacity, uint32_t heads, uint32_t hd, float scale, int round_bf16,
-                                     cudaStream_t stream) {
-    if ((uint64_t)ceil_div(chunk, 32u) * heads * sessions >= 148 &&
+static bool launch_strict_tile_width(uint32_t tile, const float* q, const void* kc, const void* vc, float* out, uint32_t sessions, uint32_t chunk,
+                                     uint32_t position, const uint32_t* d_position, uint32_t capacity, uint32_t heads, uint32_t hd, float scale,
+                                     int round_bf16, cudaStream_t stream) {
+    if (tile == 32 &&
         launch_strict_tile_attention<KV, HP, 32>(q, kc, vc, out, sessions, chunk, position, d_position, capacity, heads, hd, scale, round_bf16, stream))
         return true;
     return launch_strict_tile_attention<KV, HP, 8>(q, kc, vc, out, sessions, chunk, position, d_position, capacity, heads, hd, scale, round_bf16, stream);
@@ -595,10 +612,12 @@ template <typename KV>
 static bool launch_strict_tile_any(const float* q, const void* kc, const void* vc, float* out, uint32_t sessions, uint32_t chunk, uint32_t position,
                                    const uint32_t* d_position, uint32_t capacity, uint32_t heads, uint32_t hd, float scale, int round_bf16,
                                    cudaStream_t stream) {
-    if (chunk < 2 || hd > 128 || heads > 65535u || sessions > 65535u) return false;
-    if (hd <= 32) return launch_strict_tile_width<KV, 32>(q, kc, vc, out, sessions, chunk, position, d_position, capacity, heads, hd, scale, round_bf16, stream);
-    if (hd <= 64) return launch_strict_tile_width<KV, 64>(q, kc, vc, out, sessions, chunk, position, d_position, capacity, heads, hd, scale, round_bf16, stream);
-    return launch_strict_tile_width<KV, 128>(q, kc, vc, out, sessions, chunk, position, d_position, capacity, heads, hd, scale, round_bf16, stream);
+    const uint32_t longest = d_position ? capacity : std::min(capacity, position + chunk);
+    const uint32_t tile = strict_tile_queries((uint64_t)sessions * heads, chunk, hd, longest);
+    if (!tile || heads > 65535u || sessions > 65535u) return false;
+    if (hd <= 32) return launch_strict_tile_width<KV, 32>(tile, q, kc, vc, out, sessions, chunk, position, d_position, capacity, heads, hd, scale, round_bf16, stream);
+    if (hd <= 64) return launch_strict_tile_width<KV, 64>(tile, q, kc, vc, out, sessions, chunk, position, d_position, capacity, heads, hd, scale, round_bf16, stream);
+    return launch_strict_tile_width<KV, 128>(tile, q, kc, vc, out, sessions, chunk, position, d_position, capacity, heads, hd, scale, round_bf16, stream);
 }
 
 int launch_attention_strict(const float* q, const void* k_cache, const void* v_cache, float* out,
