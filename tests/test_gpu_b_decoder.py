@@ -673,6 +673,34 @@ def test_strict_chunks_have_the_bits_of_single_tokens(heads, width, batch, preci
         assert np.array_equal(logits(cuts), single)
 
 
+def test_f32_chunks_behind_many_keys_are_not_one_launch():
+    """16 ids of one session with 8 heads: one launch behind few keys, operator by operator behind many, where a cluster's 16 CTAs would take
+    eight turns at the keys.  The bits are the same."""
+    from tnsr_b200 import _native
+    cfg = GptConfig(vocab_size=96, max_sequence_length=512, embed_dim=64, num_heads=8, feed_forward_dim=128, num_layers=2,
+                    layer_norm_epsilon=1e-5)
+    s = B200Session(cfg, 1, 512, logits_mode="last")
+    for i, a in enumerate(normal_model_arrays(cfg, seed=63, std=0.2)):
+        s.refresh(i, a)
+    ids = np.random.default_rng(64).integers(0, 96, size=(1, 400)).astype(np.uint32)
+    count = _native.lib().tnsr_b200_kernel_launches
+
+    def launches(chunk, position):
+        before = count()
+        logits = s.decode_full(ids[:, position:position + chunk], position, want_argmax=False)[0].copy()
+        return count() - before, logits
+
+    assert launches(16, 0)[0] == 1 and launches(16, 16)[0] == 1
+    s.decode_full(ids[:, 32:300], 32)
+    many, want = launches(16, 300)
+    assert many > 10
+    for t in range(300, 316):
+        one, got = launches(1, t)
+        assert one == 1
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+    s.close()
+
+
 def test_two_ids_of_an_f32_session_take_no_longer_than_two_steps():
     """64 sessions of 8 heads of 8 columns behind 960 keys: a tile of 32 queries per block, of which a chunk of two ids has two, took four times
     as long as a block per query (2750 us here; two single steps 820)."""

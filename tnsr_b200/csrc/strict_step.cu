@@ -422,11 +422,19 @@ constexpr uint32_t SS_MAX_ROWS = 16;
 // A cluster reads every weight through 16 SMs: beyond this many bytes of one layer the launches of strict.cu, which use all SMs, are faster.
 constexpr uint64_t SS_MAX_LAYER_BYTES = 4u << 20;
 
+// Attention is a (row, head) per CTA at a time, where the launches of strict.cu give every query an SM's share: a longer chunk of few sessions
+// with more than four of them per CTA loses once the keys take longer than the launches (8 heads of 8, one session, 16 ids, four layers, us here /
+// there: 128 keys 223 / 228, 272 keys 270 / 257, 1024 keys 508 / 362, 4096 keys 1515 / 815; 8 ids, 1024 keys 296 / 360).
+constexpr uint32_t SS_MAX_QUERIES = 4 * SS_CTAS, SS_MANY_KEYS = 128;
+
 bool strict_step_supported(const StrictStepArgs& a, bool kv_bf16) {
     if (!a.num_layers || a.num_layers > SS_MAX_LAYERS || a.d > SS_MAX_D || a.d % 4 || a.f % 4 || a.d % a.heads || (a.d / a.heads) % 4) return false;
     if ((4ull * a.d * a.d + 2ull * a.d * a.f) * 4 > SS_MAX_LAYER_BYTES || a.capacity > 16384) return false;
     const int at_once = kv_bf16 ? clusters_at_once<bf16>() : clusters_at_once<float>();
-    return at_once > 0 && (uint64_t)ceil_div(a.sessions, (uint32_t)at_once) * a.chunk <= std::min(SS_MAX_ROWS, rows_that_fit(a));
+    if (at_once <= 0) return false;
+    const uint64_t rows = (uint64_t)ceil_div(a.sessions, (uint32_t)at_once) * a.chunk;
+    if (a.chunk >= 8 && rows * a.heads > SS_MAX_QUERIES && a.position + a.chunk > SS_MANY_KEYS) return false;
+    return rows <= std::min(SS_MAX_ROWS, rows_that_fit(a));
 }
 
 // Largest vocabulary whose output head is part of the launch.
