@@ -754,10 +754,10 @@ def test_strict_step_in_one_launch_has_the_bits_of_the_operators(vocab, batch, w
 
 @pytest.mark.parametrize("batch,parts", [(128, 2), (192, 4)])
 def test_ranges_of_a_divided_step_keep_the_tcgen05_products(batch, parts):
-    """More than 32 rows in a range: products on register operands do not fit beside the other range's attention.  The sums are the tcgen05
-    engine's, bit for bit."""
+    """More than 32 rows in a range: products on register operands with more than small matrices do not fit beside the other range's attention.
+    The sums are the tcgen05 engine's, bit for bit."""
     from tnsr_b200 import _native
-    cfg = GptConfig(vocab_size=2048, max_sequence_length=64, embed_dim=256, num_heads=4, feed_forward_dim=512, num_layers=2,
+    cfg = GptConfig(vocab_size=2048, max_sequence_length=64, embed_dim=768, num_heads=12, feed_forward_dim=1024, num_layers=2,
                     layer_norm_epsilon=1e-5, activation="swiglu", weight_dtype="bf16")
     arrays = normal_model_arrays(cfg, seed=57, std=0.05)
     ids = np.random.default_rng(58).integers(0, cfg.vocab_size, size=(batch, 12)).astype(np.uint32)

@@ -871,7 +871,8 @@ static int launch_gemm_impl(const bf16* a, const bf16* bt, void* out, uint32_t l
     // In a divided step its CTAs (a block per SM from 17 rows on, up to 64 KB) have to find room beside the other ranges' scan: with more than
     // 32 rows in a range they wait longer than they save (4 layers of 768, 700 keys, us per step without / with them: 2 ranges of 64 392 / 437,
     // 4 of 64 604 / 740, 4 of 48 534 / 617; with up to 32 they gain: 2 ranges of 32 337 / 289, 4 of 24 436 / 431).
-    const bool crowded = ep.beside && m > 32;
+    // Matrices that gain at 128 rows are small enough to find it.
+    const bool crowded = ep.beside && m > 32 && !gemm_few_pays(a, bt, 128, n, k);
     if (!split_req && mode != GEMM_ARGMAX && g_gemm_engine == 0 && !ep.round_bf16 && !t_lose_gemm_stage && !narrow && !crowded &&
         gemm_few_pays(a, bt, m, n, k))
         return launch_gemm_few(a, bt, P, k, mode, stream);
