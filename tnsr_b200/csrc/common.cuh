@@ -140,6 +140,7 @@ struct GemmEpilogue {
     float* split_partials = nullptr;
     uint32_t split_k = 0;
     uint32_t split_rows = 0;
+    bool single = false;              // a call of its own (the C ABI's operators), not one of a session's chain of launches
     bool beside = false;              // another range of a divided step runs its attention on the same SMs meanwhile
 };
 

@@ -867,7 +867,7 @@ static int launch_gemm_impl(const bf16* a, const bf16* bt, void* out, uint32_t l
     // matrix with a long k, whose tiles do not give every SM one: outside a session's chain of launches, in which the weights are on their way
     // before the previous kernel ends, streaming is the faster form (us here / there, 2048 x 4096: 1 row 9.8 / 8.7, 8 rows 9.9 / 9.5;
     // 2048 x 5632: 12.9 / 11.2, 13.1 / 12.3; 2048 x 2048: 6.2 / 5.6, 6.2 / 6.4).
-    const bool narrow = streams && !t_pdl && m <= (k >= 4096 ? 8u : 4u) && n > 1024 && n <= 2304;
+    const bool narrow = streams && ep.single && m <= (k >= 4096 ? 8u : 4u) && n > 1024 && n <= 2304;
     // In a divided step its CTAs (a block per SM from 17 rows on, up to 64 KB) have to find room beside the other ranges' scan: with more than
     // 32 rows in a range they wait longer than they save (4 layers of 768, 700 keys, us per step without / with them: 2 ranges of 64 392 / 437,
     // 4 of 64 604 / 740, 4 of 48 534 / 617; with up to 32 they gain: 2 ranges of 32 337 / 289, 4 of 24 436 / 431).

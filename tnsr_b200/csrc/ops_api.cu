@@ -64,6 +64,7 @@ int tnsr_b200_gemm_bf16_ws(const void* a, const void* bt, const float* bias, con
     ep.ldr = n;
     ep.activation = activation;
     ep.out_dtype = out_dtype;
+    ep.single = true;
     if (workspace) {
         if (workspace_bytes < gemm_skinny_workspace_bytes() || (reinterpret_cast<uintptr_t>(workspace) & 15))
             return bad("gemm_bf16_ws: workspace too small or not 16-byte aligned");
@@ -107,6 +108,7 @@ int tnsr_b200_swiglu_mlp(const void* x, const void* w_gate_up_t, const float* b_
     GemmEpilogue ed;
     ed.bias = b_down;
     ed.out_dtype = TNSR_B200_BF16;
+    ed.single = true;
     return launch_gemm_bf16((const bf16*)hidden, (const bf16*)w_down_t, out, d, rows, d, f, GEMM_PLAIN, ed, nullptr, nullptr,
                             as_stream(stream));
 }
