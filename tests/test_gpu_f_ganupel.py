@@ -104,7 +104,7 @@ def run_attention(q, k, v, bias, positions, scale, window, dtype, engine=0, work
     size = lib().tnsr_b200_grouped_attention_workspace(dim, vdim)
     ws = torch.zeros(size, dtype=torch.uint8, device="cuda")
     d = [dev(x.astype(np.float32), TORCH[dtype]) for x in (q, k, v)]
-    b = dev(np.asarray(bias, np.float32))
+    b = dev(np.asarray(bias, np.float32)) if kind == "sigmoid" else None
     args = _native.GroupedAttentionArgs(d[0].data_ptr(), d[1].data_ptr(), d[2].data_ptr(), None, out.data_ptr(), ws.data_ptr() if workspace else None, None,
                                         size if workspace else 0, heads, kv_heads, dim, vdim, capacity, 0, out_ld, out_cols, scale, 0.0, dtype, engine,
                                         b.data_ptr() if kind == "sigmoid" else None, window, _native.SCORE[kind], gain, 0)
@@ -116,6 +116,28 @@ def run_attention(q, k, v, bias, positions, scale, window, dtype, engine=0, work
     assert np.array_equal(results[0], results[1])
     assert np.all(results[0][:, heads * vdim:out_cols] == 0.0) and np.all(results[0][:, out_cols:] == 7.0)
     return results[0][:, :heads * vdim].reshape(s, chunk, heads, vdim) / gain
+
+
+@pytest.mark.parametrize("dim", [16, 64, 128, 256])
+@pytest.mark.parametrize("chunk", [5, 130])
+def test_softmax_weights_of_24_bits(dim, chunk):
+    """Engine 3.  Two keys of nearly the same weight and opposite values under a third, heavier one without a value: what is left of the sum is
+    the difference of the two weights, 2^-12 of them.  Weights of 16 bits leave it off by up to 2^-17 / 2^-12, a thirty-second; of 24 bits by
+    the errors of the two scores and of exp2, 2^-20 / 2^-12 together, and by the rounding of the result, 2^-9: below 1 / 128."""
+    heads, position = 2, 20
+    q, k, v = np.zeros((1, chunk, heads, dim)), np.full((1, position + chunk, heads, dim), 0.0), np.zeros((1, position + chunk, heads, dim))
+    q[..., 0] = bf16_exact(np.linspace(0.3, 3.0, chunk * heads).astype(np.float32)).reshape(1, chunk, heads)
+    q[..., 1] = 1.0
+    k[..., 0] = -60.0                         # keys that weigh nothing
+    k[:, :3, :, 0] = [[0.0], [-1.0], [-1.0]]
+    k[:, 2, :, 1] = -2.0 ** -12
+    v[:, 1], v[:, 2] = 1.0, -1.0
+    got = run_attention(q, k, v, None, [position], 1.0, 0, BF16, engine=3, gain=1.0, kind="softmax")
+    weights = np.exp(np.einsum("sqhd,skhd->shqk", q, k))
+    for t in range(chunk):
+        weights[:, :, t, position + t + 1:] = 0.0
+    want = np.einsum("shqk,skhd->sqhd", weights / weights.sum(-1, keepdims=True), v)
+    assert np.max(np.abs(got / want - 1.0)) <= 1 / 128
 
 
 def attention_case(seed, positions, chunk, capacity, heads, kv_heads, dim, vdim, planted=None):

@@ -391,9 +391,9 @@ int layers_bf16(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chunk
                                               dec->d_status, st));
         } else if (chunk > 1 && hd <= 256 && c.prefill_mode != TNSR_B200_PREFILL_SCALAR) {
             // Paged caches and head widths other than 64: the kernels of described models, with one query head per
-            // key/value head (K/V tiles through shared memory, weights as two bf16 halves, so no bits of them are lost).
-            // The scan below reads every key once per query; 5 x 777 ids, 12 x 64 heads, pages of 64 rows, one layer on
-            // B200: 2796 us there, 51 us here.
+            // key/value head (K/V tiles through shared memory).  The scan below holds its weights in f32, so they enter the
+            // value product as three bf16 pieces here, which is all of their bits.  It reads every key once per query; 5 x 777
+            // ids, 12 x 64 heads, pages of 64 rows, one layer on B200: 2672 us there, 77 us here (69 with two pieces).
             GroupedAttention ga;
             ga.q = q; ga.k_cache = kcache; ga.v_cache = vcache; ga.out = att;
             ga.heads = ga.kv_heads = H; ga.dim = ga.vdim = hd; ga.capacity = c.capacity;
@@ -402,7 +402,7 @@ int layers_bf16(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chunk
             ga.paging = pg;
             ga.workspace = dec->grouped_ws; ga.workspace_bytes = dec->grouped_ws_bytes;
             ga.d_status = dec->d_status;
-            ga.engine = 2;
+            ga.engine = 3;
             StepPlace place;
             place.sessions = ns; place.chunk = chunk; place.position = position; place.d_position = d_position;
             RUN(dec, launch_grouped_attention(ga, place, TNSR_B200_BF16, st));

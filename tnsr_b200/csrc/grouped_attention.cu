@@ -12,8 +12,8 @@
 //  * grouped_tile_kernel    many rows (prefill): 64 rows per CTA, all warps share double-buffered key tiles.
 // Prefill with heads of 64 at a position the host knows runs on the tcgen05 kernel of prefill_tc.cu instead.
 //
-// Scores, softmax statistics and accumulators are f32; the weights enter the value product as two bf16 halves
-// (split_bf16x2), so they keep 16 bits.  A capped score costs three special-function results instead of one:
+// Scores, softmax statistics and accumulators are f32; the weights enter the value product as PARTS bf16 pieces: two, so they keep 16 bits, or
+// (engine 3, for callers whose weights were f32 all along) three, so they keep all 24.  A capped score costs three special-function results instead of one:
 // cap tanh(u) = cap (1 - 2 / (1 + exp(2u))).  Sigmoid weights (SIGMOID) need neither maximum nor sum: partial results of
 // warps and splits are added as they are.  With a window, tiles before the first row's window are never read.
 #include <algorithm>
@@ -99,7 +99,7 @@ struct SplitShape {
 };
 
 // UPPER: rows 8 .. 15 of the tile are in use (more than 8 rows).
-template <int DK, int DV, int STAGES, bool UPPER, bool SIGMOID>
+template <int DK, int DV, int STAGES, bool UPPER, bool SIGMOID, int PARTS>
 __global__ void __launch_bounds__(GA_WARPS * 32)
 grouped_split_kernel(GaParams P) {
     using S = SplitShape<DK, DV, STAGES>;
@@ -194,7 +194,7 @@ grouped_split_kernel(GaParams P) {
         for (int n = 0; n < 2; ++n)
 #pragma unroll
             for (int e = 0; e < 4; ++e) sc[n][e] += odd[n][e];
-        uint32_t hi[4] = {0u, 0u, 0u, 0u}, lo[4] = {0u, 0u, 0u, 0u};
+        uint32_t wt[PARTS][4] = {};
         if (SIGMOID) {
 #pragma unroll
             for (int n = 0; n < 2; ++n) {
@@ -205,8 +205,8 @@ grouped_split_kernel(GaParams P) {
                     const bool seen = key <= (e < 2 ? lim0 : lim1) && key >= (e < 2 ? low0 : low1);
                     w[e] = seen ? ga_sigmoid(sc[n][e], P.score.pre, e < 2 ? bias0 : bias1) : 0.0f;
                 }
-                split_bf16x2(w[0], w[1], hi[2 * n], lo[2 * n]);
-                if (UPPER) split_bf16x2(w[2], w[3], hi[2 * n + 1], lo[2 * n + 1]);
+                split_bf16_parts(w[0], w[1], wt, 2 * n);
+                if (UPPER) split_bf16_parts(w[2], w[3], wt, 2 * n + 1);
             }
         } else {
         float mx0 = m0, mx1 = m1;
@@ -237,11 +237,11 @@ grouped_split_kernel(GaParams P) {
         for (int n = 0; n < 2; ++n) {
             const float pa = mx_ex2(sc[n][0] - ms0), pb = mx_ex2(sc[n][1] - ms0);
             r0 += pa + pb;
-            split_bf16x2(pa, pb, hi[2 * n], lo[2 * n]);
+            split_bf16_parts(pa, pb, wt, 2 * n);
             if (UPPER) {
                 const float pc = mx_ex2(sc[n][2] - ms1), pd = mx_ex2(sc[n][3] - ms1);
                 r1 += pc + pd;
-                split_bf16x2(pc, pd, hi[2 * n + 1], lo[2 * n + 1]);
+                split_bf16_parts(pc, pd, wt, 2 * n + 1);
             }
         }
         l0 = l0 * c0 + r0;
@@ -249,7 +249,7 @@ grouped_split_kernel(GaParams P) {
 #pragma unroll
         for (int n = 0; n < DV / 8; ++n) { o[n][0] *= c0; o[n][1] *= c0; if (UPPER) { o[n][2] *= c1; o[n][3] *= c1; } }
         }
-        // 64 columns at a time, the two halves of a weight eight products apart: one accumulator's products wait for each other
+        // 64 columns at a time, the pieces of a weight eight products apart: one accumulator's products wait for each other
 #pragma unroll
         for (int n0 = 0; n0 < DV / 16; n0 += 4) {
             uint32_t b[4][4];
@@ -257,15 +257,12 @@ grouped_split_kernel(GaParams P) {
             for (int n = 0; n < 4; ++n)
                 mx_ldsm_t(sv + ((lane & 7) + ((lane >> 3) & 1) * 8) * S::VP + ((n0 + n) * 16 + (lane >> 4) * 8) * 2, b[n]);
 #pragma unroll
-            for (int n = 0; n < 4; ++n) {
-                mx_mma(o[2 * (n0 + n)], hi, b[n][0], b[n][1]);
-                mx_mma(o[2 * (n0 + n) + 1], hi, b[n][2], b[n][3]);
-            }
+            for (int part = 0; part < PARTS; ++part)
 #pragma unroll
-            for (int n = 0; n < 4; ++n) {
-                mx_mma(o[2 * (n0 + n)], lo, b[n][0], b[n][1]);
-                mx_mma(o[2 * (n0 + n) + 1], lo, b[n][2], b[n][3]);
-            }
+                for (int n = 0; n < 4; ++n) {
+                    mx_mma(o[2 * (n0 + n)], wt[part], b[n][0], b[n][1]);
+                    mx_mma(o[2 * (n0 + n) + 1], wt[part], b[n][2], b[n][3]);
+                }
         }
         __syncwarp();    // every lane is done with the stage that the next load may overwrite
         load(i + (STAGES - 1) * GA_WARPS, (stage + STAGES - 1) % STAGES);
@@ -368,7 +365,7 @@ struct TileShape {
     static constexpr uint32_t BYTES = Q_BYTES + 2 * (K_BYTES + V_BYTES);
 };
 
-template <int DK, int DV, int BK, bool SIGMOID>
+template <int DK, int DV, int BK, bool SIGMOID, int PARTS>
 __global__ void __launch_bounds__(128)
 grouped_tile_kernel(GaParams P) {
     using S = TileShape<DK, DV, BK>;
@@ -507,15 +504,15 @@ grouped_tile_kernel(GaParams P) {
             }
 #pragma unroll
             for (int kk = 0; kk < BK / 16; ++kk) {
-                uint32_t hi[4], lo[4];
+                uint32_t wt[PARTS][4];
 #pragma unroll
                 for (int n = 0; n < 2; ++n) {
                     const float* v = sc[2 * kk + n];
                     const float pa = SIGMOID ? v[0] : mx_ex2(v[0] - ms0), pb = SIGMOID ? v[1] : mx_ex2(v[1] - ms0);
                     const float pc = SIGMOID ? v[2] : mx_ex2(v[2] - ms1), pd = SIGMOID ? v[3] : mx_ex2(v[3] - ms1);
                     if (!SIGMOID) { l0 += pa + pb; l1 += pc + pd; }
-                    split_bf16x2(pa, pb, hi[2 * n], lo[2 * n]);
-                    split_bf16x2(pc, pd, hi[2 * n + 1], lo[2 * n + 1]);
+                    split_bf16_parts(pa, pb, wt, 2 * n);
+                    split_bf16_parts(pc, pd, wt, 2 * n + 1);
                 }
 #pragma unroll
                 for (int n0 = 0; n0 < DV / 16; n0 += 4) {
@@ -524,15 +521,12 @@ grouped_tile_kernel(GaParams P) {
                     for (int n = 0; n < 4; ++n)
                         mx_ldsm_t(sv + (kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * S::VP + ((n0 + n) * 16 + (lane >> 4) * 8) * 2, bb[n]);
 #pragma unroll
-                    for (int n = 0; n < 4; ++n) {
-                        mx_mma(o[2 * (n0 + n)], hi, bb[n][0], bb[n][1]);
-                        mx_mma(o[2 * (n0 + n) + 1], hi, bb[n][2], bb[n][3]);
-                    }
+                    for (int part = 0; part < PARTS; ++part)
 #pragma unroll
-                    for (int n = 0; n < 4; ++n) {
-                        mx_mma(o[2 * (n0 + n)], lo, bb[n][0], bb[n][1]);
-                        mx_mma(o[2 * (n0 + n) + 1], lo, bb[n][2], bb[n][3]);
-                    }
+                        for (int n = 0; n < 4; ++n) {
+                            mx_mma(o[2 * (n0 + n)], wt[part], bb[n][0], bb[n][1]);
+                            mx_mma(o[2 * (n0 + n) + 1], wt[part], bb[n][2], bb[n][3]);
+                        }
                 }
             }
         }
@@ -581,35 +575,37 @@ int allow_smem(K kernel, uint32_t bytes, bool* configured) {
     return TNSR_B200_OK;
 }
 
-template <int DK, int DV, int STAGES, bool UPPER, bool SIGMOID>
+template <int DK, int DV, int STAGES, bool UPPER, bool SIGMOID, int PARTS>
 int launch_split_kind(const GaParams& P, cudaStream_t stream) {
     static bool configured[64] = {};
     const uint32_t bytes = SplitShape<DK, DV, STAGES>::BYTES;
-    int rc = allow_smem(grouped_split_kernel<DK, DV, STAGES, UPPER, SIGMOID>, bytes, configured);
+    int rc = allow_smem(grouped_split_kernel<DK, DV, STAGES, UPPER, SIGMOID, PARTS>, bytes, configured);
     if (rc) return rc;
-    launch_kernel(grouped_split_kernel<DK, DV, STAGES, UPPER, SIGMOID>, dim3(P.splits, P.a.kv_heads * P.row_tiles, P.place.sessions), dim3(GA_WARPS * 32), bytes,
-                  stream, P);
+    launch_kernel(grouped_split_kernel<DK, DV, STAGES, UPPER, SIGMOID, PARTS>, dim3(P.splits, P.a.kv_heads * P.row_tiles, P.place.sessions), dim3(GA_WARPS * 32),
+                  bytes, stream, P);
     return TNSR_B200_OK;
 }
 
 template <int DK, int DV, int STAGES, bool UPPER>
 int launch_split(const GaParams& P, cudaStream_t stream) {
-    return P.a.score_kind == TNSR_B200_SCORE_SIGMOID ? launch_split_kind<DK, DV, STAGES, UPPER, true>(P, stream) : launch_split_kind<DK, DV, STAGES, UPPER, false>(P, stream);
+    if (P.a.score_kind == TNSR_B200_SCORE_SIGMOID) return launch_split_kind<DK, DV, STAGES, UPPER, true, 2>(P, stream);
+    return P.a.engine == 3 ? launch_split_kind<DK, DV, STAGES, UPPER, false, 3>(P, stream) : launch_split_kind<DK, DV, STAGES, UPPER, false, 2>(P, stream);
 }
 
-template <int DK, int DV, int BK, bool SIGMOID>
+template <int DK, int DV, int BK, bool SIGMOID, int PARTS>
 int launch_tile_kind(const GaParams& P, cudaStream_t stream) {
     static bool configured[64] = {};
     const uint32_t bytes = TileShape<DK, DV, BK>::BYTES;
-    int rc = allow_smem(grouped_tile_kernel<DK, DV, BK, SIGMOID>, bytes, configured);
+    int rc = allow_smem(grouped_tile_kernel<DK, DV, BK, SIGMOID, PARTS>, bytes, configured);
     if (rc) return rc;
-    launch_kernel(grouped_tile_kernel<DK, DV, BK, SIGMOID>, dim3(P.row_tiles, P.a.kv_heads, P.place.sessions), dim3(128), bytes, stream, P);
+    launch_kernel(grouped_tile_kernel<DK, DV, BK, SIGMOID, PARTS>, dim3(P.row_tiles, P.a.kv_heads, P.place.sessions), dim3(128), bytes, stream, P);
     return TNSR_B200_OK;
 }
 
 template <int DK, int DV, int BK>
 int launch_tile(const GaParams& P, cudaStream_t stream) {
-    return P.a.score_kind == TNSR_B200_SCORE_SIGMOID ? launch_tile_kind<DK, DV, BK, true>(P, stream) : launch_tile_kind<DK, DV, BK, false>(P, stream);
+    if (P.a.score_kind == TNSR_B200_SCORE_SIGMOID) return launch_tile_kind<DK, DV, BK, true, 2>(P, stream);
+    return P.a.engine == 3 ? launch_tile_kind<DK, DV, BK, false, 3>(P, stream) : launch_tile_kind<DK, DV, BK, false, 2>(P, stream);
 }
 
 uint32_t padded_width(uint32_t dim, uint32_t vdim) {

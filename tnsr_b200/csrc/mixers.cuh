@@ -74,7 +74,8 @@ struct GroupedAttention {
     void* workspace = nullptr;            // grouped_attention_workspace_bytes(), zeroed once
     uint64_t workspace_bytes = 0;
     int* d_status = nullptr;              // device status word (a bounded wait of the tcgen05 kernel gave up), may be null
-    int engine = 0;                       // 0: best kernel for the shape, 1: one warp per (row, head), 2: not the tcgen05 kernel
+    int engine = 0;                       // 0: best kernel for the shape, 1: one warp per (row, head), 2: not the tcgen05 kernel,
+                                          // 3: as 2, and softmax weights keep their 24 bits
 };
 uint64_t grouped_attention_workspace_bytes(uint32_t dim, uint32_t vdim);
 int launch_grouped_attention(const GroupedAttention& a, const StepPlace& place, int dtype, cudaStream_t stream);
@@ -258,6 +259,17 @@ __device__ __forceinline__ void split_bf16x2(float x, float y, uint32_t& hi, uin
     hi = pack_bf16x2(x, y);
     const float2 h = bf16x2_to_f32(hi);
     lo = pack_bf16x2(x - h.x, y - h.y);
+}
+// The same into PARTS pieces, element `at` of each: 8 bits of the value a piece, all 24 of an f32 in three.
+template <int PARTS>
+__device__ __forceinline__ void split_bf16_parts(float x, float y, uint32_t (&w)[PARTS][4], int at) {
+#pragma unroll
+    for (int i = 0; i < PARTS; ++i) {
+        w[i][at] = pack_bf16x2(x, y);
+        const float2 h = bf16x2_to_f32(w[i][at]);
+        x -= h.x;
+        y -= h.y;
+    }
 }
 #endif  // __CUDACC__
 
