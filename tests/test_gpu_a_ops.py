@@ -232,7 +232,7 @@ def test_gemm_bf16_register_engine_matches_f64(shape):
 
 
 @pytest.mark.parametrize("engine,shape", [(2, (32, 6144, 512)), (2, (32, 8192, 2048)), (2, (24, 16384, 1024)), (2, (17, 32000, 256)), (2, (48, 3072, 512)),
-                                          (2, (64, 3072, 512)), (2, (56, 4096, 256)), (4, (1, 2048, 4096)), (4, (8, 1536, 4096)), (4, (4, 2304, 2048))])
+                                          (2, (64, 3072, 512)), (2, (56, 4096, 256)), (2, (24, 6144, 768)), (4, (1, 2048, 4096)), (4, (8, 1536, 4096)), (4, (4, 2304, 2048))])
 def test_gemm_bf16_sizes_that_keep_the_other_engines(engine, shape):
     """Sizes at which operands on registers are the slower form: the sums of the tcgen05 engine, or of the one that streams the weights, bit for
     bit (each of the three adds in another order)."""

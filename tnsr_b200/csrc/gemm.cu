@@ -863,20 +863,22 @@ static int launch_gemm_impl(const bf16* a, const bf16* bt, void* out, uint32_t l
         }
     }
     const bool streams = !split_req && mode == GEMM_PLAIN && m <= 16 && (uint64_t)n * k >= (4ull << 20) && gemm_stream_eligible(a, bt, m, n, k, ep);
-    // Few rows: operands straight into registers (gemm_few.cu; not where a test asks this engine to lose a stage).  The exception is a narrow
-    // matrix with a long k, whose tiles do not give every SM one: outside a session's chain of launches, in which the weights are on their way
-    // before the previous kernel ends, streaming is the faster form (us here / there, 2048 x 4096: 1 row 9.8 / 8.7, 8 rows 9.9 / 9.5;
-    // 2048 x 5632: 12.9 / 11.2, 13.1 / 12.3; 2048 x 2048: 6.2 / 5.6, 6.2 / 6.4).
-    const bool narrow = streams && ep.single && m <= (k >= 4096 ? 8u : 4u) && n > 1024 && n <= 2304;
+    // Few rows: operands straight into registers (gemm_few.cu; not where a test asks this engine to lose a stage).  The exceptions are calls
+    // outside a session's chain of launches, in which the weights are on their way before the previous kernel ends: a narrow matrix with a
+    // long k, whose tiles do not give every SM one, is faster streamed (us here / there, 2048 x 4096: 1 row 9.8 / 8.7, 8 rows 9.9 / 9.5;
+    // 2048 x 5632: 12.9 / 11.2, 13.1 / 12.3; 2048 x 2048: 6.2 / 5.6, 6.2 / 6.4), and a wide one with a short k in tcgen05 tiles (6144 x 768:
+    // 17 rows 10.7 / 9.9, 31 rows 11.5 / 10.6).
+    const bool narrow = ep.single && streams && m <= (k >= 4096 ? 8u : 4u) && n > 1024 && n <= 2304;
+    const bool wide = ep.single && m > 16 && n > 32 * 148 && k < 1024;
     // In a divided step its CTAs (a block per SM from 17 rows on, up to 64 KB) have to find room beside the other ranges' scan: with more than
     // 32 rows in a range they wait longer than they save (4 layers of 768, 700 keys, us per step without / with them: 2 ranges of 64 392 / 437,
     // 4 of 64 604 / 740, 4 of 48 534 / 617; with up to 32 they gain: 2 ranges of 32 337 / 289, 4 of 24 436 / 431).
     // Matrices that gain at 128 rows are small enough to find it.
     const bool crowded = ep.beside && m > 32 && !gemm_few_pays(a, bt, 128, n, k);
-    if (!split_req && mode != GEMM_ARGMAX && g_gemm_engine == 0 && !ep.round_bf16 && !t_lose_gemm_stage && !narrow && !crowded &&
+    if (!split_req && mode != GEMM_ARGMAX && g_gemm_engine == 0 && !ep.round_bf16 && !t_lose_gemm_stage && !narrow && !wide && !crowded &&
         gemm_few_pays(a, bt, m, n, k))
         return launch_gemm_few(a, bt, P, k, mode, stream);
-    // What is left of few rows (k no multiple of 16, pointers of 16-byte alignment, the exception, a lost stage to provoke):
+    // What is left of few rows (k no multiple of 16, pointers of 16-byte alignment, the exceptions, a lost stage to provoke):
     // a handful of rows against a large weight matrix: stream the weights with the operands swapped (gemm_skinny.cu)
     // when that engine can fill the GPU, i.e. with split-K scratch lent by the caller or with at least half as many
     // 128-column tiles as SMs.  Measured inside a CUDA graph, 4096 x 4096 weights: 14.8 / 16.3 us at 1 / 8 rows against

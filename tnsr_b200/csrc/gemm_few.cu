@@ -296,7 +296,8 @@ int launch_rows(const FewParams& P, cudaStream_t stream) {
 // rows) has to hold the matrix, unless a long k makes up for it; past 64 rows only a matrix that is small altogether gains.  What that
 // leaves to the tcgen05 engine, us here / there, and two that stay:
 //     32 rows: 6144 x 512  10.4 / 8.6     6144 x 2048  19.6 / 15.5    16384 x 1024  22.3 / 14.0    32000 x 512  31.5 / 14.4
-//     24 rows: 8192 x 256   8.2 / 7.4     6144 x 768   10.9 / 10.3;   8192 x 1024   12.2 / 14.1 stays
+//     24 rows: 8192 x 256   8.2 / 7.4;    8192 x 1024  12.2 / 14.1 stays, and 6144 x 768 10.9 / 10.3 in a session, where the weights are
+//              on their way before the previous kernel ends (Bolonex, 24 sessions: a request 7.65 ms with, 7.84 ms without)
 //     64 rows: 3072 x 512   8.8 / 6.6     4096 x 512    9.3 / 7.3;    2304 x 512     5.7 / 6.5  stays
 // At most 16 rows gain at nearly any size against the streaming engine: 8 and 16 rows of 32000 x 768 19.9 / 27.7 and 20.6 / 31.0, of
 // 8192 x 8192 40.6 / 53.2 and 45.5 / 44.4, of 28672 x 4096 70.6 / 86.1 and 76.6 / 92.2 (launch_gemm_impl has the exception).  The 768 x 768
@@ -306,7 +307,7 @@ bool gemm_few_pays(const bf16* a, const bf16* w, uint32_t m, uint32_t n, uint32_
     if (reinterpret_cast<uintptr_t>(a) % 32 != 0 || reinterpret_cast<uintptr_t>(w) % 32 != 0) return false;
     const uint64_t weights = (uint64_t)n * k;
     if (m <= 16) return true;
-    if (m <= 32) return weights <= (17ull << 20) && (n <= 32 * 148 || (m < 32 && n <= 8192 && k >= 1024));
+    if (m <= 32) return weights <= (17ull << 20) && (n <= 32 * 148 || (m < 32 && n <= 8192 && k >= 768));
     if (m <= 64 && n <= 1024) return true;
     if (m <= 48 && weights <= (3ull << 20)) return n <= 16 * 148 || k >= 768;
     if (m <= 64 && weights <= (2ull << 20)) return n <= 16 * 148;
