@@ -582,7 +582,8 @@ static bool launch_strict_tile_attention(const float* q, const void* kc, const v
 
 // Queries of a block of the tiled kernel, or 0: the kernel above, with a block per query.  A tile reads every key once for its queries, but its
 // block walks all their chains: it pays when there are more queries than the GPU takes side by side, the more so the wider the head (below 32
-// columns most of a block's lanes idle; there long rows of scores, which leave room for a block or two per SM, lose at any number).  32
+// columns most of a block's lanes idle).  Long rows of scores leave room for a block or two per SM: the tiles then run in waves, which
+// have to be full (16 sessions of 4 x 32, 17 ids, 4049 keys: 3889 / 5451 us), and below 32 columns they lose at any number.  32
 // queries instead of 8 need shared memory for their scores and a chunk that fills them.  Measured on B200 over 2862 chunks (widths 8 to
 // 128, 1 to 64 sessions, 2 to 256 ids, up to 4096 keys): none more than 6 % slower than the other kernel.  Four layers, us per block and query /
 // in tiles of 8 / of 32:
@@ -595,6 +596,7 @@ static uint32_t strict_tile_queries(uint64_t units, uint32_t chunk, uint32_t hd,
     if (chunk < 2 || hd > 128) return 0;
     const uint64_t queries = units * chunk;
     if (hd >= 32 ? queries < (chunk >= 8 ? 1024 : 1536) : chunk < 8 || longest > 2048 || queries < (hd >= 16 ? 1536 : 2048)) return 0;
+    if (longest > 2048 && queries < 962 * ceil_div64(units * ceil_div(chunk, 8u), 148)) return 0;      // of a wave's 148 x 8
     return chunk >= 32 && queries >= 8192 && longest <= 640 ? 32 : 8;
 }
 
