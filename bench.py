@@ -85,7 +85,7 @@ def parse_args():
                          "restatement timed beside it (1 GPU)")
     ap.add_argument("--samples", type=int, default=20, help="timed launches per case of the operator workloads")
     ap.add_argument("--step-parts", type=int, default=0, help="session configuration: parts a single-token step is divided into (0 = automatic)")
-    ap.add_argument("--small-batch-mode", type=int, default=0, help="session configuration: 1 = operator-by-operator step also at <= 64 sessions")
+    ap.add_argument("--small-batch-mode", type=int, default=0, help="session configuration: 0 or 1, the same launches (chose between two forms of a small step once)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-e2e", action="store_true")
     return ap.parse_args()

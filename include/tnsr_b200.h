@@ -255,10 +255,10 @@ TNSR_B200_API uint64_t tnsr_b200_kernel_launches(void);
 /* GEMM engine of the bf16 path: 0 = tcgen05/TMEM kernel where the shape
  * allows it, else the CUDA-core kernel (default); 1 = always the CUDA-core
  * kernel; 2 = tcgen05 only (unsupported shapes fail); 3 = as 0, but products
- * of at most 64 rows always take the tcgen05 few-row engine with split-K (by
- * default only those shapes do for which it is the faster one); 4 = as 0, but
- * products of at most 16 rows always take the weight-streaming engine (by
- * default from 4 M weight elements up).  Process-wide.  Engine 1
+ * of at most 64 rows always take the tcgen05 few-row engine with split-K; 4 = as
+ * 0, but products of at most 16 rows always take the weight-streaming engine (by
+ * default few rows take their operands straight into registers, and these two
+ * what that engine leaves).  Process-wide.  Engine 1
  * also keeps prefill attention off tcgen05 (the warp-level mma.sync kernel
  * runs), which is how tests compare the two. */
 TNSR_B200_API int tnsr_b200_set_gemm_engine(int engine);
@@ -457,11 +457,13 @@ TNSR_B200_API int tnsr_b200_gemm_bf16(const void* a, const void* bt, const float
                                       const float* residual, void* out, uint32_t m, uint32_t n,
                                       uint32_t k, int activation, int out_dtype, void* stream);
 /* The same product with scratch lent by the caller (no reference counterpart).
- * It matters for m <= 64, where the weights are streamed once with the
- * operands of the MMA swapped: with scratch the K range of every 128-column
- * tile is divided over several CTAs so that all SMs pull on HBM, and the CTA
- * that finishes last adds the partial tiles in a fixed order (results do not
- * depend on timing).  `workspace`: tnsr_b200_gemm_workspace() bytes, 16-byte
+ * It matters for m <= 16 and large matrices that the engines for few rows do not
+ * take (k no multiple of 16, pointers that are not 32-byte aligned): there the
+ * weights are streamed once with the operands of the MMA swapped, and with scratch
+ * the K range of every 128-column tile is divided over several CTAs so that all
+ * SMs pull on HBM; the CTA that finishes last adds the partial tiles in a fixed
+ * order (results do not depend on timing).  Other shapes leave it alone.
+ * `workspace`: tnsr_b200_gemm_workspace() bytes, 16-byte
  * aligned, zeroed once before the first use (every launch that completes leaves
  * it zeroed; zero it again if a launch was cut short by a device error);
  * launches that may overlap on the GPU must not share it. */

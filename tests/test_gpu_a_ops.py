@@ -211,7 +211,7 @@ def test_gemm_bf16_epilogues(engine):
 def test_gemm_bf16_register_engine_matches_f64(shape):
     """Few rows, k a multiple of 16: 16 to 64 rows and 8 to 32 columns per CTA, k in blocks of 64 over eight warps and, for a narrow matrix with
     a long k, over the two CTAs of a cluster; ragged rows, columns and k, several column tiles per CTA.  f32 sums of exact products: 4e-6 k.
-    A row's bits do not depend on the rows beside it."""
+    Inside the engine a row's bits do not depend on the rows beside it (here: one row alone, and half of them)."""
     m, n, k = shape
     a, bt, ref = gemm_case(m, n, k, seed=21)
     rng = np.random.default_rng(22)
@@ -221,6 +221,8 @@ def test_gemm_bf16_register_engine_matches_f64(shape):
     plain = gemm_bf16(da, dbt)
     assert np.max(np.abs(plain.cpu().numpy() - ref)) <= tol
     assert torch.equal(plain[:1], gemm_bf16(da[:1].contiguous(), dbt))
+    half = da[m // 2:].clone()                 # rows of their own at an aligned address
+    assert torch.equal(plain[m // 2:], gemm_bf16(half, dbt))
     fused = gemm_bf16(da, dbt, bias=dbias, residual=dres).cpu().numpy()
     assert np.max(np.abs(fused - (ref + bias + resid))) <= tol + 1e-5
     relu = gemm_bf16(da, dbt, bias=dbias, activation=0, out_dtype=BF16).float().cpu().numpy()

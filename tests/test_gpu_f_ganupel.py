@@ -761,8 +761,9 @@ def test_unequal_sessions_slots_and_pages_used_again(paged, dtype):
 @pytest.mark.parametrize("sessions,tokens", [(1, 500), (2, 193), (3, 769)])
 def test_prompts_divided_in_time(shape, sessions, tokens):
     """A prompt of 192 tokens and more for few sessions is scanned in segments side by side.  Against the same model on portions too short to
-    be divided, which makes the same projections (their sums do not depend on the rows beside them): the state differs by the 16 bits
-    that a written k R keeps (other chunk borders) and by f32 sums in another order, the logits by bf16 roundings that fall the other way."""
+    be divided: the state differs by the 16 bits that a written k R keeps (other chunk borders) and by f32 sums in another order -- of the scan,
+    and of the projections where a portion of up to 128 rows takes the engine for few rows -- and the logits by bf16 roundings that
+    fall the other way."""
     cfg = config(128, 160, [parallel((2, 1, 16, 16, 8, 20, 0.2), shape)])
     _, _, model = build(cfg, "bf16")
     ids = np.stack([tokens_for(cfg, tokens + 40, seed=30 + b) for b in range(sessions)])

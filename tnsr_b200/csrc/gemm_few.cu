@@ -12,7 +12,7 @@
 //    memory.  With more column tiles than CTAs the next tile's weights are on their way while this one is added up and written;
 //  * K may be divided over a cluster of CTAs (ck): each takes in 1 / ck of the rows' and the weights' bytes, the partial tiles meet
 //    through distributed shared memory, added in rank order.
-// How K is divided depends on n and k only, so the bits of an element do not depend on how many rows share the call.
+// How K is divided depends on n and k only, so within this engine the bits of an element do not depend on how many rows share the call.
 #include <algorithm>
 #include <atomic>
 
