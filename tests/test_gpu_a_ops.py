@@ -315,6 +315,28 @@ def test_gemm_bf16_in_place_residual_update_equals_out_of_place(shape, activatio
     assert torch.equal(twice, again)
 
 
+@pytest.mark.parametrize("shape", [(400, 9448, 1544), (270, 9472, 1536), (1000, 9448, 1600),      # pairs of CTAs: ragged rows, columns and k,
+                                   (400, 6000, 264), (3885, 768, 776)])                        # an empty half, two tiles each; 192 columns
+@pytest.mark.parametrize("form", ["f32", "bf16", "residual"])
+def test_gemm_bf16_tiles_of_pairs_and_of_192_columns(shape, form):
+    m, n, k = shape
+    g = torch.Generator(device="cuda").manual_seed(41)
+    a, bt = (torch.randn(r, k, device="cuda", generator=g).to(torch.bfloat16) for r in (m, n))
+    bias, resid = torch.randn(n, device="cuda", generator=g), torch.randn(m, n, device="cuda", generator=g)
+    want = a.double() @ bt.double().T + bias
+    if form == "residual":
+        got = resid.clone()
+        ok(lib().tnsr_b200_gemm_bf16(ptr(a), ptr(bt), ptr(bias), ptr(got), ptr(got), m, n, k, -1, 0, stream()))
+        want += resid
+    else:
+        got = gemm_bf16(a, bt, bias=bias, out_dtype=BF16 if form == "bf16" else F32)
+    torch.cuda.synchronize()
+    # f32 sums of k products of size 1: k^1/2 * 2^-24 * a few.  Stored bf16 has 8 significant bits: half a unit in the last place is at most
+    # 2^-8 of the value, and the sum's own error may tip it over to the next one
+    err = (got.double() - want).abs() - (want.abs() * 2.0 ** -8 if form == "bf16" else 0.0)
+    assert float(err.max()) <= 2e-3
+
+
 # ---- SwiGLU ----------------------------------------------------------------------
 def test_swiglu_elementwise(oracle):
     import json, os

@@ -7,6 +7,7 @@
 
 #include <atomic>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/tnsr_b200.h"
@@ -78,20 +79,34 @@ extern thread_local bool t_single_token_step;
 // move in beside a CTA of another stream's kernel as soon as threads, registers and shared memory allow.
 void prefer_max_shared_carveout(const void* kernel);
 
+// `cluster`: CTAs of a cluster (1: none).
 template <typename... KArgs, typename... Args>
-inline void launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+inline void launch_kernel_clusters(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, uint32_t cluster, cudaStream_t stream, Args&&... args) {
     prefer_max_shared_carveout(reinterpret_cast<const void*>(kernel));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    uint32_t count = 0;
+    if (t_pdl) {
+        attr[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[count++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[count].id = cudaLaunchAttributeClusterDimension;
+        attr[count].val.clusterDim.x = cluster;
+        attr[count].val.clusterDim.y = 1;
+        attr[count++].val.clusterDim.z = 1;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = t_pdl ? 1 : 0;
+    cfg.numAttrs = count;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline void launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+    launch_kernel_clusters(kernel, grid, block, smem, 1, stream, std::forward<Args>(args)...);
 }
 
 inline uint32_t ceil_div(uint32_t a, uint32_t b) { return (a + b - 1) / b; }

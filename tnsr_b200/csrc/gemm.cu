@@ -2,8 +2,8 @@
 //
 // Two engines share one epilogue:
 //  * gemm_tc_kernel   -- the Blackwell path: TMA (cp.async.bulk.tensor, 128-byte
-//    swizzle, one copy per CTA, no cluster forms) feeds a shared-memory ring,
-//    one thread issues tcgen05.mma (M=128, N=BN, K=16 per instruction) into
+//    swizzle; long products in pairs of CTAs that share a tile) feeds a shared-memory ring,
+//    one thread issues tcgen05.mma (M=128 or a pair's 256, N=BN, K=16 per instruction) into
 //    double-buffered TMEM accumulators, eight epilogue warps drain them with
 //    tcgen05.ld, transpose each 32x32 block through shared memory and write
 //    coalesced rows while the next tile's main loop runs.  Persistent over tiles.
@@ -16,6 +16,7 @@
 // 487-646, src/ptx/graph/matmul.rs:4-129, src/tile/graph.rs:712-1107).
 #include <cuda.h>
 
+#include <algorithm>
 #include <mutex>
 #include <unordered_map>
 
@@ -136,34 +137,37 @@ constexpr int BK = 64;            // 64 bf16 = 128 bytes = one swizzle row
 constexpr int UMMA_K = 16;        // K per tcgen05.mma for 16-bit operands
 // Epilogue warps per CTA (template parameter EPI): 8 = two per TMEM lane quarter, 16 = four per quarter; the warps of a
 // quarter take 32-column chunks in turn.  Warp 0: TMA, warp 1: MMA + TMEM owner, warps 2 .. EPI + 1: epilogue.
+constexpr uint32_t TC_SMEM_MAX = 227 * 1024;
 constexpr uint32_t TC_STAGE_TILE_BYTES = 32 * 32 * 4;  // per-warp transpose buffer: 32 rows x 32 f32 columns
 
-template <int BN, int EPI>
+template <int BN, int EPI, int CG>
 struct TcShape {
     static constexpr int THREADS = 64 + 32 * EPI;
     // 4 stages of 48 KB at BN 256 with 8 epilogue warps; 3 with 16 (their transpose buffers take 64 KB).
     // EPI 4 is the lean form of the narrow tiles (few rows, one tile per CTA: the decode step): half the shared memory
     // (about 115 KB) and at most 112 registers x 192 threads, so that a CTA of it fits on an SM beside a CTA of the lean
     // decode-attention kernel that works on the other half of the batch.
-    static constexpr int STAGES = BN >= 256 ? (EPI > 8 ? 3 : 4) : (BN >= 128 ? 6 : (EPI == 4 ? (BN >= 64 ? 4 : 5) : 8));
+    // A pair of CTAs (CG 2) holds half of the columns' operand each: 6 stages of 32 KB, or 5 with 16 epilogue warps.
     static constexpr uint32_t A_BYTES = BM * BK * 2;
-    static constexpr uint32_t B_BYTES = BN * BK * 2;
+    static constexpr uint32_t B_BYTES = BN / CG * BK * 2;
     static constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
-    static constexpr uint32_t TMEM_COLS = 2 * BN < 32 ? 32 : 2 * BN;  // two accumulators; power of two
+    static constexpr int STAGES = CG == 2 || BN == 192 ? (int)((TC_SMEM_MAX - 1280 - EPI * TC_STAGE_TILE_BYTES) / STAGE_BYTES)
+                                  : BN >= 256 ? (EPI > 8 ? 3 : 4) : (BN >= 128 ? 6 : (EPI == 4 ? (BN >= 64 ? 4 : 5) : 8));
+    static constexpr uint32_t TMEM_COLS = BN == 192 ? 512 : 2 * BN < 32 ? 32 : 2 * BN;  // two accumulators; power of two
     static constexpr uint32_t SMEM_BYTES =
         STAGES * STAGE_BYTES + 1024 /* alignment slack */ + EPI * TC_STAGE_TILE_BYTES + 256 /* barriers */;
 };
 
 // Instruction descriptor, kind::f16: f32 accumulator (bit 4), bf16 A (bit 7)
 // and B (bit 10), both K-major (bits 15, 16 clear), N/8 at bit 17, M/16 at bit 24.
-__host__ __device__ constexpr uint32_t make_idesc_bf16(uint32_t bn) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+__host__ __device__ constexpr uint32_t make_idesc_bf16(uint32_t bm, uint32_t bn) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((bn >> 3) << 17) | ((bm >> 4) << 24);
 }
 
 struct TcParams {
     EpiParams epi;
     uint32_t k;
-    uint32_t tiles_m, tiles_n;
+    uint32_t tiles_m, tiles_n;   // tiles_m: row tiles of a CTA, or of a pair of CTAs
     int* d_status;
     // 1: f32 output accumulated in place on the residual (out == residual): the epilogue hands each 32 x 32 block of
     // act(acc + bias) to a TMA reduce-add on `map_out` instead of reading, adding and storing the rows itself
@@ -524,12 +528,15 @@ __device__ __forceinline__ void epilogue_block(const EpiParams& P, float* stage,
     __syncwarp();  // the buffer is reused by the next block
 }
 
-template <int BN, int MODE, int EPI>
+// CG: CTAs that share a tile.  A pair (CG 2, a cluster) takes 256 x BN: each CTA brings in its own 128 rows and half of the columns' operand,
+// the leader (rank 0) issues products of 256 rows that read both CTAs' shared memory and leave each CTA its 128 rows x BN columns in its own
+// TMEM.  Per CTA and k block that is 128 + BN / 2 rows through L2, TMA and shared memory instead of 128 + BN.
+template <int BN, int MODE, int EPI, int CG>
 __global__ void __launch_bounds__(64 + 32 * EPI, EPI == 4 ? 3 : 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_k,
                const __grid_constant__ CUtensorMap map_v, TcParams prm) {
-    using S = TcShape<BN, EPI>;
+    using S = TcShape<BN, EPI, CG>;
     constexpr bool PLAIN = MODE == GEMM_PLAIN || MODE == GEMM_SCALED;
     constexpr int PER_QUARTER = EPI / 4;             // epilogue warps per TMEM lane quarter
     constexpr uint32_t CHUNK_STRIDE = 32 * PER_QUARTER;
@@ -548,12 +555,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t split = (PLAIN && prm.tma_reduce == 2) ? prm.split_k : 1u;
     const uint32_t num_tiles = prm.tiles_m * prm.tiles_n * split;
+    const uint32_t rank = CG == 2 ? cluster_rank() : 0u, first_tile = blockIdx.x / CG, tile_step = gridDim.x / CG;
     const uint32_t num_kb = (prm.k + BK - 1) / BK;
     const uint32_t kb_per = (num_kb + split - 1) / split;    // the host picks split so that no range is empty
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S::STAGES; ++s) { mbar_init(full_bar + s, 1); mbar_init(empty_bar + s, 1); }
-        for (int s = 0; s < 2; ++s) { mbar_init(acc_full + s, 1); mbar_init(acc_empty + s, EPI); }
+        for (int s = 0; s < 2; ++s) { mbar_init(acc_full + s, 1); mbar_init(acc_empty + s, CG * EPI); }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -561,11 +569,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     pdl_wait();
     pdl_trigger();
     if (warp == 1) {
-        tmem_alloc(tmem_slot, S::TMEM_COLS);
-        tmem_relinquish();
+        tmem_alloc<CG>(tmem_slot, S::TMEM_COLS);
+        tmem_relinquish<CG>();
     }
     tc_fence_before();
-    __syncthreads();
+    if (CG == 2) cluster_sync();      // the other CTA's barriers and TMEM are there
+    else __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
@@ -573,31 +582,45 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         // ---------------- TMA producer ----------------
         if (lane == 0) {
             uint32_t stage = 0, phase = 0;
+            const uint32_t leader_full = CG == 2 ? leader_addr(full_bar) : 0u;
             bool ok = true;
-            for (uint32_t tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
+            for (uint32_t tile = first_tile; ok && tile < num_tiles; tile += tile_step) {
                 uint32_t tm, tn;
                 tile_coords(split == 1 ? tile : tile / split, prm.tiles_m, prm.tiles_n, tm, tn);
+                const int32_t row = (int32_t)((tm * CG + rank) * BM), col = (int32_t)(tn * BN + rank * (BN / CG));
                 const uint32_t kb0 = split == 1 ? 0u : (tile % split) * kb_per, kb1 = min(num_kb, kb0 + kb_per);
                 for (uint32_t kb = kb0; kb < kb1; ++kb) {
                     if (!mbar_wait(empty_bar + stage, phase ^ 1, abort_flag, prm.wait_limit_ns)) { ok = false; break; }
                     uint8_t* sa = smem + stage * S::STAGE_BYTES;
-                    const bool lost = prm.lose_kb && blockIdx.x == 0 && tile == blockIdx.x && kb + 1 == prm.lose_kb;
+                    const bool lost = prm.lose_kb && blockIdx.x == 0 && tile == first_tile && kb + 1 == prm.lose_kb;
                     if (!lost) {   // a lost stage is never filled: its full barrier stays where it is
-                        mbar_expect_tx(full_bar + stage, S::STAGE_BYTES);
-                        tma_load_2d(sa, &map_a, (int32_t)(kb * BK), (int32_t)(tm * BM), full_bar + stage);
-                        tma_load_2d(sa + S::A_BYTES, &map_b, (int32_t)(kb * BK), (int32_t)(tn * BN), full_bar + stage);
+                        // a pair's stage is full, at the leader's barrier, when both CTAs' copies have landed
+                        if (rank == 0) mbar_expect_tx(full_bar + stage, CG * S::STAGE_BYTES);
+                        if (CG == 2) {
+                            const uint32_t bar = leader_full + 8 * stage;
+                            tma_load_2d_pair(sa, &map_a, (int32_t)(kb * BK), row, bar);
+                            tma_load_2d_pair(sa + S::A_BYTES, &map_b, (int32_t)(kb * BK), col, bar);
+                        } else {
+                            tma_load_2d(sa, &map_a, (int32_t)(kb * BK), row, full_bar + stage);
+                            tma_load_2d(sa + S::A_BYTES, &map_b, (int32_t)(kb * BK), col, full_bar + stage);
+                        }
                     }
                     if (++stage == S::STAGES) { stage = 0; phase ^= 1; }
                 }
             }
+            // the leader's signals to a pair's stages have all arrived before this CTA ends
+            for (int s = 0; CG == 2 && ok && s < S::STAGES; ++s) {
+                ok = mbar_wait(empty_bar + stage, phase ^ 1, abort_flag, prm.wait_limit_ns);
+                if (++stage == S::STAGES) { stage = 0; phase ^= 1; }
+            }
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc_bf16(BN);
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t idesc = make_idesc_bf16(BM * CG, BN);
             uint32_t stage = 0, phase = 0, it = 0;
             bool ok = true;
-            for (uint32_t tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x, ++it) {
+            for (uint32_t tile = first_tile; ok && tile < num_tiles; tile += tile_step, ++it) {
                 const uint32_t ab = it & 1, aphase = (it >> 1) & 1;
                 if (!mbar_wait(acc_empty + ab, aphase ^ 1, abort_flag, prm.wait_limit_ns)) { ok = false; break; }
                 tc_fence_after();
@@ -612,12 +635,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
                     for (uint32_t kk = 0; kk < BK / UMMA_K; ++kk) {
                         // advancing K by 16 elements = 32 bytes inside the swizzle row: +2 in the address field
-                        umma_bf16(d_tmem, adesc + kk * 2, bdesc + kk * 2, idesc, ((kb - kb0) | kk) != 0);
+                        umma_bf16<CG>(d_tmem, adesc + kk * 2, bdesc + kk * 2, idesc, ((kb - kb0) | kk) != 0);
                     }
-                    umma_commit(empty_bar + stage);  // stage reusable once these MMAs have read it
+                    umma_commit<CG>(empty_bar + stage);  // stage reusable once these MMAs have read it
                     if (++stage == S::STAGES) { stage = 0; phase ^= 1; }
                 }
-                if (ok) umma_commit(acc_full + ab);
+                if (ok) umma_commit<CG>(acc_full + ab);
             }
         }
     } else {
@@ -630,12 +653,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const uint32_t qkv_pos = (MODE == GEMM_QKV && prm.tma_store)
                                      ? (prm.epi.qkv.d_position ? *prm.epi.qkv.d_position : prm.epi.qkv.position) : 0u;
         bool ok = true;
-        for (uint32_t tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x, ++it) {
+        for (uint32_t tile = first_tile; ok && tile < num_tiles; tile += tile_step, ++it) {
             const uint32_t ab = it & 1, aphase = (it >> 1) & 1;
             uint32_t tm, tn;
             tile_coords(split == 1 ? tile : tile / split, prm.tiles_m, prm.tiles_n, tm, tn);
             const uint32_t ks = split == 1 ? 0u : tile % split;
-            const uint32_t row0 = tm * BM + quarter * 32;
+            const uint32_t row0 = (tm * CG + rank) * BM + quarter * 32;
             // f32 output with a residual: fetch this warp's first block of residual rows while the tile is still
             // being accumulated (the rows are final: only this warp rewrites them, after this read)
             float4 res_pre[8];
@@ -651,7 +674,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             // what the epilogue reads besides the accumulator (the tile's bias columns, the step's position) is asked into
             // L1 while the tile is still being accumulated: a first-touch load after the wait is a whole L2 round trip
             // on the critical path of a one-tile launch (with many tiles per CTA the loads hit anyway: not done there)
-            if (MODE != GEMM_ARGMAX && num_tiles <= gridDim.x) {
+            if (MODE != GEMM_ARGMAX && num_tiles <= tile_step) {
                 const float* bias0 = prm.epi.ep.bias ? prm.epi.ep.bias + (size_t)tn * BN : nullptr;
                 if (bias0 && lane * 32 < (uint32_t)BN && tn * BN + lane * 32 < prm.epi.n)
                     asm volatile("prefetch.global.L1 [%0];" ::"l"(bias0 + lane * 32));
@@ -703,7 +726,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(acc_empty + ab);
+            if (lane == 0) {
+                if (CG == 2) mbar_arrive_cluster(leader_addr(acc_empty + ab));     // the products that overwrite both CTAs' accumulators are issued there
+                else mbar_arrive(acc_empty + ab);
+            }
         }
         // bulk reduce operations of this warp must be complete before the CTA gives up its shared memory
         if (((PLAIN && prm.tma_reduce) || prm.tma_store) && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
@@ -719,9 +745,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (threadIdx.x == 0 && prm.d_status) atomicCAS(prm.d_status, DEV_OK, DEV_TIMEOUT);
         __syncthreads();
     }
+    if (CG == 2) cluster_sync();      // neither leaves while the other may still signal its barriers or read its operands
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, S::TMEM_COLS);
+        tmem_dealloc<CG>(tmem_base, S::TMEM_COLS);
     }
 }
 
@@ -752,20 +779,13 @@ static int sm_count() {
     return n;
 }
 
-template <int BN, int MODE, int EPI>
+template <int BN, int MODE, int EPI, int CG>
 static int launch_tc_e(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap* mo, const TcParams& prm, cudaStream_t stream) {
-    using S = TcShape<BN, EPI>;
-    static bool configured[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        if (cudaFuncSetAttribute(gemm_tc_kernel<BN, MODE, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM_BYTES) != cudaSuccess)
-            return check_launch("gemm_tc attribute");
-        if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
-    uint32_t tiles = prm.tiles_m * prm.tiles_n * (prm.tma_reduce == 2 ? prm.split_k : 1u);
-    uint32_t grid = tiles < (uint32_t)sm_count() ? tiles : (uint32_t)sm_count();
-    launch_kernel(gemm_tc_kernel<BN, MODE, EPI>, dim3(grid), dim3(S::THREADS), S::SMEM_BYTES, stream, ma, mb, mo[0], mo[1], mo[2], prm);
+    using S = TcShape<BN, EPI, CG>;
+    if (const int rc = allow_shared<gemm_tc_kernel<BN, MODE, EPI, CG>>(S::SMEM_BYTES, "gemm_tc attribute")) return rc;
+    const uint32_t tiles = prm.tiles_m * prm.tiles_n * (prm.tma_reduce == 2 ? prm.split_k : 1u);
+    const uint32_t grid = std::min(tiles, (uint32_t)sm_count() / CG) * CG;
+    launch_kernel_clusters(gemm_tc_kernel<BN, MODE, EPI, CG>, dim3(grid), dim3(S::THREADS), S::SMEM_BYTES, CG, stream, ma, mb, mo[0], mo[1], mo[2], prm);
     count_launch();
     return check_launch("gemm_tc");
 }
@@ -773,24 +793,24 @@ static int launch_tc_e(const CUtensorMap& ma, const CUtensorMap& mb, const CUten
 // Wide tiles with a bf16 epilogue (QKV routing, SwiGLU, column ranges) and a short K: the main loop of a K = 768 tile is shorter than
 // 8 warps need to drain the previous accumulator, so these run 16 epilogue warps (and 3 ring stages instead of 4, which
 // is why longer K keeps 8: there the deeper ring is worth more).
-template <int BN, int MODE>
+template <int BN, int MODE, int CG>
 static int launch_tc_t(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap* mo, const TcParams& prm, cudaStream_t stream) {
-    constexpr bool many_warps = BN == 256 && (MODE == GEMM_QKV || MODE == GEMM_SWIGLU || MODE == GEMM_SEGMENTS);
-    if (many_warps && prm.k <= 1024) return launch_tc_e<BN, MODE, many_warps ? 16 : 8>(ma, mb, mo, prm, stream);
+    constexpr bool many_warps = BN >= 192 && (MODE == GEMM_QKV || MODE == GEMM_SWIGLU || MODE == GEMM_SEGMENTS);
+    if (many_warps && prm.k <= 1024) return launch_tc_e<BN, MODE, many_warps ? 16 : 8, CG>(ma, mb, mo, prm, stream);
     // narrow tiles: one epilogue warp per TMEM lane quarter is all a 32- or 64-column tile can use
-    if (BN <= 64 && MODE != GEMM_ARGMAX) return launch_tc_e<BN, MODE, BN <= 64 ? 4 : 8>(ma, mb, mo, prm, stream);
-    return launch_tc_e<BN, MODE, 8>(ma, mb, mo, prm, stream);
+    if (BN <= 64 && MODE != GEMM_ARGMAX) return launch_tc_e<BN, MODE, BN <= 64 ? 4 : 8, CG>(ma, mb, mo, prm, stream);
+    return launch_tc_e<BN, MODE, 8, CG>(ma, mb, mo, prm, stream);
 }
 
-template <int BN>
+template <int BN, int CG>
 static int launch_tc_mode(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap* mo, const TcParams& prm, GemmMode mode, cudaStream_t stream) {
     switch (mode) {
-        case GEMM_PLAIN: return launch_tc_t<BN, GEMM_PLAIN>(ma, mb, mo, prm, stream);
-        case GEMM_SCALED: return launch_tc_t<BN, GEMM_SCALED>(ma, mb, mo, prm, stream);
-        case GEMM_QKV: return launch_tc_t<BN, GEMM_QKV>(ma, mb, mo, prm, stream);
-        case GEMM_SWIGLU: return launch_tc_t<BN, GEMM_SWIGLU>(ma, mb, mo, prm, stream);
-        case GEMM_ARGMAX: return launch_tc_t<BN, GEMM_ARGMAX>(ma, mb, mo, prm, stream);
-        case GEMM_SEGMENTS: return launch_tc_t<BN, GEMM_SEGMENTS>(ma, mb, mo, prm, stream);
+        case GEMM_PLAIN: return launch_tc_t<BN, GEMM_PLAIN, CG>(ma, mb, mo, prm, stream);
+        case GEMM_SCALED: return launch_tc_t<BN, GEMM_SCALED, CG>(ma, mb, mo, prm, stream);
+        case GEMM_QKV: return launch_tc_t<BN, GEMM_QKV, CG>(ma, mb, mo, prm, stream);
+        case GEMM_SWIGLU: return launch_tc_t<BN, GEMM_SWIGLU, CG>(ma, mb, mo, prm, stream);
+        case GEMM_ARGMAX: return launch_tc_t<BN, GEMM_ARGMAX, CG>(ma, mb, mo, prm, stream);
+        case GEMM_SEGMENTS: return launch_tc_t<BN, GEMM_SEGMENTS, CG>(ma, mb, mo, prm, stream);
     }
     return TNSR_B200_ERR_INVALID_ARGUMENT;
 }
@@ -798,6 +818,26 @@ static int launch_tc_mode(const CUtensorMap& ma, const CUtensorMap& mb, const CU
 static bool tc_eligible(const bf16* a, uint32_t lda, const bf16* bt, uint32_t k) {
     return k % 8 == 0 && lda % 8 == 0 && (reinterpret_cast<uintptr_t>(a) % 16 == 0) &&
            (reinterpret_cast<uintptr_t>(bt) % 16 == 0) && encode_fn() != nullptr;
+}
+
+// Tile width, and whether pairs of CTAs share a tile: tiles run in waves of one per SM, so what counts is waves x the time of a tile.  A tile
+// takes about what its operands take to come in, BM + bn rows of k; 192 columns do a little worse than that and a pair of 256 a little better
+// (7 % of 8192 x 8192 x 8192, 881 -> 829 us; sustained, under the power cap).  Where waves are equal the wider tile is taken.  Against widths of
+// powers of two and no pairs, us: 32768 x 768 x 768 onto the residual 66 -> 62 (7 waves of 192 for 6 of 256), x 2048 117 -> 105 (pairs),
+// 3885 x 768 x 768 16.4 -> 14.4 and x 2048 22.5 -> 20.5 (one wave of 192), 4096 x 2048 x 5632 84 -> 80, 3000 x 1536 x 6144 53.3 -> 52.0.  A pair
+// with a short k waits for two epilogues at a time: 32768 x 2304 x 768 128 -> 132, 4096 x 8192 x 1024 f32 89 -> 93.
+static void choose_tile(uint32_t m, uint32_t n, uint32_t k, uint32_t& bn, uint32_t& cg) {
+    struct Shape { uint32_t bn, cg, rows; };
+    static const Shape shapes[] = {{256, 2, 355}, {256, 1, BM + 256}, {192, 1, 322}, {128, 1, BM + 128}, {64, 1, BM + 64}, {32, 1, BM + 32}};
+    uint64_t least = ~0ull;
+    for (const Shape& s : shapes) {
+        if (s.cg == 2 && k < 1536) continue;
+        const uint64_t tiles = (uint64_t)ceil_div(m, BM * s.cg) * ceil_div(n, s.bn);
+        const uint64_t rows = ceil_div64(tiles, (uint64_t)sm_count() / s.cg) * s.rows;
+        if (rows < least) { least = rows; bn = s.bn; cg = s.cg; }
+    }
+    if (bn / 2 >= n) cg = 1;
+    while (bn > 32 && bn / 2 >= n) bn = bn == 192 ? 128 : bn >> 1;      // no wider than the matrix (a router's few columns)
 }
 
 // Shared body of the public launchers.  `tiles_n_out` (optional) receives the number of column
@@ -897,21 +937,12 @@ static int launch_gemm_impl(const bf16* a, const bf16* bt, void* out, uint32_t l
         if (pays || g_gemm_engine == 3)
             return launch_gemm_skinny(a, bt, out, ldc, m, n, k, ep, ep.skinny_ws, ep.skinny_ws_bytes, d_status, stream);
     }
-    // Tile width: a tile takes what its operands take to come in, BM + bn rows of k, and tiles run in waves of one per SM: the fewest rows
-    // through one SM, the wider tile where it is the same.  (The widest that still gives every SM a tile, the rule before, ran 186 tiles of 128
-    // columns in two waves where 93 of 256 are one.)
-    const uint32_t tiles_m = ceil_div(m, BM);
-    uint32_t bn = 256;
-    uint64_t least = ~0ull;
-    for (uint32_t w = 256; w >= 32; w >>= 1) {
-        const uint64_t rows = ceil_div64((uint64_t)tiles_m * ceil_div(n, w), (uint64_t)sm_count()) * (BM + w);
-        if (rows < least) { least = rows; bn = w; }
-    }
-    while (bn > 32 && bn / 2 >= n) bn >>= 1;      // no wider than the matrix (a router's few columns)
-    if (split_req) bn = 32;   // many small tiles: every CTA takes in as little of both operands as possible
+    uint32_t bn = 256, cg = 1;
+    choose_tile(m, n, k, bn, cg);
+    if (split_req) { bn = 32; cg = 1; }   // many small tiles: every CTA takes in as little of both operands as possible
     TcParams prm;
     prm.k = k;
-    prm.tiles_m = tiles_m;
+    prm.tiles_m = ceil_div(m, BM * cg);
     prm.tiles_n = ceil_div(n, bn);
     prm.split_k = 1;
     prm.split_rows = 0;
@@ -920,7 +951,7 @@ static int launch_gemm_impl(const bf16* a, const bf16* bt, void* out, uint32_t l
     prm.lose_kb = t_lose_gemm_stage;   // one-shot test hook, see TcParams
     t_lose_gemm_stage = 0;
     CUtensorMap ma, mb;
-    if (!make_map(&ma, a, m, k, lda, BM) || !make_map(&mb, bt, n, k, k, bn)) {
+    if (!make_map(&ma, a, m, k, lda, BM) || !make_map(&mb, bt, n, k, k, bn / cg)) {
         if (g_gemm_engine == 2) {
             set_thread_error("gemm: tensor map encoding failed");
             return TNSR_B200_ERR_CUDA;
@@ -1002,10 +1033,11 @@ static int launch_gemm_impl(const bf16* a, const bf16* bt, void* out, uint32_t l
     prm.epi = P;
     if (mode == GEMM_PLAIN && ep.scale) mode = GEMM_SCALED;
     switch (bn) {
-        case 256: return launch_tc_mode<256>(ma, mb, mo, prm, mode, stream);
-        case 128: return launch_tc_mode<128>(ma, mb, mo, prm, mode, stream);
-        case 64: return launch_tc_mode<64>(ma, mb, mo, prm, mode, stream);
-        default: return launch_tc_mode<32>(ma, mb, mo, prm, mode, stream);
+        case 256: return cg == 2 ? launch_tc_mode<256, 2>(ma, mb, mo, prm, mode, stream) : launch_tc_mode<256, 1>(ma, mb, mo, prm, mode, stream);
+        case 192: return launch_tc_mode<192, 1>(ma, mb, mo, prm, mode, stream);
+        case 128: return launch_tc_mode<128, 1>(ma, mb, mo, prm, mode, stream);
+        case 64: return launch_tc_mode<64, 1>(ma, mb, mo, prm, mode, stream);
+        default: return launch_tc_mode<32, 1>(ma, mb, mo, prm, mode, stream);
     }
 }
 
