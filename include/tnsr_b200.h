@@ -607,8 +607,8 @@ typedef struct tnsr_b200_place {
  * v_cache [.., vdim], out [sessions, chunk, out_ld], columns from heads * vdim to
  * out_cols are zeroed.  dtype: element type of q, caches and out.  engine: 0 =
  * best kernel for the shape, 1 = one warp per (query, head), 2 = warp-level tensor
- * cores only, 3 = as 2 with softmax weights of 24 bits in the value product
- * instead of 16.  A host-known position (d_positions NULL) is what the tcgen05
+ * cores only, 3 = tensor cores with softmax weights of 24 bits in the value product
+ * instead of 16 (2) or 8 (the tcgen05 kernel of engine 0).  A host-known position (d_positions NULL) is what the tcgen05
  * kernel of long chunks needs; d_status (may be NULL) receives 2 if one of its
  * bounded waits gave up.  workspace:
  * tnsr_b200_grouped_attention_workspace() bytes, zeroed once (NULL: the keys of

@@ -944,6 +944,37 @@ def test_multi_token_chunks_off_the_tiled_prefill_kernels(heads, paged, batch):
     assert rel_err(got, ref.forward(ids)) <= 2e-2
 
 
+@pytest.mark.parametrize("page", [16, 48, 192])
+def test_long_paged_prompts_over_pages_of_any_size(page):
+    """Chunks of more than 64 ids behind paged K/V run on tcgen05, whose key boxes are parts of a page: pages of one box, of an odd number of
+    boxes, of more than a block of keys.  Rows of a page behind the last id hold NaN that an earlier tenant left.  Against the scan (prefill
+    mode Scalar), whose bf16 rows may round the other way: 2^-9 of them, through two layers and the head."""
+    cfg = GptConfig(vocab_size=320, max_sequence_length=384, embed_dim=256, num_heads=4, feed_forward_dim=512, num_layers=2,
+                    layer_norm_epsilon=1e-5, activation="swiglu", weight_dtype="bf16")
+    arrays = normal_model_arrays(cfg, seed=91, std=0.05)
+    chunks, batch = [65, 130, 33, 129], 3                          # 357 ids: inside a block, across its end, a short one, across again
+    ids = np.random.default_rng(92).integers(0, cfg.vocab_size, size=(batch, sum(chunks))).astype(np.uint32)
+
+    def run(mode):
+        s = B200Session(cfg, batch, 384, GptDecoderOptions(prefill=mode), logits_mode="all", kv_page_rows=page)
+        for i, a in enumerate(arrays):
+            s.refresh(i, a)
+        for i in range(s.cache_count()):
+            s.write_cache(i, np.full(batch * 384 * cfg.embed_dim, np.nan, dtype=np.float32))
+        for b in range(batch):
+            s.release(b)
+        out, at = [], 0
+        for n in chunks:
+            out.append(s.decode_full(ids[:, at:at + n], at, want_argmax=False)[0].reshape(batch, n, -1))
+            at += n
+        s.close()
+        return np.concatenate(out, 1)
+
+    got, want = run(GptPrefillMode.Auto), run(GptPrefillMode.Scalar)
+    assert np.all(np.isfinite(got))
+    assert np.max(np.abs(got - want)) <= max(1.0, float(np.max(np.abs(want)))) / 64
+
+
 def test_paged_kv_pool_smaller_than_the_worst_case():
     """A pool of 7 pages for 4 sessions x 64 rows (worst case 16 pages): short sessions fit, a step that would need an
     eighth page is refused with ERR_CAPACITY and changes nothing, releasing a session makes room again."""

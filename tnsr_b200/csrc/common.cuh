@@ -196,6 +196,7 @@ struct GemmSegments {
 struct KvPaging {
     const uint32_t* table = nullptr;
     uint32_t page_rows = 0, pages_per_session = 0;
+    uint32_t pool_pages = 0;
 };
 #ifdef __CUDACC__
 // Physical row of logical row `r` of session `s` (contiguous layout: s * capacity + r).

@@ -340,7 +340,7 @@ int layers_bf16(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chunk
     const size_t r0 = (size_t)s0 * chunk;                       // first activation row of the range
     const size_t cache0 = dec->paged ? 0 : (size_t)s0 * c.capacity * d;   // first cache element of the range
     KvPaging pg;                                                // paged: the pools are shared, the table is per session
-    if (dec->paged) { pg.table = dec->d_table + (size_t)s0 * dec->pps; pg.page_rows = dec->page_rows; pg.pages_per_session = dec->pps; }
+    if (dec->paged) { pg.table = dec->d_table + (size_t)s0 * dec->pps; pg.page_rows = dec->page_rows; pg.pages_per_session = dec->pps; pg.pool_pages = dec->pool_pages; }
     float* h = dec->h + r0 * d;
     bf16* n = (bf16*)dec->n + r0 * d; bf16* q = (bf16*)dec->q + r0 * d; bf16* att = (bf16*)dec->att + r0 * d;
     bf16* ff = (bf16*)dec->ff + r0 * f;
@@ -393,7 +393,8 @@ int layers_bf16(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chunk
             // Paged caches and head widths other than 64: the kernels of described models, with one query head per
             // key/value head (K/V tiles through shared memory).  The scan below holds its weights in f32, so they enter the
             // value product as three bf16 pieces here, which is all of their bits.  It reads every key once per query; 5 x 777
-            // ids, 12 x 64 heads, pages of 64 rows, one layer on B200: 2672 us there, 77 us here (69 with two pieces).
+            // ids, 12 x 64 heads, pages of 64 rows, one layer on B200: 2672 us there, 77 us on warp-level tiles, 27 us on tcgen05
+            // (chunks of more than 64 ids, heads of 64).
             GroupedAttention ga;
             ga.q = q; ga.k_cache = kcache; ga.v_cache = vcache; ga.out = att;
             ga.heads = ga.kv_heads = H; ga.dim = ga.vdim = hd; ga.capacity = c.capacity;

@@ -671,7 +671,7 @@ int launch_grouped_attention(const GroupedAttention& a, const StepPlace& place, 
         if (w == 64) rc = upper ? launch_split<64, 64, 3, true>(P, stream) : launch_split<64, 64, 3, false>(P, stream);
         else if (w == 128) rc = upper ? launch_split<128, 128, 3, true>(P, stream) : launch_split<128, 128, 3, false>(P, stream);
         else rc = upper ? launch_split<256, 256, 2, true>(P, stream) : launch_split<256, 256, 2, false>(P, stream);
-    } else if (a.engine == 0 && grouped_attention_tc_eligible(a, place)) {
+    } else if ((a.engine == 0 && grouped_attention_tc_eligible(a, place)) || (a.engine == 3 && grouped_attention_exact_tc_eligible(a, place))) {
         return launch_grouped_attention_tc(a, place, stream);
     } else {
         P.row_tiles = ceil_div(P.rows, 64u);

@@ -594,7 +594,7 @@ int stack_step(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chunk,
     place.sessions = B; place.chunk = chunk; place.position = position; place.d_position = d_position;
     place.position_stride = ragged ? 1u : 0u;
     KvPaging pg;
-    if (dec->paged) { pg.table = dec->d_table; pg.page_rows = dec->page_rows; pg.pages_per_session = dec->pps; }
+    if (dec->paged) { pg.table = dec->d_table; pg.page_rows = dec->page_rows; pg.pages_per_session = dec->pps; pg.pool_pages = dec->pool_pages; }
     RUN(dec, launch_embedding(S->embed, nullptr, d_tokens, dec->h, rows, chunk, position, d_position, c.vocab_size, d, dtype,
                               dec->d_status, st, place.position_stride, S->embedding_scale));
     const bool splitk = bf && chunk == 1 && dec->split_ws;

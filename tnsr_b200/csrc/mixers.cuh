@@ -75,13 +75,15 @@ struct GroupedAttention {
     uint64_t workspace_bytes = 0;
     int* d_status = nullptr;              // device status word (a bounded wait of the tcgen05 kernel gave up), may be null
     int engine = 0;                       // 0: best kernel for the shape, 1: one warp per (row, head), 2: not the tcgen05 kernel,
-                                          // 3: as 2, and softmax weights keep their 24 bits
+                                          // 3: softmax weights keep their 24 bits
 };
 uint64_t grouped_attention_workspace_bytes(uint32_t dim, uint32_t vdim);
 int launch_grouped_attention(const GroupedAttention& a, const StepPlace& place, int dtype, cudaStream_t stream);
 
 // Many rows, heads of 64, position on the host: the tcgen05 kernel of prefill_tc.cu.
 bool grouped_attention_tc_eligible(const GroupedAttention& a, const StepPlace& place);
+// The same with weights of 24 bits, paged caches too: plain softmax scores, no window.
+bool grouped_attention_exact_tc_eligible(const GroupedAttention& a, const StepPlace& place);
 int launch_grouped_attention_tc(const GroupedAttention& a, const StepPlace& place, cudaStream_t stream);
 
 // ---- mamba2 ---------------------------------------------------------------------

@@ -41,6 +41,13 @@
 // a window the key blocks of an item start at the first one its first query sees.  Sigmoid weights (PT_SIGMOID) are not
 // normalised over keys: there is no maximum, no rescaling, and P V of all blocks accumulates in TMEM, read once per item.
 //
+// EXACT form (paged caches): softmax weights keep all their 24 bits in the value product, as in the key-by-key scan that it stands in for.  A
+// weight is the sum of three bf16 pieces, each with a product of its own.  The pieces do not fit in shared memory beside a second CTA, so they
+// are the A operand in TMEM: two of them over the scores that the same thread has just read (per 16 keys 8 columns of upper pieces, 8 of
+// middle ones), the third in the 64 columns behind the output.  S_{j+1} is issued behind P_j V_j then, which it overwrites.
+// Keys come page by page: a box is the largest power of two of rows that divides a page, up to a block; boxes behind the last live row are not
+// read, and the softmax warps zero the value rows that they would have filled.
+//
 // Every wait is bounded; a wait that gives up raises the CTA's abort flag, the
 // roles fall through to the common teardown and the status word is set.
 #include <algorithm>
@@ -59,6 +66,7 @@ constexpr uint32_t PT_XM_BYTES = 2 * 2 * 128 * 4;     // row maxima: [block pari
 constexpr uint32_t PT_SMEM_BYTES = 1024 + PT_TILE_BYTES + PT_KV_STAGES * PT_KV_BYTES + PT_TILE_BYTES + PT_XM_BYTES + 256;
 constexpr uint32_t PT_TMEM_COLS = 256;                // scores 128, outputs 64 (power of two)
 constexpr uint32_t PT_O_COL = 128;
+constexpr uint32_t PT_LOW_COL = 192;                  // EXACT: third pieces of the weights
 
 // kind::f16 instruction descriptors: f32 accumulator, bf16 operands, M = 128.
 constexpr uint32_t PT_IDESC_S = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
@@ -86,12 +94,39 @@ struct PtParams {
     float cap_pre, cap_post;   // capped scores in log2 units: cap_post - 2 cap_post / (1 + exp2(s cap_pre))
     int* d_status;
     uint64_t wait_limit_ns;
+    KvPaging paging;           // EXACT form only
+    uint32_t box_rows;         // paged: rows of a key box
 };
+
+// D = A (TMEM, 128 rows x 16 bf16 in 8 columns) . B (shared memory) + D
+__device__ __forceinline__ void umma_bf16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
+    uint32_t* r = reinterpret_cast<uint32_t*>(v);
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+          "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
+// 8 columns of this thread's TMEM lane.
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 enum : int { PT_SOFTMAX = 0, PT_CAPPED = 1, PT_SIGMOID = 2 };
 
 // WINDOW: prm.window is set (compiled apart: the masks of the unwindowed kernels stay one comparison per key).
-template <int KIND, bool WINDOW>
+template <int KIND, bool WINDOW, bool EXACT>
 __global__ void __launch_bounds__(PT_THREADS, 2)
 prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, PtParams prm) {
@@ -172,6 +207,22 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                     const uint32_t stage = g % PT_KV_STAGES;
                     if (!mbar_wait(kv_empty + stage, ((g / PT_KV_STAGES) & 1) ^ 1, abort_flag, prm.wait_limit_ns)) { ok = false; break; }
                     uint8_t* dst = kv_ring + stage * PT_KV_BYTES;
+                    if (EXACT && prm.paging.table) {
+                        // boxes of the block that hold live rows, their rows in the pool first: independent reads of the table
+                        const uint32_t key0 = (block0 + j) * PT_BK, box = prm.box_rows;
+                        const uint32_t boxes = min((uint32_t)PT_BK / box, (prm.position + prm.chunk - key0 + box - 1) / box);
+                        uint32_t rows[PT_BK / 16];
+#pragma unroll
+                        for (uint32_t i = 0; i < PT_BK / 16; ++i) rows[i] = i < boxes ? (uint32_t)kv_row(prm.paging, s, key0 + i * box, 0) : 0u;
+                        mbar_expect_tx(kv_full + stage, boxes * box * 256u);
+#pragma unroll
+                        for (uint32_t i = 0; i < PT_BK / 16; ++i) {
+                            if (i >= boxes) continue;
+                            tma_load_3d(dst + i * box * 128u, &map_k, (int32_t)(h / prm.per * PT_HD), (int32_t)rows[i], 0, kv_full + stage);
+                            tma_load_3d(dst + PT_TILE_BYTES + i * box * 128u, &map_v, (int32_t)(h / prm.per * PT_HD), (int32_t)rows[i], 0, kv_full + stage);
+                        }
+                        continue;
+                    }
                     mbar_expect_tx(kv_full + stage, PT_KV_BYTES);
                     tma_load_3d(dst, &map_k, (int32_t)(h / prm.per * PT_HD), (int32_t)((block0 + j) * PT_BK), (int32_t)s, kv_full + stage);
                     tma_load_3d(dst + PT_TILE_BYTES, &map_v, (int32_t)(h / prm.per * PT_HD), (int32_t)((block0 + j) * PT_BK), (int32_t)s, kv_full + stage);
@@ -200,7 +251,29 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 tc_fence_after();
                 issue_s(g % PT_KV_STAGES);
                 if (n_blocks == 1) umma_commit(q_empty);
-                for (uint32_t j = 0; j < n_blocks; ++j) {
+                for (uint32_t j = 0; EXACT && j < n_blocks; ++j) {
+                    const uint32_t b = g + j, stage = b % PT_KV_STAGES;
+                    if (!mbar_wait(p_full, b & 1, abort_flag, prm.wait_limit_ns)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t v_addr = smem_u32(kv_ring + stage * PT_KV_BYTES) + PT_TILE_BYTES;
+#pragma unroll
+                    for (uint32_t kk = 0; kk < PT_BK / 16; ++kk) {
+                        const uint64_t vdesc = make_mnmajor_sw128_desc(v_addr + kk * 2048, PT_TILE_BYTES, 1024);
+                        umma_bf16_ta(tmem_base + PT_O_COL, tmem_base + kk * 16, vdesc, PT_IDESC_O, kk != 0);
+                        umma_bf16_ta(tmem_base + PT_O_COL, tmem_base + kk * 16 + 8, vdesc, PT_IDESC_O, 1);
+                        umma_bf16_ta(tmem_base + PT_O_COL, tmem_base + PT_LOW_COL + kk * 8, vdesc, PT_IDESC_O, 1);
+                    }
+                    umma_commit(o_full);
+                    umma_commit(kv_empty + stage);
+                    if (j + 1 < n_blocks) {
+                        const uint32_t next = (b + 1) % PT_KV_STAGES;
+                        if (!mbar_wait(kv_full + next, ((b + 1) / PT_KV_STAGES) & 1, abort_flag, prm.wait_limit_ns)) { ok = false; break; }
+                        tc_fence_after();
+                        issue_s(next);
+                        if (j + 2 == n_blocks) umma_commit(q_empty);
+                    }
+                }
+                for (uint32_t j = 0; !EXACT && j < n_blocks; ++j) {
                     const uint32_t b = g + j, stage = b % PT_KV_STAGES;
                     // P_j is in place and the softmax warps are done with S_j
                     if (!mbar_wait(p_full, b & 1, abort_flag, prm.wait_limit_ns)) { ok = false; break; }
@@ -281,6 +354,13 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 const bool need_mask = kbase + 63 > limit || (WINDOW && kbase < low);
                 auto hidden = [&](uint32_t key) { return key > limit || (WINDOW && key < low); };
                 float corr = 0.0f, neg = 0.0f;
+                // value rows past the live ones hold whatever the ring held: a weight of 0 does not keep infinities and NaN out
+                if (EXACT && (block0 + j) * PT_BK + row >= prm.position + prm.chunk) {
+                    uint4* v_row = reinterpret_cast<uint4*>(kv_ring + (b % PT_KV_STAGES) * PT_KV_BYTES + PT_TILE_BYTES + row * 128u + half * 64u);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) v_row[i] = make_uint4(0u, 0u, 0u, 0u);
+                }
+                __syncwarp();
                 if (SIGMOID) {
                     // the previous P V must have read the upper P tile; its result stays in TMEM
                     if (j > 0 && !mbar_wait(o_full, (b - 1) & 1, abort_flag, prm.wait_limit_ns)) { ok = false; break; }
@@ -317,8 +397,36 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 // (16-byte chunk c of row r at c ^ (r & 7))
                 uint8_t* p_row = (half ? p_upper : kv_ring + (b % PT_KV_STAGES) * PT_KV_BYTES) + row * 128u;
                 float rs4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                if (EXACT) {
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
+                    for (int c = 0; c < 4; ++c) {        // 16 keys, one K step of the product
+                        float v[16];
+                        tmem_ld16(taddr + c * 16, v);
+                        tmem_ld_wait();
+                        uint32_t upper[8], middle[8], low[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            float p[2];
+#pragma unroll
+                            for (int e = 0; e < 2; ++e)
+                                p[e] = need_mask && hidden(kbase + c * 16 + 2 * i + e) ? 0.0f : pt_ex2(fmaf(v[2 * i + e], sl2, neg));
+                            rs4[i & 3] += p[0] + p[1];
+                            // what a piece leaves is exact
+                            upper[i] = pack_bf16x2(p[0], p[1]);
+                            const float2 a = bf16x2_to_f32(upper[i]);
+                            const float r0 = p[0] - a.x, r1 = p[1] - a.y;
+                            middle[i] = pack_bf16x2(r0, r1);
+                            const float2 b2 = bf16x2_to_f32(middle[i]);
+                            low[i] = pack_bf16x2(r0 - b2.x, r1 - b2.y);
+                        }
+                        tmem_st8(taddr + c * 16, upper);
+                        tmem_st8(taddr + c * 16 + 8, middle);
+                        tmem_st8(lane_taddr + PT_LOW_COL + half * 32 + c * 8, low);
+                    }
+                    tmem_st_wait();
+                }
+#pragma unroll
+                for (int c = 0; !EXACT && c < 2; ++c) {
                     float v[32];
                     tmem_ld32(taddr + c * 32, v);
                     tmem_ld_wait();
@@ -407,14 +515,14 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 }
 
 // {width, rows, sessions} bf16, `row_stride` elements between rows of one session, `session_rows`
-// rows between sessions; box = 64 columns x 128 rows x 1 session.
+// rows between sessions; box = 64 columns x 128 (or box_rows) rows x 1 session.
 static bool make_map3(CUtensorMap* map, const void* base, uint64_t width, uint64_t rows, uint64_t sessions,
-                      uint64_t session_rows) {
+                      uint64_t session_rows, uint32_t box_rows = 128) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return false;
     cuuint64_t dims[3] = {width, rows, sessions};
     cuuint64_t strides[2] = {width * 2, session_rows * width * 2};
-    cuuint32_t box[3] = {(cuuint32_t)PT_HD, 128, 1};
+    cuuint32_t box[3] = {(cuuint32_t)PT_HD, box_rows, 1};
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -432,44 +540,43 @@ bool prefill_attention_tc_eligible(uint32_t sessions, uint32_t chunk, uint32_t p
     return encode_fn() != nullptr;
 }
 
-template <int KIND, bool WINDOW>
+template <int KIND, bool WINDOW, bool EXACT>
 static int launch_pt_kind(const bf16* q, const bf16* k_cache, const bf16* v_cache, uint32_t kv_heads, uint32_t capacity, PtParams& prm, cudaStream_t stream) {
     const uint64_t width = (uint64_t)prm.heads * PT_HD, kv_width = (uint64_t)kv_heads * PT_HD;
     CUtensorMap mq, mk, mv;
-    if (!make_map3(&mq, q, width, prm.chunk, prm.sessions, prm.chunk) ||
-        !make_map3(&mk, k_cache, kv_width, (uint64_t)prm.position + prm.chunk, prm.sessions, capacity) ||
-        !make_map3(&mv, v_cache, kv_width, (uint64_t)prm.position + prm.chunk, prm.sessions, capacity)) {
+    bool mapped = make_map3(&mq, q, width, prm.chunk, prm.sessions, prm.chunk);
+    if (EXACT && prm.paging.table) {
+        const uint64_t rows = (uint64_t)prm.paging.pool_pages * prm.paging.page_rows;
+        prm.box_rows = std::min<uint32_t>(PT_BK, prm.paging.page_rows & (0u - prm.paging.page_rows));
+        mapped = mapped && make_map3(&mk, k_cache, kv_width, rows, 1, rows, prm.box_rows) && make_map3(&mv, v_cache, kv_width, rows, 1, rows, prm.box_rows);
+    } else {
+        mapped = mapped && make_map3(&mk, k_cache, kv_width, (uint64_t)prm.position + prm.chunk, prm.sessions, capacity) &&
+                 make_map3(&mv, v_cache, kv_width, (uint64_t)prm.position + prm.chunk, prm.sessions, capacity);
+    }
+    if (!mapped) {
         set_thread_error("prefill attention: tensor map encoding failed");
         return TNSR_B200_ERR_CUDA;
     }
-    static bool configured[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        if (cudaFuncSetAttribute(prefill_attention_tc_kernel<KIND, WINDOW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PT_SMEM_BYTES) != cudaSuccess ||
-            cudaFuncSetAttribute(prefill_attention_tc_kernel<KIND, WINDOW>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess)
-            return check_launch("prefill_attention_tc attribute");
-        if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
+    if (const int rc = allow_shared<prefill_attention_tc_kernel<KIND, WINDOW, EXACT>>(PT_SMEM_BYTES, "prefill_attention_tc attribute")) return rc;
     prm.q_tiles = ceil_div(prm.chunk, (uint32_t)PT_BQ);
     prm.per = prm.heads / kv_heads;
     prm.wait_limit_ns = g_wait_limit_ns.load(std::memory_order_relaxed);
     // persistent: two CTAs per SM walk the list of (query tile, head, session) items
-    int dev_sms = 0;
+    int dev = 0, dev_sms = 0;
+    cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, dev);
     if (dev_sms <= 0) dev_sms = 148;
     const uint64_t items = (uint64_t)prm.q_tiles * prm.heads * prm.sessions;
     dim3 grid((unsigned)std::min<uint64_t>(items, 2ull * dev_sms));
-    launch_kernel(prefill_attention_tc_kernel<KIND, WINDOW>, grid, dim3(PT_THREADS), (size_t)PT_SMEM_BYTES, stream, mq, mk, mv, prm);
+    launch_kernel(prefill_attention_tc_kernel<KIND, WINDOW, EXACT>, grid, dim3(PT_THREADS), (size_t)PT_SMEM_BYTES, stream, mq, mk, mv, prm);
     count_launch();
     return check_launch("prefill_attention_tc");
 }
 
 template <int KIND>
 static int launch_pt(const bf16* q, const bf16* k_cache, const bf16* v_cache, uint32_t kv_heads, uint32_t capacity, PtParams& prm, cudaStream_t stream) {
-    return prm.window ? launch_pt_kind<KIND, true>(q, k_cache, v_cache, kv_heads, capacity, prm, stream)
-                      : launch_pt_kind<KIND, false>(q, k_cache, v_cache, kv_heads, capacity, prm, stream);
+    return prm.window ? launch_pt_kind<KIND, true, false>(q, k_cache, v_cache, kv_heads, capacity, prm, stream)
+                      : launch_pt_kind<KIND, false, false>(q, k_cache, v_cache, kv_heads, capacity, prm, stream);
 }
 
 int launch_prefill_attention_tc(const bf16* q, const bf16* k_cache, const bf16* v_cache, bf16* out, uint32_t sessions,
@@ -488,11 +595,19 @@ int launch_prefill_attention_tc(const bf16* q, const bf16* k_cache, const bf16* 
     return launch_pt<PT_SOFTMAX>(q, k_cache, v_cache, heads, capacity, prm, stream);
 }
 
-bool grouped_attention_tc_eligible(const GroupedAttention& a, const StepPlace& place) {
+static bool grouped_tc_shape(const GroupedAttention& a, const StepPlace& place) {
     auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
-    return a.dim == (uint32_t)PT_HD && a.vdim == (uint32_t)PT_HD && !a.paging.table && a.scale > 0.0f && a.out_ld % 8 == 0 && aligned(a.q) &&
+    return a.dim == (uint32_t)PT_HD && a.vdim == (uint32_t)PT_HD && a.scale > 0.0f && a.out_ld % 8 == 0 && aligned(a.q) &&
            aligned(a.k_cache) && aligned(a.v_cache) && aligned(a.out) && (uint64_t)place.sessions * a.heads * ceil_div(place.chunk, (uint32_t)PT_BQ) < 0x7fffffffull &&
            prefill_attention_tc_eligible(place.sessions, place.chunk, place.position, place.d_position, a.capacity, a.heads, a.dim);
+}
+
+bool grouped_attention_tc_eligible(const GroupedAttention& a, const StepPlace& place) { return !a.paging.table && grouped_tc_shape(a, place); }
+
+bool grouped_attention_exact_tc_eligible(const GroupedAttention& a, const StepPlace& place) {
+    if (a.window || a.softcap > 0.0f || a.score_kind != TNSR_B200_SCORE_SOFTMAX) return false;
+    if (a.paging.table && ((uint64_t)a.paging.pool_pages * a.paging.page_rows > 0x7fffffffull || a.paging.pool_pages == 0 || a.paging.page_rows % 16 != 0)) return false;
+    return grouped_tc_shape(a, place);
 }
 
 int launch_grouped_attention_tc(const GroupedAttention& a, const StepPlace& place, cudaStream_t stream) {
@@ -510,7 +625,9 @@ int launch_grouped_attention_tc(const GroupedAttention& a, const StepPlace& plac
     prm.gate = a.gate;
     prm.gate_ld = a.gate_ld;
     prm.d_status = a.d_status;
+    prm.paging = a.paging;
     const bf16 *q = (const bf16*)a.q, *k = (const bf16*)a.k_cache, *v = (const bf16*)a.v_cache;
+    if (a.engine == 3) return launch_pt_kind<PT_SOFTMAX, false, true>(q, k, v, a.kv_heads, a.capacity, prm, stream);
     if (a.score_kind == TNSR_B200_SCORE_SIGMOID) {
         prm.scale_log2 = -a.scale * 1.4426950408889634f;
         prm.head_bias = a.head_bias;
