@@ -147,7 +147,7 @@ struct TcShape {
     // EPI 4 is the lean form of the narrow tiles (few rows, one tile per CTA: the decode step): half the shared memory
     // (about 115 KB) and at most 112 registers x 192 threads, so that a CTA of it fits on an SM beside a CTA of the lean
     // decode-attention kernel that works on the other half of the batch.
-    // A pair of CTAs (CG 2) holds half of the columns' operand each: 6 stages of 32 KB, or 5 with 16 epilogue warps.
+    // A pair of CTAs (CG 2) holds half of the columns' operand each: 6 stages of 32 KB.
     static constexpr uint32_t A_BYTES = BM * BK * 2;
     static constexpr uint32_t B_BYTES = BN / CG * BK * 2;
     static constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
@@ -528,15 +528,12 @@ __device__ __forceinline__ void epilogue_block(const EpiParams& P, float* stage,
     __syncwarp();  // the buffer is reused by the next block
 }
 
-// CG: CTAs that share a tile.  A pair (CG 2, a cluster) takes 256 x BN: each CTA brings in its own 128 rows and half of the columns' operand,
-// the leader (rank 0) issues products of 256 rows that read both CTAs' shared memory and leave each CTA its 128 rows x BN columns in its own
-// TMEM.  Per CTA and k block that is 128 + BN / 2 rows through L2, TMA and shared memory instead of 128 + BN.
-template <int BN, int MODE, int EPI, int CG>
+template <int BN, int MODE, int EPI>
 __global__ void __launch_bounds__(64 + 32 * EPI, EPI == 4 ? 3 : 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_k,
                const __grid_constant__ CUtensorMap map_v, TcParams prm) {
-    using S = TcShape<BN, EPI, CG>;
+    using S = TcShape<BN, EPI, 1>;
     constexpr bool PLAIN = MODE == GEMM_PLAIN || MODE == GEMM_SCALED;
     constexpr int PER_QUARTER = EPI / 4;             // epilogue warps per TMEM lane quarter
     constexpr uint32_t CHUNK_STRIDE = 32 * PER_QUARTER;
@@ -555,13 +552,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t split = (PLAIN && prm.tma_reduce == 2) ? prm.split_k : 1u;
     const uint32_t num_tiles = prm.tiles_m * prm.tiles_n * split;
-    const uint32_t rank = CG == 2 ? cluster_rank() : 0u, first_tile = blockIdx.x / CG, tile_step = gridDim.x / CG;
     const uint32_t num_kb = (prm.k + BK - 1) / BK;
     const uint32_t kb_per = (num_kb + split - 1) / split;    // the host picks split so that no range is empty
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S::STAGES; ++s) { mbar_init(full_bar + s, 1); mbar_init(empty_bar + s, 1); }
-        for (int s = 0; s < 2; ++s) { mbar_init(acc_full + s, 1); mbar_init(acc_empty + s, CG * EPI); }
+        for (int s = 0; s < 2; ++s) { mbar_init(acc_full + s, 1); mbar_init(acc_empty + s, EPI); }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -569,12 +565,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     pdl_wait();
     pdl_trigger();
     if (warp == 1) {
-        tmem_alloc<CG>(tmem_slot, S::TMEM_COLS);
-        tmem_relinquish<CG>();
+        tmem_alloc(tmem_slot, S::TMEM_COLS);
+        tmem_relinquish();
     }
     tc_fence_before();
-    if (CG == 2) cluster_sync();      // the other CTA's barriers and TMEM are there
-    else __syncthreads();
+    __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
@@ -582,45 +577,31 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         // ---------------- TMA producer ----------------
         if (lane == 0) {
             uint32_t stage = 0, phase = 0;
-            const uint32_t leader_full = CG == 2 ? leader_addr(full_bar) : 0u;
             bool ok = true;
-            for (uint32_t tile = first_tile; ok && tile < num_tiles; tile += tile_step) {
+            for (uint32_t tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
                 uint32_t tm, tn;
                 tile_coords(split == 1 ? tile : tile / split, prm.tiles_m, prm.tiles_n, tm, tn);
-                const int32_t row = (int32_t)((tm * CG + rank) * BM), col = (int32_t)(tn * BN + rank * (BN / CG));
                 const uint32_t kb0 = split == 1 ? 0u : (tile % split) * kb_per, kb1 = min(num_kb, kb0 + kb_per);
                 for (uint32_t kb = kb0; kb < kb1; ++kb) {
                     if (!mbar_wait(empty_bar + stage, phase ^ 1, abort_flag, prm.wait_limit_ns)) { ok = false; break; }
                     uint8_t* sa = smem + stage * S::STAGE_BYTES;
-                    const bool lost = prm.lose_kb && blockIdx.x == 0 && tile == first_tile && kb + 1 == prm.lose_kb;
+                    const bool lost = prm.lose_kb && blockIdx.x == 0 && tile == blockIdx.x && kb + 1 == prm.lose_kb;
                     if (!lost) {   // a lost stage is never filled: its full barrier stays where it is
-                        // a pair's stage is full, at the leader's barrier, when both CTAs' copies have landed
-                        if (rank == 0) mbar_expect_tx(full_bar + stage, CG * S::STAGE_BYTES);
-                        if (CG == 2) {
-                            const uint32_t bar = leader_full + 8 * stage;
-                            tma_load_2d_pair(sa, &map_a, (int32_t)(kb * BK), row, bar);
-                            tma_load_2d_pair(sa + S::A_BYTES, &map_b, (int32_t)(kb * BK), col, bar);
-                        } else {
-                            tma_load_2d(sa, &map_a, (int32_t)(kb * BK), row, full_bar + stage);
-                            tma_load_2d(sa + S::A_BYTES, &map_b, (int32_t)(kb * BK), col, full_bar + stage);
-                        }
+                        mbar_expect_tx(full_bar + stage, S::STAGE_BYTES);
+                        tma_load_2d(sa, &map_a, (int32_t)(kb * BK), (int32_t)(tm * BM), full_bar + stage);
+                        tma_load_2d(sa + S::A_BYTES, &map_b, (int32_t)(kb * BK), (int32_t)(tn * BN), full_bar + stage);
                     }
                     if (++stage == S::STAGES) { stage = 0; phase ^= 1; }
                 }
             }
-            // the leader's signals to a pair's stages have all arrived before this CTA ends
-            for (int s = 0; CG == 2 && ok && s < S::STAGES; ++s) {
-                ok = mbar_wait(empty_bar + stage, phase ^ 1, abort_flag, prm.wait_limit_ns);
-                if (++stage == S::STAGES) { stage = 0; phase ^= 1; }
-            }
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0 && rank == 0) {
-            constexpr uint32_t idesc = make_idesc_bf16(BM * CG, BN);
+        if (lane == 0) {
+            constexpr uint32_t idesc = make_idesc_bf16(BM, BN);
             uint32_t stage = 0, phase = 0, it = 0;
             bool ok = true;
-            for (uint32_t tile = first_tile; ok && tile < num_tiles; tile += tile_step, ++it) {
+            for (uint32_t tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x, ++it) {
                 const uint32_t ab = it & 1, aphase = (it >> 1) & 1;
                 if (!mbar_wait(acc_empty + ab, aphase ^ 1, abort_flag, prm.wait_limit_ns)) { ok = false; break; }
                 tc_fence_after();
@@ -635,12 +616,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
                     for (uint32_t kk = 0; kk < BK / UMMA_K; ++kk) {
                         // advancing K by 16 elements = 32 bytes inside the swizzle row: +2 in the address field
-                        umma_bf16<CG>(d_tmem, adesc + kk * 2, bdesc + kk * 2, idesc, ((kb - kb0) | kk) != 0);
+                        umma_bf16(d_tmem, adesc + kk * 2, bdesc + kk * 2, idesc, ((kb - kb0) | kk) != 0);
                     }
-                    umma_commit<CG>(empty_bar + stage);  // stage reusable once these MMAs have read it
+                    umma_commit(empty_bar + stage);  // stage reusable once these MMAs have read it
                     if (++stage == S::STAGES) { stage = 0; phase ^= 1; }
                 }
-                if (ok) umma_commit<CG>(acc_full + ab);
+                if (ok) umma_commit(acc_full + ab);
             }
         }
     } else {
@@ -653,12 +634,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const uint32_t qkv_pos = (MODE == GEMM_QKV && prm.tma_store)
                                      ? (prm.epi.qkv.d_position ? *prm.epi.qkv.d_position : prm.epi.qkv.position) : 0u;
         bool ok = true;
-        for (uint32_t tile = first_tile; ok && tile < num_tiles; tile += tile_step, ++it) {
+        for (uint32_t tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x, ++it) {
             const uint32_t ab = it & 1, aphase = (it >> 1) & 1;
             uint32_t tm, tn;
             tile_coords(split == 1 ? tile : tile / split, prm.tiles_m, prm.tiles_n, tm, tn);
             const uint32_t ks = split == 1 ? 0u : tile % split;
-            const uint32_t row0 = (tm * CG + rank) * BM + quarter * 32;
+            const uint32_t row0 = tm * BM + quarter * 32;
             // f32 output with a residual: fetch this warp's first block of residual rows while the tile is still
             // being accumulated (the rows are final: only this warp rewrites them, after this read)
             float4 res_pre[8];
@@ -674,7 +655,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             // what the epilogue reads besides the accumulator (the tile's bias columns, the step's position) is asked into
             // L1 while the tile is still being accumulated: a first-touch load after the wait is a whole L2 round trip
             // on the critical path of a one-tile launch (with many tiles per CTA the loads hit anyway: not done there)
-            if (MODE != GEMM_ARGMAX && num_tiles <= tile_step) {
+            if (MODE != GEMM_ARGMAX && num_tiles <= gridDim.x) {
                 const float* bias0 = prm.epi.ep.bias ? prm.epi.ep.bias + (size_t)tn * BN : nullptr;
                 if (bias0 && lane * 32 < (uint32_t)BN && tn * BN + lane * 32 < prm.epi.n)
                     asm volatile("prefetch.global.L1 [%0];" ::"l"(bias0 + lane * 32));
@@ -726,10 +707,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) {
-                if (CG == 2) mbar_arrive_cluster(leader_addr(acc_empty + ab));     // the products that overwrite both CTAs' accumulators are issued there
-                else mbar_arrive(acc_empty + ab);
-            }
+            if (lane == 0) mbar_arrive(acc_empty + ab);
         }
         // bulk reduce operations of this warp must be complete before the CTA gives up its shared memory
         if (((PLAIN && prm.tma_reduce) || prm.tma_store) && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
@@ -745,10 +723,156 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (threadIdx.x == 0 && prm.d_status) atomicCAS(prm.d_status, DEV_OK, DEV_TIMEOUT);
         __syncthreads();
     }
-    if (CG == 2) cluster_sync();      // neither leaves while the other may still signal its barriers or read its operands
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc<CG>(tmem_base, S::TMEM_COLS);
+        tmem_dealloc(tmem_base, S::TMEM_COLS);
+    }
+}
+
+// Pairs of CTAs: a cluster of two takes 256 x 256.  Each CTA brings in its own 128 rows and half of the columns' operand, the leader (rank 0)
+// issues products of 256 rows that read both CTAs' shared memory and leave each CTA its 128 rows x 256 columns in its own TMEM.  Per CTA and
+// k block that is 256 rows through L2, TMA and shared memory instead of 384, and six ring stages instead of four.
+// (A kernel of its own: as a form of the kernel above it cost that one's narrow tiles 8 % -- 93 x 3164 x 6944 35.8 -> 39.3 us -- whatever the
+// form looked like.)
+template <int MODE, int EPI>
+__global__ void __launch_bounds__(64 + 32 * EPI, 1)
+gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                    const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_k,
+                    const __grid_constant__ CUtensorMap map_v, TcParams prm) {
+    constexpr int BN = 256;
+    using S = TcShape<BN, EPI, 2>;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw_addr = smem_u32(smem_raw);
+    uint8_t* smem = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
+    float* stage_tiles = reinterpret_cast<float*>(smem + S::STAGES * S::STAGE_BYTES);
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + S::STAGES * S::STAGE_BYTES + EPI * TC_STAGE_TILE_BYTES);
+    uint64_t* empty_bar = full_bar + S::STAGES;
+    uint64_t* acc_full = empty_bar + S::STAGES;   // [2]
+    uint64_t* acc_empty = acc_full + 2;           // [2]
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank(), first_tile = blockIdx.x / 2, tile_step = gridDim.x / 2;
+    const uint32_t num_tiles = prm.tiles_m * prm.tiles_n, num_kb = (prm.k + BK - 1) / BK;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < S::STAGES; ++s) { mbar_init(full_bar + s, 1); mbar_init(empty_bar + s, 1); }
+        for (int s = 0; s < 2; ++s) { mbar_init(acc_full + s, 1); mbar_init(acc_empty + s, 2 * EPI); }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    pdl_wait();
+    pdl_trigger();
+    if (warp == 1) {
+        tmem_alloc<2>(tmem_slot, S::TMEM_COLS);
+        tmem_relinquish<2>();
+    }
+    tc_fence_before();
+    cluster_sync();               // the other CTA's barriers and TMEM are there
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp == 0) {
+        // ---------------- TMA producer, of each CTA ----------------
+        if (lane == 0) {
+            uint32_t stage = 0, phase = 0;
+            const uint32_t leader_full = leader_addr(full_bar);
+            bool ok = true;
+            for (uint32_t tile = first_tile; ok && tile < num_tiles; tile += tile_step) {
+                uint32_t tm, tn;
+                tile_coords(tile, prm.tiles_m, prm.tiles_n, tm, tn);
+                const int32_t row = (int32_t)((tm * 2 + rank) * BM), col = (int32_t)(tn * BN + rank * (BN / 2));
+                for (uint32_t kb = 0; kb < num_kb; ++kb) {
+                    if (!mbar_wait(empty_bar + stage, phase ^ 1, abort_flag, prm.wait_limit_ns)) { ok = false; break; }
+                    uint8_t* sa = smem + stage * S::STAGE_BYTES;
+                    const bool lost = prm.lose_kb && blockIdx.x == 0 && tile == first_tile && kb + 1 == prm.lose_kb;
+                    if (!lost) {
+                        // a stage is full, at the leader's barrier, when both CTAs' copies have landed
+                        if (rank == 0) mbar_expect_tx(full_bar + stage, 2 * S::STAGE_BYTES);
+                        tma_load_2d_pair(sa, &map_a, (int32_t)(kb * BK), row, leader_full + 8 * stage);
+                        tma_load_2d_pair(sa + S::A_BYTES, &map_b, (int32_t)(kb * BK), col, leader_full + 8 * stage);
+                    }
+                    if (++stage == S::STAGES) { stage = 0; phase ^= 1; }
+                }
+            }
+            // the leader's signals to these stages have all arrived before this CTA ends
+            for (int s = 0; ok && s < S::STAGES; ++s) {
+                ok = mbar_wait(empty_bar + stage, phase ^ 1, abort_flag, prm.wait_limit_ns);
+                if (++stage == S::STAGES) { stage = 0; phase ^= 1; }
+            }
+        }
+    } else if (warp == 1) {
+        // ---------------- MMA issuer, of the leader ----------------
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t idesc = make_idesc_bf16(2 * BM, BN);
+            uint32_t stage = 0, phase = 0, it = 0;
+            bool ok = true;
+            for (uint32_t tile = first_tile; ok && tile < num_tiles; tile += tile_step, ++it) {
+                const uint32_t ab = it & 1, aphase = (it >> 1) & 1;
+                if (!mbar_wait(acc_empty + ab, aphase ^ 1, abort_flag, prm.wait_limit_ns)) { ok = false; break; }
+                tc_fence_after();
+                const uint32_t d_tmem = tmem_base + ab * BN;
+                for (uint32_t kb = 0; kb < num_kb; ++kb) {
+                    if (!mbar_wait(full_bar + stage, phase, abort_flag, prm.wait_limit_ns)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t sa = smem_u32(smem + stage * S::STAGE_BYTES);
+                    const uint64_t adesc = make_kmajor_sw128_desc(sa), bdesc = make_kmajor_sw128_desc(sa + S::A_BYTES);
+#pragma unroll
+                    for (uint32_t kk = 0; kk < BK / UMMA_K; ++kk) umma_bf16<2>(d_tmem, adesc + kk * 2, bdesc + kk * 2, idesc, (kb | kk) != 0);
+                    umma_commit<2>(empty_bar + stage);
+                    if (++stage == S::STAGES) { stage = 0; phase ^= 1; }
+                }
+                if (ok) umma_commit<2>(acc_full + ab);
+            }
+        }
+    } else {
+        // ---------------- epilogue warps, of each CTA: as in the kernel above ----------------
+        const uint32_t quarter = warp & 3, half = (warp - 2) >> 2;
+        float* stage = stage_tiles + (warp - 2) * (TC_STAGE_TILE_BYTES / 4);
+        uint32_t it = 0, store_parity = 0;
+        const bool reduce = (MODE == GEMM_PLAIN || MODE == GEMM_SCALED) && prm.tma_reduce;
+        const uint32_t qkv_pos = (MODE == GEMM_QKV && prm.tma_store)
+                                     ? (prm.epi.qkv.d_position ? *prm.epi.qkv.d_position : prm.epi.qkv.position) : 0u;
+        for (uint32_t tile = first_tile; tile < num_tiles; tile += tile_step, ++it) {
+            const uint32_t ab = it & 1, aphase = (it >> 1) & 1;
+            uint32_t tm, tn;
+            tile_coords(tile, prm.tiles_m, prm.tiles_n, tm, tn);
+            const uint32_t row0 = (tm * 2 + rank) * BM + quarter * 32;
+            if (!mbar_wait(acc_full + ab, aphase, abort_flag, prm.wait_limit_ns)) break;
+            tc_fence_after();
+            const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + ab * BN;
+#pragma unroll 1
+            for (uint32_t c = half * 32; c < BN; c += 8 * EPI) {
+                float acc[32];
+                tmem_ld32(taddr + c, acc);
+                tmem_ld_wait();
+                const uint32_t col0 = tn * BN + c;
+                if (row0 >= prm.epi.m || col0 >= prm.epi.n) continue;
+                if (reduce) epilogue_block_reduce<MODE == GEMM_SCALED>(prm.epi, &map_out, stage, row0, col0, acc, lane);
+                else if (prm.tma_store) epilogue_block_store<MODE>(prm.epi, &map_out, &map_k, &map_v, stage, row0, col0, acc, lane, store_parity++, qkv_pos);
+                else epilogue_block<MODE>(prm.epi, stage, row0, col0, acc, lane);
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(leader_addr(acc_empty + ab));     // where the products that overwrite it are issued
+        }
+        if ((reduce || prm.tma_store) && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    }
+
+    // ---------------- teardown ----------------
+    tc_fence_before();
+    __syncthreads();
+    if (*abort_flag) {
+        const uint64_t start = global_timer_ns();
+        while (global_timer_ns() - start < 200000ull) __nanosleep(1000);
+        if (threadIdx.x == 0 && prm.d_status) atomicCAS(prm.d_status, DEV_OK, DEV_TIMEOUT);
+        __syncthreads();
+    }
+    cluster_sync();               // neither leaves while the other may still signal its barriers or read its operands
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc<2>(tmem_base, S::TMEM_COLS);
     }
 }
 
@@ -779,40 +903,62 @@ static int sm_count() {
     return n;
 }
 
-template <int BN, int MODE, int EPI, int CG>
+template <int BN, int MODE, int EPI>
 static int launch_tc_e(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap* mo, const TcParams& prm, cudaStream_t stream) {
-    using S = TcShape<BN, EPI, CG>;
-    if (const int rc = allow_shared<gemm_tc_kernel<BN, MODE, EPI, CG>>(S::SMEM_BYTES, "gemm_tc attribute")) return rc;
-    const uint32_t tiles = prm.tiles_m * prm.tiles_n * (prm.tma_reduce == 2 ? prm.split_k : 1u);
-    const uint32_t grid = std::min(tiles, (uint32_t)sm_count() / CG) * CG;
-    launch_kernel_clusters(gemm_tc_kernel<BN, MODE, EPI, CG>, dim3(grid), dim3(S::THREADS), S::SMEM_BYTES, CG, stream, ma, mb, mo[0], mo[1], mo[2], prm);
+    using S = TcShape<BN, EPI, 1>;
+    if (const int rc = allow_shared<gemm_tc_kernel<BN, MODE, EPI>>(S::SMEM_BYTES, "gemm_tc attribute")) return rc;
+    uint32_t tiles = prm.tiles_m * prm.tiles_n * (prm.tma_reduce == 2 ? prm.split_k : 1u);
+    uint32_t grid = tiles < (uint32_t)sm_count() ? tiles : (uint32_t)sm_count();
+    launch_kernel(gemm_tc_kernel<BN, MODE, EPI>, dim3(grid), dim3(S::THREADS), S::SMEM_BYTES, stream, ma, mb, mo[0], mo[1], mo[2], prm);
     count_launch();
     return check_launch("gemm_tc");
+}
+
+template <int MODE, int EPI>
+static int launch_pair_e(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap* mo, const TcParams& prm, cudaStream_t stream) {
+    using S = TcShape<256, EPI, 2>;
+    if (const int rc = allow_shared<gemm_tc_pair_kernel<MODE, EPI>>(S::SMEM_BYTES, "gemm_tc_pair attribute")) return rc;
+    const uint32_t grid = 2 * std::min(prm.tiles_m * prm.tiles_n, (uint32_t)sm_count() / 2);
+    launch_kernel_clusters(gemm_tc_pair_kernel<MODE, EPI>, dim3(grid), dim3(S::THREADS), S::SMEM_BYTES, 2, stream, ma, mb, mo[0], mo[1], mo[2], prm);
+    count_launch();
+    return check_launch("gemm_tc_pair");
 }
 
 // Wide tiles with a bf16 epilogue (QKV routing, SwiGLU, column ranges) and a short K: the main loop of a K = 768 tile is shorter than
 // 8 warps need to drain the previous accumulator, so these run 16 epilogue warps (and 3 ring stages instead of 4, which
 // is why longer K keeps 8: there the deeper ring is worth more).
-template <int BN, int MODE, int CG>
+template <int BN, int MODE>
 static int launch_tc_t(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap* mo, const TcParams& prm, cudaStream_t stream) {
     constexpr bool many_warps = BN >= 192 && (MODE == GEMM_QKV || MODE == GEMM_SWIGLU || MODE == GEMM_SEGMENTS);
-    if (many_warps && prm.k <= 1024) return launch_tc_e<BN, MODE, many_warps ? 16 : 8, CG>(ma, mb, mo, prm, stream);
+    if (many_warps && prm.k <= 1024) return launch_tc_e<BN, MODE, many_warps ? 16 : 8>(ma, mb, mo, prm, stream);
     // narrow tiles: one epilogue warp per TMEM lane quarter is all a 32- or 64-column tile can use
-    if (BN <= 64 && MODE != GEMM_ARGMAX) return launch_tc_e<BN, MODE, BN <= 64 ? 4 : 8, CG>(ma, mb, mo, prm, stream);
-    return launch_tc_e<BN, MODE, 8, CG>(ma, mb, mo, prm, stream);
+    if (BN <= 64 && MODE != GEMM_ARGMAX) return launch_tc_e<BN, MODE, BN <= 64 ? 4 : 8>(ma, mb, mo, prm, stream);
+    return launch_tc_e<BN, MODE, 8>(ma, mb, mo, prm, stream);
 }
 
-template <int BN, int CG>
+template <int BN>
 static int launch_tc_mode(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap* mo, const TcParams& prm, GemmMode mode, cudaStream_t stream) {
     switch (mode) {
-        case GEMM_PLAIN: return launch_tc_t<BN, GEMM_PLAIN, CG>(ma, mb, mo, prm, stream);
-        case GEMM_SCALED: return launch_tc_t<BN, GEMM_SCALED, CG>(ma, mb, mo, prm, stream);
-        case GEMM_QKV: return launch_tc_t<BN, GEMM_QKV, CG>(ma, mb, mo, prm, stream);
-        case GEMM_SWIGLU: return launch_tc_t<BN, GEMM_SWIGLU, CG>(ma, mb, mo, prm, stream);
-        case GEMM_ARGMAX: return launch_tc_t<BN, GEMM_ARGMAX, CG>(ma, mb, mo, prm, stream);
-        case GEMM_SEGMENTS: return launch_tc_t<BN, GEMM_SEGMENTS, CG>(ma, mb, mo, prm, stream);
+        case GEMM_PLAIN: return launch_tc_t<BN, GEMM_PLAIN>(ma, mb, mo, prm, stream);
+        case GEMM_SCALED: return launch_tc_t<BN, GEMM_SCALED>(ma, mb, mo, prm, stream);
+        case GEMM_QKV: return launch_tc_t<BN, GEMM_QKV>(ma, mb, mo, prm, stream);
+        case GEMM_SWIGLU: return launch_tc_t<BN, GEMM_SWIGLU>(ma, mb, mo, prm, stream);
+        case GEMM_ARGMAX: return launch_tc_t<BN, GEMM_ARGMAX>(ma, mb, mo, prm, stream);
+        case GEMM_SEGMENTS: return launch_tc_t<BN, GEMM_SEGMENTS>(ma, mb, mo, prm, stream);
     }
     return TNSR_B200_ERR_INVALID_ARGUMENT;
+}
+
+// Products with a long k only: eight epilogue warps are enough.
+static int launch_pair_mode(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap* mo, const TcParams& prm, GemmMode mode, cudaStream_t stream) {
+    switch (mode) {
+        case GEMM_PLAIN: return launch_pair_e<GEMM_PLAIN, 8>(ma, mb, mo, prm, stream);
+        case GEMM_SCALED: return launch_pair_e<GEMM_SCALED, 8>(ma, mb, mo, prm, stream);
+        case GEMM_QKV: return launch_pair_e<GEMM_QKV, 8>(ma, mb, mo, prm, stream);
+        case GEMM_SWIGLU: return launch_pair_e<GEMM_SWIGLU, 8>(ma, mb, mo, prm, stream);
+        case GEMM_SEGMENTS: return launch_pair_e<GEMM_SEGMENTS, 8>(ma, mb, mo, prm, stream);
+        default: return TNSR_B200_ERR_INVALID_ARGUMENT;
+    }
 }
 
 static bool tc_eligible(const bf16* a, uint32_t lda, const bf16* bt, uint32_t k) {
@@ -825,13 +971,14 @@ static bool tc_eligible(const bf16* a, uint32_t lda, const bf16* bt, uint32_t k)
 // (7 % of 8192 x 8192 x 8192, 881 -> 829 us; sustained, under the power cap).  Where waves are equal the wider tile is taken.  Against widths of
 // powers of two and no pairs, us: 32768 x 768 x 768 onto the residual 66 -> 62 (7 waves of 192 for 6 of 256), x 2048 117 -> 105 (pairs),
 // 3885 x 768 x 768 16.4 -> 14.4 and x 2048 22.5 -> 20.5 (one wave of 192), 4096 x 2048 x 5632 84 -> 80, 3000 x 1536 x 6144 53.3 -> 52.0.  A pair
-// with a short k waits for two epilogues at a time: 32768 x 2304 x 768 128 -> 132, 4096 x 8192 x 1024 f32 89 -> 93.
-static void choose_tile(uint32_t m, uint32_t n, uint32_t k, uint32_t& bn, uint32_t& cg) {
+// with a shorter k waits for two epilogues at a time: 32768 x 2304 x 768 128 -> 132, 4096 x 8192 x 1024 f32 89 -> 93, SwiGLU 973 x 1600 -> 4544
+// 47 -> 50.
+static void choose_tile(uint32_t m, uint32_t n, uint32_t k, GemmMode mode, uint32_t& bn, uint32_t& cg) {
     struct Shape { uint32_t bn, cg, rows; };
     static const Shape shapes[] = {{256, 2, 355}, {256, 1, BM + 256}, {192, 1, 322}, {128, 1, BM + 128}, {64, 1, BM + 64}, {32, 1, BM + 32}};
     uint64_t least = ~0ull;
     for (const Shape& s : shapes) {
-        if (s.cg == 2 && k < 1536) continue;
+        if (s.cg == 2 && (k < 2048 || mode == GEMM_ARGMAX)) continue;
         const uint64_t tiles = (uint64_t)ceil_div(m, BM * s.cg) * ceil_div(n, s.bn);
         const uint64_t rows = ceil_div64(tiles, (uint64_t)sm_count() / s.cg) * s.rows;
         if (rows < least) { least = rows; bn = s.bn; cg = s.cg; }
@@ -938,7 +1085,7 @@ static int launch_gemm_impl(const bf16* a, const bf16* bt, void* out, uint32_t l
             return launch_gemm_skinny(a, bt, out, ldc, m, n, k, ep, ep.skinny_ws, ep.skinny_ws_bytes, d_status, stream);
     }
     uint32_t bn = 256, cg = 1;
-    choose_tile(m, n, k, bn, cg);
+    choose_tile(m, n, k, mode, bn, cg);
     if (split_req) { bn = 32; cg = 1; }   // many small tiles: every CTA takes in as little of both operands as possible
     TcParams prm;
     prm.k = k;
@@ -1032,12 +1179,13 @@ static int launch_gemm_impl(const bf16* a, const bf16* bt, void* out, uint32_t l
     }
     prm.epi = P;
     if (mode == GEMM_PLAIN && ep.scale) mode = GEMM_SCALED;
+    if (cg == 2) return launch_pair_mode(ma, mb, mo, prm, mode, stream);
     switch (bn) {
-        case 256: return cg == 2 ? launch_tc_mode<256, 2>(ma, mb, mo, prm, mode, stream) : launch_tc_mode<256, 1>(ma, mb, mo, prm, mode, stream);
-        case 192: return launch_tc_mode<192, 1>(ma, mb, mo, prm, mode, stream);
-        case 128: return launch_tc_mode<128, 1>(ma, mb, mo, prm, mode, stream);
-        case 64: return launch_tc_mode<64, 1>(ma, mb, mo, prm, mode, stream);
-        default: return launch_tc_mode<32, 1>(ma, mb, mo, prm, mode, stream);
+        case 256: return launch_tc_mode<256>(ma, mb, mo, prm, mode, stream);
+        case 192: return launch_tc_mode<192>(ma, mb, mo, prm, mode, stream);
+        case 128: return launch_tc_mode<128>(ma, mb, mo, prm, mode, stream);
+        case 64: return launch_tc_mode<64>(ma, mb, mo, prm, mode, stream);
+        default: return launch_tc_mode<32>(ma, mb, mo, prm, mode, stream);
     }
 }
 
