@@ -420,6 +420,30 @@ def test_decode_attention_live_prefix_and_poisoned_slots(oracle, heads, hd):
     assert np.max(np.abs(got - expected)) <= scale / 128
 
 
+@pytest.mark.parametrize("heads,hd,batch", [(12, 64, 7), (1, 64, 7), (3, 32, 7), (5, 128, 7), (16, 64, 30)])
+def test_decode_attention_of_few_keys_equals_the_streaming_kernel(oracle, heads, hd, batch):
+    """Few keys in all take a launch of clusters; a larger capacity, with the same lengths, the streaming kernel.  Lengths at the edges of a
+    pass, of a cluster's shares, none, the whole capacity; slots past a length hold NaN."""
+    capacity, large = 300, 400000 // (batch * heads) + 16
+    lengths = np.asarray(([1, 63, 64, 65, 129, 0, 300] * 5)[:batch], dtype=np.uint32)
+    rng = np.random.default_rng(71)
+    q = rng.standard_normal((batch, heads * hd)).astype(np.float32)
+    k, v = (rng.standard_normal((batch, capacity, heads * hd)).astype(np.float32) for _ in range(2))
+    for b, n in enumerate(lengths):
+        k[b, n:] = v[b, n:] = np.nan
+    few = run_decode_attention(q, k, v, lengths, heads)
+    wide = [np.full((batch, max(large, capacity), heads * hd), np.nan, dtype=np.float32) for _ in range(2)]
+    for w, x in zip(wide, (k, v)):
+        w[:, :capacity] = x
+    many = run_decode_attention(q, *wide, lengths, heads)
+    want = oracle.decode_attention(bf16_round(q), np.nan_to_num(bf16_round(k)), np.nan_to_num(bf16_round(v)), lengths, heads)
+    assert np.all(few[lengths == 0] == 0.0)
+    # both round an f32 result to bf16 (8 bits: half a unit is at most 2^-8 of the value) and may differ by one such step
+    assert np.max(np.abs(few - many) - np.abs(many) * 2.0 ** -7) <= 1e-5
+    live = lengths > 0
+    assert rel_err(few[live], want[live]) <= 2.0 ** -8 + 1e-5
+
+
 def test_decode_attention_ragged_long_context(oracle):
     """Configuration 3 in miniature: per-session lengths uniform in [1, capacity]."""
     heads, hd, batch, capacity = 16, 64, 12, 4096

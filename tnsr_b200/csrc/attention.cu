@@ -16,6 +16,8 @@
 //
 // HBM traffic per decode step is the live K and V rows once: 4 * d bytes per
 // live key per session (d = heads * head_dim) plus q / out / partials.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace tb {
@@ -737,6 +739,232 @@ decode_attention_kernel(DaParams P) {
     }
 }
 
+// ===========================================================================
+// Few keys in all: one launch, no plan, no workspace
+// ===========================================================================
+// With a few MB of keys the kernel above is a chain of latencies: work list, ring, partial results to L2, counters, merge (12 us for one
+// session of 1000 keys x 12 heads, whose 3 MB are 0.5 us of HBM).  Here a cluster of CTAs shares one (session, head): rank r takes an even share
+// of its keys, 16 bytes per lane straight into registers, up to 64 keys per CTA and pass, the next pass on its way while one is summed up.
+// All keys but a session's newest are older than the previous kernel (the QKV product): their first pass is asked for before it ends.
+// Partial (maximum, sum, numerator) go to rank 0 through distributed shared memory, which adds them in rank order.
+constexpr uint32_t DS_THREADS = 256, DS_WARPS = DS_THREADS / 32;
+constexpr int DS_U = 4;                      // keys of a lane group per pass
+
+struct DsParams {
+    const bf16* q;
+    const bf16* kc;
+    const bf16* vc;
+    const uint32_t* lengths;
+    const uint32_t* d_position;
+    bf16* out;
+    uint32_t extra, capacity, heads, ck;     // ck: CTAs of a cluster
+    float scale_log2;
+    int* d_status;
+    KvPaging paging;
+    uint32_t early;                          // the previous kernel writes no key but every session's newest
+};
+
+__device__ __forceinline__ uint4 ds_load(const bf16* p) {
+    uint4 v;
+    asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void ds_cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void ds_cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
+template <int HD>
+__global__ void __launch_bounds__(DS_THREADS, 3)
+decode_attention_short_kernel(const __grid_constant__ DsParams P) {
+    constexpr uint32_t LPK = HD / 8, KPW = 32 / LPK, PASS = DS_WARPS * KPW;   // lanes per key, keys of a warp and of the CTA side by side
+    constexpr uint32_t PART = HD + 2;
+    __shared__ float warp_part[DS_WARPS][PART], cta_part[8][PART];           // numerator, maximum, sum
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane / LPK, sub = lane % LPK;
+    const uint32_t rank = blockIdx.x % P.ck, unit = blockIdx.x / P.ck, h = unit % P.heads, session = unit / P.heads, d = P.heads * HD;
+    if (P.ck > 1) ds_cluster_arrive();
+    if (!P.early) pdl_wait();
+    uint32_t L = (P.lengths ? __ldcg(P.lengths + session) : (P.d_position ? __ldcg(P.d_position) : 0u)) + P.extra;
+    if (L > P.capacity) {
+        if (threadIdx.x == 0 && P.d_status) atomicCAS(P.d_status, DEV_OK, DEV_BAD_LENGTH);
+        L = P.capacity;
+    }
+    // an even share, but half a pass at least: how many CTAs a short session is given does not show in its bits
+    const uint32_t share = max((L + P.ck - 1) / P.ck, DS_U * PASS / 2), k0 = min(L, rank * share), k1 = min(L, k0 + share);
+    const uint32_t mine = k0 + warp * KPW + grp;        // this lane group's keys: mine, mine + PASS, ...
+    const size_t col = (size_t)h * HD + sub * 8;
+    uint4 kx[DS_U], vx[DS_U];
+    const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+    auto at = [&](uint32_t key) { return kv_row_l2(P.paging, session, key, P.capacity) * d + col; };
+    const uint32_t ahead = P.early ? L - 1 : k1;        // keys below it may be read now (a session of a step has one at least)
+#pragma unroll
+    for (int u = 0; u < DS_U; ++u) {
+        const uint32_t key = mine + u * PASS;
+        kx[u] = vx[u] = none;
+        if (key < k1 && key < ahead) {
+            const size_t o = at(key);
+            kx[u] = ds_load(P.kc + o);
+            vx[u] = ds_load(P.vc + o);
+        }
+    }
+    if (P.early) pdl_wait();
+    pdl_trigger();
+    const uint4 qq = ds_load(P.q + (size_t)session * d + col);
+    if (P.early && k1 == L) {
+#pragma unroll
+        for (int u = 0; u < DS_U; ++u) {
+            if (mine + u * PASS != L - 1) continue;
+            const size_t o = at(L - 1);
+            kx[u] = ds_load(P.kc + o);
+            vx[u] = ds_load(P.vc + o);
+        }
+    }
+    float qf[8], acc[8], m = -INFINITY, l = 0.0f;
+    {
+        const uint32_t w[4] = {qq.x, qq.y, qq.z, qq.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float2 f = bf16x2_to_f32(w[e]);
+            qf[2 * e] = f.x * P.scale_log2;
+            qf[2 * e + 1] = f.y * P.scale_log2;
+            acc[2 * e] = acc[2 * e + 1] = 0.0f;
+        }
+    }
+    for (uint32_t base = 0; k0 + base < k1; base += DS_U * PASS) {
+        float sc[DS_U];
+        float m_new = m;
+        size_t next[DS_U];                       // the next pass: its pages are looked up before this one's sums
+#pragma unroll
+        for (int u = 0; u < DS_U; ++u) {
+            const uint32_t key = mine + base + (DS_U + u) * PASS;
+            next[u] = key < k1 ? at(key) : ~(size_t)0;
+        }
+#pragma unroll
+        for (int u = 0; u < DS_U; ++u) {
+            const uint32_t w[4] = {kx[u].x, kx[u].y, kx[u].z, kx[u].w};
+            float part = 0.0f;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 f = bf16x2_to_f32(w[e]);
+                part = fmaf(qf[2 * e], f.x, part);
+                part = fmaf(qf[2 * e + 1], f.y, part);
+            }
+#pragma unroll
+            for (uint32_t o = LPK / 2; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+            sc[u] = mine + base + u * PASS < k1 ? part : -INFINITY;
+            m_new = fmaxf(m_new, sc[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < DS_U; ++u) kx[u] = next[u] != ~(size_t)0 ? ds_load(P.kc + next[u]) : none;
+        const float m_safe = m_new == -INFINITY ? 0.0f : m_new, corr = ex2(m - m_safe);
+        m = m_new;
+        l *= corr;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] *= corr;
+#pragma unroll
+        for (int u = 0; u < DS_U; ++u) {
+            const float p = ex2(sc[u] - m_safe);        // 0 for keys past the range
+            l += p;
+            const uint32_t w[4] = {vx[u].x, vx[u].y, vx[u].z, vx[u].w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 f = bf16x2_to_f32(w[e]);
+                acc[2 * e] = fmaf(p, f.x, acc[2 * e]);
+                acc[2 * e + 1] = fmaf(p, f.y, acc[2 * e + 1]);
+            }
+            vx[u] = next[u] != ~(size_t)0 ? ds_load(P.vc + next[u]) : none;
+        }
+    }
+    // lane groups of the warp, warps of the CTA, CTAs of the cluster
+    float mm = m;
+#pragma unroll
+    for (uint32_t o = LPK; o < 32; o <<= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, o));
+    const float f = ex2(m - (mm == -INFINITY ? 0.0f : mm));
+    l *= f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[e] *= f;
+#pragma unroll
+    for (uint32_t o = LPK; o < 32; o <<= 1) {
+        l += __shfl_xor_sync(0xffffffffu, l, o);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
+    }
+    if (grp == 0) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) warp_part[warp][sub * 8 + e] = acc[e];
+        if (sub == 0) { warp_part[warp][HD] = mm; warp_part[warp][HD + 1] = l; }
+    }
+    __syncthreads();
+    if (threadIdx.x >= HD && P.ck == 1) return;
+    // sums `parts` partials of dimension c: (numerator, maximum, sum)
+    auto join = [&](const float (*part)[PART], uint32_t parts, uint32_t c) {
+        float top = -INFINITY, num = 0.0f, sum = 0.0f;
+        for (uint32_t i = 0; i < parts; ++i) top = fmaxf(top, part[i][HD]);
+        const float safe = top == -INFINITY ? 0.0f : top;
+        for (uint32_t i = 0; i < parts; ++i) {
+            const float w = ex2(part[i][HD] - safe);
+            num = fmaf(part[i][c], w, num);
+            sum = fmaf(part[i][HD + 1], w, sum);
+        }
+        return make_float3(num, top, sum);
+    };
+    const uint32_t c = threadIdx.x;
+    float3 all = make_float3(0.0f, -INFINITY, 0.0f);
+    if (c < HD) all = join(warp_part, DS_WARPS, c);
+    if (P.ck > 1) {
+        ds_cluster_wait();                       // rank 0 is there
+        if (c < HD) {
+            uint32_t to;
+            const uint32_t from = (uint32_t)__cvta_generic_to_shared(&cta_part[rank][0]);
+            asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(to) : "r"(from));
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to + 4 * c), "f"(all.x) : "memory");
+            if (c == 0) {
+                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to + 4 * HD), "f"(all.y) : "memory");
+                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to + 4 * HD + 4), "f"(all.z) : "memory");
+            }
+        }
+        ds_cluster_arrive();
+        ds_cluster_wait();
+        if (rank != 0 || c >= HD) return;
+        all = join(cta_part, P.ck, c);
+    }
+    // a session without keys: zeros
+    P.out[(size_t)session * d + h * HD + c] = __float2bfloat16_rn(L ? all.x / all.z : 0.0f);
+}
+
+static int da_sm_count() {
+    static int n = 0;
+    if (!n) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        if (n <= 0) n = 148;
+    }
+    return n;
+}
+
+// CTAs per (session, head): what fits the GPU at once, three per SM, and at most a portable cluster.
+static uint32_t ds_cluster(uint32_t units) { return std::max(1u, std::min(8u, 3u * (uint32_t)da_sm_count() / units)); }
+
+// Whether the launch above is the faster one: `longest` keys that a session can have, `chained` in a session's step (no plan to save there, as
+// that is made once for all layers).  Its CTAs are not balanced by length and their many short streams stop at 4 TB/s, so what ends it is keys x
+// heads in all.  us with the streaming kernel / here, B200:
+//     operator, sessions x heads x capacity, lengths anywhere     a step of 12 layers x 12 heads, sessions @ keys
+//       1 x 12 x 64     13.8 / 6.2     16 x 12 x 1000  20.7 / 15.9    1 @ 100   295 / 241     16 @ 1000  408 / 390
+//       1 x 12 x 1000   17.1 / 7.3     32 x 12 x 1000  23.6 / 22.2    1 @ 1000  332 / 247     32 @ 100   401 / 353
+//       1 x 16 x 4096   28.5 / 11.6    48 x 12 x 900   25.7 / 24.5    4 @ 1000  349 / 284     32 @ 1000  554 / 593
+//       4 x 12 x 4096   25.7 / 15.4    64 x 16 x 300   22.3 / 18.4    8 @ 300   327 / 275     64 @ 500   638 / 689
+//       8 x 12 x 2048   23.2 / 15.0    16 x 16 x 4096  34.9 / 49.3    8 @ 1000  363 / 316     48, lengths to 900  781 / 955
+//       16 x 12 x 300   18.3 / 9.4     64 x 16 x 1000  34.8 / 39.3    16 @ 300  361 / 312     16, lengths to 1000 489 / 498
+static bool ds_pays(uint32_t batch, uint32_t heads, uint32_t longest, bool chained) {
+    return (uint64_t)batch * heads * longest <= (chained ? 180000u : 400000u);
+}
+
+template <int HD>
+static int launch_ds(const DsParams& P, uint32_t units, cudaStream_t stream) {
+    launch_kernel_clusters(decode_attention_short_kernel<HD>, dim3(units * P.ck), dim3(DS_THREADS), 0, P.ck, stream, P);
+    count_launch();
+    return check_launch("decode_attention_short");
+}
+
 template <int HD, int HPW, int KS>
 static int launch_da_t(const DaParams& P, uint32_t threads, size_t smem, uint32_t grid, cudaStream_t stream) {
     static size_t configured[64] = {};
@@ -768,17 +996,6 @@ static int launch_da_t(const DaParams& P, uint32_t threads, size_t smem, uint32_
     return check_launch("decode_attention");
 }
 
-static int da_sm_count() {
-    static int n = 0;
-    if (!n) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 148;
-    }
-    return n;
-}
-
 // lengths may be nullptr: then every session holds (d_position ? *d_position : 0) + extra keys.
 int launch_decode_attention_ex(const bf16* q, const bf16* k_cache, const bf16* v_cache, const uint32_t* d_lengths,
                                const uint32_t* d_position, uint32_t extra, bf16* out, void* workspace,
@@ -799,6 +1016,22 @@ int launch_decode_attention_ex(const bf16* q, const bf16* k_cache, const bf16* v
     if (L.bytes > workspace_bytes) {
         set_thread_error("decode attention: workspace too small");
         return TNSR_B200_ERR_INVALID_ARGUMENT;
+    }
+    if (paging && paging->table && (paging->page_rows == 0 || paging->page_rows % DA_KS != 0)) {
+        set_thread_error("decode attention: the page size must be a multiple of 16 rows");
+        return TNSR_B200_ERR_INVALID_ARGUMENT;
+    }
+    if (!lean && !t_attention_timer && ds_pays(batch, heads, capacity, t_pdl && extra > 0)) {
+        DsParams S;
+        S.q = q; S.kc = k_cache; S.vc = v_cache; S.out = out;
+        S.lengths = d_lengths; S.d_position = d_position; S.extra = extra;
+        S.capacity = capacity; S.heads = heads; S.ck = ds_cluster(batch * heads);
+        S.scale_log2 = (1.0f / sqrtf((float)head_dim)) * 1.4426950408889634f;
+        S.d_status = d_status;
+        if (paging && paging->table) S.paging = *paging;
+        S.early = t_pdl && extra > 0;
+        return head_dim == 32 ? launch_ds<32>(S, batch * heads, stream) : head_dim == 64 ? launch_ds<64>(S, batch * heads, stream)
+                                                                                        : launch_ds<128>(S, batch * heads, stream);
     }
     uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
     uint32_t* header = reinterpret_cast<uint32_t*>(ws);
@@ -853,13 +1086,7 @@ int launch_decode_attention_ex(const bf16* q, const bf16* k_cache, const bf16* v
     P.d_status = d_status;
     P.wait_limit_ns = g_wait_limit_ns.load(std::memory_order_relaxed);
     P.early = !plan && t_pdl;
-    if (paging && paging->table) {
-        if (paging->page_rows == 0 || paging->page_rows % DA_KS != 0) {
-            set_thread_error("decode attention: the page size must be a multiple of 16 rows");
-            return TNSR_B200_ERR_INVALID_ARGUMENT;
-        }
-        P.paging = *paging;
-    }
+    if (paging && paging->table) P.paging = *paging;
     const uint32_t threads = (consumers + 1) * 32;
     if (lean) {
         if (hpw == 1) {
