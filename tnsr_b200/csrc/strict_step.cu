@@ -10,8 +10,9 @@
 //
 // Arithmetic is strict.cu's, operation by operation: all threads form the rounded products of an output side by side in shared
 // memory, one lane per output adds them up in order.  What is left is chains: sums, and the f64 exp and log of a LayerNorm and of the
-// scores.  One step of one session at 4 x 128 columns and 60 keys, ids in to logits out, B200: 197 us in 38 launches, 125 us here; 48
-// sessions 246 and 154 us.
+// scores -- and instructions: straight-line code that runs once per phase does not stay in the nearest instruction cache, so a layer's phases are
+// rounds of one loop and the sums are a function.  (All phases inlined 84 us a step on the device, so 63; inlined, with loads further ahead, 115.)
+// One step of one session at 4 x 128 columns and 60 keys, ids in to logits out, B200: 197 us in 38 launches, 105 us here; 48 sessions 246 and 140 us.
 #include <algorithm>
 
 #include "strict.cuh"
@@ -29,6 +30,7 @@ constexpr uint32_t SS_VALUES = 8192;        // weight x value products of a head
 struct SsParams {
     StrictStepArgs a;
     uint32_t sessions_per_cluster;
+    float part;                          // 1 / d, if that is exact
 };
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
@@ -98,71 +100,88 @@ __device__ __forceinline__ void form_products(const Matrix& m, const Share& s, c
     for (; p < k; p += 4 * groups) put(p, weights4(w + (size_t)p * m.width, m.width));
 }
 
-// sum of terms[0 .. n) in order from a zero start, n a multiple of 4 (16-byte aligned): sixteen loads ahead of sixteen sums.
-__device__ __forceinline__ float add_up(const float* terms, uint32_t n) {
-    const float4* t = reinterpret_cast<const float4*>(terms);
+// sum of terms[0 .. n) in order from a zero start, n a multiple of 4, terms 16-byte aligned in shared memory: eight values on their way while
+// eight are added.
+__device__ __noinline__ float add_up(uint32_t terms, uint32_t n) {
+    auto quad = [](uint32_t at) {
+        float4 v;
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
+        return v;
+    };
     float sum = 0.0f;
-    float4 v[4];
-    const uint32_t quads = n / 4, whole = quads & ~3u;
-#pragma unroll
-    for (uint32_t i = 0; i < 4; ++i) v[i] = t[min(i, quads - 1)];
-    for (uint32_t q = 0; q < whole; q += 4) {
-        float4 u[4];
-#pragma unroll
-        for (uint32_t i = 0; i < 4; ++i) u[i] = t[min(q + 4 + i, quads - 1)];
-#pragma unroll
-        for (uint32_t i = 0; i < 4; ++i) {
-            sum = sum + v[i].x;
-            sum = sum + v[i].y;
-            sum = sum + v[i].z;
-            sum = sum + v[i].w;
-            v[i] = u[i];
+    auto add = [&](const float4& v) {
+        sum = sum + v.x;
+        sum = sum + v.y;
+        sum = sum + v.z;
+        sum = sum + v.w;
+    };
+    const uint32_t end = terms + 4 * n;
+    uint32_t at = terms;
+    if (at + 32 <= end) {
+        float4 u0 = quad(at), u1 = quad(at + 16);
+        at += 32;
+#pragma unroll 1
+        for (; at + 64 <= end; at += 64) {
+            const float4 v0 = quad(at), v1 = quad(at + 16);
+            add(u0);
+            add(u1);
+            u0 = quad(at + 32);
+            u1 = quad(at + 48);
+            add(v0);
+            add(v1);
         }
+        add(u0);
+        add(u1);
     }
-    for (uint32_t q = whole; q < quads; ++q) {
-        const float4 x = t[q];
-        sum = sum + x.x;
-        sum = sum + x.y;
-        sum = sum + x.z;
-        sum = sum + x.w;
-    }
+#pragma unroll 1
+    for (; at < end; at += 16) add(quad(at));
     return sum;
 }
+__device__ __forceinline__ float add_up(const float* terms, uint32_t n) { return add_up((uint32_t)__cvta_generic_to_shared(terms), n); }
 
-// LayerNorm of row r (x + r * d) by warp r, in strict.cu's order, into xs; `term`: d floats per row.
-__device__ __forceinline__ void norm_rows(float* xs, float* term, const float* x, uint32_t stride, const float* __restrict__ w, const float* __restrict__ b,
-                                          uint32_t rows, uint32_t d, float eps) {
-    const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    if (warp >= rows) return;
-    constexpr uint32_t V = SS_MAX_D / 32;
-    const float nf = (float)d;
-    float v[V], wv[V], bv[V];
-    float* mine = term + warp * d;
+// Scale and shift of a LayerNorm, asked for before the phase's barrier: a warp per row, lane l holds columns l, l + 32, ...
+template <uint32_t V>
+__device__ __forceinline__ void ask_norm(const float* __restrict__ w, const float* __restrict__ b, uint32_t rows, uint32_t d, float (&wv)[V], float (&bv)[V]) {
+    if (threadIdx.x / 32 >= rows) return;
 #pragma unroll
     for (uint32_t i = 0; i < V; ++i) {
-        const uint32_t c = lane + 32 * i;
-        wv[i] = c < d ? __ldg(w + c) : 0.0f;
-        bv[i] = c < d ? __ldg(b + c) : 0.0f;
+        const uint32_t c = threadIdx.x % 32 + 32 * i;
+        if (c < d) wv[i] = __ldg(w + c), bv[i] = __ldg(b + c);
     }
+}
+// LayerNorm of row r (x + r * stride) by warp r, in strict.cu's order, into xs; `term`: d floats per row.  With a width of 2^n a term is divided
+// by multiplying with `part` = 2^-n (0: another width): the same value, rounded once.
+template <uint32_t V>
+__device__ __forceinline__ void norm_rows(float* xs, float* term, const float* x, uint32_t stride, const float (&wv)[V], const float (&bv)[V],
+                                          uint32_t rows, uint32_t d, float eps, float part) {
+    const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    if (warp >= rows) return;
+    const float nf = (float)d;
+    const bool whole = part != 0.0f;
+    float v[V], t[V], mean = 0.0f, inv = 0.0f;
+    float* mine = term + warp * d;
 #pragma unroll
     for (uint32_t i = 0; i < V; ++i)
-        if (lane + 32 * i < d) {
-            v[i] = x[warp * stride + lane + 32 * i];
-            mine[lane + 32 * i] = v[i] / nf;
+        if (lane + 32 * i < d) t[i] = v[i] = x[warp * stride + lane + 32 * i];
+#pragma unroll 1
+    for (uint32_t pass = 0; pass < 2; ++pass) {      // mean, variance
+#pragma unroll
+        for (uint32_t i = 0; i < V; ++i)
+            if (lane + 32 * i < d) mine[lane + 32 * i] = whole ? t[i] * part : t[i] / nf;
+        __syncwarp();
+        const float sum = __shfl_sync(0xffffffffu, lane == 0 ? add_up(mine, d) : 0.0f, 0);
+        __syncwarp();
+        if (pass) {
+            inv = strict_expf(strict_logf(sum + eps) * -0.5f);
+            break;
         }
-    __syncwarp();
-    const float mean = __shfl_sync(0xffffffffu, lane == 0 ? add_up(mine, d) : 0.0f, 0);
-    __syncwarp();
+        mean = sum;
 #pragma unroll
-    for (uint32_t i = 0; i < V; ++i)
-        if (lane + 32 * i < d) {
+        for (uint32_t i = 0; i < V; ++i) {
             const float c = v[i] - mean;
-            const float sq = c * c;
-            mine[lane + 32 * i] = sq / nf;
+            t[i] = c * c;
         }
-    __syncwarp();
-    const float var = __shfl_sync(0xffffffffu, lane == 0 ? add_up(mine, d) : 0.0f, 0);
-    const float inv = strict_expf(strict_logf(var + eps) * -0.5f);
+    }
 #pragma unroll
     for (uint32_t i = 0; i < V; ++i)
         if (lane + 32 * i < d) {
@@ -197,7 +216,7 @@ __device__ __forceinline__ float attend(const StrictStepArgs& a, const KV* kb, c
     for (uint32_t j = tid; j < total; j += SS_THREADS) {
         float sum = 0.0f;
         const KV* row = kb + (size_t)j * d;
-#pragma unroll 8
+#pragma unroll 4
         for (uint32_t c = 0; c < hd; c += 4) {
             const float4 k = load_kv4(row + c), v = *reinterpret_cast<const float4*>(qs + c);
             sum = sum + v.x * k.x;
@@ -220,7 +239,7 @@ __device__ __forceinline__ float attend(const StrictStepArgs& a, const KV* kb, c
     for (uint32_t j = tid; j < total; j += SS_THREADS) sc[j] = strict_expf(sc[j] - mx);
     __syncthreads();
     if (tid == 0) {
-        float sum = total >= 4 ? add_up(sc, total & ~3u) : 0.0f;
+        float sum = add_up(sc, total & ~3u);
         for (uint32_t j = total & ~3u; j < total; ++j) sum = sum + sc[j];
         red[SS_WARPS] = sum;
     }
@@ -245,20 +264,9 @@ __device__ __forceinline__ float attend(const StrictStepArgs& a, const KV* kb, c
         for (; e < keys * quads; e += SS_THREADS) put(e, load_kv4(vb + (size_t)(j0 + e / quads) * d + 4 * (e % quads)));
         __syncthreads();
         if (tid < hd) {
-            float v[16];
-#pragma unroll
-            for (uint32_t i = 0; i < 16; ++i) v[i] = prod[min(i, keys - 1) * hd + tid];
-            uint32_t j = 0;
-            for (; j + 16 <= keys; j += 16) {
-                float u[16];
-#pragma unroll
-                for (uint32_t i = 0; i < 16; ++i) u[i] = prod[min(j + 16 + i, keys - 1) * hd + tid];
-#pragma unroll
-                for (uint32_t i = 0; i < 16; ++i) { acc = acc + v[i]; v[i] = u[i]; }
-            }
-#pragma unroll
-            for (uint32_t i = 0; i < 16; ++i)
-                if (j + i < keys) acc = acc + v[i];
+            const float* p = prod + tid;
+#pragma unroll 8
+            for (uint32_t j = 0; j < keys; ++j, p += hd) acc = acc + *p;
         }
     }
     __syncthreads();
@@ -268,7 +276,8 @@ __device__ __forceinline__ float attend(const StrictStepArgs& a, const KV* kb, c
 // Shared floats of one row: residual, queries, attention output, normalised row, its terms, hidden row.
 __host__ __device__ __forceinline__ uint32_t floats_per_row(uint32_t d, uint32_t f) { return 5 * d + f; }
 
-template <typename KV>
+// V: columns of a row that a lane of a LayerNorm holds.
+template <typename KV, uint32_t V>
 __global__ void __launch_bounds__(SS_THREADS, 1)
 strict_step_kernel(const __grid_constant__ SsParams P) {
     extern __shared__ __align__(16) float smem[];
@@ -284,7 +293,6 @@ strict_step_kernel(const __grid_constant__ SsParams P) {
     float* ff = term + rows * d;             // [rows][f]
     float* prod = ff + rows * f;
     float4 ahead[2];
-
     for (uint32_t r = 0; r < rows; ++r) {    // every CTA keeps the residual rows
         const uint32_t id = a.ids[row0 + r], position = a.position + r % a.chunk;
         if (id >= a.vocab && tid == 0 && rank == 0) atomicCAS(a.d_status, DEV_OK, DEV_TOKEN_RANGE);
@@ -292,69 +300,95 @@ strict_step_kernel(const __grid_constant__ SsParams P) {
     }
     __syncthreads();
     cluster_arrive();
-    // One phase: rows of k values (the LayerNorm of h, or `src`) times the CTA's columns; `store` takes the sums.
-    auto phase = [&](const Matrix& m, const float* src, const float* lnw, const float* lnb, auto&& store) {
-        ask_weights(m, share_of(m.n, rank, 0), ahead);
+    // A layer is four products, each of rows of k values (a LayerNorm of h, or what the phase before left) and the CTA's columns of a matrix;
+    // attention follows the first one.  The round behind the last layer ends with the rows of the output head.
+    enum : uint32_t { QKV = 0, OUT = 1, UP = 2, DOWN = 3 };
+    const uint32_t products = 4 * a.num_layers, wanted = a.last_only ? ns : rows;
+    auto matrix = [&](uint32_t step) {
+        const StrictStepLayer& L = P.a.layers[step / 4];
+        switch (step % 4) {
+            case QKV: return Matrix{L.wq, L.wk, L.wv, d, 3 * d, d};
+            case OUT: return Matrix{L.wo, nullptr, nullptr, d, d, d};
+            case UP: return Matrix{L.w_in, nullptr, nullptr, d, f, f};
+            default: return Matrix{L.w_out, nullptr, nullptr, f, d, d};
+        }
+    };
+#pragma unroll 1
+    for (uint32_t step = 0;; ++step) {
+        const uint32_t kind = step % 4;
+        const bool head = step == products;
+        const StrictStepLayer& L = P.a.layers[head ? 0 : step / 4];
+        const Matrix m = matrix(head ? 0 : step);
+        const float* bias_of = kind == OUT ? L.bo : kind == UP ? L.b_in : L.b_out;
+        float wv[V], bv[V];
+        if (!head) ask_weights(m, share_of(m.n, rank, 0), ahead);
+        if (head) ask_norm(a.fnw, a.fnb, wanted, d, wv, bv);
+        else if (kind == QKV || kind == UP) ask_norm(kind == QKV ? L.ln1w : L.ln2w, kind == QKV ? L.ln1b : L.ln2b, rows, d, wv, bv);
+        float bias = 0.0f;
+        auto ask_bias = [&](const Share& s) {
+            if (warp >= rows || lane >= s.cols) return;
+            const uint32_t col = s.col0 + lane;
+            bias = kind != QKV ? __ldg(bias_of + col) : __ldg(col < d ? L.bq + col : col < 2 * d ? L.bk + (col - d) : L.bv + (col - 2 * d));
+        };
+        if (!head) ask_bias(share_of(m.n, rank, 0));
         cluster_wait();
-        if (lnw) norm_rows(xs, term, h, d, lnw, lnb, rows, d, a.eps);
-        const float* x = lnw ? xs : src;
+        if (head && !a.logits) break;
+        if (head) norm_rows(xs, term, a.last_only ? h + (a.chunk - 1) * d : h, a.last_only ? a.chunk * d : d, wv, bv, wanted, d, a.eps, P.part);
+        else if (kind == QKV || kind == UP) norm_rows(xs, term, h, d, wv, bv, rows, d, a.eps, P.part);
+        if (head) break;
+        const float* x = kind == OUT ? att : kind == DOWN ? ff : xs;
         const uint32_t rounds = (per_cta(m.n) + SS_COLS - 1) / SS_COLS;
+#pragma unroll 1
         for (uint32_t round = 0; round < rounds; ++round) {
             const Share s = share_of(m.n, rank, round);
+            if (round) ask_bias(s);
             __syncthreads();
             form_products(m, s, ahead, round == 0, x, prod, rows);
             __syncthreads();
-            if (warp < rows && lane < s.cols) store(warp, s.col0 + lane, add_up(prod + (((warp << s.log2_pad) + lane) * (m.k + 4)), m.k));
-        }
-        cluster_arrive();
-    };
-    for (uint32_t l = 0; l < a.num_layers; ++l) {
-        const StrictStepLayer& L = P.a.layers[l];
-        KV* kcache = reinterpret_cast<KV*>(L.kcache);
-        KV* vcache = reinterpret_cast<KV*>(L.vcache);
-        phase(Matrix{L.wq, L.wk, L.wv, d, 3 * d, d}, nullptr, L.ln1w, L.ln1b, [&](uint32_t r, uint32_t col, float sum) {
-            const uint32_t part = col < d ? 0 : col < 2 * d ? 1 : 2, c = col - part * d;
-            float v = sum + (part == 0 ? L.bq : part == 1 ? L.bk : L.bv)[c];
-            if (a.round_bf16) v = round_to_bf16(v);
-            if (part == 0) {
-                store_to_all(q + r * d + c, v);
+            if (warp >= rows || lane >= s.cols) continue;
+            const uint32_t r = warp, col = s.col0 + lane;
+            const float sum = add_up(prod + (((warp << s.log2_pad) + lane) * (m.k + 4)), m.k);
+            float v = sum + bias;
+            float* to = h + r * d + col;
+            if (kind == QKV) {
+                const uint32_t part = col < d ? 0 : col < 2 * d ? 1 : 2, c = col - part * d;
+                if (a.round_bf16) v = round_to_bf16(v);
+                to = q + r * d + c;
+                if (part != 0) {
+                    KV* cache = reinterpret_cast<KV*>(part == 1 ? L.kcache : L.vcache);
+                    const size_t at = ((size_t)(s0 + r / a.chunk) * a.capacity + a.position + r % a.chunk) * d + c;
+                    if constexpr (sizeof(KV) == 2) cache[at] = __float2bfloat16_rn(v);
+                    else cache[at] = v;
+                    continue;
+                }
+            } else if (kind == UP) {
+                v = a.activation == ACT_GELU ? strict_gelu(v) : fmaxf(v, 0.0f);
+                to = ff + r * f + col;
             } else {
-                KV* cache = part == 1 ? kcache : vcache;
-                const size_t at = ((size_t)(s0 + r / a.chunk) * a.capacity + a.position + r % a.chunk) * d + c;
-                if constexpr (sizeof(KV) == 2) cache[at] = __float2bfloat16_rn(v);
-                else cache[at] = v;
+                v = *to + v;
             }
-        });
-        cluster_wait();
-        for (uint32_t i = rank; i < rows * a.heads; i += SS_CTAS) {
-            const uint32_t r = i / a.heads, head = i % a.heads;
-            const size_t base = (size_t)(s0 + r / a.chunk) * a.capacity * d + (size_t)head * hd;
-            const uint32_t at = r * d + head * hd;
-            const float v = attend<KV>(a, kcache + base, vcache + base, q + at, min(a.position + r % a.chunk + 1, a.capacity), prod);
-            if (tid < hd) store_to_all(att + at + tid, v);
+            store_to_all(to, v);
         }
         cluster_arrive();
-        auto add_to_residual = [&](const float* bias) {
-            return [&, bias](uint32_t r, uint32_t col, float sum) {
-                const float v = sum + bias[col];
-                store_to_all(h + r * d + col, h[r * d + col] + v);
-            };
-        };
-        phase(Matrix{L.wo, nullptr, nullptr, d, d, d}, att, nullptr, nullptr, add_to_residual(L.bo));
-        phase(Matrix{L.w_in, nullptr, nullptr, d, f, f}, nullptr, L.ln2w, L.ln2b, [&](uint32_t r, uint32_t col, float sum) {
-            const float v = sum + L.b_in[col];
-            store_to_all(ff + r * f + col, a.activation == ACT_GELU ? strict_gelu(v) : fmaxf(v, 0.0f));
-        });
-        phase(Matrix{L.w_out, nullptr, nullptr, f, d, d}, ff, nullptr, nullptr, add_to_residual(L.b_out));
+        if (kind != QKV) continue;
+        const KV* kcache = reinterpret_cast<const KV*>(L.kcache);
+        const KV* vcache = reinterpret_cast<const KV*>(L.vcache);
+        cluster_wait();
+#pragma unroll 1
+        for (uint32_t i = rank; i < rows * a.heads; i += SS_CTAS) {
+            const uint32_t r = i / a.heads, head_at = r * d + i % a.heads * hd;
+            const size_t base = (size_t)(s0 + r / a.chunk) * a.capacity * d + (size_t)(i % a.heads) * hd;
+            const float v = attend<KV>(a, kcache + base, vcache + base, q + head_at, min(a.position + r % a.chunk + 1, a.capacity), prod);
+            if (tid < hd) store_to_all(att + head_at + tid, v);
+        }
+        cluster_arrive();
     }
-    cluster_wait();
     if (!a.logits) {                        // a large vocabulary: the head is a launch of its own
         for (uint32_t i = rank * SS_THREADS + tid; i < rows * d; i += SS_CTAS * SS_THREADS) a.h[(size_t)row0 * d + i] = h[i];
         return;
     }
     // the tied head: rows of the token table [vocab, d], so lanes run along d; every row, or the last one of each session
-    const uint32_t wanted = a.last_only ? ns : rows, per = per_cta(a.vocab), col0 = rank * per, cols = col0 < a.vocab ? min(per, a.vocab - col0) : 0u;
-    norm_rows(xs, term, a.last_only ? h + (a.chunk - 1) * d : h, a.last_only ? a.chunk * d : d, a.fnw, a.fnb, wanted, d, a.eps);
+    const uint32_t per = per_cta(a.vocab), col0 = rank * per, cols = col0 < a.vocab ? min(per, a.vocab - col0) : 0u;
     for (uint32_t c0 = 0; c0 < cols; c0 += SS_COLS) {
         const uint32_t nc = min(SS_COLS, cols - c0);
         __syncthreads();
@@ -387,8 +421,8 @@ uint32_t rows_that_fit(const StrictStepArgs& a) {
     return std::min({SS_WARPS, floats / (each + products), (floats - head) / each});
 }
 
-template <typename KV>
-int clusters_at_once() {
+template <typename KV, uint32_t V>
+int clusters_at_once_kind() {
     static std::atomic<int> known[64];      // per device: clusters of 16 CTAs that run side by side, -1: none, 0: not asked yet
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
@@ -404,15 +438,18 @@ int clusters_at_once() {
         attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        const bool fits = cudaFuncSetAttribute(strict_step_kernel<KV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SS_SMEM) == cudaSuccess &&
-                          cudaFuncSetAttribute(strict_step_kernel<KV>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                          cudaOccupancyMaxActiveClusters(&n, strict_step_kernel<KV>, &cfg) == cudaSuccess && n > 0;
+        const bool fits = cudaFuncSetAttribute(strict_step_kernel<KV, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SS_SMEM) == cudaSuccess &&
+                          cudaFuncSetAttribute(strict_step_kernel<KV, V>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                          cudaOccupancyMaxActiveClusters(&n, strict_step_kernel<KV, V>, &cfg) == cudaSuccess && n > 0;
         if (!fits) cudaGetLastError();
         n = fits ? n : -1;
         known[dev].store(n, std::memory_order_release);
     }
     return std::max(0, n);
 }
+
+template <typename KV>
+int clusters_at_once(uint32_t d) { return d <= 128 ? clusters_at_once_kind<KV, 4>() : clusters_at_once_kind<KV, SS_MAX_D / 32>(); }
 
 }  // namespace
 
@@ -430,7 +467,7 @@ constexpr uint32_t SS_MAX_QUERIES = 4 * SS_CTAS, SS_MANY_KEYS = 128;
 bool strict_step_supported(const StrictStepArgs& a, bool kv_bf16) {
     if (!a.num_layers || a.num_layers > SS_MAX_LAYERS || a.d > SS_MAX_D || a.d % 4 || a.f % 4 || a.d % a.heads || (a.d / a.heads) % 4) return false;
     if ((4ull * a.d * a.d + 2ull * a.d * a.f) * 4 > SS_MAX_LAYER_BYTES || a.capacity > 16384) return false;
-    const int at_once = kv_bf16 ? clusters_at_once<bf16>() : clusters_at_once<float>();
+    const int at_once = kv_bf16 ? clusters_at_once<bf16>(a.d) : clusters_at_once<float>(a.d);
     if (at_once <= 0) return false;
     const uint64_t rows = (uint64_t)ceil_div(a.sessions, (uint32_t)at_once) * a.chunk;
     if (a.chunk >= 8 && rows * a.heads > SS_MAX_QUERIES && a.position + a.chunk > SS_MANY_KEYS) return false;
@@ -444,7 +481,8 @@ template <typename KV>
 static int launch_strict_step_kind(const StrictStepArgs& a, cudaStream_t stream) {
     SsParams P;
     P.a = a;
-    const int at_once = std::max(1, clusters_at_once<KV>());
+    const int at_once = std::max(1, clusters_at_once<KV>(a.d));
+    P.part = (a.d & (a.d - 1)) == 0 ? 1.0f / (float)a.d : 0.0f;
     P.sessions_per_cluster = ceil_div(a.sessions, (uint32_t)at_once);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ceil_div(a.sessions, P.sessions_per_cluster) * SS_CTAS);
@@ -457,7 +495,8 @@ static int launch_strict_step_kind(const StrictStepArgs& a, cudaStream_t stream)
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, strict_step_kernel<KV>, P);
+    if (a.d <= 128) cudaLaunchKernelEx(&cfg, strict_step_kernel<KV, 4>, P);
+    else cudaLaunchKernelEx(&cfg, strict_step_kernel<KV, SS_MAX_D / 32>, P);
     count_launch();
     return check_launch("strict_step");
 }
