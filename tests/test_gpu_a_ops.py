@@ -337,6 +337,33 @@ def test_gemm_bf16_tiles_of_pairs_and_of_192_columns(shape, form):
     assert float(err.max()) <= 2e-3
 
 
+@pytest.mark.parametrize("m,n,k", [(8, 4096, 4096), (1, 512, 512), (4, 2048, 4096), (5, 4096, 1032), (48, 2304, 768), (200, 768, 2048), (600, 9472, 2048)])
+def test_gemm_bf16_call_reads_nothing_before_the_kernel_ahead_of_it_has_ended(m, n, k):
+    """Operator launches are made ready while the kernel before them drains, which may be the one that writes the weights (here a transposition,
+    whose blocks let the next launch in early).  Every engine; the same bits as with a wait in between."""
+    g = torch.Generator(device="cuda").manual_seed(43)
+    a = torch.randn(m, k, device="cuda", generator=g).to(torch.bfloat16)
+    sources = [torch.randn(k, n, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2)]
+    weights, outs = torch.zeros(n, k, device="cuda", dtype=torch.bfloat16), [torch.empty(m, n, device="cuda") for _ in range(8)]
+
+    def call(i, out):
+        ok(lib().tnsr_b200_transpose_bf16(ptr(sources[i % 2]), ptr(weights), k, n, stream()))
+        ok(lib().tnsr_b200_gemm_bf16(ptr(a), ptr(weights), None, None, ptr(out), m, n, k, -1, 0, stream()))
+
+    want = []
+    for i in range(2):
+        want.append(torch.empty(m, n, device="cuda"))
+        ok(lib().tnsr_b200_transpose_bf16(ptr(sources[i]), ptr(weights), k, n, stream()))
+        torch.cuda.synchronize()
+        ok(lib().tnsr_b200_gemm_bf16(ptr(a), ptr(weights), None, None, ptr(want[i]), m, n, k, -1, 0, stream()))
+        torch.cuda.synchronize()
+    for i, out in enumerate(outs):
+        call(i, out)
+    torch.cuda.synchronize()
+    for i, out in enumerate(outs):
+        assert torch.equal(out, want[i % 2]), i
+
+
 # ---- SwiGLU ----------------------------------------------------------------------
 def test_swiglu_elementwise(oracle):
     import json, os

@@ -156,6 +156,7 @@ struct GemmEpilogue {
     uint32_t split_k = 0;
     uint32_t split_rows = 0;
     bool single = false;              // a call of its own (the C ABI's operators), not one of a session's chain of launches
+    bool wait_first = false;          // the kernel before may be anyone's and write any operand: nothing is read before it has ended
     bool beside = false;              // another range of a divided step runs its attention on the same SMs meanwhile
 };
 

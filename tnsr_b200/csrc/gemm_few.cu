@@ -91,6 +91,7 @@ gemm_few_kernel(const __grid_constant__ FewParams P) {
         for (int j = 0; j < NT; ++j) w[j][s] = ok && col + j * col_step < n ? fw_load_weights(p + (size_t)j * col_step * k) : fw_zero();
     };
     uint32_t tile = blockIdx.x / P.ck;
+    if (P.epi.ep.wait_first) pdl_wait();
 #pragma unroll
     for (int s = 0; s < S; ++s) load_w(s, tile, b0 + s);
     // A thread finishes elements tid, tid + 256, ... of the (ck = 1) tile, all of one column: its bias and scale

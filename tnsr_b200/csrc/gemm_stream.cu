@@ -41,6 +41,7 @@ struct GsParams {
     uint32_t ldr;
     int activation, out_dtype;
     uint32_t stages;
+    bool wait_first;
 };
 
 __device__ __forceinline__ uint32_t gs_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -112,7 +113,8 @@ gemm_stream_kernel(GsParams P) {
         }
         gs_commit();        // a group per slot, also when it is empty: the wait counts stay uniform
     };
-    // The weights do not depend on the previous kernel: request the whole ring before waiting for it.
+    // The weights of a session do not depend on the previous kernel: request the whole ring before waiting for it.
+    if (P.wait_first) pdl_wait();
     for (uint32_t s = 0; s + 1 < P.stages; ++s) issue(s);
     pdl_wait();
     pdl_trigger();
@@ -241,7 +243,7 @@ int launch_gemm_stream(const bf16* a, const bf16* bt, void* out, uint32_t ldc, u
     (void)d_status;      // nothing in this kernel waits on another agent: there is no time-out to report
     GsParams P = {};
     P.a = a; P.w = bt; P.out = out; P.ldc = ldc; P.m = m; P.n = n; P.k = k;
-    P.bias = ep.bias; P.scale = ep.scale; P.residual = ep.residual; P.ldr = ep.ldr; P.activation = ep.activation; P.out_dtype = ep.out_dtype;
+    P.bias = ep.bias; P.scale = ep.scale; P.residual = ep.residual; P.ldr = ep.ldr; P.activation = ep.activation; P.out_dtype = ep.out_dtype; P.wait_first = ep.wait_first;
     return m <= 8 ? gs_launch<8>(P, stream) : gs_launch<16>(P, stream);
 }
 
