@@ -169,6 +169,10 @@ uint32_t gemm_split_k(const bf16* a, const bf16* bt, uint32_t m, uint32_t n, uin
 int launch_gemm_strict(const float* a, const float* b, void* out, uint32_t ldc, uint32_t m, uint32_t k,
                        uint32_t n, bool b_transposed, const GemmEpilogue& ep, cudaStream_t stream);
 
+// Three products of one left-hand side, each with its own matrix [k, n], destination and epilogue, in one launch.
+int launch_gemm_strict_three(const float* a, const float* const* b, void* const* out, uint32_t ldc, uint32_t m, uint32_t k, uint32_t n,
+                             const GemmEpilogue* ep, cudaStream_t stream);
+
 // bf16 operands, f32 accumulation.  `bt` is [n, k] K-major.  `mode` selects the
 // epilogue family.
 enum GemmMode : int {

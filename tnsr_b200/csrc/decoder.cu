@@ -264,18 +264,17 @@ int strict_layers(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chu
     float* n = (float*)dec->n; float* q = (float*)dec->q; float* att = (float*)dec->att; float* ff = (float*)dec->ff;
     for (Layer& L : dec->layers) {
         RUN(dec, launch_layernorm(dec->h, L.ln1w, L.ln1b, n, rows, d, c.layer_norm_epsilon, TNSR_B200_F32, true, st));
-        GemmEpilogue eq;
-        eq.bias = L.bq;
-        eq.round_bf16 = dec->kv_bf16;
-        RUN(dec, launch_gemm_strict(n, (const float*)L.wq, q, d, rows, d, d, false, eq, st));
-        GemmEpilogue ek;
-        ek.round_bf16 = dec->kv_bf16;
-        ek.out_dtype = kvdt;
-        ek.rows_per_session = chunk; ek.out_session_rows = c.capacity; ek.row_offset = position; ek.d_row_offset = d_position;
-        ek.bias = L.bk;
-        RUN(dec, launch_gemm_strict(n, (const float*)L.wk, L.kcache, d, rows, d, d, false, ek, st));
-        ek.bias = L.bv;
-        RUN(dec, launch_gemm_strict(n, (const float*)L.wv, L.vcache, d, rows, d, d, false, ek, st));
+        GemmEpilogue e[3];                       // queries, keys, values
+        for (GemmEpilogue& x : e) x.round_bf16 = dec->kv_bf16;
+        e[0].bias = L.bq;
+        e[1].out_dtype = kvdt;
+        e[1].rows_per_session = chunk; e[1].out_session_rows = c.capacity; e[1].row_offset = position; e[1].d_row_offset = d_position;
+        e[2] = e[1];
+        e[1].bias = L.bk;
+        e[2].bias = L.bv;
+        const float* w[3] = {(const float*)L.wq, (const float*)L.wk, (const float*)L.wv};
+        void* to[3] = {q, L.kcache, L.vcache};
+        RUN(dec, launch_gemm_strict_three(n, w, to, d, rows, d, d, e, st));
         RUN(dec, launch_attention_strict(q, L.kcache, L.vcache, att, B, chunk, position, d_position, c.capacity, H, d / H, kvdt,
                                          dec->kv_bf16, st));
         GemmEpilogue eo;
