@@ -123,6 +123,16 @@ def test_strict_matmul_tiles_bit_exact(oracle, shape):
     assert np.array_equal(run_strict(a, np.ascontiguousarray(b.T), bias, transposed=True).view(np.uint32), expected)
 
 
+@pytest.mark.parametrize("transposed", [False, True])
+@pytest.mark.parametrize("shape", [(2369, 37, 257), (2401, 33, 130), (9473, 9, 66), (90, 40, 6400)])     # 32 x 64 tiles, their ragged edges; 64 x 64 ones
+def test_strict_matmul_tiles_of_two_shapes_bit_exact(oracle, shape, transposed):
+    m, k, n = shape
+    rng = np.random.default_rng(19)
+    a, b = (rng.standard_normal(x).astype(np.float32) for x in ((m, k), (k, n)))
+    got = run_strict(a, np.ascontiguousarray(b.T) if transposed else b, transposed=transposed)
+    assert np.array_equal(got.view(np.uint32), oracle.matmul(a, b).view(np.uint32))
+
+
 @pytest.mark.parametrize("shape", [(1, 128, 128), (16, 128, 512), (7, 13, 8), (33, 37, 35), (3, 512, 96)])
 def test_strict_matmul_random_shapes_bit_exact(oracle, shape):
     m, k, n = shape

@@ -15,8 +15,8 @@
 namespace tb {
 
 // ---------------------------------------------------------------------------
-// GEMM: a block of 256 threads owns a T x T tile of the output, a thread R x R of its elements (R = T / 16), K is walked in
-// order through 32-deep shared tiles.  An output is one chain of rounded products and rounded sums; the R * R chains of a
+// GEMM: a block of 256 threads owns a TM x TN tile of the output, a thread RM x RN of its elements (a sixteenth of each), K is walked in
+// order through 32-deep shared tiles.  An output is one chain of rounded products and rounded sums; the RM * RN chains of a
 // thread are independent of each other and hide each other's latency.  Two columns go through one packed instruction whose halves
 // round as the scalar ones do: mul.rn.f32x2, then fma.rn.f32x2 with a factor of one that only the launch knows, because the
 // assembler joins a packed product and a packed sum into one operation with one rounding.  The rows' values are stored twice side
@@ -56,67 +56,76 @@ struct StrictSets {
     GemmEpilogue ep[3];
 };
 
-template <int T, bool BT>
+template <int TM, int TN, bool BT>
 __global__ void __launch_bounds__(256)
 gemm_strict_tile_kernel(const float* __restrict__ a, const __grid_constant__ StrictSets sets, uint32_t ldc, uint32_t m,
                         uint32_t k, uint32_t n, bool vec_a, bool vec_b, float one) {
     const float* __restrict__ b = sets.b[blockIdx.z];
-    constexpr uint32_t R = T / 16, LOADS = T * SK / 4 / 256;      // float4 loads per thread and operand tile (1 or 2)
-    __shared__ __align__(16) float as[SK][2 * T];                 // every value twice
-    __shared__ __align__(16) float bs[SK][T];
-    const uint32_t tid = threadIdx.x, tx = tid % 16, ty = tid / 16, row0 = blockIdx.y * T, col0 = blockIdx.x * T;
-    float4 ra[LOADS], rb[LOADS];
+    constexpr uint32_t RM = TM / 16, RN = TN / 16, LA = TM * SK / 4 / 256, LB = TN * SK / 4 / 256;      // LA, LB: float4 loads per thread (1 or 2)
+    __shared__ __align__(16) float as[SK][2 * TM];                // every value twice
+    __shared__ __align__(16) float bs[SK][TN];
+    const uint32_t tid = threadIdx.x, tx = tid % 16, ty = tid / 16, row0 = blockIdx.y * TM, col0 = blockIdx.x * TN;
+    float4 ra[LA], rb[LB];
     auto fetch = [&](uint32_t k0) {
 #pragma unroll
-        for (uint32_t i = 0; i < LOADS; ++i) {
-            const uint32_t e = tid + i * 256, r = e % T, q = e / T;      // along k: lanes on different rows, so that stores do not collide
+        for (uint32_t i = 0; i < LA; ++i) {
+            const uint32_t e = tid + i * 256, r = e % TM, q = e / TM;    // along k: lanes on different rows, so that stores do not collide
             ra[i] = strict_load4(a + (size_t)(row0 + r) * k, k0 + 4 * q, k, row0 + r < m, vec_a);
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < LB; ++i) {
+            const uint32_t e = tid + i * 256;
             if (BT) {
+                const uint32_t r = e % TN, q = e / TN;
                 rb[i] = strict_load4(b + (size_t)(col0 + r) * k, k0 + 4 * q, k, col0 + r < n, vec_b);
             } else {
-                const uint32_t p = e / (T / 4), c = e % (T / 4);
+                const uint32_t p = e / (TN / 4), c = e % (TN / 4);
                 rb[i] = strict_load4(b + (size_t)(k0 + p) * n, col0 + 4 * c, n, k0 + p < k, vec_b);
             }
         }
     };
-    uint64_t acc[R][R / 2];
+    uint64_t acc[RM][RN / 2];
 #pragma unroll
-    for (uint32_t i = 0; i < R; ++i)
+    for (uint32_t i = 0; i < RM; ++i)
 #pragma unroll
-        for (uint32_t j = 0; j < R / 2; ++j) acc[i][j] = 0;
+        for (uint32_t j = 0; j < RN / 2; ++j) acc[i][j] = 0;
     const uint64_t one2 = (uint64_t)__float_as_uint(one) << 32 | __float_as_uint(one);
     fetch(0);
     for (uint32_t k0 = 0; k0 < k; k0 += SK) {
         __syncthreads();
 #pragma unroll
-        for (uint32_t i = 0; i < LOADS; ++i) {
-            const uint32_t e = tid + i * 256, r = e % T, q = e / T;
-            const float va[4] = {ra[i].x, ra[i].y, ra[i].z, ra[i].w}, vb[4] = {rb[i].x, rb[i].y, rb[i].z, rb[i].w};
+        for (uint32_t i = 0; i < LA; ++i) {
+            const uint32_t e = tid + i * 256, r = e % TM, q = e / TM;
+            const float va[4] = {ra[i].x, ra[i].y, ra[i].z, ra[i].w};
 #pragma unroll
-            for (uint32_t j = 0; j < 4; ++j) {
-                *reinterpret_cast<float2*>(&as[4 * q + j][2 * r]) = make_float2(va[j], va[j]);
-                if (BT) bs[4 * q + j][r] = vb[j];
-            }
-            if (!BT) *reinterpret_cast<float4*>(&bs[e / (T / 4)][4 * (e % (T / 4))]) = rb[i];
+            for (uint32_t j = 0; j < 4; ++j) *reinterpret_cast<float2*>(&as[4 * q + j][2 * r]) = make_float2(va[j], va[j]);
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < LB; ++i) {
+            const uint32_t e = tid + i * 256, r = e % TN, q = e / TN;
+            const float vb[4] = {rb[i].x, rb[i].y, rb[i].z, rb[i].w};
+            if (!BT) *reinterpret_cast<float4*>(&bs[e / (TN / 4)][4 * (e % (TN / 4))]) = rb[i];
+#pragma unroll
+            for (uint32_t j = 0; BT && j < 4; ++j) bs[4 * q + j][r] = vb[j];
         }
         __syncthreads();
         if (k0 + SK < k) fetch(k0 + SK);
         auto step = [&](uint32_t p) {
-            uint64_t av[R], bv[R / 2];
-            const ulonglong2* ap = reinterpret_cast<const ulonglong2*>(&as[p][2 * R * ty]);
+            uint64_t av[RM], bv[RN / 2];
+            const ulonglong2* ap = reinterpret_cast<const ulonglong2*>(&as[p][2 * RM * ty]);
 #pragma unroll
-            for (uint32_t i = 0; i < R / 2; ++i) { const ulonglong2 v = ap[i]; av[2 * i] = v.x; av[2 * i + 1] = v.y; }
-            if (R == 2) {
+            for (uint32_t i = 0; i < RM / 2; ++i) { const ulonglong2 v = ap[i]; av[2 * i] = v.x; av[2 * i + 1] = v.y; }
+            if (RN == 2) {
                 bv[0] = *reinterpret_cast<const uint64_t*>(&bs[p][2 * tx]);
             } else {
-                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&bs[p][R * tx]);
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&bs[p][RN * tx]);
                 bv[0] = v.x;
-                bv[R / 2 - 1] = v.y;
+                bv[RN / 2 - 1] = v.y;
             }
 #pragma unroll
-            for (uint32_t i = 0; i < R; ++i)
+            for (uint32_t i = 0; i < RM; ++i)
 #pragma unroll
-                for (uint32_t j = 0; j < R / 2; ++j) acc[i][j] = add_f32x2(acc[i][j], mul_f32x2(av[i], bv[j]), one2);
+                for (uint32_t j = 0; j < RN / 2; ++j) acc[i][j] = add_f32x2(acc[i][j], mul_f32x2(av[i], bv[j]), one2);
         };
         if (k - k0 >= SK) {
 #pragma unroll 8
@@ -126,24 +135,24 @@ gemm_strict_tile_kernel(const float* __restrict__ a, const __grid_constant__ Str
         }
     }
 #pragma unroll
-    for (uint32_t i = 0; i < R; ++i)
+    for (uint32_t i = 0; i < RM; ++i)
 #pragma unroll
-        for (uint32_t j = 0; j < R; ++j) {
-            const uint32_t row = row0 + R * ty + i, col = col0 + R * tx + j;
+        for (uint32_t j = 0; j < RN; ++j) {
+            const uint32_t row = row0 + RM * ty + i, col = col0 + RN * tx + j;
             const uint32_t bits = (uint32_t)(acc[i][j / 2] >> (j % 2 ? 32 : 0));
             if (row < m && col < n) strict_finish(sets.ep[blockIdx.z], __uint_as_float(bits), row, col, sets.out[blockIdx.z], ldc);
         }
 }
 
-template <int T>
+template <int TM, int TN>
 static void launch_strict_tile(const float* a, const StrictSets& sets, uint32_t count, uint32_t ldc, uint32_t m, uint32_t k, uint32_t n, bool b_transposed,
                                cudaStream_t stream) {
     const bool vec_a = k % 4 == 0 && reinterpret_cast<uintptr_t>(a) % 16 == 0;
     bool vec_b = (b_transposed ? k : n) % 4 == 0;
     for (uint32_t i = 0; i < count; ++i) vec_b = vec_b && reinterpret_cast<uintptr_t>(sets.b[i]) % 16 == 0;
-    const dim3 grid(ceil_div(n, (uint32_t)T), ceil_div(m, (uint32_t)T), count);
-    if (b_transposed) gemm_strict_tile_kernel<T, true><<<grid, 256, 0, stream>>>(a, sets, ldc, m, k, n, vec_a, vec_b, 1.0f);
-    else gemm_strict_tile_kernel<T, false><<<grid, 256, 0, stream>>>(a, sets, ldc, m, k, n, vec_a, vec_b, 1.0f);
+    const dim3 grid(ceil_div(n, (uint32_t)TN), ceil_div(m, (uint32_t)TM), count);
+    if (b_transposed) gemm_strict_tile_kernel<TM, TN, true><<<grid, 256, 0, stream>>>(a, sets, ldc, m, k, n, vec_a, vec_b, 1.0f);
+    else gemm_strict_tile_kernel<TM, TN, false><<<grid, 256, 0, stream>>>(a, sets, ldc, m, k, n, vec_a, vec_b, 1.0f);
 }
 
 // Few rows (decode steps, short prefills): one block per (row, 32 output columns).  The sum of an output is
@@ -199,14 +208,20 @@ static int launch_gemm_strict_sets(const float* a, const StrictSets& sets, uint3
         count_launch();
         return check_launch("gemm_strict_rows");
     }
-    // 64 x 64 tiles if there are enough of them for every SM, else 32 x 32
-    const uint64_t tiles = (uint64_t)ceil_div(m, 64u) * ceil_div(n, 64u) * count;
     if (ceil_div(m, 16u) > 65535u) {
         set_thread_error("strict GEMM: too many rows for one launch");
         return TNSR_B200_ERR_UNSUPPORTED;
     }
-    if (tiles >= 148) launch_strict_tile<64>(a, sets, count, ldc, m, k, n, b_transposed, stream);
-    else launch_strict_tile<32>(a, sets, count, ldc, m, k, n, b_transposed, stream);
+    // A block is latency first: what a tile costs is its first wave and, less, every further one of an SM.  us at k = 512 by blocks per SM
+    // (1, 2, 3, 4): 64 x 64 tiles 37, 63, 90, 117; 32 x 64 22, 39, 57, 74; 32 x 32 17, 29, 41, 52.  (64 x 64 wherever there was one for every SM, else
+    // 32 x 32, the rule before: 5808 x 512 x 128 63 us, 56 here; 2000 x 512 x 128 29 / 25; 700 x 768 x 768 77 / 53; 5808 x 128 x 96 23 / 18.)
+    auto cost = [&](uint32_t tm, uint32_t tn, uint32_t first, uint32_t wave) {
+        return first + wave * ceil_div64((uint64_t)ceil_div(m, tm) * ceil_div(n, tn) * count, 148u);
+    };
+    const uint64_t c64 = cost(64, 64, 110, 262), c48 = cost(32, 64, 42, 175), c32 = cost(32, 32, 46, 119);
+    if (c64 <= std::min(c48, c32)) launch_strict_tile<64, 64>(a, sets, count, ldc, m, k, n, b_transposed, stream);
+    else if (c48 <= c32) launch_strict_tile<32, 64>(a, sets, count, ldc, m, k, n, b_transposed, stream);
+    else launch_strict_tile<32, 32>(a, sets, count, ldc, m, k, n, b_transposed, stream);
     count_launch();
     return check_launch("gemm_strict");
 }
