@@ -519,9 +519,11 @@ int step_bf16(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chunk, 
     return TNSR_B200_OK;
 }
 
-// Rows up to which a step's kernels are launched ahead of their predecessors' end.  About 90 launches of a prompt gain 1 to 2 us each: 5 x 777
-// ids 2.35 -> 2.21 ms; with long kernels the early blocks only take room: 64 x 512 ids 8.19 -> 8.33 ms.
-constexpr uint32_t kPdlMaxRows = 4096;
+// Rows up to which a step's kernels are launched ahead of their predecessors' end.  About 90 launches of a prompt gain 1 to 2 us each; with long
+// kernels the early blocks only take room.  us without / with: 5 x 777 ids 2350 / 2210, 10 x 500 1765 / 1633, 16 x 500 2248 / 2113 (in pages 2465 / 2351),
+// 30 x 400 3010 / 2933, 8 x 1900 level, 64 x 512 8190 / 8330.  Described models, whose kernels wait more on memory: 24 x 301 (Bolonex) 3335 / 3347,
+// 16 x 500 (Ganupel) 4248 / 4368.
+constexpr uint32_t kPdlMaxRows = 12288, kPdlMaxStackRows = 4096;
 
 int run_step_direct(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chunk, uint32_t position,
                     const uint32_t* d_position, uint32_t* d_argmax_out) {
@@ -531,7 +533,7 @@ int run_step_direct(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t c
     const bool sampling = dec->sample_temperature > 0.0f;
     const bool fuse_ids = dec->bf16_path && c.logits_mode == TNSR_B200_LOGITS_NONE && d_argmax_out && dec->lm_candidates && !sampling;
     t_attention_timer = dec->profile_attention ? &dec->attention_timer : nullptr;
-    t_pdl = dec->use_pdl && dec->bf16_path && rows <= kPdlMaxRows;
+    t_pdl = dec->use_pdl && dec->bf16_path && rows <= (dec->stack ? kPdlMaxStackRows : kPdlMaxRows);
     t_single_token_step = chunk == 1;
     int rc = dec->stack ? stack_step(dec, d_tokens, chunk, position, d_position, false, logit_rows, fuse_ids ? d_argmax_out : nullptr)
            : dec->bf16_path ? step_bf16(dec, d_tokens, chunk, position, d_position, logit_rows, fuse_ids ? d_argmax_out : nullptr)
