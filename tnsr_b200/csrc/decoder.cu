@@ -392,7 +392,7 @@ int layers_bf16(tnsr_b200_decoder* dec, const uint32_t* d_tokens, uint32_t chunk
             // Paged caches and head widths other than 64: the kernels of described models, with one query head per
             // key/value head (K/V tiles through shared memory).  The scan below holds its weights in f32, so they enter the
             // value product as three bf16 pieces here, which is all of their bits.  It reads every key once per query; 5 x 777
-            // ids, 12 x 64 heads, pages of 64 rows, one layer on B200: 2672 us there, 77 us on warp-level tiles, 27 us on tcgen05
+            // ids, 12 x 64 heads, pages of 64 rows, one layer on B200: 2672 us there, 77 us on warp-level tiles, 42 us on tcgen05
             // (chunks of more than 64 ids, heads of 64).
             GroupedAttention ga;
             ga.q = q; ga.k_cache = kcache; ga.v_cache = vcache; ga.out = att;
