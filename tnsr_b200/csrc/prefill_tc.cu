@@ -46,8 +46,8 @@
 // are the A operand in TMEM: two of them over the scores that the same thread has just read (per 16 keys 8 columns of upper pieces, 8 of
 // middle ones), the third in the 64 columns behind the output.  S_{j+1} is issued behind P_j V_j then, which it overwrites.
 // Keys come page by page: a box is the largest power of two of rows that divides a page, up to a block; boxes behind the last live row are not
-// read, and the softmax warps zero the value rows that they would have filled.  What bounds it is the chain of a block (scores, maximum, weights, product, fold: 5 us); 5
-// x 777 ids, 12 heads, a layer: 77 us on warp-level tiles, 42 here.
+// read, and the softmax warps zero the value rows that they would have filled.  What bounds it is the chain of a block (scores, maximum,
+// weights, product, fold: 5 us); 5 x 777 ids, 12 heads, a layer: 77 us on warp-level tiles, 42 here.
 //
 // Every wait is bounded; a wait that gives up raises the CTA's abort flag, the
 // roles fall through to the common teardown and the status word is set.
