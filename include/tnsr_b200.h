@@ -408,8 +408,9 @@ TNSR_B200_API int tnsr_b200_decoder_write_cache(tnsr_b200_decoder* dec, uint32_t
 
 /* Measurement aid (no reference counterpart; the reference times kernels from
  * outside with CUDA events, src/ptx/linear/mod.rs:425-437).  While enabled, the
- * session brackets every launch of its split-KV decode-attention kernel with a
- * pair of CUDA events on its stream.  `attention_profile` waits for the stream,
+ * session brackets every launch of a decode-attention kernel of a GPT decoder,
+ * the one that an unprofiled undivided step of it launches, with a pair of CUDA
+ * events on its stream.  `attention_profile` waits for the stream,
  * returns the summed device time in milliseconds and the number of launches
  * since the last call, and clears the record. */
 TNSR_B200_API int tnsr_b200_decoder_profile_attention(tnsr_b200_decoder* dec, int enable);

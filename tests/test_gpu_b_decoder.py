@@ -16,6 +16,7 @@ from tests.helpers import close, cpu_decoder, cpu_forward, cpu_generate, kv_mode
 from tests.test_kv_cache_host import chunks_match, validate_inputs_and_weights  # noqa: E402
 from tests.workloads import (config0_model, config0_prompt, kv_test_tokens, normal_model_arrays,  # noqa: E402
                              set_model_arrays)
+from tnsr_b200 import _native  # noqa: E402
 from tnsr_b200.nn import (Backend, Gpt, GptAttentionPrecision, GptConfig, GptDecoder, GptDecoderOptions,  # noqa: E402
                           argmax_last,
                           GptPrefillMode, model_parameters)
@@ -973,6 +974,31 @@ def test_long_paged_prompts_over_pages_of_any_size(page):
     got, want = run(GptPrefillMode.Auto), run(GptPrefillMode.Scalar)
     assert np.all(np.isfinite(got))
     assert np.max(np.abs(got - want)) <= max(1.0, float(np.max(np.abs(want)))) / 64
+
+
+@pytest.mark.parametrize("capacity", [320, 4096])                 # the launch of clusters, the streaming kernel
+def test_the_attention_record_is_of_the_kernels_that_run_without_it(capacity):
+    cfg = GptConfig(vocab_size=300, max_sequence_length=capacity, embed_dim=256, num_heads=4, feed_forward_dim=256, num_layers=3,
+                    layer_norm_epsilon=1e-5, activation="swiglu", weight_dtype="bf16")
+    arrays = normal_model_arrays(cfg, seed=61, std=0.05)
+    batch = 12
+    ids = np.random.default_rng(62).integers(0, cfg.vocab_size, size=(batch, 301)).astype(np.uint32)
+    seen = []
+    for record in (False, True):
+        s = B200Session(cfg, batch, capacity, logits_mode="last")
+        for i, a in enumerate(arrays):
+            s.refresh(i, a)
+        s.decode_full(ids[:, :300], 0)
+        s.profile_attention(record)
+        before = _native.lib().tnsr_b200_kernel_launches()
+        logits = s.decode_full(ids[:, 300:], 300)[0].copy()
+        seen.append((_native.lib().tnsr_b200_kernel_launches() - before, logits.view(np.uint32)))
+        if record:
+            milliseconds, launches = s.attention_profile()
+            assert launches == cfg.num_layers and milliseconds > 0.0
+        s.close()
+    assert seen[0][0] == seen[1][0]
+    assert np.array_equal(seen[0][1], seen[1][1])
 
 
 def test_paged_kv_pool_smaller_than_the_worst_case():

@@ -958,11 +958,32 @@ static bool ds_pays(uint32_t batch, uint32_t heads, uint32_t longest, bool chain
     return (uint64_t)batch * heads * longest <= (chained ? 180000u : 400000u);
 }
 
+// Launches an attention kernel, between two events of the handle's record while one is kept: the same kernel either way.
+template <typename Launch>
+static int launch_timed(cudaStream_t stream, const char* name, Launch&& launch) {
+    KernelTimer* timer = t_attention_timer;
+    size_t at = 0;
+    if (timer) {
+        while (timer->used + 2 > timer->events.size()) {
+            cudaEvent_t e;
+            if (cudaEventCreate(&e) != cudaSuccess) return check_launch("decode_attention event");
+            timer->events.push_back(e);
+        }
+        at = timer->used;
+        timer->used += 2;
+        cudaEventRecord(timer->events[at], stream);
+    }
+    launch();
+    if (timer) cudaEventRecord(timer->events[at + 1], stream);
+    count_launch();
+    return check_launch(name);
+}
+
 template <int HD>
 static int launch_ds(const DsParams& P, uint32_t units, cudaStream_t stream) {
-    launch_kernel_clusters(decode_attention_short_kernel<HD>, dim3(units * P.ck), dim3(DS_THREADS), 0, P.ck, stream, P);
-    count_launch();
-    return check_launch("decode_attention_short");
+    return launch_timed(stream, "decode_attention_short", [&] {
+        launch_kernel_clusters(decode_attention_short_kernel<HD>, dim3(units * P.ck), dim3(DS_THREADS), 0, P.ck, stream, P);
+    });
 }
 
 template <int HD, int HPW, int KS>
@@ -975,25 +996,7 @@ static int launch_da_t(const DaParams& P, uint32_t threads, size_t smem, uint32_
             return check_launch("decode_attention attribute");
         if (dev >= 0 && dev < 64) configured[dev] = smem;
     }
-    KernelTimer* timer = t_attention_timer;
-    cudaEvent_t start = nullptr, stop = nullptr;
-    if (timer) {
-        if (timer->used + 2 > timer->events.size()) {
-            for (int i = 0; i < 2; ++i) {
-                cudaEvent_t e;
-                if (cudaEventCreate(&e) != cudaSuccess) return check_launch("decode_attention event");
-                timer->events.push_back(e);
-            }
-        }
-        start = timer->events[timer->used];
-        stop = timer->events[timer->used + 1];
-        timer->used += 2;
-        cudaEventRecord(start, stream);
-    }
-    launch_kernel(decode_attention_kernel<HD, HPW, KS>, dim3(grid), dim3(threads), smem, stream, P);
-    if (timer) cudaEventRecord(stop, stream);
-    count_launch();
-    return check_launch("decode_attention");
+    return launch_timed(stream, "decode_attention", [&] { launch_kernel(decode_attention_kernel<HD, HPW, KS>, dim3(grid), dim3(threads), smem, stream, P); });
 }
 
 // lengths may be nullptr: then every session holds (d_position ? *d_position : 0) + extra keys.
@@ -1021,7 +1024,7 @@ int launch_decode_attention_ex(const bf16* q, const bf16* k_cache, const bf16* v
         set_thread_error("decode attention: the page size must be a multiple of 16 rows");
         return TNSR_B200_ERR_INVALID_ARGUMENT;
     }
-    if (!lean && !t_attention_timer && ds_pays(batch, heads, capacity, t_pdl && extra > 0)) {
+    if (!lean && ds_pays(batch, heads, capacity, t_pdl && extra > 0)) {
         DsParams S;
         S.q = q; S.kc = k_cache; S.vc = v_cache; S.out = out;
         S.lengths = d_lengths; S.d_position = d_position; S.extra = extra;
