@@ -1001,6 +1001,41 @@ def test_the_attention_record_is_of_the_kernels_that_run_without_it(capacity):
     assert np.array_equal(seen[0][1], seen[1][1])
 
 
+@pytest.mark.parametrize("batch,heads,width,capacity", [(24, 12, 768, 1024),      # the streaming kernel: keys asked for ahead, list kept for all layers
+                                                        (2, 4, 256, 4096), (3, 2, 256, 3008)])    # clusters: several passes of a CTA, heads of 64 and 128
+def test_steps_behind_many_keys_have_the_same_bits_however_they_are_launched(monkeypatch, batch, heads, width, capacity):
+    """Replayed and direct steps, with and without early launches, contiguous and paged caches: steps at a common position and ragged ones.  Pages
+    were another tenant's before."""
+    cfg = GptConfig(vocab_size=300, max_sequence_length=capacity, embed_dim=width, num_heads=heads, feed_forward_dim=256, num_layers=2,
+                    layer_norm_epsilon=1e-5, activation="swiglu", weight_dtype="bf16")
+    arrays = normal_model_arrays(cfg, seed=63, std=0.05)
+    rng = np.random.default_rng(64)
+    prompt, steps = capacity - 40, 6
+    old, ids = (rng.integers(0, cfg.vocab_size, size=(batch, capacity)).astype(np.uint32) for _ in range(2))
+    ragged = np.asarray([(prompt if b % 3 == 0 else 1 + (b * 131) % prompt) for b in range(batch)], dtype=np.uint32)
+
+    def run(switches, **kw):
+        for name in ("TNSR_B200_NO_GRAPH", "TNSR_B200_NO_PDL"):
+            monkeypatch.setenv(name, "1") if name in switches else monkeypatch.delenv(name, raising=False)
+        # the scan: its chunks are the same kernel behind pages and behind a contiguous cache
+        s = B200Session(cfg, batch, capacity, GptDecoderOptions(prefill=GptPrefillMode.Scalar), logits_mode="last", **kw)
+        for i, a in enumerate(arrays):
+            s.refresh(i, a)
+        if kw:
+            s.decode_full(old[:, :128], 0)
+            for b in reversed(range(batch)):
+                s.release(b)
+        s.decode_full(ids[:, :prompt], 0)
+        out = [s.decode_full(ids[:, t:t + 1], t)[0].copy() for t in range(prompt, prompt + steps)]
+        out += [s.decode_ragged(ids[:, t], ragged + t)[0].copy() for t in range(steps)]
+        s.close()
+        return np.stack(out).view(np.uint32)
+
+    want = run(())
+    for switches, kw in ((("TNSR_B200_NO_GRAPH",), {}), (("TNSR_B200_NO_GRAPH", "TNSR_B200_NO_PDL"), {}), ((), {"kv_page_rows": 32})):
+        assert np.array_equal(run(switches, **kw), want), (switches, kw)
+
+
 def test_paged_kv_pool_smaller_than_the_worst_case():
     """A pool of 7 pages for 4 sessions x 64 rows (worst case 16 pages): short sessions fit, a step that would need an
     eighth page is refused with ERR_CAPACITY and changes nothing, releasing a session makes room again."""

@@ -1024,7 +1024,7 @@ int launch_decode_attention_ex(const bf16* q, const bf16* k_cache, const bf16* v
         set_thread_error("decode attention: the page size must be a multiple of 16 rows");
         return TNSR_B200_ERR_INVALID_ARGUMENT;
     }
-    if (!lean && ds_pays(batch, heads, capacity, t_pdl && extra > 0)) {
+    if (!lean && ds_pays(batch, heads, capacity, extra > 0)) {       // a step's newest key comes on top of the lengths
         DsParams S;
         S.q = q; S.kc = k_cache; S.vc = v_cache; S.out = out;
         S.lengths = d_lengths; S.d_position = d_position; S.extra = extra;
