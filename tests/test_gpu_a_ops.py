@@ -347,31 +347,98 @@ def test_gemm_bf16_tiles_of_pairs_and_of_192_columns(shape, form):
     assert float(err.max()) <= 2e-3
 
 
-@pytest.mark.parametrize("m,n,k", [(8, 4096, 4096), (1, 512, 512), (4, 2048, 4096), (5, 4096, 1032), (48, 2304, 768), (200, 768, 2048), (600, 9472, 2048)])
-def test_gemm_bf16_call_reads_nothing_before_the_kernel_ahead_of_it_has_ended(m, n, k):
-    """Operator launches are made ready while the kernel before them drains, which may be the one that writes the weights (here a transposition,
-    whose blocks let the next launch in early).  Every engine; the same bits as with a wait in between."""
-    g = torch.Generator(device="cuda").manual_seed(43)
-    a = torch.randn(m, k, device="cuda", generator=g).to(torch.bfloat16)
-    sources = [torch.randn(k, n, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2)]
-    weights, outs = torch.zeros(n, k, device="cuda", dtype=torch.bfloat16), [torch.empty(m, n, device="cuda") for _ in range(8)]
+# ---- operator launches that are made ready early ----------------------------------
+class Writer:
+    """Fills a tensor with one of two contents by a product, which lets the next launch in at its start and writes at its end: in several
+    waves of tiles, behind a long k.  What runs next and does not wait for it reads the other content."""
 
-    def call(i, out):
-        ok(lib().tnsr_b200_transpose_bf16(ptr(sources[i % 2]), ptr(weights), k, n, stream()))
-        ok(lib().tnsr_b200_gemm_bf16(ptr(a), ptr(weights), None, None, ptr(out), m, n, k, -1, 0, stream()))
+    def __init__(self, rows, cols, dtype, seed, std=1.0, k=4096):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        self.k, self.dtype = k, dtype
+        self.left = [(torch.randn(rows, k, device="cuda", generator=g) * (std * k ** -0.5)).to(torch.bfloat16) for _ in range(2)]
+        self.right = torch.randn(cols, k, device="cuda", generator=g).to(torch.bfloat16)
+        self.out = torch.zeros(rows, cols, device="cuda", dtype=torch.float32 if dtype == F32 else torch.bfloat16)
 
+    def __call__(self, which):
+        rows, cols = self.out.shape
+        ok(lib().tnsr_b200_gemm_bf16(ptr(self.left[which]), ptr(self.right), None, None, ptr(self.out), rows, cols, self.k, -1, self.dtype, stream()))
+
+
+def same_bits_as_with_waits(writer, call, out):
+    """call() behind writer(which), back to back and with a wait in between."""
     want = []
-    for i in range(2):
-        want.append(torch.empty(m, n, device="cuda"))
-        ok(lib().tnsr_b200_transpose_bf16(ptr(sources[i]), ptr(weights), k, n, stream()))
+    for which in range(2):
+        writer(which)
         torch.cuda.synchronize()
-        ok(lib().tnsr_b200_gemm_bf16(ptr(a), ptr(weights), None, None, ptr(want[i]), m, n, k, -1, 0, stream()))
+        call()
         torch.cuda.synchronize()
-    for i, out in enumerate(outs):
-        call(i, out)
+        want.append(out.clone())
+    assert not torch.equal(want[0], want[1])
+    got = []
+    for i in range(8):
+        writer(i % 2)
+        call()
+        got.append(out.clone())
     torch.cuda.synchronize()
-    for i, out in enumerate(outs):
-        assert torch.equal(out, want[i % 2]), i
+    for i, x in enumerate(got):
+        assert torch.equal(x, want[i % 2]), i
+
+
+@pytest.mark.parametrize("m,n,k", [(8, 4096, 4096), (1, 512, 512), (4, 2048, 4096), (5, 4096, 1032), (48, 2304, 768), (200, 768, 2048), (600, 9472, 2048),
+                                   (400, 9472, 2048), (70, 300, 333)])
+@pytest.mark.parametrize("operand", ["weights", "rows", "bias", "residual"])
+def test_gemm_bf16_call_reads_nothing_before_the_product_ahead_of_it_has_ended(m, n, k, operand):
+    """Operator launches are made ready while the kernel before them drains, which may be the one that writes an operand.  Every engine (few rows,
+    streamed, tcgen05 tiles and pairs of CTAs, CUDA cores); the same bits as with a wait in between."""
+    g = torch.Generator(device="cuda").manual_seed(43)
+    a, bt = (torch.randn(r, k, device="cuda", generator=g).to(torch.bfloat16) for r in (m, n))
+    bias, resid, out = torch.randn(n, device="cuda", generator=g), torch.randn(m, n, device="cuda", generator=g), torch.empty(m, n, device="cuda")
+    shape, dtype = {"weights": ((n, k), BF16), "rows": ((m, k), BF16), "bias": ((1, n), F32), "residual": ((m, n), F32)}[operand]
+    writer = Writer(*shape, dtype, seed=44)
+    a, bt, bias, resid = (writer.out if operand == x else t for x, t in (("rows", a), ("weights", bt), ("bias", bias), ("residual", resid)))
+    same_bits_as_with_waits(writer, lambda: ok(lib().tnsr_b200_gemm_bf16(ptr(a), ptr(bt), ptr(bias), ptr(resid), ptr(out), m, n, k, -1, 0, stream())), out)
+
+
+@pytest.mark.parametrize("rows", [8, 48, 300])
+@pytest.mark.parametrize("operand", ["x", "gate_up", "down", "gate_up bias", "down bias"])
+def test_swiglu_mlp_call_reads_nothing_before_the_product_ahead_of_it_has_ended(rows, operand):
+    """The second product of the block asks for its weights before its own wait; the first one's wait is before it."""
+    d, f = 1024, 2816
+    g = torch.Generator(device="cuda").manual_seed(45)
+    shapes = {"x": ((rows, d), BF16, 1.0), "gate_up": ((2 * f, d), BF16, d ** -0.5), "down": ((d, f), BF16, f ** -0.5),
+              "gate_up bias": ((1, 2 * f), F32, 1.0), "down bias": ((1, d), F32, 1.0)}
+    t = {name: torch.randn(shape, device="cuda", generator=g).mul_(std).to(torch.float32 if dtype == F32 else torch.bfloat16)
+         for name, (shape, dtype, std) in shapes.items()}
+    shape, dtype, std = shapes[operand]
+    writer = Writer(*shape, dtype, seed=46, std=std)
+    t[operand] = writer.out
+    hidden, out = torch.empty((rows, f), device="cuda", dtype=torch.bfloat16), torch.empty((rows, d), device="cuda", dtype=torch.bfloat16)
+    same_bits_as_with_waits(writer, lambda: ok(lib().tnsr_b200_swiglu_mlp(ptr(t["x"]), ptr(t["gate_up"]), ptr(t["gate_up bias"]), ptr(t["down"]),
+                                                                          ptr(t["down bias"]), ptr(hidden), ptr(out), rows, d, f, stream())), out)
+
+
+@pytest.mark.parametrize("batch,capacity", [(4, 512), (24, 1536)])            # the launch of clusters; plan and streaming kernel
+@pytest.mark.parametrize("operand", ["q", "k", "v", "lengths"])
+def test_decode_attention_call_reads_nothing_before_the_kernel_ahead_of_it_has_ended(batch, capacity, operand):
+    heads, hd = 12, 64
+    d = heads * hd
+    g = torch.Generator(device="cuda").manual_seed(48)
+    t = {"q": torch.randn(batch, d, device="cuda", generator=g).to(torch.bfloat16)}
+    t["k"], t["v"] = (torch.randn(batch * capacity, d, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    t["lengths"] = torch.randint(1, capacity + 1, (batch,), device="cuda", generator=g, dtype=torch.int32)
+    if operand == "lengths":
+        # greedy ids of two sets of logits: a kernel that lets the next launch in at its start too
+        logits = [torch.rand(batch, capacity, device="cuda", generator=g) for _ in range(2)]
+
+        def writer(which):
+            ok(lib().tnsr_b200_argmax(ptr(logits[which]), ptr(t["lengths"]), batch, capacity, stream()))
+    else:
+        writer = Writer(*t[operand].shape, BF16, seed=49, k=1024)
+        t[operand] = writer.out
+    space = lib().tnsr_b200_decode_attention_workspace(batch, capacity, heads, hd)
+    workspace, out = torch.zeros(space, device="cuda", dtype=torch.uint8), torch.empty(batch, d, device="cuda", dtype=torch.bfloat16)
+    same_bits_as_with_waits(writer, lambda: ok(lib().tnsr_b200_decode_attention(ptr(t["q"]), ptr(t["k"]), ptr(t["v"]), ptr(t["lengths"]), ptr(out),
+                                                                                ptr(workspace), space, batch, capacity, heads, hd, stream())), out)
 
 
 # ---- SwiGLU ----------------------------------------------------------------------

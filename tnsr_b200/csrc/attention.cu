@@ -186,7 +186,7 @@ bool decode_attention_supported(uint32_t heads, uint32_t head_dim) {
 // ---- plan: one block ---------------------------------------------------------------
 // Session b has lengths[b] + extra keys; lengths == nullptr means (d_position ? *d_position : 0) + extra for all.
 __global__ void __launch_bounds__(1024)
-da_plan_kernel(const uint32_t* __restrict__ lengths, const uint32_t* __restrict__ d_position, uint32_t extra,
+da_plan_kernel(const uint32_t* lengths, const uint32_t* d_position, uint32_t extra,
                uint32_t batch, uint32_t heads, uint32_t capacity, uint32_t grid, uint32_t ks, uint32_t* __restrict__ header,
                uint32_t* __restrict__ first, uint32_t* __restrict__ count, uint32_t* __restrict__ done,
                uint32_t* __restrict__ sstart, uint32_t* __restrict__ cta_begin, DaItem* __restrict__ items,

@@ -34,7 +34,7 @@ constexpr int SB = 64, SK = 16;
 
 template <int MODE>
 __global__ void __launch_bounds__(256)
-gemm_simple_kernel(const bf16* __restrict__ a, uint32_t lda, const bf16* __restrict__ bt, EpiParams P, uint32_t k) {
+gemm_simple_kernel(const bf16* a, uint32_t lda, const bf16* bt, EpiParams P, uint32_t k) {
     __shared__ float as[SK][SB + 4];
     __shared__ float bs[SK][SB + 4];
     __shared__ float cs[SB][SB + 1];
@@ -245,35 +245,36 @@ template <bool SCALED>
 __device__ __forceinline__ void epilogue_block_reduce(const EpiParams& P, const CUtensorMap* map_out, float* stage,
                                                       uint32_t row0, uint32_t col0, const float* acc, uint32_t lane,
                                                       bool store = false, bool with_bias = true, uint32_t row_out = 0) {
+    const bool bias_vec = with_bias && P.ep.bias && (reinterpret_cast<uintptr_t>(P.ep.bias) & 15) == 0 && col0 + 32 <= P.n;
+    const bool scale_vec = SCALED && (reinterpret_cast<uintptr_t>(P.ep.scale) & 15) == 0 && col0 + 32 <= P.n;
+    float4 v[8];        // bias and scale are asked for ahead of the wait and of the stores, which plain loads do not pass
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+        const uint32_t c = col0 + 4 * g;
+        float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (bias_vec) {
+            b = *reinterpret_cast<const float4*>(P.ep.bias + c);
+        } else if (with_bias && P.ep.bias) {
+            b = make_float4(c < P.n ? P.ep.bias[c] : 0.f, c + 1 < P.n ? P.ep.bias[c + 1] : 0.f,
+                            c + 2 < P.n ? P.ep.bias[c + 2] : 0.f, c + 3 < P.n ? P.ep.bias[c + 3] : 0.f);
+        }
+        v[g] = act4(make_float4(acc[4 * g] + b.x, acc[4 * g + 1] + b.y, acc[4 * g + 2] + b.z, acc[4 * g + 3] + b.w), P.ep.activation);
+        if (SCALED) {
+            if (scale_vec) {
+                const float4 f = *reinterpret_cast<const float4*>(P.ep.scale + c);
+                v[g] = make_float4(v[g].x * f.x, v[g].y * f.y, v[g].z * f.z, v[g].w * f.w);
+            } else {
+                v[g] = make_float4(c < P.n ? v[g].x * P.ep.scale[c] : 0.f, c + 1 < P.n ? v[g].y * P.ep.scale[c + 1] : 0.f,
+                                   c + 2 < P.n ? v[g].z * P.ep.scale[c + 2] : 0.f, c + 3 < P.n ? v[g].w * P.ep.scale[c + 3] : 0.f);
+            }
+        }
+    }
     // the previous box of this warp must have been read out of the buffer
     if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     __syncwarp();
     float4* row = reinterpret_cast<float4*>(stage) + lane * 8;
-    const bool bias_vec = with_bias && P.ep.bias && (reinterpret_cast<uintptr_t>(P.ep.bias) & 15) == 0 && col0 + 32 <= P.n;
-    const bool scale_vec = SCALED && (reinterpret_cast<uintptr_t>(P.ep.scale) & 15) == 0 && col0 + 32 <= P.n;
 #pragma unroll
-    for (int g = 0; g < 8; ++g) {
-        float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (bias_vec) {
-            b = __ldg(reinterpret_cast<const float4*>(P.ep.bias + col0 + 4 * g));
-        } else if (with_bias && P.ep.bias) {
-            const uint32_t c = col0 + 4 * g;
-            b = make_float4(c < P.n ? P.ep.bias[c] : 0.f, c + 1 < P.n ? P.ep.bias[c + 1] : 0.f,
-                            c + 2 < P.n ? P.ep.bias[c + 2] : 0.f, c + 3 < P.n ? P.ep.bias[c + 3] : 0.f);
-        }
-        float4 v = act4(make_float4(acc[4 * g] + b.x, acc[4 * g + 1] + b.y, acc[4 * g + 2] + b.z, acc[4 * g + 3] + b.w), P.ep.activation);
-        if (SCALED) {
-            const uint32_t c = col0 + 4 * g;
-            if (scale_vec) {
-                const float4 f = __ldg(reinterpret_cast<const float4*>(P.ep.scale + c));
-                v = make_float4(v.x * f.x, v.y * f.y, v.z * f.z, v.w * f.w);
-            } else {
-                v = make_float4(c < P.n ? v.x * P.ep.scale[c] : 0.f, c + 1 < P.n ? v.y * P.ep.scale[c + 1] : 0.f,
-                                c + 2 < P.n ? v.z * P.ep.scale[c + 2] : 0.f, c + 3 < P.n ? v.w * P.ep.scale[c + 3] : 0.f);
-            }
-        }
-        row[(g ^ lane) & 7] = v;     // 16-byte chunk g of row r sits at g ^ (r & 7)
-    }
+    for (int g = 0; g < 8; ++g) row[(g ^ lane) & 7] = v[g];     // 16-byte chunk g of row r sits at g ^ (r & 7)
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
     if (lane == 0) {
@@ -304,7 +305,7 @@ __device__ __forceinline__ void epilogue_block_store(const EpiParams& P, const C
     if (P.ep.bias && (reinterpret_cast<uintptr_t>(P.ep.bias) & 15) == 0 && col0 + 32 <= P.n) {
 #pragma unroll
         for (int g = 0; g < 8; ++g) {
-            const float4 t = __ldg(reinterpret_cast<const float4*>(P.ep.bias + col0 + 4 * g));
+            const float4 t = *reinterpret_cast<const float4*>(P.ep.bias + col0 + 4 * g);
             b[4 * g] = t.x; b[4 * g + 1] = t.y; b[4 * g + 2] = t.z; b[4 * g + 3] = t.w;
         }
     } else {
@@ -382,8 +383,8 @@ __device__ __forceinline__ void epilogue_block(const EpiParams& P, float* stage,
             bf16* out = reinterpret_cast<bf16*>(base);
             float4 b0 = make_float4(0.f, 0.f, 0.f, 0.f), b1 = b0;
             if (P.ep.bias) {
-                b0 = __ldg(reinterpret_cast<const float4*>(P.ep.bias + col0 + c8));
-                b1 = __ldg(reinterpret_cast<const float4*>(P.ep.bias + col0 + c8 + 4));
+                b0 = *reinterpret_cast<const float4*>(P.ep.bias + col0 + c8);
+                b1 = *reinterpret_cast<const float4*>(P.ep.bias + col0 + c8 + 4);
             }
 #pragma unroll
             for (uint32_t it = 0; it < 4; ++it) {
@@ -408,8 +409,8 @@ __device__ __forceinline__ void epilogue_block(const EpiParams& P, float* stage,
         if (full_cols && P.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 7) == 0) {
             float4 bg = make_float4(0.f, 0.f, 0.f, 0.f), bu = bg;
             if (P.ep.bias) {
-                bg = __ldg(reinterpret_cast<const float4*>(P.ep.bias + col0 + 4 * j));
-                bu = __ldg(reinterpret_cast<const float4*>(P.ep.bias + col0 + 16 + 4 * j));
+                bg = *reinterpret_cast<const float4*>(P.ep.bias + col0 + 4 * j);
+                bu = *reinterpret_cast<const float4*>(P.ep.bias + col0 + 16 + 4 * j);
             }
             const uint32_t ocol = col0 / 2 + 4 * j;
 #pragma unroll
@@ -448,8 +449,8 @@ __device__ __forceinline__ void epilogue_block(const EpiParams& P, float* stage,
         if (fast) {
             float4 b0 = make_float4(0.f, 0.f, 0.f, 0.f), b1 = b0;
             if (P.ep.bias) {
-                b0 = __ldg(reinterpret_cast<const float4*>(P.ep.bias + col0 + c8));
-                b1 = __ldg(reinterpret_cast<const float4*>(P.ep.bias + col0 + c8 + 4));
+                b0 = *reinterpret_cast<const float4*>(P.ep.bias + col0 + c8);
+                b1 = *reinterpret_cast<const float4*>(P.ep.bias + col0 + c8 + 4);
             }
             const int act = MODE == GEMM_QKV ? ACT_NONE : P.ep.activation;
 #pragma unroll
@@ -494,11 +495,11 @@ __device__ __forceinline__ void epilogue_block(const EpiParams& P, float* stage,
                 load_residual_block(P, row0, col0, lane, r4);
             }
             float4 bv = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (P.ep.bias) bv = __ldg(reinterpret_cast<const float4*>(P.ep.bias + col0 + c4));
+            if (P.ep.bias) bv = *reinterpret_cast<const float4*>(P.ep.bias + col0 + c4);
             float4 sv = make_float4(1.f, 1.f, 1.f, 1.f);
             if (MODE == GEMM_SCALED) {
                 const float* f = P.ep.scale + col0 + c4;       // any alignment
-                sv = make_float4(__ldg(f), __ldg(f + 1), __ldg(f + 2), __ldg(f + 3));
+                sv = make_float4(f[0], f[1], f[2], f[3]);
             }
 #pragma unroll
             for (uint32_t it = 0; it < 8; ++it) {
@@ -517,8 +518,8 @@ __device__ __forceinline__ void epilogue_block(const EpiParams& P, float* stage,
 #pragma unroll
             for (int rr = 0; rr < 32; ++rr)
                 rv[rr] = (res && col_ok && (uint32_t)rr < rows) ? res[(size_t)(row0 + rr) * P.ep.ldr + col] : 0.0f;
-            const float bv = (P.ep.bias && col_ok) ? __ldg(P.ep.bias + col) : 0.0f;
-            const float sv = (MODE == GEMM_SCALED && col_ok) ? __ldg(P.ep.scale + col) : 1.0f;
+            const float bv = (P.ep.bias && col_ok) ? P.ep.bias[col] : 0.0f;
+            const float sv = (MODE == GEMM_SCALED && col_ok) ? P.ep.scale[col] : 1.0f;
 #pragma unroll
             for (int rr = 0; rr < 32; ++rr)
                 if (col_ok && (uint32_t)rr < rows)

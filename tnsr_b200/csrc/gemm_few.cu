@@ -38,9 +38,11 @@ struct FewParams {
 struct Words { uint32_t x[8]; };
 
 __device__ __forceinline__ Words fw_zero() { return {{0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u}}; }
+// Weights and rows alike may be what a kernel wrote before which this grid was resident already: no form of load that takes them for constant
+// (.nc, __ldg), here or in the other kernels of a product.
 __device__ __forceinline__ Words fw_load_weights(const bf16* p) {
     Words v;
-    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+    asm volatile("ld.global.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=r"(v.x[0]), "=r"(v.x[1]), "=r"(v.x[2]), "=r"(v.x[3]), "=r"(v.x[4]), "=r"(v.x[5]), "=r"(v.x[6]), "=r"(v.x[7]) : "l"(p));
     return v;
 }
@@ -91,23 +93,41 @@ gemm_few_kernel(const __grid_constant__ FewParams P) {
         for (int j = 0; j < NT; ++j) w[j][s] = ok && col + j * col_step < n ? fw_load_weights(p + (size_t)j * col_step * k) : fw_zero();
     };
     uint32_t tile = blockIdx.x / P.ck;
-    if (P.epi.ep.wait_first) pdl_wait();
-#pragma unroll
-    for (int s = 0; s < S; ++s) load_w(s, tile, b0 + s);
     // A thread finishes elements tid, tid + 256, ... of the (ck = 1) tile, all of one column: its bias and scale
     const uint32_t threads = FW_THREADS * P.ck, tid = rank * FW_THREADS + threadIdx.x;
     const uint32_t my_cols = swiglu ? COLS / 2 : COLS, my_col = tid % my_cols;
+    float bias = 0.0f, bias_up = 0.0f, scale = 1.0f;
+    auto load_col = [&](uint32_t col) {
+        if (col >= n) return;
+        if (P.epi.ep.bias) {
+            bias = P.epi.ep.bias[col];
+            if (swiglu) bias_up = P.epi.ep.bias[col + 16];
+        }
+        if (P.mode == GEMM_PLAIN && P.epi.ep.scale) scale = P.epi.ep.scale[col];
+    };
+    if (P.epi.ep.wait_first) {
+        // L2 may have what is at the weights' places now: whoever still writes them does so there (1 x 4096 x 4096 back to back 11.5 us without,
+        // 10.4 with; 1 x 4096 x 1024 4.4 / 3.7)
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            const uint32_t c = first_col(tile) + g, b = b0 + s;
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+                if (tile < P.tiles && b < b1 && b * FW_BLOCK + 16 * t < k && c + j * col_step < n)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(P.w + (size_t)(c + j * col_step) * k + b * FW_BLOCK + 16 * t));
+        }
+        pdl_wait();
+    }
+#pragma unroll
+    for (int s = 0; s < S; ++s) load_w(s, tile, b0 + s);
+    load_col(first_col(tile) + my_col);
 
     pdl_wait();
     pdl_trigger();
     const bf16* ap = P.a + (size_t)(row0 + g) * k + 16 * t;       // rows g, g + 8, g + 16 ... of the tile
-    for (; tile < P.tiles; tile += tile_step) {
+    for (bool first = true; tile < P.tiles; tile += tile_step, first = false) {
         const uint32_t col0 = first_col(tile), col = col0 + my_col;
-        float bias = 0.0f, bias_up = 0.0f;
-        if (P.epi.ep.bias && col < n) {
-            bias = __ldg(P.epi.ep.bias + col);
-            if (swiglu) bias_up = __ldg(P.epi.ep.bias + col + 16);
-        }
+        if (!first) load_col(col);
         // what the end of the tile reads from memory per element: the residual, or the row of the cache
         uint32_t early[MINE];
 #pragma unroll
@@ -215,7 +235,7 @@ gemm_few_kernel(const __grid_constant__ FewParams P) {
                     if (ep.out_dtype == TNSR_B200_BF16) {
                         reinterpret_cast<bf16*>(P.epi.out)[o] = __float2bfloat16_rn(v);
                     } else {
-                        if (ep.scale) v *= __ldg(ep.scale + col);
+                        if (ep.scale) v *= scale;
                         if (ep.residual) v += __uint_as_float(early[i]);
                         reinterpret_cast<float*>(P.epi.out)[o] = v;
                     }

@@ -62,12 +62,12 @@ struct SkParams {
 
 __device__ __forceinline__ void sk_store(const SkParams& P, uint32_t row, uint32_t col, float acc) {
     float v = acc;
-    if (P.bias) v += __ldg(P.bias + col);
+    if (P.bias) v += P.bias[col];
     v = apply_activation(v, P.activation);
     if (P.out_dtype == TNSR_B200_BF16) {
         reinterpret_cast<bf16*>(P.out)[(size_t)row * P.ldc + col] = __float2bfloat16_rn(v);
     } else {
-        if (P.scale) v *= __ldg(P.scale + col);
+        if (P.scale) v *= P.scale[col];
         if (P.residual) v += P.residual[(size_t)row * P.ldr + col];
         reinterpret_cast<float*>(P.out)[(size_t)row * P.ldc + col] = v;
     }

@@ -177,12 +177,12 @@ gemm_stream_kernel(GsParams P) {
                 for (int w = 0; w < GS_THREADS / 32; ++w) v += red[(size_t)w * GS_ROWS * MT + c * MT + m];
                 const uint32_t colg = n0 + c;
                 if (m < P.m && colg < P.n) {
-                    if (P.bias) v += __ldg(P.bias + colg);
+                    if (P.bias) v += P.bias[colg];
                     v = apply_activation(v, P.activation);
                     if (P.out_dtype == TNSR_B200_BF16) {
                         reinterpret_cast<bf16*>(P.out)[(size_t)m * P.ldc + colg] = __float2bfloat16_rn(v);
                     } else {
-                        if (P.scale) v *= __ldg(P.scale + colg);
+                        if (P.scale) v *= P.scale[colg];
                         if (P.residual) v += P.residual[(size_t)m * P.ldr + colg];
                         reinterpret_cast<float*>(P.out)[(size_t)m * P.ldc + colg] = v;
                     }
