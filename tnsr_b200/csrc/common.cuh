@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <cstdlib>
 #include <string>
 #include <utility>
 #include <vector>
@@ -107,6 +108,12 @@ inline void launch_kernel_clusters(void (*kernel)(KArgs...), dim3 grid, dim3 blo
 template <typename... KArgs, typename... Args>
 inline void launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
     launch_kernel_clusters(kernel, grid, block, smem, 1, stream, std::forward<Args>(args)...);
+}
+
+// A debugging switch of the environment: set, and to 1.
+inline bool switched_on(const char* name) {
+    const char* v = std::getenv(name);
+    return v && v[0] == '1';
 }
 
 inline uint32_t ceil_div(uint32_t a, uint32_t b) { return (a + b - 1) / b; }

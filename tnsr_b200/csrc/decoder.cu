@@ -31,10 +31,7 @@ void prefer_max_shared_carveout(const void* kernel) {
         cudaGetLastError();   // a hint only: the launch itself does not depend on it
 }
 bool debug_sync_enabled() {
-    static const bool on = [] {
-        const char* v = std::getenv("TNSR_B200_DEBUG_SYNC");
-        return v && v[0] == '1';
-    }();
+    static const bool on = switched_on("TNSR_B200_DEBUG_SYNC");
     return on;
 }
 }  // namespace tb
@@ -750,11 +747,8 @@ static int create_decoder(const tnsr_b200_config* config, const tnsr_b200_stack*
         if ((rc = dev_alloc(dec, &dec->lm_candidates, lm_head_argmax_scratch_bytes(config->batch, config->vocab_size), false)))
             return bail(rc);
     {
-        const char* v = std::getenv("TNSR_B200_NO_GRAPH");
-        if (v && v[0] == '1') dec->use_graphs = false;
-        v = std::getenv("TNSR_B200_NO_PDL");
-        if (v && v[0] == '1') dec->use_pdl = false;
-
+        if (switched_on("TNSR_B200_NO_GRAPH")) dec->use_graphs = false;
+        if (switched_on("TNSR_B200_NO_PDL")) dec->use_pdl = false;
     }
     if (cudaMallocHost((void**)&dec->h_status, 16 + (size_t)config->batch * 4) != cudaSuccess ||
         cudaMallocHost((void**)&dec->h_logits, kStagedLogitBytes) != cudaSuccess)

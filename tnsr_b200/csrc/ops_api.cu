@@ -1,8 +1,6 @@
 // extern "C" wrappers of the individual kernels (operator-level entry points of
 // include/tnsr_b200.h).  They queue work on the caller's stream and never
 // synchronise or allocate.
-#include <cstdlib>
-
 #include "common.cuh"
 #include "feed_forward.cuh"
 #include "mixers.cuh"
@@ -25,7 +23,7 @@ struct OverlapLaunches {
     explicit OverlapLaunches(cudaStream_t stream) {
         cudaStreamCaptureStatus status = cudaStreamCaptureStatusActive;
         if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) cudaGetLastError();
-        static const bool off = std::getenv("TNSR_B200_NO_PDL") != nullptr;
+        static const bool off = switched_on("TNSR_B200_NO_PDL");      // as it was at the first call
         t_pdl = !off && status == cudaStreamCaptureStatusNone;
     }
     ~OverlapLaunches() { t_pdl = before; }
