@@ -2,11 +2,13 @@
 //
 // Two engines share one epilogue:
 //  * gemm_tc_kernel   -- the Blackwell path: TMA (cp.async.bulk.tensor, 128-byte
-//    swizzle; long products in pairs of CTAs that share a tile) feeds a shared-memory ring,
-//    one thread issues tcgen05.mma (M=128 or a pair's 256, N=BN, K=16 per instruction) into
+//    swizzle, one copy per CTA, no cluster forms) feeds a shared-memory ring,
+//    one thread issues tcgen05.mma (M=128, N=BN, K=16 per instruction) into
 //    double-buffered TMEM accumulators, eight epilogue warps drain them with
 //    tcgen05.ld, transpose each 32x32 block through shared memory and write
 //    coalesced rows while the next tile's main loop runs.  Persistent over tiles.
+//    gemm_tc_pair_kernel is the same for products with a long k: two CTAs of a
+//    cluster share a tile (cta_group::2, M=256).
 //  * gemm_simple_kernel -- CUDA-core kernel for shapes TMA cannot address
 //    (k not a multiple of 8, unaligned pointers) and as the cross-check of the
 //    tensor-core engine.
@@ -738,8 +740,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 template <int MODE, int EPI>
 __global__ void __launch_bounds__(64 + 32 * EPI, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                    const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_k,
-                    const __grid_constant__ CUtensorMap map_v, TcParams prm) {
+                    const __grid_constant__ CUtensorMap map_out, TcParams prm) {
     constexpr int BN = 256;
     using S = TcShape<BN, EPI, 2>;
     extern __shared__ uint8_t smem_raw[];
@@ -828,13 +829,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             }
         }
     } else {
-        // ---------------- epilogue warps, of each CTA: as in the kernel above ----------------
+        // ---------------- epilogue warps, of each CTA: as in the kernel above, without the bulk stores of a short k ----------------
         const uint32_t quarter = warp & 3, half = (warp - 2) >> 2;
         float* stage = stage_tiles + (warp - 2) * (TC_STAGE_TILE_BYTES / 4);
-        uint32_t it = 0, store_parity = 0;
+        uint32_t it = 0;
         const bool reduce = (MODE == GEMM_PLAIN || MODE == GEMM_SCALED) && prm.tma_reduce;
-        const uint32_t qkv_pos = (MODE == GEMM_QKV && prm.tma_store)
-                                     ? (prm.epi.qkv.d_position ? *prm.epi.qkv.d_position : prm.epi.qkv.position) : 0u;
         for (uint32_t tile = first_tile; tile < num_tiles; tile += tile_step, ++it) {
             const uint32_t ab = it & 1, aphase = (it >> 1) & 1;
             uint32_t tm, tn;
@@ -851,14 +850,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 const uint32_t col0 = tn * BN + c;
                 if (row0 >= prm.epi.m || col0 >= prm.epi.n) continue;
                 if (reduce) epilogue_block_reduce<MODE == GEMM_SCALED>(prm.epi, &map_out, stage, row0, col0, acc, lane);
-                else if (prm.tma_store) epilogue_block_store<MODE>(prm.epi, &map_out, &map_k, &map_v, stage, row0, col0, acc, lane, store_parity++, qkv_pos);
                 else epilogue_block<MODE>(prm.epi, stage, row0, col0, acc, lane);
             }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(leader_addr(acc_empty + ab));     // where the products that overwrite it are issued
         }
-        if ((reduce || prm.tma_store) && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        if (reduce && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
 
     // ---------------- teardown ----------------
@@ -920,7 +918,7 @@ static int launch_pair_e(const CUtensorMap& ma, const CUtensorMap& mb, const CUt
     using S = TcShape<256, EPI, 2>;
     if (const int rc = allow_shared<gemm_tc_pair_kernel<MODE, EPI>>(S::SMEM_BYTES, "gemm_tc_pair attribute")) return rc;
     const uint32_t grid = 2 * std::min(prm.tiles_m * prm.tiles_n, (uint32_t)sm_count() / 2);
-    launch_kernel_clusters(gemm_tc_pair_kernel<MODE, EPI>, dim3(grid), dim3(S::THREADS), S::SMEM_BYTES, 2, stream, ma, mb, mo[0], mo[1], mo[2], prm);
+    launch_kernel_clusters(gemm_tc_pair_kernel<MODE, EPI>, dim3(grid), dim3(S::THREADS), S::SMEM_BYTES, 2, stream, ma, mb, mo[0], prm);
     count_launch();
     return check_launch("gemm_tc_pair");
 }
