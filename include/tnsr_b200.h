@@ -276,6 +276,12 @@ TNSR_B200_API int tnsr_b200_set_wait_limit_ns(uint64_t ns);
  * out after the wait limit and the kernel returns through its time-out path,
  * which is the only way to exercise that path on healthy hardware. */
 TNSR_B200_API int tnsr_b200_test_lose_gemm_stage(uint32_t k_block);
+/* Test hook (no reference counterpart): the tile that the tcgen05 GEMM takes for
+ * an [m, n] product over k (`argmax`: the greedy head) -- its columns, and how
+ * many CTAs share one (1 or 2) -- so that a test of a tile can tell that it
+ * reaches it.  Launches nothing. */
+TNSR_B200_API int tnsr_b200_test_gemm_tile(uint32_t m, uint32_t n, uint32_t k, int argmax,
+                                           uint32_t* columns, uint32_t* ctas);
 
 /* ---- session: replaces cuda::CudaDecoder -------------------------------- */
 

@@ -325,11 +325,20 @@ def test_gemm_bf16_in_place_residual_update_equals_out_of_place(shape, activatio
     assert torch.equal(twice, again)
 
 
-@pytest.mark.parametrize("shape", [(400, 9448, 1544), (270, 9472, 1536), (1000, 9448, 1600),      # pairs of CTAs: ragged rows, columns and k,
-                                   (400, 6000, 264), (3885, 768, 776)])                        # an empty half, two tiles each; 192 columns
+def gemm_tile(m, n, k, argmax=0):
+    """(columns of a tile, CTAs that share one) of the tcgen05 engine."""
+    columns, ctas = C.c_uint32(), C.c_uint32()
+    ok(lib().tnsr_b200_test_gemm_tile(m, n, k, argmax, C.byref(columns), C.byref(ctas)))
+    return columns.value, ctas.value
+
+
+# pairs of CTAs: ragged rows, columns and k, an empty half (rows 257 .. 270 are the first CTA's), more tiles than pairs; then 192 columns
+@pytest.mark.parametrize("shape,tile", [((400, 9448, 2056), (256, 2)), ((270, 9472, 2048), (256, 2)), ((1000, 9448, 2064), (256, 2)),
+                                        ((400, 6000, 264), (192, 1)), ((3885, 768, 776), (192, 1))])
 @pytest.mark.parametrize("form", ["f32", "bf16", "residual"])
-def test_gemm_bf16_tiles_of_pairs_and_of_192_columns(shape, form):
+def test_gemm_bf16_tiles_of_pairs_and_of_192_columns(shape, tile, form):
     m, n, k = shape
+    assert gemm_tile(m, n, k) == tile
     g = torch.Generator(device="cuda").manual_seed(41)
     a, bt = (torch.randn(r, k, device="cuda", generator=g).to(torch.bfloat16) for r in (m, n))
     bias, resid = torch.randn(n, device="cuda", generator=g), torch.randn(m, n, device="cuda", generator=g)
@@ -345,6 +354,30 @@ def test_gemm_bf16_tiles_of_pairs_and_of_192_columns(shape, form):
     # 2^-8 of the value, and the sum's own error may tip it over to the next one
     err = (got.double() - want).abs() - (want.abs() * 2.0 ** -8 if form == "bf16" else 0.0)
     assert float(err.max()) <= 2e-3
+
+
+@pytest.mark.parametrize("rows,d,f,tile", [(1100, 2064, 5616, (256, 2)), (700, 2048, 5632, (256, 2)), (200, 776, 5616, (192, 1))])
+def test_swiglu_mlp_in_tiles_of_pairs_and_of_192_columns(rows, d, f, tile):
+    """Ragged rows, k and a last column tile that is partly empty."""
+    assert gemm_tile(rows, 2 * f, d) == tile
+    g = torch.Generator(device="cuda").manual_seed(47)
+
+    def normal(*shape, std):
+        return (torch.randn(shape, device="cuda", generator=g) * std).to(torch.bfloat16)
+
+    x, gate, up, down = normal(rows, d, std=1.0), normal(d, f, std=d ** -0.5), normal(d, f, std=d ** -0.5), normal(f, d, std=f ** -0.5)
+    bias_gate, bias_up, bias_down = (torch.randn(w, device="cuda", generator=g) for w in (f, f, d))
+    packed, packed_bias = torch.empty((2 * f, d), device="cuda", dtype=torch.bfloat16), torch.empty(2 * f, device="cuda")
+    ok(lib().tnsr_b200_pack_gate_up(ptr(gate), ptr(up), ptr(bias_gate), ptr(bias_up), ptr(packed), ptr(packed_bias), d, f, stream()))
+    down_t, hidden = down.T.contiguous(), torch.empty((rows, f), device="cuda", dtype=torch.bfloat16)
+    out = torch.empty((rows, d), device="cuda", dtype=torch.bfloat16)
+    ok(lib().tnsr_b200_swiglu_mlp(ptr(x), ptr(packed), ptr(packed_bias), ptr(down_t), ptr(bias_down), ptr(hidden), ptr(out), rows, d, f, stream()))
+    torch.cuda.synchronize()
+    want = torch.nn.functional.silu(x.double() @ gate.double() + bias_gate) * (x.double() @ up.double() + bias_up)
+    # bf16 of an f32 result: half a unit is at most 2^-8 of the value; the f32 sums and the sigmoid are good to 1e-5 of values of size 10
+    assert float(((hidden.double() - want).abs() - want.abs() * 2.0 ** -8).max()) <= 2e-4
+    want = hidden.double() @ down.double() + bias_down
+    assert float(((out.double() - want).abs() - want.abs() * 2.0 ** -8).max()) <= 2e-4
 
 
 # ---- operator launches that are made ready early ----------------------------------
@@ -524,12 +557,16 @@ def test_decode_attention_live_prefix_and_poisoned_slots(oracle, heads, hd):
     assert np.max(np.abs(got - expected)) <= scale / 128
 
 
-@pytest.mark.parametrize("heads,hd,batch", [(12, 64, 7), (1, 64, 7), (3, 32, 7), (5, 128, 7), (16, 64, 30)])
-def test_decode_attention_of_few_keys_equals_the_streaming_kernel(oracle, heads, hd, batch):
+@pytest.mark.parametrize("heads,hd,capacity,lengths", [
+    *((h, hd, 300, ([1, 63, 64, 65, 129, 0, 300] * 5)[:b]) for h, hd, b in ((12, 64, 7), (1, 64, 7), (3, 32, 7), (5, 128, 7), (16, 64, 30))),
+    (2, 64, 300, [127, 128, 129, 255, 256, 257]),                              # whole passes of a CTA's 128 keys
+    (12, 64, 4000, [4000, 3999, 1025, 1024]), (20, 64, 4000, [4000, 8, 2049, 3000]),      # clusters of 8 and of 5, several passes each
+    (5, 128, 4000, [4000, 513, 511, 2050]), (12, 32, 8000, [8000, 2049, 4097, 100])])     # 64 and 256 keys a pass
+def test_decode_attention_of_few_keys_equals_the_streaming_kernel(oracle, heads, hd, capacity, lengths):
     """Few keys in all take a launch of clusters; a larger capacity, with the same lengths, the streaming kernel.  Lengths at the edges of a
     pass, of a cluster's shares, none, the whole capacity; slots past a length hold NaN."""
-    capacity, large = 300, 400000 // (batch * heads) + 16
-    lengths = np.asarray(([1, 63, 64, 65, 129, 0, 300] * 5)[:batch], dtype=np.uint32)
+    lengths, batch = np.asarray(lengths, dtype=np.uint32), len(lengths)
+    large = 400000 // (batch * heads) * max(1, 64 // hd) + 16
     rng = np.random.default_rng(71)
     q = rng.standard_normal((batch, heads * hd)).astype(np.float32)
     k, v = (rng.standard_normal((batch, capacity, heads * hd)).astype(np.float32) for _ in range(2))

@@ -1001,9 +1001,9 @@ def test_the_attention_record_is_of_the_kernels_that_run_without_it(capacity):
     assert np.array_equal(seen[0][1], seen[1][1])
 
 
-@pytest.mark.parametrize("batch,heads,width,capacity", [(24, 12, 768, 1024),      # the streaming kernel: keys asked for ahead, list kept for all layers
-                                                        (2, 4, 256, 4096), (3, 2, 256, 3008)])    # clusters: several passes of a CTA, heads of 64 and 128
-def test_steps_behind_many_keys_have_the_same_bits_however_they_are_launched(monkeypatch, batch, heads, width, capacity):
+@pytest.mark.parametrize("batch,heads,width,capacity,page", [(24, 12, 768, 1024, 32),      # the streaming kernel: keys asked for ahead, list kept for all layers
+                                                             (2, 4, 256, 4096, 64), (3, 2, 256, 3024, 48)])    # clusters: several passes, heads of 64 and 128
+def test_steps_behind_many_keys_have_the_same_bits_however_they_are_launched(monkeypatch, batch, heads, width, capacity, page):
     """Replayed and direct steps, with and without early launches, contiguous and paged caches: steps at a common position and ragged ones.  Pages
     were another tenant's before."""
     cfg = GptConfig(vocab_size=300, max_sequence_length=capacity, embed_dim=width, num_heads=heads, feed_forward_dim=256, num_layers=2,
@@ -1032,8 +1032,92 @@ def test_steps_behind_many_keys_have_the_same_bits_however_they_are_launched(mon
         return np.stack(out).view(np.uint32)
 
     want = run(())
-    for switches, kw in ((("TNSR_B200_NO_GRAPH",), {}), (("TNSR_B200_NO_GRAPH", "TNSR_B200_NO_PDL"), {}), ((), {"kv_page_rows": 32})):
+    for switches, kw in ((("TNSR_B200_NO_GRAPH",), {}), (("TNSR_B200_NO_GRAPH", "TNSR_B200_NO_PDL"), {}), ((), {"kv_page_rows": page})):
         assert np.array_equal(run(switches, **kw), want), (switches, kw)
+
+
+def wide_layer():
+    """One layer of 2048 columns: with 700 rows its query/key/value and gate/up products are pairs of CTAs."""
+    cfg = GptConfig(vocab_size=512, max_sequence_length=400, embed_dim=2048, num_heads=32, feed_forward_dim=5632, num_layers=1,
+                    layer_norm_epsilon=1e-5, activation="swiglu", weight_dtype="bf16")
+    columns, ctas = _native.C.c_uint32(), _native.C.c_uint32()
+    for n in (3 * 2048, 2 * 5632):
+        assert _native.lib().tnsr_b200_test_gemm_tile(700, n, 2048, 0, columns, ctas) == 0
+        assert (columns.value, ctas.value) == (256, 2)
+    return cfg, normal_model_arrays(cfg, seed=65, std=0.02), np.random.default_rng(66).integers(0, 512, size=(2, 350)).astype(np.uint32)
+
+
+@pytest.mark.parametrize("paged", [False, True])
+def test_a_layer_whose_products_are_pairs_of_ctas(paged):
+    """Against the products of the CUDA-core engine: rows of the caches, which are the QKV product's bf16 results (sums in another order may
+    round to the next value, 2^-8 of it), and the logits behind attention and the SwiGLU block."""
+    cfg, arrays, ids = wide_layer()
+
+    def run(engine):
+        s = B200Session(cfg, 2, 400, logits_mode="all", **({"kv_page_rows": 16} if paged else {}))
+        for i, a in enumerate(arrays):
+            s.refresh(i, a)
+        assert _native.lib().tnsr_b200_set_gemm_engine(engine) == 0
+        try:
+            logits = s.decode_full(ids, 0)[0].reshape(2, 350, -1)
+        finally:
+            _native.lib().tnsr_b200_set_gemm_engine(0)
+        caches = [s.read_cache(i)[:, :350].copy() for i in range(2)]
+        s.close()
+        return logits, caches
+
+    (got, got_caches), (want, want_caches) = run(0), run(1)
+    for g, w in zip(got_caches, want_caches):
+        assert np.max(np.abs(g - w) - np.abs(w) * 2.0 ** -7) <= 1e-4
+    assert rel_err(got, want) <= 2e-2
+
+
+def test_a_wait_of_a_pair_that_runs_out_fails_the_session_until_reset():
+    """As test_a_wait_that_runs_out_fails_the_session_until_reset, for two CTAs that share a tile: the first one's copies of a stage are left out,
+    both CTAs' waits run out, each by itself, and the kernel returns."""
+    cfg, arrays, ids = wide_layer()
+    lib = _native.lib()
+    s = B200Session(cfg, 2, 400)
+    for i, a in enumerate(arrays):
+        s.refresh(i, a)
+    want = s.decode_full(ids, 0)[0].copy()
+    s.reset()
+    assert lib.tnsr_b200_set_wait_limit_ns(2_000_000) == 0
+    try:
+        assert lib.tnsr_b200_test_lose_gemm_stage(2) == 0
+        u32p, fp = _native.C.POINTER(_native.C.c_uint32), _native.C.POINTER(_native.C.c_float)
+        logits = np.empty(2 * 350 * cfg.vocab_size, dtype=np.float32)
+        assert lib.tnsr_b200_decoder_decode(s.handle, ids.ctypes.data_as(u32p), 350, 0, logits.ctypes.data_as(fp), None) == -7
+        assert lib.tnsr_b200_decoder_decode(s.handle, ids.ctypes.data_as(u32p), 350, 0, logits.ctypes.data_as(fp), None) == -6
+    finally:
+        assert lib.tnsr_b200_set_wait_limit_ns(2_000_000_000) == 0
+    s.reset()
+    assert np.array_equal(s.decode_full(ids, 0)[0].view(np.uint32), want.view(np.uint32))
+    s.close()
+
+
+def test_greedy_ids_of_a_head_in_tiles_of_192_columns():
+    cfg = GptConfig(vocab_size=20011, max_sequence_length=16, embed_dim=64, num_heads=1, feed_forward_dim=64, num_layers=1, layer_norm_epsilon=1e-5,
+                    activation="swiglu", weight_dtype="bf16")
+    columns, ctas = _native.C.c_uint32(), _native.C.c_uint32()
+    assert _native.lib().tnsr_b200_test_gemm_tile(40, 20011, 64, 1, columns, ctas) == 0
+    assert (columns.value, ctas.value) == (192, 1)
+    arrays = normal_model_arrays(cfg, seed=67, std=0.05)
+    ids = np.random.default_rng(68).integers(0, cfg.vocab_size, size=(40, 5)).astype(np.uint32)
+    picks = []
+    for mode in ("none", "last"):
+        s = B200Session(cfg, 40, 16, logits_mode=mode)
+        for i, a in enumerate(arrays):
+            s.refresh(i, a)
+        logits, greedy = s.decode_full(ids, 0)
+        picks.append(greedy.copy())
+        if mode == "last":
+            rows = logits.reshape(40, -1)
+            top = np.sort(rows, axis=1)[:, -2:]
+            clear = top[:, 1] - top[:, 0] > 1e-4 * np.abs(top[:, 1])     # f32 sums of 64 products in another order
+        s.close()
+    assert clear.sum() >= 30
+    assert np.array_equal(picks[0][clear], picks[1][clear])
 
 
 def test_paged_kv_pool_smaller_than_the_worst_case():

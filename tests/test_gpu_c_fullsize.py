@@ -193,16 +193,22 @@ def test_config4_full_width_chunking_invariance_and_determinism():
     assert whole.min() >= 0 and whole.max() < cfg.vocab_size
 
 
-def test_config4_wide_tile_epilogues_agree_with_narrow_tile_epilogues():
-    """32 sessions x 96 tokens give the projections enough rows for 256-column tiles, whose QKV and SwiGLU epilogues run
-    sixteen warps and write through bulk tensor stores; 8 sessions take narrower tiles with per-lane stores.  The
-    accumulation order over K does not depend on the tile shape, so the first 8 sessions must come out bit-identical:
-    K/V rows of the first and the last layer and the greedy continuation."""
+@pytest.mark.parametrize("sessions,qkv,gate_up,down", [(32, (192, 1), (256, 1), (128, 1)), (36, (256, 1), (256, 1), (192, 1)),
+                                                       (52, (256, 1), (256, 1), (256, 2))])
+def test_config4_wide_tile_epilogues_agree_with_narrow_tile_epilogues(sessions, qkv, gate_up, down):
+    """32 sessions x 96 tokens and more give the projections enough rows for tiles of 192 and 256 columns, whose QKV and SwiGLU epilogues run
+    sixteen warps and, at 256, write through bulk tensor stores, and for pairs of CTAs; 8 sessions take narrower tiles with per-lane stores.
+    The accumulation order over K does not depend on the tile shape, so the first 8 sessions must come out bit-identical: K/V rows of the
+    first and the last layer and the greedy continuation."""
     cfg = GptConfig(vocab_size=32000, max_sequence_length=2048, embed_dim=768, num_heads=12, feed_forward_dim=2048,
                     num_layers=12, layer_norm_epsilon=1e-5, activation="swiglu", weight_dtype="bf16")
     arrays = normal_model_arrays(cfg, seed=5, std=0.02)
     prompt_len, steps = 96, 6
-    ids = np.random.default_rng(56).integers(0, cfg.vocab_size, size=(32, prompt_len)).astype(np.uint32)
+    ids = np.random.default_rng(56).integers(0, cfg.vocab_size, size=(sessions, prompt_len)).astype(np.uint32)
+    columns, ctas = C.c_uint32(), C.c_uint32()
+    for n, k, tile in ((3 * 768, 768, qkv), (2 * 2048, 768, gate_up), (768, 2048, down)):
+        ok(lib().tnsr_b200_test_gemm_tile(sessions * prompt_len, n, k, 0, C.byref(columns), C.byref(ctas)))
+        assert (columns.value, ctas.value) == tile
 
     def run(batch):
         s = B200Session(cfg, batch, 128, logits_mode="none")
@@ -217,7 +223,7 @@ def test_config4_wide_tile_epilogues_agree_with_narrow_tile_epilogues():
         s.close()
         return np.stack(out), caches
 
-    wide_ids, wide = run(32)
+    wide_ids, wide = run(sessions)
     narrow_ids, narrow = run(8)
     for w, n in zip(wide, narrow):
         assert np.array_equal(w[:8, :prompt_len].view(np.uint32), n[:, :prompt_len].view(np.uint32))

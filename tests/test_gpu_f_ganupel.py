@@ -625,6 +625,18 @@ def test_layers_wide_enough_for_the_few_row_products(dtype):
         assert close(row_errors(logits_of(decoder, ids, portions), want), dtype), portions
 
 
+def test_products_in_pairs_of_ctas():
+    """2048 channels and 1856 rows: column ranges, layer scales and single ranges in tiles that two CTAs share."""
+    cfg, tensors, model = build(config(2048, 64, [rglru(2048, 16, 4, dense(2048))]), "bf16")
+    columns, ctas = C.c_uint32(), C.c_uint32()
+    for n in (4096, 2048):
+        ok(lib().tnsr_b200_test_gemm_tile(1856, n, 2048, 0, C.byref(columns), C.byref(ctas)))
+        assert (columns.value, ctas.value) == (256, 2)
+    ids = tokens_for(cfg, 1856)
+    want, _ = plain.forward(cfg, tensors, ids)
+    assert close(row_errors(logits_of(model.decoder_with_capacity(Backend.Cuda, 1, 1856), ids), want), "bf16")
+
+
 @pytest.mark.parametrize("name", ["mixed", "even"])
 def test_scalar_prefill_is_the_same_function(name):
     cfg, tensors, model = build(name, "bf16")

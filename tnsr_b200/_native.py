@@ -113,6 +113,7 @@ SIGNATURES = {
     "tnsr_b200_set_gemm_engine": (_i, [_i]),
     "tnsr_b200_set_wait_limit_ns": (_i, [_u64]),
     "tnsr_b200_test_lose_gemm_stage": (_i, [_u32]),
+    "tnsr_b200_test_gemm_tile": (_i, [_u32, _u32, _u32, _i, _u32p, _u32p]),
     "tnsr_b200_decoder_create": (_i, [C.POINTER(Config), C.POINTER(_vp)]),
     "tnsr_b200_decoder_create_stack": (_i, [C.POINTER(Config), C.POINTER(StackDesc), C.POINTER(_vp)]),
     "tnsr_b200_decoder_destroy": (None, [_vp]),

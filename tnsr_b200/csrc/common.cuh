@@ -21,6 +21,8 @@ typedef __nv_bfloat16 bf16;
 
 extern std::atomic<uint64_t> g_launches;       // kernels launched by this library
 extern std::atomic<uint64_t> g_wait_limit_ns;  // bound of every device-side barrier wait; launchers copy it into kernel parameters
+// Tile of the tcgen05 GEMM: columns, CTAs that share one.
+void gemm_tile(uint32_t m, uint32_t n, uint32_t k, bool argmax, uint32_t& columns, uint32_t& ctas);
 // Test hook: when non-zero, the next tcgen05 GEMM launched from this thread loses the copies of k-block (value - 1) of
 // its first tile, so a bounded wait runs out and the kernel reports DEV_TIMEOUT; the launcher clears it.
 extern thread_local uint32_t t_lose_gemm_stage;

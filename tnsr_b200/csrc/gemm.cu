@@ -986,6 +986,10 @@ static void choose_tile(uint32_t m, uint32_t n, uint32_t k, GemmMode mode, uint3
     while (bn > 32 && bn / 2 >= n) bn = bn == 192 ? 128 : bn >> 1;      // no wider than the matrix (a router's few columns)
 }
 
+void gemm_tile(uint32_t m, uint32_t n, uint32_t k, bool argmax, uint32_t& columns, uint32_t& ctas) {
+    choose_tile(m, n, k, argmax ? GEMM_ARGMAX : GEMM_PLAIN, columns, ctas);
+}
+
 // Shared body of the public launchers.  `tiles_n_out` (optional) receives the number of column
 // tiles the chosen engine used, which GEMM_ARGMAX callers need to read the candidates back.
 static int launch_gemm_impl(const bf16* a, const bf16* bt, void* out, uint32_t ldc, uint32_t m, uint32_t n, uint32_t k,

@@ -154,6 +154,12 @@ int tnsr_b200_decode_attention(const void* q, const void* k_cache, const void* v
                                    workspace_bytes, batch, capacity, heads, head_dim, d_status, as_stream(stream));
 }
 
+int tnsr_b200_test_gemm_tile(uint32_t m, uint32_t n, uint32_t k, int argmax, uint32_t* columns, uint32_t* ctas) {
+    if (!m || !n || !k || !columns || !ctas) return bad("gemm_tile: empty product or null pointer");
+    gemm_tile(m, n, k, argmax != 0, *columns, *ctas);
+    return TNSR_B200_OK;
+}
+
 int tnsr_b200_prefill_attention(const void* q, const void* k_cache, const void* v_cache, void* out, uint32_t batch,
                                 uint32_t chunk, uint32_t position, uint32_t capacity, uint32_t heads, uint32_t head_dim,
                                 void* stream) {
