@@ -137,6 +137,40 @@ __device__ __noinline__ float add_up(uint32_t terms, uint32_t n) {
     for (; at < end; at += 16) add(quad(at));
     return sum;
 }
+// acc + the n values at `at`, `at` + stride bytes, ... in shared memory, in order, eight on their way while eight are added: behind thousands of keys
+// these sums are half of a step.  (Eight loaded and then added, as rows of more than 128 columns have it, whose registers are full: 16 sessions x
+// 6 heads of 16 x 4096 keys 788 us a step, 721 so.)
+__device__ __noinline__ float add_column(uint32_t at, uint32_t stride, uint32_t n, float acc) {
+    float u[8], v[8];
+    auto load = [&](float (&x)[8]) {
+#pragma unroll
+        for (uint32_t i = 0; i < 8; ++i, at += stride) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x[i]) : "r"(at) : "memory");
+    };
+    auto add = [&](const float (&x)[8]) {
+#pragma unroll
+        for (uint32_t i = 0; i < 8; ++i) acc = acc + x[i];
+    };
+    if (n >= 8) {
+        load(u);
+#pragma unroll 1
+        for (n -= 8; n >= 16; n -= 16) {
+            load(v);
+            add(u);
+            load(u);
+            add(v);
+        }
+        if (n >= 8) load(v);
+        add(u);
+        if (n >= 8) add(v), n -= 8;
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < 7; ++i, at += stride)
+        if (i < n) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(u[i]) : "r"(at) : "memory");
+#pragma unroll
+    for (uint32_t i = 0; i < 7; ++i)
+        if (i < n) acc = acc + u[i];
+    return acc;
+}
 __device__ __forceinline__ float add_up(const float* terms, uint32_t n) { return add_up((uint32_t)__cvta_generic_to_shared(terms), n); }
 
 // Scale and shift of a LayerNorm, asked for before the phase's barrier: a warp per row, lane l holds columns l, l + 32, ...
@@ -198,7 +232,7 @@ __device__ __forceinline__ float4 load_kv4(const bf16* p) {
 
 // Attention of one (row, head) by the whole CTA, in the order of attention_strict_kernel: thread c < head width returns output c.
 // `scratch`: scores, then products.
-template <typename KV>
+template <typename KV, bool AHEAD>
 __device__ __forceinline__ float attend(const StrictStepArgs& a, const KV* kb, const KV* vb, const float* qs, uint32_t total, float* scratch) {
     __shared__ float red[SS_WARPS + 1];
     const uint32_t tid = threadIdx.x, lane = tid % 32, warp = tid / 32, hd = a.d / a.heads, quads = hd / 4, d = a.d;
@@ -264,9 +298,13 @@ __device__ __forceinline__ float attend(const StrictStepArgs& a, const KV* kb, c
         for (; e < keys * quads; e += SS_THREADS) put(e, load_kv4(vb + (size_t)(j0 + e / quads) * d + 4 * (e % quads)));
         __syncthreads();
         if (tid < hd) {
-            const float* p = prod + tid;
+            if (AHEAD) {
+                acc = add_column((uint32_t)__cvta_generic_to_shared(prod + tid), 4 * hd, keys, acc);
+            } else {
+                const float* p = prod + tid;
 #pragma unroll 8
-            for (uint32_t j = 0; j < keys; ++j, p += hd) acc = acc + *p;
+                for (uint32_t j = 0; j < keys; ++j, p += hd) acc = acc + *p;
+            }
         }
     }
     __syncthreads();
@@ -276,7 +314,7 @@ __device__ __forceinline__ float attend(const StrictStepArgs& a, const KV* kb, c
 // Shared floats of one row: residual, queries, attention output, normalised row, its terms, hidden row.
 __host__ __device__ __forceinline__ uint32_t floats_per_row(uint32_t d, uint32_t f) { return 5 * d + f; }
 
-// V: columns of a row that a lane of a LayerNorm holds.
+// V: columns of a row that a lane of a LayerNorm holds; with 4 there are registers left for values on their way in attention.
 template <typename KV, uint32_t V>
 __global__ void __launch_bounds__(SS_THREADS, 1)
 strict_step_kernel(const __grid_constant__ SsParams P) {
@@ -378,7 +416,7 @@ strict_step_kernel(const __grid_constant__ SsParams P) {
         for (uint32_t i = rank; i < rows * a.heads; i += SS_CTAS) {
             const uint32_t r = i / a.heads, head_at = r * d + i % a.heads * hd;
             const size_t base = (size_t)(s0 + r / a.chunk) * a.capacity * d + (size_t)(i % a.heads) * hd;
-            const float v = attend<KV>(a, kcache + base, vcache + base, q + head_at, min(a.position + r % a.chunk + 1, a.capacity), prod);
+            const float v = attend<KV, V == 4>(a, kcache + base, vcache + base, q + head_at, min(a.position + r % a.chunk + 1, a.capacity), prod);
             if (tid < hd) store_to_all(att + head_at + tid, v);
         }
         cluster_arrive();
