@@ -744,11 +744,13 @@ decode_attention_kernel(DaParams P) {
 // ===========================================================================
 // With a few MB of keys the kernel above is a chain of latencies: work list, ring, partial results to L2, counters, merge (12 us for one
 // session of 1000 keys x 12 heads, whose 3 MB are 0.5 us of HBM).  Here a cluster of CTAs shares one (session, head): rank r takes an even share
-// of its keys, 16 bytes per lane straight into registers, up to 64 keys per CTA and pass, the next pass on its way while one is summed up.
+// of its keys, 16 bytes per lane straight into registers, 32 KB of keys (256, 128 or 64 of them) per CTA and pass, the next pass on its way while
+// one is summed up.
 // All keys but a session's newest are older than the previous kernel (the QKV product): their first pass is asked for before it ends.
 // Partial (maximum, sum, numerator) go to rank 0 through distributed shared memory, which adds them in rank order.
 constexpr uint32_t DS_THREADS = 256, DS_WARPS = DS_THREADS / 32;
 constexpr int DS_U = 4;                      // keys of a lane group per pass
+constexpr uint32_t DS_PAGES = 1536;          // pages that a CTA's share of keys may touch (ds_pays)
 
 struct DsParams {
     const bf16* q;
@@ -762,6 +764,7 @@ struct DsParams {
     int* d_status;
     KvPaging paging;
     uint32_t early;                          // the previous kernel writes no key but every session's newest
+    uint32_t page_inverse;                   // 2^32 / page_rows rounded up: finds the page of every key, as capacity * page_rows <= 2^32
 };
 
 __device__ __forceinline__ uint4 ds_load(const bf16* p) {
@@ -778,6 +781,7 @@ decode_attention_short_kernel(const __grid_constant__ DsParams P) {
     constexpr uint32_t LPK = HD / 8, KPW = 32 / LPK, PASS = DS_WARPS * KPW;   // lanes per key, keys of a warp and of the CTA side by side
     constexpr uint32_t PART = HD + 2;
     __shared__ float warp_part[DS_WARPS][PART], cta_part[8][PART];           // numerator, maximum, sum
+    __shared__ uint32_t page_row[DS_PAGES];                                  // first rows of the pages of this CTA's keys
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane / LPK, sub = lane % LPK;
     const uint32_t rank = blockIdx.x % P.ck, unit = blockIdx.x / P.ck, h = unit % P.heads, session = unit / P.heads, d = P.heads * HD;
     if (P.ck > 1) ds_cluster_arrive();
@@ -793,14 +797,30 @@ decode_attention_short_kernel(const __grid_constant__ DsParams P) {
     const size_t col = (size_t)h * HD + sub * 8;
     uint4 kx[DS_U], vx[DS_U];
     const uint4 none = make_uint4(0u, 0u, 0u, 0u);
-    auto at = [&](uint32_t key) { return kv_row_l2(P.paging, session, key, P.capacity) * d + col; };
+    // The pages of the share are looked up once, all side by side: a look-up per key and pass is a chain of its own (a step of 20 sessions x 12 heads
+    // of 64 at 575 keys, 4 layers, 168 us so, 156 from here; the streaming kernel 143).  Rows fit 32 bits: 2^32 of the narrowest are 256 GB.
+    auto page_of = [&](uint32_t key) { return __umulhi(key, P.page_inverse); };
+    const uint32_t first_page = P.paging.table ? page_of(k0) : 0u;
+    if (P.paging.table) {
+        const uint32_t pages = k1 > k0 ? page_of(k1 - 1) - first_page + 1 : 0u;
+        const uint32_t* table = P.paging.table + (size_t)session * P.paging.pages_per_session + first_page;
+        for (uint32_t i = threadIdx.x; i < pages; i += DS_THREADS) page_row[i] = __ldcg(table + i) * P.paging.page_rows;
+        __syncthreads();
+    }
+    auto row_of = [&](uint32_t key) -> uint32_t {
+        if (!P.paging.table) return session * P.capacity + key;
+        const uint32_t page = page_of(key);
+        return page_row[page - first_page] + (key - page * P.paging.page_rows);
+    };
+    auto at = [&](uint32_t row) { return (size_t)row * d + col; };
+    constexpr uint32_t NO_ROW = ~0u;
     const uint32_t ahead = P.early ? L - 1 : k1;        // keys below it may be read now (a session of a step has one at least)
 #pragma unroll
     for (int u = 0; u < DS_U; ++u) {
         const uint32_t key = mine + u * PASS;
         kx[u] = vx[u] = none;
         if (key < k1 && key < ahead) {
-            const size_t o = at(key);
+            const size_t o = at(row_of(key));
             kx[u] = ds_load(P.kc + o);
             vx[u] = ds_load(P.vc + o);
         }
@@ -812,7 +832,7 @@ decode_attention_short_kernel(const __grid_constant__ DsParams P) {
 #pragma unroll
         for (int u = 0; u < DS_U; ++u) {
             if (mine + u * PASS != L - 1) continue;
-            const size_t o = at(L - 1);
+            const size_t o = at(row_of(L - 1));
             kx[u] = ds_load(P.kc + o);
             vx[u] = ds_load(P.vc + o);
         }
@@ -831,11 +851,11 @@ decode_attention_short_kernel(const __grid_constant__ DsParams P) {
     for (uint32_t base = 0; k0 + base < k1; base += DS_U * PASS) {
         float sc[DS_U];
         float m_new = m;
-        size_t next[DS_U];                       // the next pass: its pages are looked up before this one's sums
+        uint32_t row[DS_U];                      // of the next pass
 #pragma unroll
         for (int u = 0; u < DS_U; ++u) {
             const uint32_t key = mine + base + (DS_U + u) * PASS;
-            next[u] = key < k1 ? at(key) : ~(size_t)0;
+            row[u] = key < k1 ? row_of(key) : NO_ROW;
         }
 #pragma unroll
         for (int u = 0; u < DS_U; ++u) {
@@ -853,7 +873,7 @@ decode_attention_short_kernel(const __grid_constant__ DsParams P) {
             m_new = fmaxf(m_new, sc[u]);
         }
 #pragma unroll
-        for (int u = 0; u < DS_U; ++u) kx[u] = next[u] != ~(size_t)0 ? ds_load(P.kc + next[u]) : none;
+        for (int u = 0; u < DS_U; ++u) kx[u] = row[u] != NO_ROW ? ds_load(P.kc + at(row[u])) : none;
         const float m_safe = m_new == -INFINITY ? 0.0f : m_new, corr = ex2(m - m_safe);
         m = m_new;
         l *= corr;
@@ -870,7 +890,7 @@ decode_attention_short_kernel(const __grid_constant__ DsParams P) {
                 acc[2 * e] = fmaf(p, f.x, acc[2 * e]);
                 acc[2 * e + 1] = fmaf(p, f.y, acc[2 * e + 1]);
             }
-            vx[u] = next[u] != ~(size_t)0 ? ds_load(P.vc + next[u]) : none;
+            vx[u] = row[u] != NO_ROW ? ds_load(P.vc + at(row[u])) : none;
         }
     }
     // lane groups of the warp, warps of the CTA, CTAs of the cluster
@@ -941,21 +961,58 @@ static int da_sm_count() {
     return n;
 }
 
-// CTAs per (session, head): what fits the GPU at once, three per SM, and at most a portable cluster.
-static uint32_t ds_cluster(uint32_t units) { return std::max(1u, std::min(8u, 3u * (uint32_t)da_sm_count() / units)); }
+// Clusters of `ck` CTAs that run side by side (they do not cross a GPC: 444, 222, 142, 104, 82, 71, 56, 48 of 1 to 8 on a B200, not 444 / ck).
+template <int HD>
+static uint32_t ds_clusters_at_once(uint32_t ck) {
+    static std::atomic<int> known[64][9];          // 0: not asked yet
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    int n = known[dev][ck].load(std::memory_order_relaxed);
+    if (n == 0) {
+        prefer_max_shared_carveout(reinterpret_cast<const void*>(decode_attention_short_kernel<HD>));
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(ck);
+        cfg.blockDim = dim3(DS_THREADS);
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = ck;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&n, decode_attention_short_kernel<HD>, &cfg) != cudaSuccess) cudaGetLastError();
+        if (n <= 0) n = -1;
+        known[dev][ck].store(n, std::memory_order_relaxed);
+    }
+    return n > 0 ? (uint32_t)n : 0u;
+}
+// CTAs per (session, head): the largest cluster, portable ones, of which all run at once.  (One too large is a second wave: a step of 12 sessions x
+// 12 heads at 1215 keys 156 us in clusters of three, 138 in clusters of two.)
+template <int HD>
+static uint32_t ds_cluster(uint32_t units) {
+    uint32_t ck = 8;
+    while (ck > 1 && units > ds_clusters_at_once<HD>(ck)) --ck;
+    return ck;
+}
 
 // Whether the launch above is the faster one: `longest` keys that a session can have, `chained` in a session's step (no plan to save there, as
 // that is made once for all layers).  Its CTAs are not balanced by length and their many short streams stop at 4 TB/s, so what ends it is keys x
-// heads in all.  us with the streaming kernel / here, B200:
-//     operator, sessions x heads x capacity, lengths anywhere     a step of 12 layers x 12 heads, sessions @ keys
-//       1 x 12 x 64     13.8 / 6.2     16 x 12 x 1000  20.7 / 15.9    1 @ 100   295 / 241     16 @ 1000  408 / 390
-//       1 x 12 x 1000   17.1 / 7.3     32 x 12 x 1000  23.6 / 22.2    1 @ 1000  332 / 247     32 @ 100   401 / 353
-//       1 x 16 x 4096   28.5 / 11.6    48 x 12 x 900   25.7 / 24.5    4 @ 1000  349 / 284     32 @ 1000  554 / 593
-//       4 x 12 x 4096   25.7 / 15.4    64 x 16 x 300   22.3 / 18.4    8 @ 300   327 / 275     64 @ 500   638 / 689
-//       8 x 12 x 2048   23.2 / 15.0    16 x 16 x 4096  34.9 / 49.3    8 @ 1000  363 / 316     48, lengths to 900  781 / 955
-//       16 x 12 x 300   18.3 / 9.4     64 x 16 x 1000  34.8 / 39.3    16 @ 300  361 / 312     16, lengths to 1000 489 / 498
-static bool ds_pays(uint32_t batch, uint32_t heads, uint32_t longest, bool chained) {
-    return (uint64_t)batch * heads * longest <= (chained ? 180000u : 400000u);
+// heads in all.  us with the streaming kernel / here, B200, operator, sessions x heads of 64 x capacity, lengths anywhere:
+//       1 x 12 x 64     13.8 / 6.2     16 x 12 x 1000  20.7 / 15.9    1 x 16 x 4096   28.5 / 11.6    64 x 16 x 300   22.3 / 18.4
+//       1 x 12 x 1000   17.1 / 7.3     32 x 12 x 1000  23.6 / 22.2    4 x 12 x 4096   25.7 / 15.4    16 x 16 x 4096  34.9 / 49.3
+//       16 x 12 x 300   18.3 / 9.4     48 x 12 x 900   25.7 / 24.5    8 x 12 x 2048   23.2 / 15.0    64 x 16 x 1000  34.8 / 39.3
+// so 400 K (at that line 0.82 of the streaming kernel's time on average and 0.98 at most, heads of 32 0.77 and 0.99).  Heads of 128 have twice the bytes:
+// 0.87 on average at 300 K, 0.97 at 400 K; chains of more than 20 passes lose there (4 x 4 x 12496 39.1 / 42.1), but with few rows (1 x 4 x 12496 38.7 / 30.7).
+// In a step, measured over 1160 handles of 4 layers, heads of 32, 64 and 128, contiguous and in pages, at their last key and at a third of it: 180 K keys x
+// heads; two waves at most (48 x 24 heads of 32 at 21 keys 1.08 times as long); and no chain of more than 12 passes (four where a CTA has a session's
+// head alone and few are there to hide it), unless the rows are few, where the streaming kernel is a chain itself.  At the last key / at a third of
+// it, time here over time there: 0.87 / 0.84 on average inside these lines, 1.06 at worst; past them
+//       sessions x heads x capacity   20 x 12 x 64, 576: 1.07 / 0.92 (4.5 passes, alone)      2 x 4 x 128, 7488: 1.07 / 0.72 (14.6 passes)
+//       64 x 12 x 32, 448 (344 K): 1.09 / 0.95                                                 1 x 8 x 128, 7488: 0.75 / 0.68 (14.6 passes, few rows: taken)
+static bool ds_pays(uint32_t batch, uint32_t heads, uint32_t ck, uint32_t longest, uint32_t head_dim, bool chained) {
+    const uint64_t units = (uint64_t)batch * heads, keys = units * longest, rows = (uint64_t)batch * longest;
+    const uint32_t pass = 8192 / head_dim, passes = ceil_div(ceil_div(longest, ck), pass);
+    if (!chained) return head_dim <= 64 ? keys <= 400000u : keys <= 300000u && (passes <= 20u || rows <= 16384u);
+    return keys <= 180000u && units <= 888u && (ck == 1 ? passes <= 4u : passes <= 12u || rows <= 8192u);
 }
 
 // Launches an attention kernel, between two events of the handle's record while one is kept: the same kernel either way.
@@ -1024,17 +1081,22 @@ int launch_decode_attention_ex(const bf16* q, const bf16* k_cache, const bf16* v
         set_thread_error("decode attention: the page size must be a multiple of 16 rows");
         return TNSR_B200_ERR_INVALID_ARGUMENT;
     }
-    if (!lean && ds_pays(batch, heads, capacity, extra > 0)) {       // a step's newest key comes on top of the lengths
+    const uint32_t units = batch * heads;
+    const uint32_t ck = head_dim == 32 ? ds_cluster<32>(units) : head_dim == 64 ? ds_cluster<64>(units) : ds_cluster<128>(units);
+    const bool paged = paging && paging->table;
+    const bool addressed = !paged || ((uint64_t)capacity * paging->page_rows <= 1ull << 32 && ceil_div(capacity, ck) / paging->page_rows + 2 <= DS_PAGES);
+    // a step's newest key comes on top of the lengths
+    if (!lean && addressed && ds_pays(batch, heads, ck, capacity, head_dim, extra > 0)) {
         DsParams S;
         S.q = q; S.kc = k_cache; S.vc = v_cache; S.out = out;
         S.lengths = d_lengths; S.d_position = d_position; S.extra = extra;
-        S.capacity = capacity; S.heads = heads; S.ck = ds_cluster(batch * heads);
+        S.capacity = capacity; S.heads = heads; S.ck = ck;
         S.scale_log2 = (1.0f / sqrtf((float)head_dim)) * 1.4426950408889634f;
         S.d_status = d_status;
-        if (paging && paging->table) S.paging = *paging;
+        if (paged) S.paging = *paging;
+        S.page_inverse = paged ? (uint32_t)(((1ull << 32) + paging->page_rows - 1) / paging->page_rows) : 0u;
         S.early = t_pdl && extra > 0;
-        return head_dim == 32 ? launch_ds<32>(S, batch * heads, stream) : head_dim == 64 ? launch_ds<64>(S, batch * heads, stream)
-                                                                                        : launch_ds<128>(S, batch * heads, stream);
+        return head_dim == 32 ? launch_ds<32>(S, units, stream) : head_dim == 64 ? launch_ds<64>(S, units, stream) : launch_ds<128>(S, units, stream);
     }
     uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
     uint32_t* header = reinterpret_cast<uint32_t*>(ws);
