@@ -1002,10 +1002,10 @@ static uint32_t ds_cluster(uint32_t units) {
 //       16 x 12 x 300   18.3 / 9.4     48 x 12 x 900   25.7 / 24.5    8 x 12 x 2048   23.2 / 15.0    64 x 16 x 1000  34.8 / 39.3
 // so 400 K (at that line 0.82 of the streaming kernel's time on average and 0.98 at most, heads of 32 0.77 and 0.99).  Heads of 128 have twice the bytes:
 // 0.87 on average at 300 K, 0.97 at 400 K; chains of more than 20 passes lose there (4 x 4 x 12496 39.1 / 42.1), but with few rows (1 x 4 x 12496 38.7 / 30.7).
-// In a step, measured over 1160 handles of 4 layers, heads of 32, 64 and 128, contiguous and in pages, at their last key and at a third of it: 180 K keys x
+// In a step, measured over 1328 handles of 4 layers, heads of 32, 64 and 128, contiguous and in pages, at their last key and at a third of it: 180 K keys x
 // heads; two waves at most (48 x 24 heads of 32 at 21 keys 1.08 times as long); and no chain of more than 12 passes (four where a CTA has a session's
 // head alone and few are there to hide it), unless the rows are few, where the streaming kernel is a chain itself.  At the last key / at a third of
-// it, time here over time there: 0.87 / 0.84 on average inside these lines, 1.06 at worst; past them
+// it, time here over time there: 0.87 / 0.83 on average inside these lines, 1.06 at worst; past them
 //       sessions x heads x capacity   20 x 12 x 64, 576: 1.07 / 0.92 (4.5 passes, alone)      2 x 4 x 128, 7488: 1.07 / 0.72 (14.6 passes)
 //       64 x 12 x 32, 448 (344 K): 1.09 / 0.95                                                 1 x 8 x 128, 7488: 0.75 / 0.68 (14.6 passes, few rows: taken)
 static bool ds_pays(uint32_t batch, uint32_t heads, uint32_t ck, uint32_t longest, uint32_t head_dim, bool chained) {
