@@ -16,7 +16,7 @@ inline int bad(const char* msg) {
 
 // The launches of an operator may be made ready while the caller's kernel before them drains, as a session's are.  What comes before is the
 // caller's, so the first kernel of a call reads nothing until that has ended (GemmEpilogue::wait_first).  Back to back, us per call without /
-// with: 8 x 4096 x 4096 14.1 / 10.5, 100 x 3000 x 2048 18.5 / 16.2, 900 x 3000 x 2048 22.8 / 20.0, SwiGLU 300 x 1024 -> 4096 38.9 / 32.4, decode
+// with: 8 x 4096 x 4096 14.1 / 10.7, 100 x 3000 x 2048 18.5 / 16.2, 900 x 3000 x 2048 22.8 / 20.0, SwiGLU 300 x 1024 -> 4096 38.9 / 32.4, decode
 // attention 30 x 16 x 3000 42.1 / 40.3.  Not while the stream is being captured: what is before the first node is up to the caller's graph.
 struct OverlapLaunches {
     const bool before = t_pdl;
