@@ -43,9 +43,9 @@ __device__ __forceinline__ float warp_sum_f(float v) {
 constexpr int GEN_MAX_SLOTS = 8;  // head_dim <= 256
 
 __global__ void __launch_bounds__(128)
-attention_generic_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kc, const bf16* __restrict__ vc,
+attention_generic_kernel(const bf16* q, const bf16* kc, const bf16* vc,
                          bf16* __restrict__ out, uint32_t total_queries, uint32_t chunk, uint32_t position,
-                         const uint32_t* __restrict__ d_position, uint32_t capacity, uint32_t heads, uint32_t hd,
+                         const uint32_t* d_position, uint32_t capacity, uint32_t heads, uint32_t hd,
                          float scale_log2, KvPaging paging) {
     pdl_wait();
     pdl_trigger();

@@ -383,6 +383,8 @@ __device__ __forceinline__ int total_order_key(float x) {
     return bits ^ (int)(((unsigned)(bits >> 31)) >> 1);
 }
 // First statement of every kernel that may be launched with programmatic stream serialization.
+// What earlier kernels write is read by plain loads (no __ldg, no .nc, no const T* __restrict__ parameter): memory that is taken for constant while the
+// grid lives may be read ahead of the wait.  Weights may.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Lets the next kernel in the stream be scheduled (it still waits for this one's completion in its own pdl_wait).
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

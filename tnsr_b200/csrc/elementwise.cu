@@ -37,9 +37,9 @@ __device__ __forceinline__ float load1<bf16>(const bf16* p) { return __bfloat162
 
 template <typename T>
 __global__ void __launch_bounds__(128)
-embedding_kernel(const T* __restrict__ tok, const T* __restrict__ pos, const uint32_t* __restrict__ ids,
+embedding_kernel(const T* __restrict__ tok, const T* __restrict__ pos, const uint32_t* ids,
                  float* __restrict__ out, uint32_t chunk, uint32_t position0,
-                 const uint32_t* __restrict__ d_position, uint32_t position_stride, uint32_t vocab, uint32_t width,
+                 const uint32_t* d_position, uint32_t position_stride, uint32_t vocab, uint32_t width,
                  float scale, int* __restrict__ d_status) {
     pdl_wait();
     pdl_trigger();
@@ -110,7 +110,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 // RMS: y = x / sqrt(mean(x^2) + eps) * (w_add + w) -- no mean, no shift; w_add is 1 for weights stored around zero.
 template <bool OUT_BF16, bool RMS>
 __global__ void __launch_bounds__(128)
-layernorm_warp_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b,
+layernorm_warp_kernel(const float* x, const float* __restrict__ w, const float* __restrict__ b,
                       void* __restrict__ out, uint32_t rows, uint32_t width, float eps, float w_add) {
     pdl_wait();
     pdl_trigger();
@@ -182,7 +182,7 @@ __device__ __forceinline__ float ln_fold_block_sum(float x, float* red) {
 
 template <bool RMS>
 __global__ void __launch_bounds__(LN_FOLD_THREADS)
-layernorm_fold_kernel(float* __restrict__ h, const float* __restrict__ partials, uint32_t split_k, uint32_t split_rows,
+layernorm_fold_kernel(float* __restrict__ h, const float* partials, uint32_t split_k, uint32_t split_rows,
                       const float* __restrict__ w, const float* __restrict__ b, bf16* __restrict__ out, uint32_t rows,
                       uint32_t width, float eps, float w_add) {
     __shared__ float red[LN_FOLD_THREADS / 32];
@@ -223,7 +223,7 @@ layernorm_fold_kernel(float* __restrict__ h, const float* __restrict__ partials,
 // Any width: one block per row, three passes over global memory (L2-resident).
 template <bool OUT_BF16, bool RMS>
 __global__ void __launch_bounds__(256)
-layernorm_block_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b,
+layernorm_block_kernel(const float* x, const float* __restrict__ w, const float* __restrict__ b,
                        void* __restrict__ out, uint32_t width, float eps, float w_add) {
     __shared__ float red[8];
     __shared__ float bc;
@@ -345,7 +345,7 @@ int launch_rmsnorm_fold(float* h, const float* partials, uint32_t split_k, uint3
 }
 
 // ---------------------------------------------------------------------------
-__global__ void gather_last_rows_kernel(const float* __restrict__ x, float* __restrict__ out, uint32_t chunk,
+__global__ void gather_last_rows_kernel(const float* x, float* __restrict__ out, uint32_t chunk,
                                         uint32_t width) {
     pdl_wait();
     pdl_trigger();
@@ -368,7 +368,7 @@ int launch_gather_last_rows(const float* x, float* out, uint32_t sessions, uint3
 // patterns, compared as signed integers; ties prefer the larger index.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024)
-argmax_kernel(const float* __restrict__ logits, uint32_t* __restrict__ out, uint32_t vocab, uint32_t row_stride) {
+argmax_kernel(const float* logits, uint32_t* __restrict__ out, uint32_t vocab, uint32_t row_stride) {
     __shared__ int keys[32];
     __shared__ uint32_t idxs[32];
     pdl_wait();
@@ -440,7 +440,7 @@ int launch_argmax(const float* logits, uint32_t* out, uint32_t rows, uint32_t vo
 // 6 bytes of traffic per element.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-swiglu_kernel(const bf16* __restrict__ gate, const bf16* __restrict__ up, bf16* __restrict__ out, uint64_t elems) {
+swiglu_kernel(const bf16* gate, const bf16* up, bf16* __restrict__ out, uint64_t elems) {
     pdl_wait();
     pdl_trigger();
     const uint64_t nvec = elems >> 3;

@@ -49,7 +49,7 @@ __device__ __forceinline__ PolySums pn_total(PolySums s) {
 
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(PN_THREADS)
-polynorm_kernel(const T* __restrict__ z, const float* __restrict__ act, T* __restrict__ out, uint32_t width, uint32_t out_ld, uint32_t out_cols,
+polynorm_kernel(const T* z, const float* __restrict__ act, T* __restrict__ out, uint32_t width, uint32_t out_ld, uint32_t out_cols,
                 float eps) {
     pdl_wait();
     pdl_trigger();
@@ -105,7 +105,7 @@ polynorm_kernel(const T* __restrict__ z, const float* __restrict__ act, T* __res
 constexpr int PN_WARP_CHUNKS = 16;
 template <int CHUNKS>
 __global__ void __launch_bounds__(128)
-polynorm_warp_kernel(const bf16* __restrict__ z, const float* __restrict__ act, bf16* __restrict__ out, uint32_t rows, uint32_t width, uint32_t out_ld,
+polynorm_warp_kernel(const bf16* z, const float* __restrict__ act, bf16* __restrict__ out, uint32_t rows, uint32_t width, uint32_t out_ld,
                      uint32_t out_cols, float eps) {
     pdl_wait();
     pdl_trigger();
@@ -323,8 +323,8 @@ experts_offsets_kernel(uint32_t* counts, uint32_t* offsets, uint32_t blocks, uin
 // A warp per (row, slot): fixes its place and copies the row there.
 template <typename V>
 __global__ void __launch_bounds__(256)
-experts_gather_kernel(const V* __restrict__ h, V* __restrict__ out, uint32_t* __restrict__ place, const uint32_t* __restrict__ rank,
-                      const uint32_t* __restrict__ counts, uint32_t pairs, uint32_t top, uint32_t experts, uint32_t words) {
+experts_gather_kernel(const V* h, V* __restrict__ out, uint32_t* __restrict__ place, const uint32_t* rank,
+                      const uint32_t* counts, uint32_t pairs, uint32_t top, uint32_t experts, uint32_t words) {
     pdl_wait();
     pdl_trigger();
     const uint32_t lane = threadIdx.x & 31, pair = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -448,7 +448,7 @@ experts_choose_kernel(ChooseParams P) {
 // every block counts for its eight pairs, the first one also makes the group offsets.
 template <typename V>
 __global__ void __launch_bounds__(256)
-experts_gather_few_kernel(const V* __restrict__ h, V* __restrict__ out, uint32_t* __restrict__ place, const uint32_t* __restrict__ ids,
+experts_gather_few_kernel(const V* h, V* __restrict__ out, uint32_t* __restrict__ place, const uint32_t* ids,
                           uint32_t* __restrict__ offsets, uint32_t pairs, uint32_t top, uint32_t experts, uint32_t words) {
     __shared__ uint32_t before[8][8], hist[kMaxExperts], first[kMaxExperts + 1];
     pdl_wait();
@@ -498,8 +498,8 @@ constexpr int EC_KEEP = 4;
 
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(EC_THREADS)
-experts_combine_kernel(float* __restrict__ x, const T* __restrict__ y, const T* h, const uint32_t* __restrict__ place,
-                       const float* __restrict__ weights, const float* __restrict__ layer_scale, const float* __restrict__ norm_w, T* norm_out,
+experts_combine_kernel(float* __restrict__ x, const T* y, const T* h, const uint32_t* place,
+                       const float* weights, const float* __restrict__ layer_scale, const float* __restrict__ norm_w, T* norm_out,
                        uint32_t pairs, uint32_t top, uint32_t d, float norm_offset, float eps) {
     __shared__ uint32_t s_place[kMaxTop];
     __shared__ float s_weight[kMaxTop], red[EC_THREADS / 32];
@@ -587,8 +587,8 @@ experts_combine_kernel(float* __restrict__ x, const T* __restrict__ y, const T* 
 // Many rows of at most 1024 columns: a warp per row.
 template <typename T>
 __global__ void __launch_bounds__(128)
-experts_combine_warp_kernel(float* __restrict__ x, const T* __restrict__ y, const T* h, const uint32_t* __restrict__ place,
-                            const float* __restrict__ weights, const float* __restrict__ layer_scale, const float* __restrict__ norm_w, T* norm_out,
+experts_combine_warp_kernel(float* __restrict__ x, const T* y, const T* h, const uint32_t* place,
+                            const float* weights, const float* __restrict__ layer_scale, const float* __restrict__ norm_w, T* norm_out,
                             uint32_t rows, uint32_t top, uint32_t d, float norm_offset, float eps) {
     constexpr int KEEP = 8;
     pdl_wait();

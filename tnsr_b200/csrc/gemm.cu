@@ -1224,7 +1224,7 @@ int launch_gemm_segments(const bf16* a, const bf16* bt, uint32_t m, uint32_t n, 
 // One warp per row folds the per-tile candidates; ties between tiles go to the larger index,
 // which is the later tile, so the result is the last index of the row maximum.
 __global__ void __launch_bounds__(128)
-argmax_finish_kernel(const uint2* __restrict__ cand, uint32_t* __restrict__ ids, uint32_t rows, uint32_t tiles) {
+argmax_finish_kernel(const uint2* cand, uint32_t* __restrict__ ids, uint32_t rows, uint32_t tiles) {
     pdl_wait();
     pdl_trigger();
     const uint32_t lane = threadIdx.x & 31;

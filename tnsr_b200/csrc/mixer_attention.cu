@@ -393,7 +393,7 @@ int launch_attention_prep(const AttentionPrep& a, const StepPlace& place, int dt
 // ---- convolution inputs of a multi-token chunk into the session's ring ---------------------
 template <typename T>
 __global__ void __launch_bounds__(256)
-conv_ring_kernel(const T* __restrict__ rows, uint32_t ld, uint32_t channels, uint32_t taps, T* __restrict__ ring, StepPlace place) {
+conv_ring_kernel(const T* rows, uint32_t ld, uint32_t channels, uint32_t taps, T* __restrict__ ring, StepPlace place) {
     pdl_wait();
     pdl_trigger();
     const uint32_t s = blockIdx.y, keep = min(place.chunk, taps);

@@ -145,7 +145,7 @@ bool hgrn2_supported(uint32_t heads, uint32_t dim, uint32_t vdim) {
 // ---- norm of wide heads: a block per (row, head) -----------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(128)
-head_norm_kernel(const float* __restrict__ raw, const float* __restrict__ w, T* __restrict__ out, uint32_t heads, uint32_t vdim, uint32_t out_ld,
+head_norm_kernel(const float* raw, const float* __restrict__ w, T* __restrict__ out, uint32_t heads, uint32_t vdim, uint32_t out_ld,
                  uint32_t out_cols, float eps, float gain) {
     __shared__ float red[4];
     pdl_wait();

@@ -30,7 +30,7 @@ __device__ __forceinline__ float act_silu<bf16>(float x) { return mx_silu(x); }
 // A thread owns two neighbouring channels of a run of tokens.
 template <typename T, int TAPS, bool SILU>
 __global__ void __launch_bounds__(128)
-short_conv_kernel(const T* __restrict__ rows, uint32_t ld, uint32_t channels, uint32_t taps, const float* __restrict__ conv_w,
+short_conv_kernel(const T* rows, uint32_t ld, uint32_t channels, uint32_t taps, const float* __restrict__ conv_w,
                   const float* __restrict__ conv_b, T* __restrict__ ring, T* __restrict__ out, uint32_t part, StepPlace place,
                   uint32_t run, uint32_t vec) {
     const uint32_t c = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
@@ -262,7 +262,7 @@ bool mamba2_supported(uint32_t heads, uint32_t vdim, uint32_t state) {
 // registers between the sum and the scaling (gated_norm_warp_kernel).
 template <typename T>
 __global__ void __launch_bounds__(256)
-gated_norm_kernel(const T* __restrict__ gated, const float* __restrict__ w, T* __restrict__ out, uint32_t inner, uint32_t groups,
+gated_norm_kernel(const T* gated, const float* __restrict__ w, T* __restrict__ out, uint32_t inner, uint32_t groups,
                   uint32_t out_ld, uint32_t out_cols, float eps) {
     __shared__ float red[8];
     pdl_wait();
@@ -287,7 +287,7 @@ gated_norm_kernel(const T* __restrict__ gated, const float* __restrict__ w, T* _
 
 constexpr uint32_t GN_VEC = 8;   // 16-byte chunks per lane: parts of up to 2048 values, one warp each
 __global__ void __launch_bounds__(128)
-gated_norm_warp_kernel(const bf16* __restrict__ gated, const float* __restrict__ w, bf16* __restrict__ out, uint32_t rows, uint32_t inner,
+gated_norm_warp_kernel(const bf16* gated, const float* __restrict__ w, bf16* __restrict__ out, uint32_t rows, uint32_t inner,
                        uint32_t groups, uint32_t out_ld, uint32_t out_cols, float eps) {
     pdl_wait();
     pdl_trigger();

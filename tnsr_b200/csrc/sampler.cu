@@ -41,8 +41,8 @@ __device__ __forceinline__ uint32_t philox_first(uint32_t c0, uint32_t c1, uint3
 }
 
 __global__ void __launch_bounds__(SAMPLE_THREADS)
-sample_top_k_kernel(const float* __restrict__ logits, uint32_t vocab, uint32_t row_stride, float temperature, uint32_t top_k,
-                    uint32_t seed_lo, uint32_t seed_hi, const uint32_t* __restrict__ d_step, uint32_t step_stride,
+sample_top_k_kernel(const float* logits, uint32_t vocab, uint32_t row_stride, float temperature, uint32_t top_k,
+                    uint32_t seed_lo, uint32_t seed_hi, const uint32_t* d_step, uint32_t step_stride,
                     uint32_t step_add, uint32_t first_session, uint32_t* __restrict__ out) {
     __shared__ uint32_t hist[256];
     __shared__ uint32_t s_prefix, s_remaining, s_eq_total;
@@ -64,7 +64,7 @@ sample_top_k_kernel(const float* __restrict__ logits, uint32_t vocab, uint32_t r
         __syncthreads();
         const uint32_t prefix = s_prefix;
         for (uint32_t i = tid; i < vocab; i += SAMPLE_THREADS) {
-            const uint32_t uk = ordered_key(__ldg(row + i));
+            const uint32_t uk = ordered_key(row[i]);
             if ((uk & mask) == prefix) atomicAdd(&hist[(uk >> shift) & 255u], 1u);
         }
         __syncthreads();
@@ -93,7 +93,7 @@ sample_top_k_kernel(const float* __restrict__ logits, uint32_t vocab, uint32_t r
         float v = 0.0f;
         uint32_t uk = 0;
         const bool in = i < vocab;
-        if (in) { v = __ldg(row + i); uk = ordered_key(v); }
+        if (in) { v = row[i]; uk = ordered_key(v); }
         const bool eq = in && uk == threshold;
         const uint32_t eq_ballot = __ballot_sync(0xffffffffu, eq);
         if (lane == 0) warp_eq[warp] = __popc(eq_ballot);

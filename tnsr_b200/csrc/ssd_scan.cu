@@ -236,7 +236,7 @@ ssd_scan_kernel(Mamba2 m, StepPlace place, uint32_t vec) {
                     for (int nt = 0; nt < 2; ++nt) {
                         uint32_t v = 0u;
                         if ((uint32_t)rr * 8 < live && c0 + nt * 8 < width) {
-                            if (vec) v = __ldg(reinterpret_cast<const uint32_t*>(src + nt * 8));
+                            if (vec) v = *reinterpret_cast<const uint32_t*>(src + nt * 8);
                             else v = (uint32_t)__bfloat16_as_ushort(src[nt * 8]) | (c0 + nt * 8 + 1 < width ? (uint32_t)__bfloat16_as_ushort(src[nt * 8 + 1]) << 16 : 0u);
                         }
                         z[rr >> 1][rr & 1][nt] = v;
