@@ -238,7 +238,7 @@ gemm_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 // ---- CUDA cores: 32 x 32 tile, a thread owns 2 x 2 outputs -------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(256)
-gemm_grouped_simple_kernel(const T* __restrict__ a, const T* __restrict__ w, GgParams P) {
+gemm_grouped_simple_kernel(const T* a, const T* __restrict__ w, GgParams P) {
     constexpr uint32_t TS = 32, KS = 32;
     __shared__ float as[KS][TS + 1], ws[KS][TS + 1];
     __shared__ uint32_t offs[GG_MAX_GROUPS + 1], first[GG_MAX_GROUPS + 1];
